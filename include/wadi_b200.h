@@ -322,7 +322,8 @@ typedef struct {
     int32_t row_offset, col_offset;
     const double* npix; /* per-pixel Manning n aligned with z (NaN: the cell's own), or NULL */
     const double* nman; /* (ny, nx) */
-    const double *xcrest, *xlen, *xc, *ycrest, *ylen, *yc; /* CrestFaces, wadi2d/tables/builder.py:62-80 */
+    /* CrestFaces, wadi2d/tables/builder.py:62-80; each may be NULL: no face edited (crest NaN, length 1, coefficient 0) */
+    const double *xcrest, *xlen, *xc, *ycrest, *ylen, *yc;
     const uint8_t *xwall, *ywall;                         /* or NULL */
     const uint8_t* mask;
     const int32_t* tiles; /* (ntiles, 2) */
@@ -333,7 +334,7 @@ typedef struct {
 /* Outputs: (ntiles, 32, 32[, rows[, 2]]) float32 in the reference's GridTables layout (tile 0 left as the caller
  * set it: zeros, and ones for efx, efy), and (ny, nx) float64 grids zmin, rel (mean bed over zmin), zfx, zfy (face
  * inverts) that the caller zeroed. ws: scratch of w2b_table_workspace_doubles(k + 2 margin, ws_threads) doubles,
- * ws_threads a multiple of 128 (the face kernel's thread count); needed when local != 0. */
+ * ws_threads a multiple of 128; needed when local != 0. */
 typedef struct {
     float *hc, *dtab, *efx, *efy, *ftabx, *ftaby, *zcx, *zcy;
     float *flx, *frx, *glx, *grx, *cwx, *fly, *fry, *gly, *gry, *cwy;
@@ -346,31 +347,22 @@ typedef struct {
  * a larger one is refused with W2B_EINVAL. */
 #define W2B_TABLE_MARGIN_MAX (1 << 20)
 
-/* Doubles of table-builder scratch for lines of up to nmax pixels and the given face-kernel thread count. */
+/* Doubles of table-builder scratch for lines of up to nmax pixels and the given count of threads (128 suffice: the
+ * scratch then holds 576 CTAs' lines). */
 int64_t w2b_table_workspace_doubles(int32_t nmax, int64_t threads);
 
 /* Replaces build_tables (wadi2d/tables/builder.py:131-258): cell tables, face tables (strips, or the local
- * hydraulic radius when local != 0), centre beds, inverts, closed faces and natural crests, on the GPU. The local
- * radius works in shared memory when a face's line (k + 2 margin pixels) is at most about 2,800 pixels, and in
- * out->ws beyond that; out->ws is required with local != 0 either way. */
+ * hydraulic radius when local != 0), centre beds, inverts, closed faces and natural crests, on the GPU. A face's line
+ * (k + 2 margin pixels) lies in shared memory up to about 11,000 pixels, and in out->ws beyond that; out->ws is
+ * required with local != 0 either way. */
 int32_t w2b_build_tables(const W2BTableIn* in, const W2BTableOut* out, void* stream);
 
 /* w2b_build_tables for callers that cannot allocate device memory. It has no counterpart in the reference. A
  * library embedded in a host program whose device memory belongs to someone else (a pool or caching allocator it
  * does not control, a memory cap, an FFI binding with no allocator of its own) still passes its inputs and outputs,
  * but has no way to hand over the builder's scratch; this entry point allocates nothing (no cudaMalloc, cudaFree or
- * allocating library call) and uses instead a 32 MiB array of file-scope device memory, which every GPU that loads
- * the library holds until the process exits. out->ws and out->ws_threads are ignored.
- *  - Limit: a face's line (k + 2 margin pixels) of at most 3,639 pixels; longer lines are refused with W2B_EINVAL
- *    and a message. Lines that fit the builder's shared-memory workspace (up to 2,843 pixels) do not touch the array.
- *    Lines of 2,844 to 3,639 pixels do, and the array holds the workspaces of only 128 to 155 threads: the face
- *    tables are then built by a single CTA of 128 threads, correct but far slower than with a caller's workspace.
- *  - The first call on a device looks the array's address up (cudaGetSymbolAddress) with that device current;
- *    make that first call before any stream capture. The address is kept for the life of the process: it is not
- *    valid across a cudaDeviceReset.
- *  - Every call shares the one array and it keeps the last call's contents; the kernels write every scratch slot
- *    before reading it, so nothing has to start at zero. Calls that overlap on the GPU (two streams, two threads)
- *    race on it: serialise them. */
+ * allocating library call) and needs none: a face's line (k + 2 margin pixels) of at most 3,639 pixels works in shared
+ * memory; longer lines are refused with W2B_EINVAL and a message. out->ws and out->ws_threads are ignored. */
 int32_t w2b_build_tables_noalloc(const W2BTableIn* in, const W2BTableOut* out, void* stream);
 
 /* The device loop's launch schedule and its tuner. No counterpart in the reference, whose step launches each kernel

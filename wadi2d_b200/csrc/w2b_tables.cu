@@ -10,7 +10,6 @@
 // ArrayBed hold (wadi2d/tables/builder.py:47-50): a window that reaches past the bed repeats its edge pixel.
 #include <cmath>
 #include <cstdio>
-#include <mutex>
 
 #include "w2b_common.cuh"
 
@@ -22,7 +21,7 @@ struct TableArgs {
     int32_t roff, coff;
     const double* npix;  // per-pixel Manning n aligned with z (NaN: the cell's own), or null
     const double* nman;  // (ny, nx)
-    const double *xcrest, *xlen, *xc, *ycrest, *ylen, *yc;  // (ny, nx)
+    const double *xcrest, *xlen, *xc, *ycrest, *ylen, *yc;  // (ny, nx), or null: no face edited
     const uint8_t *xwall, *ywall, *mask;                    // (ny, nx); walls may be null
     const int32_t* tiles;
     int32_t ntiles, ny, nx, k, rows, local, margin, nmax;
@@ -32,7 +31,7 @@ struct TableArgs {
     float *flx, *frx, *glx, *grx, *cwx, *fly, *fry, *gly, *gry, *cwy;
     // outputs, dense (ny, nx) float64
     double *zmin, *rel, *zfx, *zfy;
-    // workspace of the local radius: 9 * (nmax + 1) doubles per thread of the face kernel
+    // workspace for face lines beyond shared memory: 9 * (nmax + 1) doubles per thread the caller counts
     double* ws;
     int64_t ws_threads;
 };
@@ -174,227 +173,236 @@ __global__ void __launch_bounds__(128) cell_tables_kernel(TableArgs A) {
     }
 }
 
-// ------------------------------------------------------------------ face tables (one thread per face)
-
-// _face_table, wadi2d/tables/core.py:44-79, into tab[2 * rows] (FP64). prof is raised to the crest in place.
-__device__ void face_table(double* prof, int m, double crest, double pixel, double n_inv, const double* weight,
-                           double length, double e_lo, double e_hi, int rows, double* tab, double& zf_out,
-                           double& top_out) {
-    if (!isnan(crest))
-        for (int q = 0; q < m; ++q) prof[q] = prof[q] >= crest ? prof[q] : crest;
-    double zf = prof[0];
-    for (int q = 1; q < m; ++q) zf = prof[q] < zf ? prof[q] : zf;
-    double relmax = prof[0] - zf;
-    for (int q = 1; q < m; ++q) {
-        const double v = prof[q] - zf;
-        relmax = v > relmax ? v : relmax;
-    }
-    const double lo = relmax <= e_hi ? relmax : e_hi;
-    const double top = lo >= e_lo ? lo : e_lo;
-    const int last = rows - 1;
-    for (int r = 0; r < rows; ++r) {
-        const double x = (double)r / (double)last;
-        const double e = top * (x * x);
-        double area = 0.0, conv = 0.0;
-        for (int q = 0; q < m; ++q) {
-            const double dep = e - (prof[q] - zf);
-            if (dep > 0.0) {
-                area += dep;
-                const double cb = cbrt(dep);
-                conv += weight[q] * dep * (cb * cb);
-            }
-        }
-        tab[2 * r] = pixel * area * length;
-        tab[2 * r + 1] = pow(pixel * n_inv * conv * length, 0.6);
-    }
-    zf_out = zf;
-    top_out = top;
-}
-
-// _local_radius_conveyance, wadi2d/tables/core.py:82-179, on the line ext[0..n) held in the workspace (array 0);
-// overwrites tab's conveyance column. W(a, i) is this thread's slot i of workspace array a.
-struct Work {
-    double* ws;
-    int64_t stride;  // threads
-    int64_t tid;
-    int nmax;
-    __device__ __forceinline__ double& operator()(int a, int i) const {
-        return ws[((int64_t)a * (nmax + 1) + i) * stride + tid];
-    }
-};
-
-enum { W_EXT = 0, W_D, W_PER, W_S0, W_S1, W_P0, W_P1, W_LO, W_HI };
-
-__device__ void local_radius(const Work& W, int n, int i0, int i1, double zf, double top, double pixel,
-                             double n_inv, const double* weight, double length, double beta, int rows, double* tab) {
-    const double pix2 = pixel * pixel;
-    const int last = rows - 1;
-    for (int t = 0; t < n; ++t) {
-        W(W_LO, t) = 0.0;
-        W(W_HI, t) = 0.0;
-    }
-    W(W_S0, 0) = W(W_S1, 0) = W(W_P0, 0) = W(W_P1, 0) = 0.0;
-    for (int r = 0; r < rows; ++r) {
-        const double x = (double)r / (double)last;
-        const double level = zf + top * (x * x);
-        for (int t = 0; t < n; ++t) {
-            const double dep = level - W(W_EXT, t);
-            W(W_D, t) = dep > 0.0 ? dep : 0.0;
-            W(W_PER, t) = 0.0;
-        }
-        if (W(W_D, 0) > 0.0) W(W_PER, 0) += 0.5 * pixel;
-        if (W(W_D, n - 1) > 0.0) W(W_PER, n - 1) += 0.5 * pixel;
-        for (int t = 0; t < n - 1; ++t) {
-            const double da = W(W_D, t), db = W(W_D, t + 1);
-            const bool wa = da > 0.0, wb = db > 0.0;
-            if (!(wa || wb)) continue;
-            const double rise = W(W_EXT, t + 1) - W(W_EXT, t);
-            const double seg = sqrt(pix2 + rise * rise);
-            if (wa && wb) {
-                W(W_PER, t) += 0.5 * seg;
-                W(W_PER, t + 1) += 0.5 * seg;
-            } else if (wa) {
-                if (rise > 0.0) {
-                    const double f = da / rise;
-                    W(W_PER, t) += (f <= 1.0 ? f : 1.0) * seg;
-                } else {
-                    W(W_PER, t) += 0.5 * pixel;
-                }
-            } else if (-rise > 0.0) {
-                const double f = db / -rise;
-                W(W_PER, t + 1) += (f <= 1.0 ? f : 1.0) * seg;
-            } else {
-                W(W_PER, t + 1) += 0.5 * pixel;
-            }
-        }
-        int start = -1;
-        for (int t = 0; t < n; ++t) {
-            if (W(W_D, t) > 0.0) {
-                if (start < 0) start = t;
-                W(W_LO, t) = (double)start;
-            } else {
-                start = -1;
-            }
-        }
-        int end = -1;
-        for (int t = n - 1; t >= 0; --t) {
-            if (W(W_D, t) > 0.0) {
-                if (end < 0) end = t;
-                W(W_HI, t) = (double)end;
-            } else {
-                end = -1;
-            }
-        }
-        for (int t = 0; t < n; ++t) {
-            const double d = W(W_D, t), per = W(W_PER, t);
-            W(W_S0, t + 1) = W(W_S0, t) + d;
-            W(W_S1, t + 1) = W(W_S1, t) + (double)t * d;
-            W(W_P0, t + 1) = W(W_P0, t) + per;
-            W(W_P1, t + 1) = W(W_P1, t) + (double)t * per;
-        }
-        double conv = 0.0;
-        for (int i = i0; i < i1; ++i) {
-            const double di = W(W_D, i);
-            if (di <= 0.0) continue;
-            double w = beta * di / pixel;
-            if (w < 1e-9) w = 1e-9;
-            int lo = (int)ceil((double)i - w);
-            const int rlo = (int)W(W_LO, i);
-            lo = rlo > lo ? rlo : lo;
-            int hi = (int)floor((double)i + w);
-            const int rhi = (int)W(W_HI, i);
-            hi = rhi < hi ? rhi : hi;
-            const double fi = (double)i;
-            double a_sum = (1.0 - fi / w) * (W(W_S0, i + 1) - W(W_S0, lo)) + (W(W_S1, i + 1) - W(W_S1, lo)) / w;
-            a_sum += (1.0 + fi / w) * (W(W_S0, hi + 1) - W(W_S0, i + 1)) - (W(W_S1, hi + 1) - W(W_S1, i + 1)) / w;
-            double p_sum = (1.0 - fi / w) * (W(W_P0, i + 1) - W(W_P0, lo)) + (W(W_P1, i + 1) - W(W_P1, lo)) / w;
-            p_sum += (1.0 + fi / w) * (W(W_P0, hi + 1) - W(W_P0, i + 1)) - (W(W_P1, hi + 1) - W(W_P1, i + 1)) / w;
-            const double radius = p_sum > 0.0 ? pixel * a_sum / p_sum : di;
-            const double cb = cbrt(radius);
-            conv += weight[i - i0] * di * (cb * cb);
-        }
-        tab[2 * r + 1] = pow(pixel * n_inv * conv * length, 0.6);
-    }
-}
+// ------------------------------------------------------------------ face tables
 
 constexpr int KMAX = 32;
-constexpr int64_t FACE_SMEM_BYTES = 200 * 1024;  // the shared workspace a CTA of the face-table kernel may take
 constexpr int ROWS_MAX = 64;
+constexpr int FACE_THREADS = 256;
+constexpr int64_t FACE_SMEM_BYTES = 200 * 1024;  // the shared memory a CTA of the face-table kernel may take
+constexpr int64_t FACE_TERM_BYTES = 24 * 1024;   // of it for the pixels' conveyance terms (at least one face's)
 
-// SMEM: the local radius's workspace in this CTA's shared memory (interleaved across its threads as the global one is
-// across the grid's), else in the caller's device workspace. The arithmetic is the same either way.
-template <bool SMEM>
-__global__ void __launch_bounds__(128) face_tables_kernel(TableArgs A) {
-    extern __shared__ double sws[];
-    const int64_t nface = (int64_t)(A.ntiles - 1) * TILE2 * 2;
-    const int k = A.k, rows = A.rows;
-    double prof[KMAX], weight[KMAX], tab[2 * ROWS_MAX];
-    const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const Work W = SMEM ? Work{sws, (int64_t)blockDim.x, (int64_t)threadIdx.x, A.nmax} : Work{A.ws, A.ws_threads, tid, A.nmax};
-    for (int64_t f = tid; f < nface; f += (int64_t)gridDim.x * blockDim.x) {
-        const int axis = (int)(f & 1);
-        const int64_t c = f >> 1;
-        const int t = (int)(c / TILE2) + 1;
-        const int local = (int)(c % TILE2);
-        const int64_t j = (int64_t)A.tiles[2 * t] * TILE + local / TILE;
-        const int64_t i = (int64_t)A.tiles[2 * t + 1] * TILE + local % TILE;
-        const int64_t r0 = j * k, c0 = i * k;
-        const int64_t g = j * A.nx + i;
-        const double nm = A.nman[g];
-        // the higher of the two pixels meeting along the face, and its lining (wadi2d/tables/core.py:249-264)
-        for (int q = 0; q < k; ++q) {
-            int64_t nr, nc, fr, fc;
-            if (axis == 0) {
-                nr = r0 + q, nc = c0, fr = r0 + q, fc = c0 - 1;
-            } else {
-                nr = r0, nc = c0 + q, fr = r0 - 1, fc = c0 + q;
-            }
-            const double near = zpix(A, nr, nc), far = zpix(A, fr, fc);
-            prof[q] = far >= near ? far : near;
-            weight[q] = A.npix ? lined(far > near ? npix_at(A, fr, fc) : npix_at(A, nr, nc), nm) : 1.0;
-        }
-        const double crest = axis == 0 ? A.xcrest[g] : A.ycrest[g];
-        const double length = axis == 0 ? A.xlen[g] : A.ylen[g];
-        double zf, top;
-        face_table(prof, k, crest, A.pixel, 1.0 / nm, weight, length, A.e_lo, A.e_hi, rows, tab, zf, top);
-        if (A.local && isnan(crest)) {
-            // wadi2d/tables/core.py:324-351: the face's line reaches margin pixels past both ends
-            const int nfull = k + 2 * A.margin;
-            double hi = -INFINITY;
-            for (int s = 0; s < nfull; ++s) {
-                double x0, x1;
-                if (axis == 0) {
-                    x0 = zpix(A, r0 + s - A.margin, c0 - 1);
-                    x1 = zpix(A, r0 + s - A.margin, c0);
+// The higher of the two pixels meeting along a face's line (wadi2d/tables/core.py:249-264): position p along the
+// line, from the first pixel of the face's cell; (r0, c0) is the cell's first pixel.
+__device__ __forceinline__ double edge_pixel(const TableArgs& A, int axis, int64_t r0, int64_t c0, int64_t p) {
+    const double far = axis == 0 ? zpix(A, r0 + p, c0 - 1) : zpix(A, r0 - 1, c0 + p);
+    const double near = axis == 0 ? zpix(A, r0 + p, c0) : zpix(A, r0, c0 + p);
+    return far >= near ? far : near;
+}
+
+// The lining weight of pixel q of a face, from the pixel that edge_pixel took.
+__device__ __forceinline__ double edge_weight(const TableArgs& A, int axis, int64_t r0, int64_t c0, int q, double nm) {
+    if (!A.npix) return 1.0;
+    const int64_t nr = axis == 0 ? r0 + q : r0, nc = axis == 0 ? c0 : c0 + q;
+    const int64_t fr = axis == 0 ? r0 + q : r0 - 1, fc = axis == 0 ? c0 - 1 : c0 + q;
+    return lined(zpix(A, fr, fc) > zpix(A, nr, nc) ? npix_at(A, fr, fc) : npix_at(A, nr, nc), nm);
+}
+
+// One pixel's conveyance term weight d cbrt(R)^2 at one level (_local_radius_conveyance, wadi2d/tables/core.py:
+// 82-179): E is the face's conveyance line (n pixels), HS half the length of the bed between pixels t and t + 1. The
+// local radius R weighs depth and wetted perimeter by a tent of half-width w = beta d / pixel pixels around pixel i,
+// inside its wet stretch; its sums are differences of running sums taken from the line's start, so the sums run in
+// that order here too: over [0, i] with their values kept at the tent's first pixel lo, then over (i, hi]. A dry pixel
+// adds nothing to a sum and starts a new stretch, so lo moves behind it; the first dry pixel after i ends the sweep.
+__device__ __forceinline__ double local_term(const double* __restrict__ E, const double* __restrict__ HS, int n, int i,
+                                             double level, double pixel, double beta, double weight) {
+    const double di = level - E[i];
+    if (!(di > 0.0)) return 0.0;
+    double w = beta * di / pixel;
+    if (w < 1e-9) w = 1e-9;
+    const int lo = (int)ceil((double)i - w);
+    int hi = (int)floor((double)i + w);
+    hi = hi < n - 1 ? hi : n - 1;
+    const double half = 0.5 * pixel;
+    double s0 = 0.0, s1 = 0.0, p0 = 0.0, p1 = 0.0, ft = 0.0;
+    double da = level - E[0];  // depth of pixel t, and cr: the perimeter it has from its west segment or the line's end
+    da = da > 0.0 ? da : 0.0;
+    double cr = da > 0.0 ? half : 0.0;
+    if (n == 1) cr = da > 0.0 ? half + half : 0.0;
+    auto step = [&](int t) {
+        double db = 0.0, nr = 0.0, per = cr;
+        if (t + 1 < n) {
+            db = level - E[t + 1];
+            db = db > 0.0 ? db : 0.0;
+            if (da > 0.0 && db > 0.0) {
+                nr = HS[t];
+                per += nr;
+            } else if (da > 0.0) {
+                const double rise = E[t + 1] - E[t];
+                if (rise > 0.0) {
+                    const double f = da / rise;
+                    per += (f <= 1.0 ? f : 1.0) * (2.0 * HS[t]);
                 } else {
-                    x0 = zpix(A, r0 - 1, c0 + s - A.margin);
-                    x1 = zpix(A, r0, c0 + s - A.margin);
+                    per += half;
                 }
-                const double v = x0 >= x1 ? x0 : x1;
-                W(W_EXT, s) = v;
-                hi = v > hi ? v : hi;
+            } else if (db > 0.0) {
+                const double rise = E[t + 1] - E[t];
+                if (-rise > 0.0) {
+                    const double f = db / -rise;
+                    nr = (f <= 1.0 ? f : 1.0) * (2.0 * HS[t]);
+                } else {
+                    nr = half;
+                }
             }
-            // _raise_top and window_top, wadi2d/tables/core.py:354-371
-            const double relw = hi - zf;
-            const double cap = relw <= A.e_hi ? relw : A.e_hi;
-            const double wtop = top >= cap ? top : cap;
-            if (wtop > top) {
-                for (int q = 0; q < k; ++q) prof[q] = W(W_EXT, A.margin + q);
-                face_table(prof, k, NAN, A.pixel, 1.0 / nm, weight, length, wtop, A.e_hi, rows, tab, zf, top);
-            }
-            int e = (int)ceil(A.beta * top / A.pixel);
-            e = e > A.margin ? A.margin : e;
-            // the conveyance line is full[margin - e : margin + k + e]: shift it to the front of the workspace
-            const int off = A.margin - e;
-            const int nn = k + 2 * e;
-            if (off > 0)
-                for (int s = 0; s < nn; ++s) W(W_EXT, s) = W(W_EXT, s + off);
-            local_radius(W, nn, e, e + k, zf, top, A.pixel, 1.0 / nm, weight, length, A.beta, rows, tab);
+            if (t + 2 == n && db > 0.0) nr = half + nr;
         }
-        float* out = (axis == 0 ? A.ftabx : A.ftaby) + ((size_t)t * TILE2 + local) * rows * 2;
-        for (int r = 0; r < 2 * rows; ++r) out[r] = (float)tab[r];
-        (axis == 0 ? A.efx : A.efy)[(size_t)t * TILE2 + local] = (float)top;
-        (axis == 0 ? A.zfx : A.zfy)[g] = zf;
+        if (da > 0.0) {
+            s0 += da;
+            s1 += ft * da;
+            p0 += per;
+            p1 += ft * per;
+        }
+        da = db;
+        cr = nr;
+        ft += 1.0;
+    };
+    double l0 = 0.0, l1 = 0.0, l2 = 0.0, l3 = 0.0;
+    for (int t = 0; t <= i; ++t) {
+        const bool dry = !(da > 0.0);
+        if (t == lo) l0 = s0, l1 = s1, l2 = p0, l3 = p1;
+        step(t);
+        if (dry && t >= lo) l0 = s0, l1 = s1, l2 = p0, l3 = p1;
+    }
+    const double m0 = s0, m1 = s1, m2 = p0, m3 = p1;
+    for (int t = i + 1; t <= hi && da > 0.0; ++t) step(t);
+    const double fi = (double)i;
+    double a_sum = (1.0 - fi / w) * (m0 - l0) + (m1 - l1) / w;
+    a_sum += (1.0 + fi / w) * (s0 - m0) - (s1 - m1) / w;
+    double p_sum = (1.0 - fi / w) * (m2 - l2) + (m3 - l3) / w;
+    p_sum += (1.0 + fi / w) * (p0 - m2) - (p1 - m3) / w;
+    const double radius = p_sum > 0.0 ? pixel * a_sum / p_sum : di;
+    const double cb = cbrt(radius);
+    return weight * di * (cb * cb);
+}
+
+// The face tables (_face_table, wadi2d/tables/core.py:44-79, and the local radius's conveyance), a group of GF faces
+// in a row along their own line at a time (GF divides 32: a column of a tile's west faces, a row of its north faces).
+// The faces of a group share one line of GF k + 2 margin pixels, read once; then every (face, row, pixel) is a thread's
+// own sweep along it (local_term), and every (face, row) a thread that adds its pixels' terms in order. The work is
+// FP64 and the sweeps' instructions bound it. A thread a face with its nine line arrays in shared memory, as this was
+// first written, left 63 threads a SM on lines of 44 pixels and 9 on lines of 298.
+// LINE_SMEM: the group's line in shared memory, else (a line too long for it) in the caller's workspace, GF = 1.
+struct FaceShape {
+    int gf, fc;      // faces a group; of them, whose terms are held at a time
+    int line;        // pixels of a group's line
+};
+template <bool LINE_SMEM>
+__global__ void __launch_bounds__(FACE_THREADS) face_tables_kernel(TableArgs A, FaceShape F) {
+    extern __shared__ double sws[];
+    __shared__ double s_zf[TILE], s_top[TILE];
+    __shared__ int s_e[TILE];  // pixels the conveyance line reaches past the face's ends, -1: the strips' sum
+    const int k = A.k, rows = A.rows, last = rows - 1, GF = F.gf, tid = threadIdx.x;
+    double* terms = sws;
+    double* ext = LINE_SMEM ? sws + (size_t)F.fc * rows * k : A.ws + (size_t)blockIdx.x * 2 * F.line;
+    double* hs = ext + F.line;
+    const int per = TILE / GF;
+    const int64_t groups = (int64_t)(A.ntiles - 1) * 2 * TILE * per;
+    for (int64_t g = blockIdx.x; g < groups; g += gridDim.x) {
+        const int sub = (int)(g % per), c = (int)(g / per % TILE), axis = (int)(g / (per * TILE) & 1);
+        const int t = (int)(g / (per * TILE * 2)) + 1;
+        // the group's first face, and the step from one to the next
+        const int jj0 = axis == 0 ? sub * GF : c, ii0 = axis == 0 ? c : sub * GF;
+        const int64_t j0 = (int64_t)A.tiles[2 * t] * TILE + jj0, i0 = (int64_t)A.tiles[2 * t + 1] * TILE + ii0;
+        const int dj = axis == 0, di = axis != 0;
+        for (int s = tid; s < F.line; s += FACE_THREADS) ext[s] = edge_pixel(A, axis, j0 * k, i0 * k, s - A.margin);
+        __syncthreads();
+        if (A.local)
+            for (int s = tid; s < F.line - 1; s += FACE_THREADS) {
+                const double rise = ext[s + 1] - ext[s];
+                hs[s] = 0.5 * sqrt(A.pixel * A.pixel + rise * rise);
+            }
+        const double* crests = axis == 0 ? A.xcrest : A.ycrest;
+        for (int f = tid >> 5; f < GF; f += FACE_THREADS / 32) {
+            const int lane = tid & 31;
+            const int64_t cell = (j0 + f * dj) * A.nx + i0 + f * di;
+            const double crest = crests ? crests[cell] : NAN;
+            const bool natural = isnan(crest);
+            double hi = -INFINITY;
+            if (A.local && natural) {
+                for (int s = lane; s < A.nmax; s += 32) {
+                    const double v = ext[f * k + s];
+                    hi = v > hi ? v : hi;
+                }
+                for (int o = 16; o > 0; o >>= 1) {
+                    const double v = __shfl_xor_sync(0xffffffffu, hi, o);
+                    hi = v > hi ? v : hi;
+                }
+            }
+            if (lane == 0) {
+                const double* prof = ext + f * k + A.margin;
+                auto at = [&](int q) { return natural || prof[q] >= crest ? prof[q] : crest; };
+                double zf = at(0);
+                for (int q = 1; q < k; ++q) zf = at(q) < zf ? at(q) : zf;
+                double relmax = at(0) - zf;
+                for (int q = 1; q < k; ++q) {
+                    const double v = at(q) - zf;
+                    relmax = v > relmax ? v : relmax;
+                }
+                const double cut = relmax <= A.e_hi ? relmax : A.e_hi;
+                double top = cut >= A.e_lo ? cut : A.e_lo;
+                int e = -1;
+                if (A.local && natural) {
+                    // _raise_top and window_top, wadi2d/tables/core.py:354-371
+                    const double relw = hi - zf;
+                    const double cap = relw <= A.e_hi ? relw : A.e_hi;
+                    const double wtop = top >= cap ? top : cap;
+                    if (wtop > top) top = cut >= wtop ? cut : wtop;
+                    e = (int)ceil(A.beta * top / A.pixel);
+                    e = e > A.margin ? A.margin : e;
+                }
+                s_zf[f] = zf;
+                s_top[f] = top;
+                s_e[f] = e;
+                const size_t o = (size_t)t * TILE2 + (jj0 + f * dj) * TILE + ii0 + f * di;
+                (axis == 0 ? A.efx : A.efy)[o] = (float)top;
+                (axis == 0 ? A.zfx : A.zfy)[cell] = zf;
+            }
+        }
+        __syncthreads();
+        for (int f0 = 0; f0 < GF; f0 += F.fc) {
+            const int nf = GF - f0 < F.fc ? GF - f0 : F.fc;
+            for (int x = tid; x < nf * rows * k && A.local; x += FACE_THREADS) {
+                const int q = x % k, f = f0 + x / k % nf, r = x / (k * nf);
+                const int e = s_e[f];
+                if (e < 0) continue;
+                const double xr = (double)r / (double)last;
+                const double level = s_zf[f] + s_top[f] * (xr * xr);
+                const int at = f * k + A.margin - e;
+                const int64_t j = j0 + f * dj, i = i0 + f * di;
+                const double weight = A.npix ? edge_weight(A, axis, j * k, i * k, q, A.nman[j * A.nx + i]) : 1.0;
+                terms[x] = local_term(ext + at, hs + at, k + 2 * e, e + q, level, A.pixel, A.beta, weight);
+            }
+            __syncthreads();
+            for (int x = tid; x < nf * rows; x += FACE_THREADS) {
+                const int r = x % rows, fl = x / rows, f = f0 + fl;
+                const int64_t j = j0 + f * dj, i = i0 + f * di, cell = j * A.nx + i;
+                const double nm = A.nman[cell];
+                const double crest = crests ? crests[cell] : NAN;
+                const double* lengths = axis == 0 ? A.xlen : A.ylen;
+                const double length = lengths ? lengths[cell] : 1.0;
+                const double* prof = ext + f * k + A.margin;
+                const double zf = s_zf[f], xr = (double)r / (double)last;
+                const double e = s_top[f] * (xr * xr);
+                const bool strips = s_e[f] < 0;
+                double area = 0.0, conv = 0.0;
+                for (int q = 0; q < k; ++q) {
+                    const double v = prof[q] >= crest || isnan(crest) ? prof[q] : crest;
+                    const double dep = e - (v - zf);
+                    if (dep > 0.0) {
+                        area += dep;
+                        if (strips) {
+                            const double cb = cbrt(dep);
+                            conv += edge_weight(A, axis, j * k, i * k, q, nm) * dep * (cb * cb);
+                        }
+                    }
+                    if (!strips) conv += terms[(r * nf + fl) * k + q];
+                }
+                const size_t o = (size_t)t * TILE2 + (jj0 + f * dj) * TILE + ii0 + f * di;
+                float* out = (axis == 0 ? A.ftabx : A.ftaby) + (o * rows + r) * 2;
+                out[0] = (float)(A.pixel * area * length);
+                out[1] = (float)pow(A.pixel * (1.0 / nm) * conv * length, 0.6);
+            }
+            __syncthreads();  // the terms, and at the end the line and the faces' numbers, are read by every thread
+        }
     }
 }
 
@@ -423,7 +431,8 @@ __global__ void close_faces_kernel(TableArgs A) {
         const double gl = open ? zf - zbar_n : 0.0;
         const double gr = open ? zf - zbar : 0.0;
         const bool natural = open && (gl > A.tol) && (gr > A.tol);
-        const double given = axis == 0 ? A.xc[g] : A.yc[g];
+        const double* coeff = axis == 0 ? A.xc : A.yc;
+        const double given = coeff ? coeff[g] : 0.0;
         double cw = given != 0.0 ? given : (natural ? 1.7046 : 0.0);
         cw = open ? cw : 0.0;
         const size_t o = (size_t)t * TILE2 + local;
@@ -443,11 +452,13 @@ extern "C" {
 
 int64_t w2b_table_workspace_doubles(int32_t nmax, int64_t threads) { return 9 * (int64_t)(nmax + 1) * threads; }
 
-int32_t w2b_build_tables(const W2BTableIn* in, const W2BTableOut* out, void* stream) {
+}  // extern "C"
+
+// The build itself; out->ws may be null where no face line needs it.
+static int32_t build(const W2BTableIn* in, const W2BTableOut* out, void* stream) {
     if (!in || !out || !in->z || !in->nman || !in->mask || !in->tiles || in->k < 1 || in->k > KMAX || in->rows < 4 ||
         in->rows > ROWS_MAX || in->ntiles < 1 || in->ny % TILE || in->nx % TILE || in->zh < 1 || in->zw < 1)
         return W2B_EINVAL;
-    if (in->local && (!out->ws || out->ws_threads < 1)) return W2B_EINVAL;
     if (in->local && (in->margin < 0 || in->margin > W2B_TABLE_MARGIN_MAX)) return W2B_EINVAL;
     TableArgs A;
     A.z = in->z;
@@ -504,7 +515,6 @@ int32_t w2b_build_tables(const W2BTableIn* in, const W2BTableOut* out, void* str
     A.zfy = out->zfy;
     A.ws = out->ws;
     A.ws_threads = out->ws_threads;
-    if (in->local && out->ws_threads % 128) return W2B_EINVAL;
     cudaStream_t s = (cudaStream_t)stream;
     const int n = in->k * in->k;
     const int cblocks = 148 * 8;
@@ -514,33 +524,36 @@ int32_t w2b_build_tables(const W2BTableIn* in, const W2BTableOut* out, void* str
         cell_tables_kernel<256><<<cblocks, 128, 0, s>>>(A);
     else
         cell_tables_kernel<1024><<<cblocks, 128, 0, s>>>(A);
-    // the local radius's workspace: in shared memory when a CTA of at least one thread fits it (a face line of up to
-    // about 2,800 pixels), else in the caller's workspace
-    const int64_t per_thread = 9 * (int64_t)(A.nmax + 1) * (int64_t)sizeof(double);
-    const int64_t smem_threads = in->local ? FACE_SMEM_BYTES / per_thread : 0;
-    if (in->local && smem_threads >= 1) {
-        const int threads = smem_threads > 128 ? 128 : (int)smem_threads;
-        const size_t bytes = (size_t)threads * (size_t)per_thread;
-        int dev = 0, sms = 148;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (cudaFuncSetAttribute(face_tables_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) !=
-            cudaSuccess) {
-            fprintf(stderr, "libwadi_b200: w2b_build_tables: shared workspace: %s\n",
-                    cudaGetErrorString(cudaGetLastError()));
-            return W2B_ECUDA;
-        }
-        // as many CTAs a SM as their workspaces allow: short face lines leave room for several
-        int occ = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, face_tables_kernel<true>, threads, bytes) !=
-                cudaSuccess ||
-            occ < 1)
-            occ = 1;
-        face_tables_kernel<true><<<sms * occ, threads, bytes, s>>>(A);
-    } else {
-        const int64_t fthreads = in->local ? out->ws_threads : (int64_t)148 * 8 * 128;
-        face_tables_kernel<false><<<(unsigned)(fthreads / 128), 128, 0, s>>>(A);
+    // the face kernel's groups: as many faces in a row as their line and at least one face's terms fit shared memory;
+    // a single face's line beyond that (about 11,000 pixels) lies in the caller's workspace, which holds its two arrays
+    // for every CTA (each thread's share of the workspace is nine arrays of a line)
+    FaceShape F;
+    F.gf = TILE;
+    const int64_t face_terms = (int64_t)in->rows * in->k * (int64_t)sizeof(double);
+    int64_t term_faces = FACE_TERM_BYTES / face_terms;
+    term_faces = term_faces < 1 ? 1 : (term_faces > TILE ? TILE : term_faces);
+    auto line_bytes = [&](int gf) { return 2 * ((int64_t)gf * in->k + 2 * A.margin) * (int64_t)sizeof(double); };
+    while (F.gf > 1 && line_bytes(F.gf) + term_faces * face_terms > FACE_SMEM_BYTES) F.gf /= 2;
+    F.fc = (int)(term_faces < F.gf ? term_faces : F.gf);
+    F.line = (int)(F.gf * in->k + 2 * A.margin);
+    const bool line_smem = line_bytes(F.gf) + F.fc * face_terms <= FACE_SMEM_BYTES;
+    const size_t bytes = (size_t)(F.fc * face_terms + (line_smem ? line_bytes(F.gf) : 0));
+    int dev = 0, sms = 148, occ = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    auto kernel = line_smem ? face_tables_kernel<true> : face_tables_kernel<false>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, FACE_THREADS, bytes) != cudaSuccess) {
+        fprintf(stderr, "libwadi_b200: w2b_build_tables: face tables: %s\n", cudaGetErrorString(cudaGetLastError()));
+        return W2B_ECUDA;
     }
+    const int64_t groups = (int64_t)(in->ntiles - 1) * 2 * TILE * (TILE / F.gf);
+    int64_t fblocks = (int64_t)sms * (occ > 0 ? occ : 1);
+    if (!line_smem) {
+        const int64_t held = out->ws_threads * 9 * (int64_t)(A.nmax + 1) / (2 * (int64_t)F.line);
+        fblocks = fblocks < held ? fblocks : held;
+    }
+    if (groups > 0) kernel<<<(unsigned)(fblocks < groups ? fblocks : groups), FACE_THREADS, bytes, s>>>(A, F);
     close_faces_kernel<<<148 * 8, 256, 0, s>>>(A);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
@@ -550,61 +563,29 @@ int32_t w2b_build_tables(const W2BTableIn* in, const W2BTableOut* out, void* str
     return W2B_OK;
 }
 
-}  // extern "C"
+extern "C" int32_t w2b_build_tables(const W2BTableIn* in, const W2BTableOut* out, void* stream) {
+    if (!in || !out) return W2B_EINVAL;
+    if (in->local && (!out->ws || out->ws_threads < 1 || out->ws_threads % 128)) return W2B_EINVAL;
+    return build(in, out, stream);
+}
 
 // ------------------------------------------------------------------ the table build without allocation
 
-// Scratch of w2b_build_tables_noalloc: 32 MiB of file-scope device memory. Every GPU on which a process loads this
-// library holds it until the process exits, whether the entry point is called or not.
-constexpr size_t NOALLOC_SCRATCH_BYTES = (size_t)32 << 20;
-static __device__ __align__(256) double noalloc_scratch[NOALLOC_SCRATCH_BYTES / sizeof(double)];
-
-// The array's device address, looked up once per device with that device current and kept for the life of the
-// process (a cudaDeviceReset makes it stale). In host code the name noalloc_scratch is a host-side stand-in, not a
-// device address: a kernel given it would fault or read the wrong memory, so only this address is ever passed on.
-static std::mutex noalloc_mutex;
-static void* noalloc_address[256];
-
-static int noalloc_scratch_address(void** out) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 256) return W2B_ECUDA;
-    std::lock_guard<std::mutex> lock(noalloc_mutex);
-    if (!noalloc_address[dev]) {
-        void* p = nullptr;
-        const cudaError_t e = cudaGetSymbolAddress(&p, noalloc_scratch);
-        if (e != cudaSuccess || !p) {
-            fprintf(stderr, "libwadi_b200: w2b_build_tables_noalloc: cudaGetSymbolAddress: %s\n",
-                    cudaGetErrorString(e));
-            return W2B_ECUDA;
-        }
-        noalloc_address[dev] = p;
-    }
-    *out = noalloc_address[dev];
-    return W2B_OK;
-}
+// The longest face line (k + 2 margin pixels) w2b_build_tables_noalloc takes. Such a line and a face's terms fit a
+// CTA's shared memory at every k and number of rows, so the build needs no scratch at all.
+constexpr int64_t NOALLOC_LINE_MAX = 3639;
+static_assert(2 * NOALLOC_LINE_MAX * 8 + (int64_t)KMAX * ROWS_MAX * 8 <= FACE_SMEM_BYTES, "a line in shared memory");
 
 extern "C" int32_t w2b_build_tables_noalloc(const W2BTableIn* in, const W2BTableOut* out, void* stream) {
     if (!in || !out) return W2B_EINVAL;
     if (in->local && (in->margin < 0 || in->margin > W2B_TABLE_MARGIN_MAX)) return W2B_EINVAL;
+    if (in->local && in->k + 2 * (int64_t)in->margin > NOALLOC_LINE_MAX) {
+        fprintf(stderr, "libwadi_b200: w2b_build_tables_noalloc: face lines of %lld pixels: at most %lld\n",
+                (long long)(in->k + 2 * (int64_t)in->margin), (long long)NOALLOC_LINE_MAX);
+        return W2B_EINVAL;
+    }
     W2BTableOut o = *out;
     o.ws = nullptr;
     o.ws_threads = 0;
-    if (in->local) {
-        const int64_t per_thread = 9 * ((int64_t)in->k + 2 * (int64_t)in->margin + 1) * (int64_t)sizeof(double);
-        const int64_t threads = (int64_t)(NOALLOC_SCRATCH_BYTES / (size_t)per_thread) / 128 * 128;
-        if (threads < 128) {
-            fprintf(stderr,
-                    "libwadi_b200: w2b_build_tables_noalloc: face lines of %d pixels need %lld bytes of scratch for "
-                    "128 threads; the static scratch holds %zu (at most %lld pixels a line)\n",
-                    in->k + 2 * in->margin, (long long)(per_thread * 128), NOALLOC_SCRATCH_BYTES,
-                    (long long)(NOALLOC_SCRATCH_BYTES / (128 * 9 * sizeof(double)) - 1));
-            return W2B_EINVAL;
-        }
-        void* ws = nullptr;
-        const int st = noalloc_scratch_address(&ws);
-        if (st != W2B_OK) return st;
-        o.ws = static_cast<double*>(ws);
-        o.ws_threads = threads;
-    }
-    return w2b_build_tables(in, &o, stream);
+    return build(in, &o, stream);
 }

@@ -15,7 +15,6 @@ from wadi2d_b200.grid import TileGrid
 TILE_FIELDS = ("hc", "dtab", "efx", "efy", "ftabx", "ftaby", "zcx", "zcy", "flx", "frx", "glx", "grx", "cwx", "fly",
                "fry", "gly", "gry", "cwy")  # fmt: skip
 GRID_FIELDS = ("zmin", "zbar")
-WS_BYTES_MAX = 2 << 30
 
 
 class TableIn(ctypes.Structure):
@@ -102,16 +101,16 @@ def build_tables_gpu(grid: TileGrid, bed, cfg=None, manning=0.035, crest=None, l
     if not isinstance(bed.z, torch.Tensor):
         zt = d64(z)
     npt = d64(npix) if npix is not None else None
-    nman = d64(np.full((ny, nx), float(manning)) if np.isscalar(manning) else manning)
-    if crest is None:
-        nan = np.full((ny, nx), np.nan)
-        cr = dict(xcrest=nan, xlen=np.ones((ny, nx)), xc=np.zeros((ny, nx)), ycrest=nan, ylen=np.ones((ny, nx)),
-                  yc=np.zeros((ny, nx)))  # fmt: skip
-        walls = (None, None)
+    if np.isscalar(manning):
+        nman = torch.full((ny, nx), float(manning), dtype=torch.float64, device=dev)
+    else:
+        nman = d64(manning)
+    if crest is None:  # null arrays: no face edited
+        cr, walls = dict.fromkeys(("xcrest", "xlen", "xc", "ycrest", "ylen", "yc")), (None, None)
     else:
         cr = dict(xcrest=crest.xz, xlen=crest.xlen, xc=crest.xc, ycrest=crest.yz, ylen=crest.ylen, yc=crest.yc)
         walls = (crest.xwall, crest.ywall)
-    crt = {n: d64(a) for n, a in cr.items()}
+    crt = {n: None if a is None else d64(a) for n, a in cr.items()}
     wt = [u8(w) if w is not None else None for w in walls]
     mask = u8(grid.mask)
     tiles = torch.as_tensor(np.ascontiguousarray(grid.tiles, np.int32), device=dev)
@@ -121,14 +120,13 @@ def build_tables_gpu(grid: TileGrid, bed, cfg=None, manning=0.035, crest=None, l
         shape = {"dtab": (nt, 32, 32, rows), "ftabx": (nt, 32, 32, rows, 2), "ftaby": (nt, 32, 32, rows, 2)}.get(
             n, (nt, 32, 32)
         )
-        out[n] = torch.full(shape, 1.0 if n in ("efx", "efy") else 0.0, dtype=torch.float32, device=dev)
+        out[n] = torch.empty(shape, dtype=torch.float32, device=dev)  # the build writes every tile but the void one
+        out[n][0] = 1.0 if n in ("efx", "efy") else 0.0
     dense = {n: torch.zeros((ny, nx), dtype=torch.float64, device=dev) for n in ("zmin", "rel", "zfx", "zfy")}
     local = cfg.face_conveyance == "local_radius"
     margin = tile_margin(cfg, pixel, max(zshape))
     nmax = k + 2 * margin
-    threads = 148 * 8 * 128
-    per_thread = int(_L.w2b_table_workspace_doubles(nmax, 1)) * 8
-    threads = max(128, min(threads, (WS_BYTES_MAX // per_thread) // 128 * 128))
+    threads = 128  # scratch of 576 CTAs for face lines too long for shared memory
     ws = torch.empty(int(_L.w2b_table_workspace_doubles(nmax, threads)) if local else 1, dtype=torch.float64,
                      device=dev)  # fmt: skip
 
@@ -137,7 +135,7 @@ def build_tables_gpu(grid: TileGrid, bed, cfg=None, manning=0.035, crest=None, l
 
     tin = TableIn(
         zt.data_ptr(), zshape[0], zshape[1], int(getattr(bed, "row_offset", 0)), int(getattr(bed, "col_offset", 0)),
-        ptr(npt), nman.data_ptr(), *(crt[n].data_ptr() for n in ("xcrest", "xlen", "xc", "ycrest", "ylen", "yc")),
+        ptr(npt), nman.data_ptr(), *(ptr(crt[n]) for n in ("xcrest", "xlen", "xc", "ycrest", "ylen", "yc")),
         ptr(wt[0]), ptr(wt[1]), mask.data_ptr(), tiles.data_ptr(), nt, ny, nx, k, rows, int(local), margin, pixel,
         float(cfg.face_depth_min), float(cfg.face_depth_max), float(cfg.local_radius_beta), float(cfg.crest_tolerance),
     )  # fmt: skip
