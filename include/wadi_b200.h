@@ -413,6 +413,45 @@ int32_t w2b_advance_runs(void* handle, const W2BStepper* cfg, const double* t_en
  * a and b 16-byte aligned. status (device int32) is set to W2B_ETIMEOUT if a bounded wait gave up. */
 int32_t w2b_mma_gemm(const void* a, const void* b, int32_t m, int32_t n, int32_t k, const float* bias, float* c,
                      int32_t* status, void* stream);
+/* One product of the network with the element-wise work that follows it. The product: m x n = A B^T over k, with A
+ * row-major m x k (BF16), or with a_mn k x m, and B row-major n x k, or with b_mn k x n; n, k (and with a_mn m) as
+ * w2b_mma_gemm. With x, A is instead the FP32 rows x (k wide) rounded to BF16: row r the data set's row r, or with rows
+ * row rows[*step * batch + r] (step NULL: 0); rows from `valid` on are zero; h0 (m x k, BF16, or NULL) takes them.
+ * Then, v being the product plus bias (n, or NULL), each of these that is not NULL:
+ *  - w, mw, vw, wb: one Adam step of the weights w (m x n) with gradient v (step size lr, or lr_table[*step]), wb their
+ *    BF16 copy; and with gb, mb, vb one of the biases gb (m) with the column sums of A (a_mn), rows in order;
+ *  - gb without w: those column sums into gb;
+ *  - c: v (FP32);
+ *  - h (BF16): with t, scale (v - t) on the valid rows of the targets t (rows of n, picked as x's), 0 on the rest, and
+ *    partial[tile] (FP64) the squared errors of each 128 x 32 tile; else v where z (with z NULL, v itself) is positive,
+ *    0 elsewhere.
+ * x, h0, a, b, h, z, t, w, mw, vw and wb 16-byte aligned. */
+typedef struct {
+    const void *a, *b;
+    int32_t m, n, k, a_mn, b_mn;
+    int32_t valid, batch;
+    const float* x;
+    const int64_t *rows, *step;
+    void* h0;
+    const float *bias, *z, *t;
+    float* c;
+    void* h;
+    double* partial;
+    float *w, *mw, *vw, *gb, *mb, *vb;
+    void* wb;
+    const float* lr_table;
+    float scale, lr, b1, b2, eps;
+} W2BMlpOp;
+#define W2B_MLP_OPS_MAX 4
+/* Up to W2B_MLP_OPS_MAX products (host array; none reads what another writes) in one launch. */
+int32_t w2b_mlp_ops(const W2BMlpOp* ops, int32_t count, int32_t* status, void* stream);
+/* iters training steps back to back without the host: each launches the products of `ops` in `launches` launches of
+ * sizes[l] products, in order, then w2b_mlp_tick. ops and sizes are host arrays, read before the call returns. */
+int32_t w2b_mlp_train(const W2BMlpOp* ops, const int32_t* sizes, int32_t launches, int32_t iters,
+                      const double* partial, int32_t n, double count, double* loss, int64_t* step, int32_t* status,
+                      void* stream);
+/* The end of a training step: loss[*step] = (sum of partial[0 .. n) in order) / count, then *step += 1. */
+int32_t w2b_mlp_tick(const double* partial, int32_t n, double count, double* loss, int64_t* step, void* stream);
 /* out (BF16) = relu(z) (relu = 1) or z, n elements. */
 int32_t w2b_bf16_act(const float* z, int64_t n, int32_t relu, void* out, void* stream);
 /* dz (BF16) = g where z > 0, else 0. */

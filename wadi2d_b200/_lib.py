@@ -68,12 +68,23 @@ class Rain(ctypes.Structure):
 
 
 PARTIALS = 296
+MLP_OPS_MAX = 4
 INFLOWS_MAX, INFLOW_CELLS_MAX = 64, 4096
 
 
 class Inflow(ctypes.Structure):
     _fields_ = [("n", c_i32), ("start", c_vp), ("lowest", c_vp), ("min_depth", c_vp), ("cells", c_vp),
                 ("rained", c_vp), ("area", c_f64), ("volume", c_vp)]  # fmt: skip
+
+
+class MlpOp(ctypes.Structure):
+    _fields_ = (
+        [("a", c_vp), ("b", c_vp)]
+        + [(n, c_i32) for n in ("m", "n", "k", "a_mn", "b_mn", "valid", "batch")]
+        + [(n, c_vp) for n in ("x", "rows", "step", "h0", "bias", "z", "t", "c", "h", "partial", "w", "mw", "vw", "gb",
+                               "mb", "vb", "wb", "lr_table")]
+        + [(n, c_f32) for n in ("scale", "lr", "b1", "b2", "eps")]
+    )  # fmt: skip
 
 
 class Clock(ctypes.Structure):
@@ -116,6 +127,9 @@ _SIGNATURES = {
     "w2b_loop_tuning": [c_vp, c_i32, c_i32, c_i32, c_i32],
     "w2b_loop_config": [c_vp, c_vp],
     "w2b_mma_gemm": [c_vp, c_vp, c_i32, c_i32, c_i32, c_vp, c_vp, c_vp, c_vp],
+    "w2b_mlp_ops": [c_vp, c_i32, c_vp, c_vp],
+    "w2b_mlp_train": [c_vp, c_vp, c_i32, c_i32, c_vp, c_i32, c_f64, c_vp, c_vp, c_vp, c_vp],
+    "w2b_mlp_tick": [c_vp, c_i32, c_f64, c_vp, c_vp, c_vp],
     "w2b_bf16_act": [c_vp, c_i64, c_i32, c_vp, c_vp],
     "w2b_relu_back": [c_vp, c_vp, c_i64, c_vp, c_vp],
     "w2b_transpose_bf16": [c_vp, c_i32, c_i32, c_i32, c_vp, c_vp],
