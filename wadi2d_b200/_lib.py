@@ -126,6 +126,7 @@ _SIGNATURES = {
     "w2b_face_waves": [c_vp, c_i32, c_f32, c_vp, c_vp],
     "w2b_loop_tuning": [c_vp, c_i32, c_i32, c_i32, c_i32],
     "w2b_loop_config": [c_vp, c_vp],
+    "w2b_loop_resident": [c_vp, c_vp],
     "w2b_mma_gemm": [c_vp, c_vp, c_i32, c_i32, c_i32, c_vp, c_vp, c_vp, c_vp],
     "w2b_mlp_ops": [c_vp, c_i32, c_vp, c_vp],
     "w2b_mlp_train": [c_vp, c_vp, c_i32, c_i32, c_vp, c_i32, c_f64, c_vp, c_vp, c_vp, c_vp],

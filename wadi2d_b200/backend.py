@@ -380,16 +380,22 @@ class B200Backend:
         _lib.call("w2b_loop_config", self.handle, out.ctypes.data)
         keys = ("faces_per_sm", "update_per_sm", "steps_per_graph", "tuning", "faces_occupancy", "update_occupancy",
                 "strips", "strips16_occupancy", "strips8_occupancy")  # fmt: skip
-        return {k: int(v) for k, v in zip(keys, out, strict=True)}
+        res = np.zeros(4, np.int32)
+        _lib.call("w2b_loop_resident", self.handle, res.ctypes.data)
+        cfg = {k: int(v) for k, v in zip(keys, out, strict=True)}
+        cfg.update({f"resident{rows}_occupancy": int(v) for rows, v in zip((16, 8, 4), res[1:], strict=True)})
+        return {**cfg, "resident": int(res[0]), "strips4_occupancy": int(res[3])}  # 4-row strips: the resident loop alone
 
     def set_loop(self, tune: bool = True, faces_per_sm: int = 0, update_per_sm: int = 0, steps: int = 0,
-                 strips: int = 0) -> None:  # fmt: skip
+                 strips: int = 0, resident: bool = False) -> None:  # fmt: skip
         """Start the launch tuner again (``tune``), or fix the device loop's launch schedule (w2b_loop_tuning): the face
         pass's CTAs a SM in its tile form, or with ``strips`` (16 or 8) in its strip form of that many rows, the
-        update pass's CTAs a SM, steps a graph."""
-        if strips not in (0, 8, 16):
-            raise ValueError("strips: 0 (the tile form), 16 or 8")
-        code = 1 if tune else {0: 0, 16: 2, 8: 3}[strips]
+        update pass's CTAs a SM, steps a graph; with ``resident``, the resident loop of that strip form, steps a
+        launch."""
+        forms = {16: 4, 8: 5, 4: 6} if resident else {0: 0, 16: 2, 8: 3}
+        if strips not in forms:
+            raise ValueError("strips: 0 (the tile form), 16 or 8; 16, 8 or 4 in the resident loop")
+        code = 1 if tune else forms[strips]
         _lib.call("w2b_loop_tuning", self.handle, code, int(faces_per_sm), int(update_per_sm), int(steps))
 
     def max_wave(self) -> float:

@@ -1,13 +1,13 @@
 // extern "C" entry points of libwadi_b200 (declared in include/wadi_b200.h) and the host side of the handle.
 //
-// The handle binds caller-owned device buffers; the only memory it allocates is its own host record and the CUDA
-// graphs of the device loop. Ping-pong pairs (h, u, v, mx, my) are resolved through the handle's parity, which
+// The handle binds caller-owned device buffers; the only memory it allocates is its own host record (with a pinned copy
+// of the run table for the loop's read-back), the CUDA graphs of the device loop and the index of the boundary cells. Ping-pong pairs (h, u, v, mx, my) are resolved through the handle's parity, which
 // flips after every step: the reference swaps its arrays the same way (wadi2d/solver/gpu/backend.py:185-188).
 #include <cstddef>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <new>
-#include <vector>
 
 #include <cuda.h>
 
@@ -25,7 +25,10 @@ namespace w2b {
     int update_occupancy();                                                         \
     void launch_update(const TMaps& M, const StepArgs& A, int grid, cudaStream_t s); \
     int strips_occupancy(int rows);                                                 \
-    void launch_strips(int rows, const TMaps& M, const StepArgs& A, int grid, cudaStream_t s);
+    void launch_strips(int rows, const TMaps& M, const StepArgs& A, int grid, cudaStream_t s); \
+    cudaError_t resident_setup();                                                   \
+    int resident_occupancy(int rows);                                               \
+    cudaError_t launch_resident(int rows, const ResidentMaps& M, const StepArgs& A, int grid, int max_steps, cudaStream_t s);
 namespace exact {
 W2B_PASSES_DECL
 }
@@ -44,13 +47,18 @@ struct Passes {
     void (*launch_update)(const TMaps&, const StepArgs&, int, cudaStream_t);
     int (*strips_occupancy)(int);
     void (*launch_strips)(int, const TMaps&, const StepArgs&, int, cudaStream_t);
+    cudaError_t (*resident_setup)();
+    int (*resident_occupancy)(int);
+    cudaError_t (*launch_resident)(int, const ResidentMaps&, const StepArgs&, int, int, cudaStream_t);
 };
 static const Passes EXACT_PASSES = {exact::faces_setup,  exact::launch_probe,     exact::faces_occupancy,
                                     exact::launch_faces, exact::update_setup,     exact::update_occupancy,
-                                    exact::launch_update, exact::strips_occupancy, exact::launch_strips};
+                                    exact::launch_update, exact::strips_occupancy, exact::launch_strips,
+                                    exact::resident_setup, exact::resident_occupancy, exact::launch_resident};
 static const Passes FAST_PASSES = {fast::faces_setup,  fast::launch_probe,     fast::faces_occupancy,
                                    fast::launch_faces, fast::update_setup,     fast::update_occupancy,
-                                   fast::launch_update,  fast::strips_occupancy,  fast::launch_strips};
+                                   fast::launch_update,  fast::strips_occupancy,  fast::launch_strips,
+                                   fast::resident_setup, fast::resident_occupancy, fast::launch_resident};
 static const Passes& passes(const W2BParams& P) { return P.arith == W2B_ARITH_FAST ? FAST_PASSES : EXACT_PASSES; }
 
 void launch_cbrt_check(uint32_t first, uint32_t count, unsigned long long* out, cudaStream_t s);
@@ -58,11 +66,11 @@ void launch_wait_check(uint32_t polls, long long* out, cudaStream_t s);
 void launch_momentum(const StepArgs& A, int sms, cudaStream_t s);
 __global__ void boundary_kernel(StepArgs A, int control);
 __global__ void envelope_kernel(StepArgs A);
-__global__ void control_kernel(StepArgs A);
-__global__ void prestep_kernel(StepArgs A);
+__global__ void control_kernel(const __grid_constant__ StepArgs A);
+__global__ void begin_kernel(const __grid_constant__ StepArgs A, Ctl c, W2BClock one, double t_end, long long max_steps,
+                             const W2BClock* clocks, const double* t_ends);
 __global__ void setstep_kernel(StepArgs A, float dtf, int want_wave, int want_wet, int nact);
 __global__ void endstep_kernel(StepArgs A);
-__global__ void activity_kernel(StepArgs A, int only_work);
 __global__ void plan_kernel(StepArgs A, const int32_t* list, int count);
 __global__ void maxima_kernel(StepArgs A, float time, float arrive, float deep, int nact);
 __global__ void tally_kernel(StepArgs A, double dt);
@@ -72,18 +80,21 @@ __global__ void native_to_ref_kernel(const float* nat, float* ref, const int32_t
 __global__ void pack_tables_kernel(const float* dtab, const float* ftabx, const float* ftaby, float2* dtab2,
                                    float4* fx, float4* fy, int ntiles, int rows);
 __global__ void bmark_kernel(StepArgs A, int clear_words);
+__global__ void boundary_index_kernel(StepArgs A, int32_t* start, int32_t* item, int32_t* next);
 
 // A launch configuration of the device loop: the face pass's form (whole tiles, or the strip form: half tiles in
-// smaller CTAs), its CTAs a SM, the update pass's CTAs a SM, and loop steps a captured graph. Every configuration
-// computes the same bits (a face's arithmetic does not depend on the form or the grid, and the wave maximum is an
-// order-free integer max); they differ only in time.
+// smaller CTAs), its CTAs a SM, the update pass's CTAs a SM, and loop steps a launch: a captured graph of the passes'
+// kernels, or (resident) one cooperative launch that takes the steps itself, with the strip form's units. Every
+// configuration computes the same bits (a face's arithmetic does not depend on the form or the grid, and the wave
+// maximum is an order-free integer max); they differ only in time.
 struct LoopConfig {
     int faces_per_sm, update_per_sm, steps;
     int strips;  // the face pass's form: 0 whole tiles, else strips of this many rows (16 or 8)
+    int resident;
 };
-constexpr int TUNE_CANDIDATES = 7;               // the default, one change of each knob either way, two strip forms
+constexpr int TUNE_CANDIDATES = 7;  // the default, it with more steps a graph, two strip forms, three resident ones
 constexpr int FORCED = TUNE_CANDIDATES;          // the slot of a configuration the caller fixes
-constexpr int TUNE_SAMPLES = 3;                  // timed graph launches a candidate before the tuner settles
+constexpr int TUNE_SAMPLES = 3;                  // timed launches a candidate before the tuner settles
 constexpr int MAX_GRAPH_STEPS = 64;
 constexpr double TUNE_MARGIN = 0.02;
 
@@ -108,6 +119,9 @@ struct Loop {
         for (auto& v : version) v = ~0u;
     }
 };
+
+constexpr int RESIDENT_ROWS[3] = {16, 8, 4};  // the resident loop's strip heights
+static int resident_index(int rows) { return rows == 16 ? 0 : (rows == 8 ? 1 : 2); }
 
 struct Handle {
     W2BGridDesc g{};
@@ -134,7 +148,12 @@ struct Handle {
     int faces_blocks = 296;  // resident CTAs of the face pass
     int faces_occ = 2, update_occ = 1;  // resident CTAs a SM of the two passes
     int strips16_occ = 4, strips8_occ = 8;  // resident CTAs a SM of the face pass's strip forms
+    int resident_occ[3] = {1, 1, 1};  // and of the resident loop's, in the order of RESIDENT_ROWS
+    int32_t *bstart = nullptr, *bitem = nullptr;  // the boundary cells by tile (StepArgs::bstart, bitem)
+    int bitem_held = 0;
+    char* host = nullptr;  // pinned: the run table and the control block as read back, and a batch's clocks and ends
     TMaps tmaps;
+    ResidentMaps rmaps[3];
     unsigned version = 0;   // bumped whenever a graph would capture stale arguments
     Loop loop;
     cudaStream_t cap = nullptr;  // private stream the loop graphs are captured on (a legacy stream cannot be)
@@ -200,6 +219,8 @@ static StepArgs make_args(const Handle& H) {
     A.bkind = H.bkind;
     A.bd0 = H.bd0;
     A.bh0 = H.bh0;
+    A.bstart = H.nb ? H.bstart : nullptr;
+    A.bitem = H.bitem;
     A.ntally = H.ntally;
     A.tface = H.tface;
     A.taxis = H.taxis;
@@ -301,8 +322,8 @@ static int build_tmaps(Handle& H) {
     // the strip forms' boxes, 40 columns of the rows the face arithmetic reads around a strip of `rows` rows: the
     // velocities rows + 4 (two above, two below), the y discharge rows + 2, the x lip rows, depth, mean depth, x
     // discharge and y lip rows + 1 (one above); 32 x rows for the momenta
-    for (const int rows : {16, 8}) {
-        StripMaps& S = rows == 16 ? H.tmaps.s16 : H.tmaps.s8;
+    for (const int rows : RESIDENT_ROWS) {
+        StripMaps& S = H.rmaps[resident_index(rows)].s;
         auto strip = [&](CUtensorMap* m, const float* q, int extra) {
             if (st == W2B_OK) st = encode_2d(enc, m, q, H.g, H.L, 40, (uint32_t)(rows + extra));
         };
@@ -321,7 +342,16 @@ static int build_tmaps(Handle& H) {
             strip_own(&S.mx[p], B.mx[p]);
             strip_own(&S.my[p], B.my[p]);
         }
+        // the resident loop's update of a strip: one row above to two below; its own rows of the residual and source
+        UpdateMaps& U = H.rmaps[resident_index(rows)].u;
+        strip(&U.qx1, B.qx1, 3);
+        strip(&U.qy1, B.qy1, 3);
+        for (int p = 0; p < 2; ++p) strip(&U.h[p], B.h[p], 3);
+        strip_own(&U.res, B.res);
+        strip_own(&U.src, B.src);
     }
+    H.tmaps.s16 = H.rmaps[0].s;
+    H.tmaps.s8 = H.rmaps[1].s;
     return st;
 }
 
@@ -337,20 +367,19 @@ static void drop_graphs(Handle& H) {
     for (int c = 0; c <= TUNE_CANDIDATES; ++c) drop_graph(H, c);
 }
 
-// The tuner's candidates: the occupancy-given default (both passes at their resident CTAs a SM, 16 steps a graph),
-// and from it one CTA a SM fewer in the face pass, half the update pass's, 8 and 32 steps a graph, and the face pass
-// in its strip form at its resident CTAs a SM.
+// The tuner's candidates: the occupancy-given default (both passes at their resident CTAs a SM, 16 steps a graph), it
+// with 32 steps a graph, the face pass in its strip forms, and the resident loop with each strip height.
 static void init_loop(Handle& H) {
     Loop& L = H.loop;
     const int F = H.faces_occ, U = H.update_occ;
+    auto fit = [&](int occ) { return occ < U ? occ : U; };
     L.ncand = 0;
-    L.cand[L.ncand++] = {F, U, 16, 0};
-    if (F > 1) L.cand[L.ncand++] = {F - 1, U, 16, 0};
-    if (U > 1) L.cand[L.ncand++] = {F, (U + 1) / 2, 16, 0};
-    L.cand[L.ncand++] = {F, U, 8, 0};
-    L.cand[L.ncand++] = {F, U, 32, 0};
-    L.cand[L.ncand++] = {H.strips16_occ, U, 16, 16};
-    L.cand[L.ncand++] = {H.strips8_occ, U, 16, 8};
+    L.cand[L.ncand++] = {F, U, 16, 0, 0};
+    L.cand[L.ncand++] = {F, U, 32, 0, 0};
+    L.cand[L.ncand++] = {H.strips16_occ, U, 16, 16, 0};
+    L.cand[L.ncand++] = {H.strips8_occ, U, 16, 8, 0};
+    for (int i = 0; i < 3; ++i)
+        L.cand[L.ncand++] = {H.resident_occ[i], fit(H.resident_occ[i]), 32, RESIDENT_ROWS[i], 1};
     L.cand[FORCED] = L.cand[0];
     for (int c = 0; c < TUNE_CANDIDATES; ++c) {
         L.sec[c] = 0.0;
@@ -378,7 +407,7 @@ static int boundary_grid(const Handle& H, int control) {
 // which set the launch grids and the tuner's candidates.
 static int set_passes(Handle& H) {
     for (const Passes* X : {&EXACT_PASSES, &FAST_PASSES}) {
-        if (X->update_setup() != cudaSuccess || X->faces_setup() != cudaSuccess)
+        if (X->update_setup() != cudaSuccess || X->faces_setup() != cudaSuccess || X->resident_setup() != cudaSuccess)
             return cuda_status(cudaGetLastError(), "pass setup");
     }
     const Passes& X = passes(H.P);
@@ -388,10 +417,19 @@ static int set_passes(Handle& H) {
     H.faces_occ = focc > 0 ? focc : 1;
     H.strips16_occ = s16 > 0 ? s16 : 1;
     H.strips8_occ = s8 > 0 ? s8 : 1;
+    for (int i = 0; i < 3; ++i) {
+        const int occ = X.resident_occupancy(RESIDENT_ROWS[i]);
+        H.resident_occ[i] = occ > 0 ? occ : 1;
+    }
     H.step_blocks = H.sms * H.update_occ;
     H.faces_blocks = H.sms * H.faces_occ;
     init_loop(H);
     return W2B_OK;
+}
+
+// The pinned buffer: the run table, the control block, a batch's clocks and end times.
+static size_t host_bytes(int nruns) {
+    return run_table_bytes(nruns) + W2B_CTL_BYTES + (sizeof(W2BClock) + sizeof(double)) * (size_t)nruns;
 }
 
 // The face pass of a host-driven step (w2b_step, w2b_step_timed) over n tiles: in the form and at the CTAs a SM the
@@ -399,8 +437,10 @@ static int set_passes(Handle& H) {
 static void launch_faces_host(Handle& H, const StepArgs& A, int n, cudaStream_t s) {
     const LoopConfig& C = H.loop.cand[H.loop.chosen];
     if (!H.loop.tuning && C.strips) {
-        const int g = H.sms * C.faces_per_sm, units = (TILE / C.strips) * n;
-        passes(H.P).launch_strips(C.strips, H.tmaps, A, units < g ? units : g, s);
+        const int rows = C.strips == 16 ? 16 : 8;
+        const int occ = !C.resident ? C.faces_per_sm : (rows == 16 ? H.strips16_occ : H.strips8_occ);
+        const int g = H.sms * occ, units = (TILE / rows) * n;
+        passes(H.P).launch_strips(rows, H.tmaps, A, units < g ? units : g, s);
     } else {
         passes(H.P).launch_faces(H.tmaps, A, faces_grid(H, n), s);
     }
@@ -410,7 +450,6 @@ static void launch_faces_host(Handle& H, const StepArgs& A, int n, cudaStream_t 
 static int launch_loop_step(Handle& H, const LoopConfig& C, cudaStream_t s) {
     StepArgs A = make_args(H);
     A.list = A.work;
-    const dim3 blk(32, 8);
     const int grid = blocks_for(H, H.g.ntiles - 1);
     const int tiles = H.g.ntiles - 1 > 0 ? H.g.ntiles - 1 : 1;
     const int fgrid = H.sms * C.faces_per_sm, ugrid = H.sms * C.update_per_sm;
@@ -423,8 +462,32 @@ static int launch_loop_step(Handle& H, const LoopConfig& C, cudaStream_t s) {
     envelope_kernel<<<H.sms * 2, TILE2, 0, s>>>(A);
     boundary_kernel<<<boundary_grid(H, 1), 256, 0, s>>>(A, 1);
     control_kernel<<<1, 1024, 0, s>>>(A);  // clocks, rebuild and work list, the next step's settings
-    plan_kernel<<<grid, blk, 0, s>>>(A, A.woken, -1);
+    plan_kernel<<<grid, 256, 0, s>>>(A, A.woken, -1);
     CKL("loop step");
+    return W2B_OK;
+}
+
+// Up to C.steps steps of the resident loop. Its CTAs wait for one another, so two such launches of one process must
+// not share a GPU half resident each: every launch waits for the one before it on the device, whatever its stream.
+static int launch_loop_resident(Handle& H, const LoopConfig& C, cudaStream_t s) {
+    static struct {
+        std::mutex mutex;
+        cudaEvent_t last = nullptr;
+    } lanes[64];
+    const int64_t units = (int64_t)(TILE / C.strips) * (H.g.ntiles - 1);
+    const int64_t most = (int64_t)H.sms * C.faces_per_sm - 1;
+    const int workers = (int)(units < most ? (units > 0 ? units : 1) : most);
+    int dev = 0;
+    CK(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64 || workers < 1) return W2B_EINVAL;
+    auto& lane = lanes[dev];
+    std::lock_guard<std::mutex> lock(lane.mutex);
+    if (!lane.last)
+        CK(cudaEventCreateWithFlags(&lane.last, cudaEventDisableTiming));
+    else
+        CK(cudaStreamWaitEvent(s, lane.last, 0));
+    CK(passes(H.P).launch_resident(C.strips, H.rmaps[resident_index(C.strips)], make_args(H), workers + 1, C.steps, s));
+    CK(cudaEventRecord(lane.last, s));
     return W2B_OK;
 }
 
@@ -527,11 +590,20 @@ int32_t w2b_create(const W2BGridDesc* grid, const W2BParams* params, const W2BBu
         delete H;
         return cuda_status(cudaGetLastError(), "w2b_create control block");
     }
+    if (cudaMemset(reinterpret_cast<char*>(H->ctl()) + GRID_STATE_AT, 0, sizeof(GridState)) != cudaSuccess) {
+        delete H;
+        return cuda_status(cudaGetLastError(), "w2b_create grid state");
+    }
     if (H->nruns == 1 && cudaMemcpy(H->R.dx, &H->P.dx, sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess) {
         delete H;
         return cuda_status(cudaGetLastError(), "w2b_create run table");
     }
+    if (cudaMallocHost(&H->host, host_bytes(H->nruns)) != cudaSuccess) {
+        delete H;
+        return cuda_status(cudaGetLastError(), "w2b_create read-back");
+    }
     if (cudaStreamCreateWithFlags(&H->cap, cudaStreamNonBlocking) != cudaSuccess) {
+        cudaFreeHost(H->host);
         delete H;
         return cuda_status(cudaGetLastError(), "w2b_create stream");
     }
@@ -540,6 +612,7 @@ int32_t w2b_create(const W2BGridDesc* grid, const W2BParams* params, const W2BBu
         for (auto& e : H->loop.ev)
             if (e) cudaEventDestroy(e);
         cudaStreamDestroy(H->cap);
+        cudaFreeHost(H->host);
         delete H;
         return cuda_status(cudaGetLastError(), "w2b_create events");
     }
@@ -559,6 +632,9 @@ int32_t w2b_destroy(void* handle) {
     for (auto& e : H->loop.ev)
         if (e) cudaEventDestroy(e);
     if (H->cap) cudaStreamDestroy(H->cap);
+    if (H->host) cudaFreeHost(H->host);
+    if (H->bstart) cudaFree(H->bstart);
+    if (H->bitem) cudaFree(H->bitem);
     delete H;
     return W2B_OK;
 }
@@ -606,6 +682,14 @@ int32_t w2b_set_boundary(void* handle, int32_t n, const int32_t* cell, const int
                          const float* d0, const float* h0) {
     if (!handle || n < 0 || (n && (!cell || !ref || !kind || !d0 || !h0))) return W2B_EINVAL;
     Handle* H = static_cast<Handle*>(handle);
+    if (n && !H->bstart) CK(cudaMalloc(&H->bstart, sizeof(int32_t) * (2 * (size_t)H->g.ntiles + 2)));
+    if (n > H->bitem_held) {  // the index may be in use by steps in flight: cudaFree waits for them
+        if (H->bitem) CK(cudaFree(H->bitem));
+        H->bitem = nullptr;
+        H->bitem_held = 0;
+        CK(cudaMalloc(&H->bitem, sizeof(int32_t) * (size_t)n));
+        H->bitem_held = n;
+    }
     H->nb = n;
     H->bcell = cell;
     H->bref = ref;
@@ -615,7 +699,10 @@ int32_t w2b_set_boundary(void* handle, int32_t n, const int32_t* cell, const int
     H->version++;
     const StepArgs A = make_args(*H);
     bmark_kernel<<<64, 256>>>(A, H->g.ntiles * TILE);
-    if (n) bmark_kernel<<<64, 256>>>(A, 0);
+    if (n) {
+        bmark_kernel<<<64, 256>>>(A, 0);
+        boundary_index_kernel<<<1, 1024>>>(A, H->bstart, H->bitem, H->bstart + H->g.ntiles + 2);
+    }
     CKL("w2b_set_boundary");
     return W2B_OK;
 }
@@ -722,7 +809,7 @@ int32_t w2b_refresh_plan(void* handle, const int32_t* tiles, int32_t n, void* st
     Handle* H = static_cast<Handle*>(handle);
     if (!n) return W2B_OK;
     const StepArgs A = make_args(*H);
-    plan_kernel<<<blocks_for(*H, n), dim3(32, 8), 0, (cudaStream_t)stream>>>(A, tiles, n);
+    plan_kernel<<<blocks_for(*H, n), 256, 0, (cudaStream_t)stream>>>(A, tiles, n);
     CKL("w2b_refresh_plan");
     return W2B_OK;
 }
@@ -908,25 +995,9 @@ static void tune_sample(Handle& H, int c, long long live, float ms) {
         if (k != best) drop_graph(H, k);
 }
 
-// A single run's loop settings and clock, written by one thread from its arguments. A copy from the host would be
-// queued on a copy engine behind any large upload in flight on another stream (the next window's source, staged while
-// this window steps) and wait for it; kernel arguments travel with the launch. The stored-momenta flag stays.
-__global__ void advance_setup_kernel(Ctl c, double t, double dt, double t_end, long long nsteps, long long max_steps,
-                                     int32_t refresh_due, Ctl* ctl, RunTab R) {
-    c.m_stored = ctl->m_stored;
-    *ctl = c;
-    R.t[0] = t;
-    R.dt[0] = dt;
-    R.t_end[0] = t_end;
-    R.nsteps[0] = nsteps;
-    R.steps_run[0] = 0;
-    R.max_steps[0] = max_steps;
-    R.refresh_due[0] = refresh_due;
-    R.status[0] = 0;
-}
-
-// The device-resident loop. Steps run in chunks of a captured graph (the launch configuration's steps), every running
-// run advancing one of its own steps each graph step; after each chunk the host reads the runs' clocks once.
+// The device-resident loop. Steps run in chunks (a captured graph, or one launch of the resident loop, of the launch
+// configuration's steps), every running run advancing one of its own steps each loop step; after each chunk the host
+// reads the run table and the control block once, into pinned memory.
 static int advance_runs(Handle* H, const W2BStepper* cfg, const double* t_end, int64_t max_steps, W2BClock* clocks,
                         cudaStream_t s) {
     const int n = H->nruns;
@@ -944,59 +1015,49 @@ static int advance_runs(Handle* H, const W2BStepper* cfg, const double* t_end, i
     c.wave_floor = cfg->wave_floor;
     c.dt_max = cfg->dt_max;
     c.dt_min = cfg->dt_min;
-    std::vector<double> t(n), dt(n), te(t_end, t_end + n);
-    std::vector<long long> ns(n), zero(n, 0), ms(n, (long long)max_steps);
-    std::vector<int32_t> rd(n), st(n, 0);
-    for (int r = 0; r < n; ++r) {
-        t[r] = clocks[r].t;
-        dt[r] = clocks[r].dt;
-        ns[r] = clocks[r].nsteps;
-        rd[r] = clocks[r].refresh_due;
+    // A single run's settings and clock travel as kernel arguments: a copy from the host would be queued on a copy
+    // engine behind any large upload in flight on another stream (the next window's source, staged while this window
+    // steps) and wait for it. A batch's are read from the pinned buffer by the kernel itself.
+    char* const held = H->host;
+    Ctl* const hctl = reinterpret_cast<Ctl*>(held + run_table_bytes(n));
+    W2BClock* const hclocks = reinterpret_cast<W2BClock*>(held + run_table_bytes(n) + W2B_CTL_BYTES);
+    double* const hends = reinterpret_cast<double*>(hclocks + n);
+    if (n > 1) {
+        memcpy(hclocks, clocks, sizeof(W2BClock) * n);
+        memcpy(hends, t_end, sizeof(double) * n);
     }
-    const RunTab& R = H->R;
-    if (n == 1) {  // by kernel arguments: no host-to-device copy (see advance_setup_kernel)
-        advance_setup_kernel<<<1, 1, 0, s>>>(c, t[0], dt[0], te[0], ns[0], ms[0], rd[0], H->ctl(), R);
-        CKL("advance settings");
-    } else {
-        CK(cudaMemcpyAsync(H->ctl(), &c, offsetof(Ctl, m_stored), cudaMemcpyHostToDevice, s));  // the flag stays
-        CK(cudaMemcpyAsync(R.t, t.data(), 8 * n, cudaMemcpyHostToDevice, s));
-        CK(cudaMemcpyAsync(R.dt, dt.data(), 8 * n, cudaMemcpyHostToDevice, s));
-        CK(cudaMemcpyAsync(R.t_end, te.data(), 8 * n, cudaMemcpyHostToDevice, s));
-        CK(cudaMemcpyAsync(R.nsteps, ns.data(), 8 * n, cudaMemcpyHostToDevice, s));
-        CK(cudaMemcpyAsync(R.steps_run, zero.data(), 8 * n, cudaMemcpyHostToDevice, s));
-        CK(cudaMemcpyAsync(R.max_steps, ms.data(), 8 * n, cudaMemcpyHostToDevice, s));
-        CK(cudaMemcpyAsync(R.refresh_due, rd.data(), 4 * n, cudaMemcpyHostToDevice, s));
-        CK(cudaMemcpyAsync(R.status, st.data(), 4 * n, cudaMemcpyHostToDevice, s));
-    }
-    activity_kernel<<<1, 1024, 0, s>>>(make_args(*H), 1);  // the work list of the runs that take a step
-    prestep_kernel<<<1, 1024, 0, s>>>(make_args(*H));      // the first step's settings; each step sets the next's
-    CKL("advance work list");
+    // the work list of the runs that take a step, and the first step's settings; each step sets the next's
+    begin_kernel<<<1, 1024, 0, s>>>(make_args(*H), c, clocks[0], t_end[0], (long long)max_steps,
+                                    n > 1 ? hclocks : nullptr, n > 1 ? hends : nullptr);
+    CKL("advance begin");
+    const RunTab T = run_table(held, n);
     Loop& L = H->loop;
-    std::vector<long long> run(n);
     long long ran_before = 0;  // loop steps so far in this call (the largest steps_run of any run)
-    int32_t gstatus = 0;
     int end = 1, have_prev = 0;  // ev[end] takes this launch's end; ev[3 - end] holds the last one's, if have_prev
     if (L.tuning)  // every candidate's graph before the first timed launch: no capture falls inside a timing
         for (int k = 0; k < L.ncand; ++k) {
-            const int stc = loop_graph(*H, k);
+            const int stc = L.cand[k].resident ? W2B_OK : loop_graph(*H, k);
             if (stc != W2B_OK) return stc;
         }
     for (;;) {
         const bool timed = L.tuning != 0;
         const int c = timed ? L.next : L.chosen;
-        const int stc = loop_graph(*H, c);
+        const bool resident = L.cand[c].resident != 0;
+        int stc = resident ? W2B_OK : loop_graph(*H, c);
         if (stc != W2B_OK) return stc;
         if (timed && !have_prev) CK(cudaEventRecord(L.ev[0], s));
-        CK(cudaGraphLaunch(L.exec[c], s));
+        if (resident)
+            stc = launch_loop_resident(*H, L.cand[c], s);
+        else
+            CK(cudaGraphLaunch(L.exec[c], s));
+        if (stc != W2B_OK) return stc;
         if (timed) CK(cudaEventRecord(L.ev[end], s));
-        CK(cudaMemcpyAsync(t.data(), R.t, 8 * n, cudaMemcpyDeviceToHost, s));
-        CK(cudaMemcpyAsync(run.data(), R.steps_run, 8 * n, cudaMemcpyDeviceToHost, s));
-        CK(cudaMemcpyAsync(st.data(), R.status, 4 * n, cudaMemcpyDeviceToHost, s));
-        CK(cudaMemcpyAsync(&gstatus, &H->ctl()->status, 4, cudaMemcpyDeviceToHost, s));
+        CK(cudaMemcpyAsync(held, H->B.runs, run_table_bytes(n), cudaMemcpyDeviceToHost, s));
+        CK(cudaMemcpyAsync(hctl, H->ctl(), sizeof(Ctl), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
         if (timed) {
             long long ran = 0;
-            for (int r = 0; r < n; ++r) ran = run[r] > ran ? run[r] : ran;
+            for (int r = 0; r < n; ++r) ran = T.steps_run[r] > ran ? T.steps_run[r] : ran;
             float ms = 0.0f;
             CK(cudaEventElapsedTime(&ms, have_prev ? L.ev[3 - end] : L.ev[0], L.ev[end]));
             tune_sample(*H, c, ran - ran_before, ms);
@@ -1006,37 +1067,29 @@ static int advance_runs(Handle* H, const W2BStepper* cfg, const double* t_end, i
         } else {
             have_prev = 0;
         }
-        bool done = gstatus != 0;
+        bool done = hctl->status != 0;
         if (!done) {
             done = true;
             for (int r = 0; r < n; ++r)
-                if (st[r] == 0 && t[r] < te[r] - 1e-9 && run[r] < ms[r]) done = false;
+                if (T.status[r] == 0 && T.t[r] < t_end[r] - 1e-9 && T.steps_run[r] < max_steps) done = false;
         }
         if (done) break;
     }
-    std::vector<uint32_t> wb(n);
-    std::vector<int32_t> par(n);
-    CK(cudaMemcpyAsync(dt.data(), R.dt, 8 * n, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(ns.data(), R.nsteps, 8 * n, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(wb.data(), R.wave_last, 4 * n, cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(par.data(), R.parity, 4 * n, cudaMemcpyDeviceToHost, s));
-    int32_t nact = 0;
-    CK(cudaMemcpyAsync(&nact, &H->ctl()->nact, 4, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    H->nact = nact;
-    H->cur = par[0];
+    const int32_t gstatus = hctl->status;
+    if (gstatus)  // a wait gave up: the grid barrier's counters may be anything
+        CK(cudaMemsetAsync(reinterpret_cast<char*>(H->ctl()) + GRID_STATE_AT, 0, sizeof(GridState), s));
+    H->nact = hctl->nact;
+    H->cur = T.parity[0];
     int32_t first = gstatus;
     for (int r = 0; r < n; ++r) {
-        clocks[r].t = t[r];
-        clocks[r].dt = dt[r];
-        clocks[r].nsteps = ns[r];
+        clocks[r].t = T.t[r];
+        clocks[r].dt = T.dt[r];
+        clocks[r].nsteps = T.nsteps[r];
         clocks[r].refresh_due = 0;
-        clocks[r].status = st[r] != 0 ? st[r] : gstatus;
-        float w;
-        memcpy(&w, &wb[r], 4);
-        clocks[r].wave_max = w;
-        clocks[r].nact = nact;
-        if (!first && st[r]) first = st[r];
+        clocks[r].status = T.status[r] != 0 ? T.status[r] : gstatus;
+        clocks[r].wave_max = T.wave_last[r];
+        clocks[r].nact = hctl->nact;
+        if (!first && T.status[r]) first = T.status[r];
     }
     return first;
 }
@@ -1065,13 +1118,14 @@ int32_t w2b_loop_tuning(void* handle, int32_t tune, int32_t faces_per_sm, int32_
         init_loop(*H);
         return W2B_OK;
     }
-    if (tune < 0 || tune > 3) return W2B_EINVAL;
-    const int strips = tune == 2 ? 16 : (tune == 3 ? 8 : 0);
-    const int occ = strips == 16 ? H->strips16_occ : (strips == 8 ? H->strips8_occ : H->faces_occ);
+    if (tune < 0 || tune > 6) return W2B_EINVAL;
+    const int resident = tune >= 4, strips = resident ? RESIDENT_ROWS[tune - 4] : (tune == 2 ? 16 : (tune == 3 ? 8 : 0));
+    const int occ = resident ? H->resident_occ[tune - 4]
+                             : (strips == 16 ? H->strips16_occ : (strips == 8 ? H->strips8_occ : H->faces_occ));
     if (faces_per_sm < 1 || faces_per_sm > occ || update_per_sm < 1 ||
         update_per_sm > H->update_occ || steps < 1 || steps > MAX_GRAPH_STEPS)
         return W2B_EINVAL;
-    L.cand[FORCED] = {faces_per_sm, update_per_sm, steps, strips};
+    L.cand[FORCED] = {faces_per_sm, update_per_sm, steps, strips, resident};
     drop_graph(*H, FORCED);
     L.chosen = FORCED;
     L.tuning = 0;
@@ -1092,6 +1146,15 @@ int32_t w2b_loop_config(void* handle, int32_t* out) {
     out[6] = C.strips;
     out[7] = H->strips16_occ;
     out[8] = H->strips8_occ;
+    return W2B_OK;
+}
+
+int32_t w2b_loop_resident(void* handle, int32_t* out) {
+    if (!handle || !out) return W2B_EINVAL;
+    const Handle* H = static_cast<const Handle*>(handle);
+    const Loop& L = H->loop;
+    out[0] = L.cand[L.tuning ? L.next : L.chosen].resident;
+    for (int i = 0; i < 3; ++i) out[1 + i] = H->resident_occ[i];
     return W2B_OK;
 }
 

@@ -37,7 +37,15 @@ struct Ctl {
     // of the ping-pong pair). Last member: the device loop's settings overwrite the block up to it.
     int32_t m_stored;
 };
-static_assert(sizeof(Ctl) <= W2B_CTL_BYTES, "control block too large");
+// Behind it in the control block, on a line of its own: the resident loop's grid barrier (arrivals, counted up, and the
+// CTAs that have left; zero between launches) and whether the step in flight ends with a rebuild of the lists.
+struct GridState {
+    uint32_t arrived, left;
+    int32_t rebuild;
+};
+constexpr int GRID_STATE_AT = 512;
+static_assert(sizeof(Ctl) <= GRID_STATE_AT && GRID_STATE_AT + sizeof(GridState) <= W2B_CTL_BYTES,
+              "control block too large");
 
 constexpr uint32_t ANY_RUN = 1u, ANY_WAVE = 2u, ANY_ACT = 4u, ANY_MAX = 8u;
 // per-run flags of this step
@@ -52,7 +60,25 @@ struct RunTab {
     uint32_t* wave_bits;  // max wave speed of the run's tiles, as float bits (waves are never negative)
     int32_t* parity;      // the run's current half of the ping-pong pairs
     float* wave_last;     // the wave maximum of the run's last refresh step (what the clock reports)
+    // a second set of the step's settings: the resident loop forms the next step's while this one's are read
+    double *dt_tally2, *t_new, *t_new2;  // t_new: the clock at the end of the step
+    float *dtf2, *max_time2;
+    int32_t *flags2, *parity2;
+    uint32_t* wave_bits2;
 };
+
+// The settings of the step in flight, one of the two sets.
+struct StepView {
+    double *dt_tally, *t_new;
+    float *dtf, *max_time;
+    int32_t *flags, *parity;
+    uint32_t* wave_bits;
+};
+
+__device__ __forceinline__ StepView step_view(const RunTab& R, int b) {
+    return b ? StepView{R.dt_tally2, R.t_new2, R.dtf2, R.max_time2, R.flags2, R.parity2, R.wave_bits2}
+             : StepView{R.dt_tally, R.t_new, R.dtf, R.max_time, R.flags, R.parity, R.wave_bits};
+}
 
 // Whether run r takes another step (the loop test of wadi2d/solver/stepper.py:106, plus the batch's step limit).
 __device__ __forceinline__ bool live_run(const RunTab& R, int r, const Ctl* ctl) {
@@ -62,7 +88,7 @@ __device__ __forceinline__ bool live_run(const RunTab& R, int r, const Ctl* ctl)
 // Layout of a run table of nruns entries in one device block: each array 256-byte aligned.
 __host__ __device__ inline size_t run_table_bytes(int nruns) {
     const size_t a = ((size_t)nruns * 8 + 255) / 256 * 256, b = ((size_t)nruns * 4 + 255) / 256 * 256;
-    return 8 * a + 9 * b;
+    return 11 * a + 14 * b;
 }
 
 __host__ __device__ inline RunTab run_table(void* base, int nruns) {
@@ -77,7 +103,10 @@ __host__ __device__ inline RunTab run_table(void* base, int nruns) {
     R.nsteps = reinterpret_cast<long long*>(p + 5 * a);
     R.steps_run = reinterpret_cast<long long*>(p + 6 * a);
     R.max_steps = reinterpret_cast<long long*>(p + 7 * a);
-    char* q = p + 8 * a;
+    R.dt_tally2 = reinterpret_cast<double*>(p + 8 * a);
+    R.t_new = reinterpret_cast<double*>(p + 9 * a);
+    R.t_new2 = reinterpret_cast<double*>(p + 10 * a);
+    char* q = p + 11 * a;
     R.dtf = reinterpret_cast<float*>(q);
     R.max_time = reinterpret_cast<float*>(q + b);
     R.dx = reinterpret_cast<float*>(q + 2 * b);
@@ -87,6 +116,11 @@ __host__ __device__ inline RunTab run_table(void* base, int nruns) {
     R.wave_bits = reinterpret_cast<uint32_t*>(q + 6 * b);
     R.parity = reinterpret_cast<int32_t*>(q + 7 * b);
     R.wave_last = reinterpret_cast<float*>(q + 8 * b);
+    R.dtf2 = reinterpret_cast<float*>(q + 9 * b);
+    R.max_time2 = reinterpret_cast<float*>(q + 10 * b);
+    R.flags2 = reinterpret_cast<int32_t*>(q + 11 * b);
+    R.parity2 = reinterpret_cast<int32_t*>(q + 12 * b);
+    R.wave_bits2 = reinterpret_cast<uint32_t*>(q + 13 * b);
     return R;
 }
 
@@ -138,6 +172,10 @@ struct StepArgs {
     const int32_t* __restrict__ bkind;
     const float* __restrict__ bd0;
     const float* __restrict__ bh0;
+    // the boundary cells by tile: tile t's are bitem[bstart[t] .. bstart[t + 1]); bstart[ntiles + 1]: whether any
+    // follows another cell. Null without boundary cells.
+    const int32_t* __restrict__ bstart;
+    const int32_t* __restrict__ bitem;
     int32_t ntally;
     const int32_t* __restrict__ tface;
     const int32_t* __restrict__ taxis;
@@ -168,6 +206,14 @@ struct StepArgs {
 // The strip forms of the face pass (strips of H rows of a tile): 40 x (H + 4) boxes, and 32 x H for the momenta.
 struct StripMaps {
     CUtensorMap d, h[2], u[2], v[2], qx, qy, zcx, zcy, mx[2], my[2];
+};
+// The update's boxes for a strip of H rows (the resident loop): 40 x (H + 3), one row above to two below, and 32 x H.
+struct UpdateMaps {
+    CUtensorMap qx1, qy1, h[2], res, src;
+};
+struct ResidentMaps {
+    StripMaps s;
+    UpdateMaps u;
 };
 struct TMaps {
     CUtensorMap d, h[2], u[2], v[2], qx, qy, om, zcx, zcy, mx[2], my[2];

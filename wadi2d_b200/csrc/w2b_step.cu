@@ -13,6 +13,7 @@
 #include <cstdio>
 
 #include "w2b_common.cuh"
+#include "w2b_loop.cuh"
 #include "w2b_tma.cuh"
 
 namespace w2b {
@@ -385,6 +386,22 @@ __device__ __forceinline__ float block_max(float v, float* red) {
     return r;
 }
 
+// Threads' part of a table of the row constants that the table lookup forms (face_bc's rowc), one a CTA.
+__device__ __forceinline__ void fill_rowc(float* rowc, int rows) {
+    const int tid = threadIdx.x;
+    if (tid < rows - 1) {
+        const float m = (float)(rows - 1);
+        const float c0 = (float)tid / m;
+        const float c1 = (float)(tid + 1) / m;
+        rowc[2 * tid] = c0 * c0;
+        rowc[2 * tid + 1] = c1 * c1 - c0 * c0;
+    } else if (tid == rows - 1) {
+        const float m = (float)(rows - 1);
+        const float c = (m - 1.0f) / m;
+        rowc[2 * tid] = 1.0f - c * c;
+    }
+}
+
 // The face pass: both own faces of every cell of the tiles of the work list (wadi2d/solver/gpu/kernels/faces.cu:
 // 148-175). Each CTA (16 warps, a warp a tile row, two rows a warp; two CTAs a SM) stages a tile with TMA: nine
 // 40 x 36 state boxes, the two momenta (or, once a face pass has stepped, the last step's mean depth box they are
@@ -406,17 +423,7 @@ __global__ void __launch_bounds__(FACES_THREADS, 2) faces_kernel(const __grid_co
         mbar_init(&bar, 1);
         fence_barrier_init();
     }
-    if (tid < A.rows - 1) {
-        const float m = (float)(A.rows - 1);
-        const float c0 = (float)tid / m;
-        const float c1 = (float)(tid + 1) / m;
-        rowc[2 * tid] = c0 * c0;
-        rowc[2 * tid + 1] = c1 * c1 - c0 * c0;
-    } else if (tid == A.rows - 1) {
-        const float m = (float)(A.rows - 1);
-        const float c = (m - 1.0f) / m;
-        rowc[2 * tid] = 1.0f - c * c;
-    }
+    fill_rowc(rowc, A.rows);
     __syncthreads();
     const float* statics[12] = {A.fl[0], A.fr[0], A.gl[0], A.gr[0], A.ef[0], A.cw[0],
                                 A.fl[1], A.fr[1], A.gl[1], A.gr[1], A.ef[1], A.cw[1]};
@@ -521,17 +528,7 @@ __global__ void __launch_bounds__(1024) probe_kernel(StepArgs A, int t, float dt
         }
         for (int f = 0; f < 12; ++f) sm[SM_ST + f * TILE2 + idx] = statics[f][(size_t)table_of(A, t) * TILE2 + idx];
     }
-    if (tid < A.rows - 1) {
-        const float m = (float)(A.rows - 1);
-        const float c0 = (float)tid / m;
-        const float c1 = (float)(tid + 1) / m;
-        rowc[2 * tid] = c0 * c0;
-        rowc[2 * tid + 1] = c1 * c1 - c0 * c0;
-    } else if (tid == A.rows - 1) {
-        const float m = (float)(A.rows - 1);
-        const float c = (m - 1.0f) / m;
-        rowc[2 * tid] = 1.0f - c * c;
-    }
+    fill_rowc(rowc, A.rows);
     __syncthreads();
     const int jj = tid >> 5, ii = tid & 31;
     const int local = jj * TILE + ii;
@@ -558,12 +555,139 @@ void launch_probe(const StepArgs& A, int t, float dt, float* out, cudaStream_t s
 // on refresh steps only, are read from
 // global memory. A face's arithmetic is the tile form's, bit for bit. On refresh steps each strip's wave maximum goes
 // to its tile's entry and its run's maximum by integer atomic maxima on the float bits.
+// Copy c of a strip's image, from the strip's first row y and its box's first column x0: the state boxes, the momenta (or
+// the last step's mean depth box) and the twelve face scalars from table tile ts.
+constexpr int STRIP_COPIES = 22;
+template <int H>
+__device__ __forceinline__ void strip_copy(int c, const StripMaps& M, const StepArgs& A, float* sm, uint64_t* bar, int x0,
+                                           int y, int p, int mst, int ts, int row0) {
+    using L = StripImage<H>;
+    if (c < 12) {
+        const int ax = c >= 6, f = c - 6 * ax;
+        const float* from = f == 0 ? A.fl[ax] : f == 1 ? A.fr[ax] : f == 2 ? A.gl[ax] : f == 3 ? A.gr[ax]
+                          : f == 4 ? A.ef[ax] : A.cw[ax];
+        bulk_load(sm + L::ST + c * L::S, from + (size_t)ts * TILE2 + row0 * TILE, L::S * 4, bar);
+        return;
+    }
+    switch (c) {
+        case 12: tma_load_2d(sm + L::S_U, &M.u[p], x0, y - 2, bar); break;
+        case 13: tma_load_2d(sm + L::S_V, &M.v[p], x0, y - 2, bar); break;
+        case 14: tma_load_2d(sm + L::S_D, &M.d, x0, y - 1, bar); break;
+        case 15: tma_load_2d(sm + L::S_H, &M.h[p], x0, y - 1, bar); break;
+        case 16: tma_load_2d(sm + L::S_QX, &M.qx, x0, y - 1, bar); break;
+        case 17: tma_load_2d(sm + L::S_QY, &M.qy, x0, y - 1, bar); break;
+        case 18: tma_load_2d(sm + L::S_ZCX, &M.zcx, x0, y, bar); break;
+        case 19: tma_load_2d(sm + L::S_ZCY, &M.zcy, x0, y - 1, bar); break;
+        case 20:
+            if (mst)
+                tma_load_2d(sm + L::M, &M.mx[p], x0 + 4, y, bar);
+            else
+                tma_load_2d(sm + L::M, &M.h[1 - p], x0, y - 1, bar);  // the mean depth box's rows
+            break;
+        case 21:
+            if (mst) tma_load_2d(sm + L::M + L::S, &M.my[p], x0 + 4, y, bar);
+            break;
+    }
+}
+
+// One strip of tile t at (tj, ti), with the tables of tile ts, from its row row0 on: its copies, then WARPS warps' rows of
+// both faces, and on refresh steps the strip's wave maximum. SPREAD: each warp issues its share of the copies, and with
+// more warps than rows a warp takes one axis of its row. False: the copies did not land (reported; the caller leaves).
+template <int H, int WARPS, bool ON, bool SPREAD>
+__device__ __forceinline__ bool strip_unit(const StripMaps& SM_, const StepArgs& A, float* sm, uint64_t* bar,
+                                           uint32_t& phase, const float* rowc, float* red, int t, int ts, int tj, int ti,
+                                           int row0, int run, float dt, float dx, int want_wave, int p, int mst,
+                                           uint32_t* wave_bits) {
+    using L = StripImage<H>;
+    constexpr bool SPLIT = WARPS > H;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (SPREAD) {
+        if (lane == 0) {
+            fence_proxy_async();
+            if (warp == 0) mbar_expect_tx(bar, (uint32_t)(mst ? L::BYTES : L::BYTES_HO));
+            for (int c = warp; c < STRIP_COPIES; c += WARPS)
+                strip_copy<H>(c, SM_, A, sm, bar, ti * TILE + GX - 4, tj * TILE + GY + row0, p, mst, ts, row0);
+        }
+    } else if (tid == 0) {
+        const float* statics[12] = {A.fl[0], A.fr[0], A.gl[0], A.gr[0], A.ef[0], A.cw[0],
+                                    A.fl[1], A.fr[1], A.gl[1], A.gr[1], A.ef[1], A.cw[1]};
+        fence_proxy_async();
+        mbar_expect_tx(bar, (uint32_t)(mst ? L::BYTES : L::BYTES_HO));
+        // each box from its first row (the strip's row 0 is y)
+        const int x0 = ti * TILE + GX - 4, y = tj * TILE + GY + row0;
+        tma_load_2d(sm + L::S_U, &SM_.u[p], x0, y - 2, bar);
+        tma_load_2d(sm + L::S_V, &SM_.v[p], x0, y - 2, bar);
+        tma_load_2d(sm + L::S_D, &SM_.d, x0, y - 1, bar);
+        tma_load_2d(sm + L::S_H, &SM_.h[p], x0, y - 1, bar);
+        tma_load_2d(sm + L::S_QX, &SM_.qx, x0, y - 1, bar);
+        tma_load_2d(sm + L::S_QY, &SM_.qy, x0, y - 1, bar);
+        tma_load_2d(sm + L::S_ZCX, &SM_.zcx, x0, y, bar);
+        tma_load_2d(sm + L::S_ZCY, &SM_.zcy, x0, y - 1, bar);
+        if (mst) {
+            tma_load_2d(sm + L::M, &SM_.mx[p], x0 + 4, y, bar);
+            tma_load_2d(sm + L::M + L::S, &SM_.my[p], x0 + 4, y, bar);
+        } else {
+            tma_load_2d(sm + L::M, &SM_.h[1 - p], x0, y - 1, bar);  // the mean depth box's rows
+        }
+        for (int f = 0; f < 12; ++f)
+            bulk_load(sm + L::ST + f * L::S, statics[f] + (size_t)ts * TILE2 + row0 * TILE, L::S * 4, bar);
+    }
+    const bool ok = mbar_wait(bar, phase);
+    phase ^= 1u;
+    if (__syncthreads_or(!ok)) {
+        // the copies did not land: report, and give them one more bounded wait before the CTA leaves
+        if (tid == 0) atomicExch(&A.ctl->status, W2B_ETIMEOUT);
+        mbar_wait(bar, phase ^ 1u);
+        return false;
+    }
+    const int base = (tj * TILE + GY) * A.px + ti * TILE + GX;
+    float wmax = 0.0f;
+    if (SPLIT) {
+        const int js = warp >> 1, ii = lane;
+        const int jj = row0 + js;
+        const int sl = js * TILE + ii, local = jj * TILE + ii;
+        const int b = (js + 2) * BOXW + ii + 4;
+        const int k = base + jj * A.px + ii;
+        FaceA f;
+        if (warp & 1) {
+            face_a<1, ON, L>(sm, b, sl, local, A, ts, f);
+            wmax = face_bc<1, false, ON, L>(sm, b, sl, local, k, A, ts, f, dt, dx, want_wave, rowc, p, mst);
+        } else {
+            face_a<0, ON, L>(sm, b, sl, local, A, ts, f);
+            wmax = face_bc<0, false, ON, L>(sm, b, sl, local, k, A, ts, f, dt, dx, want_wave, rowc, p, mst);
+        }
+    }
+#pragma unroll 1
+    for (int c = 0; c < (SPLIT ? 0 : H / WARPS); ++c) {
+        const int js = warp + WARPS * c, ii = lane;  // the row in the strip, and in the tile
+        const int jj = row0 + js;
+        const int sl = js * TILE + ii, local = jj * TILE + ii;
+        const int b = (js + 2) * BOXW + ii + 4;
+        const int k = base + jj * A.px + ii;
+        FaceA fx, fy;
+        face_a<0, ON, L>(sm, b, sl, local, A, ts, fx);
+        face_a<1, ON, L>(sm, b, sl, local, A, ts, fy);
+        const float wx = face_bc<0, false, ON, L>(sm, b, sl, local, k, A, ts, fx, dt, dx, want_wave, rowc, p, mst);
+        const float wy = face_bc<1, false, ON, L>(sm, b, sl, local, k, A, ts, fy, dt, dx, want_wave, rowc, p, mst);
+        wmax = fmax32(wmax, fmax32(wx, wy));
+    }
+    if (want_wave) {
+        const float bm = block_max(wmax, red);
+        if (tid == 0) {
+            atomicMax(reinterpret_cast<unsigned int*>(A.wave) + t, __float_as_uint(bm));
+            atomicMax(wave_bits + run, __float_as_uint(bm));
+        }
+    } else {
+        __syncthreads();
+    }
+    return true;
+}
+
 template <int H, bool ON>
 __global__ void __launch_bounds__(StripImage<H>::THREADS, StripImage<H>::CTAS)
     strips_kernel(const __grid_constant__ TMaps M, StepArgs A) {
     using L = StripImage<H>;
     constexpr int PER = TILE / H;  // strips a tile
-    const StripMaps& SM_ = H == 16 ? M.s16 : M.s8;
     extern __shared__ __align__(128) float sm[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ float red[L::THREADS / 32];
@@ -572,96 +696,23 @@ __global__ void __launch_bounds__(StripImage<H>::THREADS, StripImage<H>::CTAS)
     if (!(ctl->any & ANY_RUN)) return;
     const int nunits = PER * ctl->nwork;
     const int mst = ctl->m_stored;
-    const int tid = threadIdx.x;
-    if (tid == 0) {
+    if (threadIdx.x == 0) {
         mbar_init(&bar, 1);
         fence_barrier_init();
     }
-    if (tid < A.rows - 1) {
-        const float m = (float)(A.rows - 1);
-        const float c0 = (float)tid / m;
-        const float c1 = (float)(tid + 1) / m;
-        rowc[2 * tid] = c0 * c0;
-        rowc[2 * tid + 1] = c1 * c1 - c0 * c0;
-    } else if (tid == A.rows - 1) {
-        const float m = (float)(A.rows - 1);
-        const float c = (m - 1.0f) / m;
-        rowc[2 * tid] = 1.0f - c * c;
-    }
+    fill_rowc(rowc, A.rows);
     __syncthreads();
-    const float* statics[12] = {A.fl[0], A.fr[0], A.gl[0], A.gr[0], A.ef[0], A.cw[0],
-                                A.fl[1], A.fr[1], A.gl[1], A.gr[1], A.ef[1], A.cw[1]};
     uint32_t phase = 0;
-    const int lane = tid & 31, warp = tid >> 5;
     for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
         const int t = A.list[u / PER];
-        const int row0 = (u % PER) * H;
         const int run = A.tile_run[t];
         const int flags = A.R.flags[run];
         if (!(flags & F_RUN)) continue;  // the tile's run has finished: uniform over the CTA
-        const float dt = A.R.dtf[run];
-        const float dx = A.R.dx[run];
-        const int want_wave = (flags & F_WAVE) != 0;
-        const int p = A.R.parity[run];
-        const int tj = A.tiles[2 * t], ti = A.tiles[2 * t + 1];
-        const int ts = table_of(A, t);
-        if (tid == 0) {
-            fence_proxy_async();
-            mbar_expect_tx(&bar, (uint32_t)(mst ? L::BYTES : L::BYTES_HO));
-            // each box from its first row (the strip's row 0 is y)
-            const int x0 = ti * TILE + GX - 4, y = tj * TILE + GY + row0;
-            tma_load_2d(sm + L::S_U, &SM_.u[p], x0, y - 2, &bar);
-            tma_load_2d(sm + L::S_V, &SM_.v[p], x0, y - 2, &bar);
-            tma_load_2d(sm + L::S_D, &SM_.d, x0, y - 1, &bar);
-            tma_load_2d(sm + L::S_H, &SM_.h[p], x0, y - 1, &bar);
-            tma_load_2d(sm + L::S_QX, &SM_.qx, x0, y - 1, &bar);
-            tma_load_2d(sm + L::S_QY, &SM_.qy, x0, y - 1, &bar);
-            tma_load_2d(sm + L::S_ZCX, &SM_.zcx, x0, y, &bar);
-            tma_load_2d(sm + L::S_ZCY, &SM_.zcy, x0, y - 1, &bar);
-            if (mst) {
-                tma_load_2d(sm + L::M, &SM_.mx[p], x0 + 4, y, &bar);
-                tma_load_2d(sm + L::M + L::S, &SM_.my[p], x0 + 4, y, &bar);
-            } else {
-                tma_load_2d(sm + L::M, &SM_.h[1 - p], x0, y - 1, &bar);  // the mean depth box's rows
-            }
-            for (int f = 0; f < 12; ++f)
-                bulk_load(sm + L::ST + f * L::S, statics[f] + (size_t)ts * TILE2 + row0 * TILE, L::S * 4, &bar);
-        }
-        const bool ok = mbar_wait(&bar, phase);
-        phase ^= 1u;
-        if (__syncthreads_or(!ok)) {
-            // the copies did not land: report, give them one more bounded wait, and leave the loop
-            if (tid == 0) atomicExch(&ctl->status, W2B_ETIMEOUT);
-            mbar_wait(&bar, phase ^ 1u);
+        if (!strip_unit<H, L::THREADS / 32, ON, false>(H == 16 ? M.s16 : M.s8, A, sm, &bar, phase, rowc, red, t,
+                                                       table_of(A, t), A.tiles[2 * t], A.tiles[2 * t + 1], (u % PER) * H,
+                                                       run, A.R.dtf[run], A.R.dx[run], (flags & F_WAVE) != 0,
+                                                       A.R.parity[run], mst, A.R.wave_bits))
             return;
-        }
-        const int base = (tj * TILE + GY) * A.px + ti * TILE + GX;
-        float wmax = 0.0f;
-#pragma unroll 1
-        for (int c = 0; c < 2; ++c) {
-            const int js = warp + (H / 2) * c, ii = lane;  // the row in the strip, and in the tile
-            const int jj = row0 + js;
-            const int sl = js * TILE + ii, local = jj * TILE + ii;
-            const int b = (js + 2) * BOXW + ii + 4;
-            const int k = base + jj * A.px + ii;
-            FaceA fx, fy;
-            face_a<0, ON, L>(sm, b, sl, local, A, ts, fx);
-            face_a<1, ON, L>(sm, b, sl, local, A, ts, fy);
-            const float wx = face_bc<0, false, ON, L>(sm, b, sl, local, k, A, ts, fx, dt, dx, want_wave, rowc,
-                                                               p, mst);
-            const float wy = face_bc<1, false, ON, L>(sm, b, sl, local, k, A, ts, fy, dt, dx, want_wave, rowc,
-                                                               p, mst);
-            wmax = fmax32(wmax, fmax32(wx, wy));
-        }
-        if (want_wave) {
-            const float bm = block_max(wmax, red);
-            if (tid == 0) {
-                atomicMax(reinterpret_cast<unsigned int*>(A.wave) + t, __float_as_uint(bm));
-                atomicMax(A.R.wave_bits + run, __float_as_uint(bm));
-            }
-        } else {
-            __syncthreads();
-        }
     }
 }
 
@@ -750,6 +801,93 @@ constexpr int UPDATE_SMEM = U_FLOATS * 4;           // 43,648 bytes: four CTAs a
 static_assert(UPDATE_SMEM == 43648, "update image size");
 constexpr int UPDATE_THREADS = 256;
 
+// The positivity ratio r (wadi2d/solver/gpu/kernels/cells.cu:4-19) of the cell at box index b, from the unscaled
+// discharges and the old depth.
+__device__ __forceinline__ float positivity(const float* QX1, const float* QY1, const float* H, int b, float dt,
+                                            float area) {
+    const float out = fmax32(QX1[b + 1], 0.0f) + fmax32(-QX1[b], 0.0f) + fmax32(QY1[b + BOXW], 0.0f) +
+                      fmax32(-QY1[b], 0.0f);
+    const float have = fmax32(H[b], 0.0f) * area;
+    return out * dt > have ? have / (out * dt) : 1.0f;
+}
+
+// What continuity hands to the level lookup: the new mean depth, its table row (-1: none, Hc <= 0), the row coordinate.
+struct CellOut {
+    float hn, sv, hc;
+    int row;
+};
+
+// Continuity (cells.cu:219-232) of the cell at box index b, own index `local` and native index k: the scaled discharges,
+// the residual and the mean depth written, and the level table's row (common.cuh cell_level): the top row above Hc.
+// row: r of the cell in the ring's image.
+__device__ __forceinline__ CellOut continuity(const StepArgs& A, const float* QX1, const float* QY1, const float* H,
+                                              const float* row, int b, int local, int k, const float* RES,
+                                              const float* SRC, const float* HC, float* h_next, float dt, float area) {
+    const int last = A.rows - 1;
+    CellOut C;
+    const float rc = row[0];
+    const float qw = scaled(QX1[b], row[-1], rc);
+    const float qe = scaled(QX1[b + 1], rc, row[1]);
+    const float qn = scaled(QY1[b], row[-RPAD], rc);
+    const float qs = scaled(QY1[b + BOXW], rc, row[RPAD]);
+    A.q[0][k] = qw;
+    A.q[1][k] = qn;
+    const float h0 = H[b];
+    const float inc = RES[local] + dt * SRC[local] - dt * (qe - qw + qs - qn) / area;
+    const float total = h0 + inc;
+    C.hn = fmax32(total, 0.0f);
+    A.res[k] = total > 0.0f ? inc - (total - h0) : 0.0f;
+    h_next[k] = C.hn;
+    const float hcv = HC[local];
+    C.hc = hcv;
+    if (hcv <= 0.0f) {
+        C.row = -1;
+        C.sv = 0.0f;
+    } else if (C.hn >= hcv) {
+        C.row = last - 1;
+        C.sv = -1.0f;
+    } else {
+        C.sv = sqrtf(C.hn / hcv) * (float)last;
+        C.row = row_of(C.sv, last);
+    }
+    return C;
+}
+
+// The cell's level pair: the cached one where its row is the cached row (about 699 cells in 700 from one step to the
+// next), else gathered from the table and cached. fid: the cell in the cache's arrays, local: in the tile's table.
+__device__ __forceinline__ float2 level_pair(const StepArgs& A, const float2* pairs_t, const float2* LP,
+                                             const uint8_t* LR, int own, int row, size_t fid, int local) {
+    if (row < 0) return make_float2(0.0f, 0.0f);
+    if (LR[own] == row) return LP[own];
+    const float2 pr = __ldg(pairs_t + (size_t)row * TILE2 + local);
+    A.lpair[fid] = pr;
+    A.lrow[fid] = (uint8_t)row;
+    return pr;
+}
+
+// The level of a cell, and its wet share into om.
+__device__ __forceinline__ float cell_out_level(const StepArgs& A, const CellOut& C, float2 q, float& om) {
+    const int last = A.rows - 1;
+    float dk;
+    om = 1.0f;
+    if (C.hc <= 0.0f) {
+        dk = C.hn;
+    } else if (C.hn >= C.hc) {
+        dk = q.y + (C.hn - C.hc);
+    } else {
+        const int r = C.row;
+        if (A.P.level_fp64 && r == 0) {
+            const double sd = sqrt((double)C.hn / (double)C.hc) * (double)last;
+            dk = (float)((double)q.x + sd * ((double)q.y - (double)q.x));
+        } else {
+            dk = q.x + (C.sv - (float)r) * (q.y - q.x);
+        }
+        const float m = (float)last;
+        om = C.hc * (float)(2 * r + 1) / (m * m) / fmax32(q.y - q.x, 1e-12f);
+    }
+    return dk;
+}
+
 // The first entry at or after a, in steps of the grid, whose run is stepping (the same for every thread of a CTA).
 __device__ __forceinline__ int next_tile(const StepArgs& A, int a, int nwork) {
     for (; a < nwork; a += gridDim.x)
@@ -788,10 +926,9 @@ __global__ void __launch_bounds__(UPDATE_THREADS) update_kernel(const __grid_con
     if (!(ctl->any & ANY_RUN)) return;
     const int nwork = ctl->nwork;
     const int px = A.px;
-    const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+    const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
     // the face pass before this one has stepped: from now on the momenta are formed from the state (Ctl::m_stored)
     if (blockIdx.x == 0 && tid == 0) ctl->m_stored = 0;
-    const int rows = A.rows, last = rows - 1;
     if (tid == 0) {
         mbar_init(&bar, 1);
         fence_barrier_init();
@@ -826,72 +963,28 @@ __global__ void __launch_bounds__(UPDATE_THREADS) update_kernel(const __grid_con
             mbar_wait(&bar, phase ^ 1u);
             return;
         }
-        // positivity ratio r (wadi2d/solver/gpu/kernels/cells.cu:4-19) of the tile and its ring, from the old h
+        // r of the tile and its ring, from the old h
         for (int idx = tid; idx < RING * RING; idx += UPDATE_THREADS) {
             const int rj = idx / RING, ri = idx - rj * RING;
-            const int b = (rj + 1) * BOXW + ri + 3;  // cell (rj - 1, ri - 1)
-            const float out = fmax32(QX1[b + 1], 0.0f) + fmax32(-QX1[b], 0.0f) + fmax32(QY1[b + BOXW], 0.0f) +
-                              fmax32(-QY1[b], 0.0f);
-            const float have = fmax32(H[b], 0.0f) * area;
-            rs[rj * RPAD + ri] = out * dt > have ? have / (out * dt) : 1.0f;
+            rs[rj * RPAD + ri] = positivity(QX1, QY1, H, (rj + 1) * BOXW + ri + 3, dt, area);  // cell (rj - 1, ri - 1)
         }
         __syncthreads();
         const int base = (tj * TILE + GY) * px + ti * TILE + GX;
-        const float2* __restrict__ pairs_t = A.dtab2 + (size_t)table_of(A, t) * (rows - 1) * TILE2;
-        // continuity (cells.cu:219-232) for the thread's four cells
-        float hn[4], sv[4], hcs[4];
-        int rr[4];
+        const float2* __restrict__ pairs_t = A.dtab2 + (size_t)table_of(A, t) * (A.rows - 1) * TILE2;
+        CellOut C[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            const int jj = threadIdx.y * 4 + c, ii = threadIdx.x;
-            const int local = jj * TILE + ii;
-            const int b = (jj + 2) * BOXW + ii + 4;
-            const int k = base + jj * px + ii;
-            const float* row = rs + (jj + 1) * RPAD + (ii + 1);
-            const float rc = row[0];
-            const float qw = scaled(QX1[b], row[-1], rc);
-            const float qe = scaled(QX1[b + 1], rc, row[1]);
-            const float qn = scaled(QY1[b], row[-RPAD], rc);
-            const float qs = scaled(QY1[b + BOXW], rc, row[RPAD]);
-            A.q[0][k] = qw;
-            A.q[1][k] = qn;
-            const float h0 = H[b];
-            const float inc = RES[local] + dt * SRC[local] - dt * (qe - qw + qs - qn) / area;
-            const float total = h0 + inc;
-            hn[c] = fmax32(total, 0.0f);
-            A.res[k] = total > 0.0f ? inc - (total - h0) : 0.0f;
-            h_next[k] = hn[c];
-            // the level table's row (common.cuh cell_level): the top row above Hc, none where Hc <= 0
-            const float hcv = HC[local];
-            hcs[c] = hcv;
-            if (hcv <= 0.0f) {
-                rr[c] = -1;
-                sv[c] = 0.0f;
-            } else if (hn[c] >= hcv) {
-                rr[c] = last - 1;
-                sv[c] = -1.0f;
-            } else {
-                sv[c] = sqrtf(hn[c] / hcv) * (float)last;
-                rr[c] = row_of(sv[c], last);
-            }
+            const int jj = ty * 4 + c, ii = tx;
+            C[c] = continuity(A, QX1, QY1, H, rs + (jj + 1) * RPAD + (ii + 1), (jj + 2) * BOXW + ii + 4, jj * TILE + ii,
+                              base + jj * px + ii, RES, SRC, HC, h_next, dt, area);
         }
-        // the level pairs: the cached one where the cell's row is the cached row (about 699 cells in 700 from one
-        // step to the next), else gathered from the table and cached
         float2 pr[4];
         const float2* LP = reinterpret_cast<const float2*>(sm + U_LP);
         const uint8_t* LR = reinterpret_cast<const uint8_t*>(sm + U_LR);
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            const int local = (threadIdx.y * 4 + c) * TILE + threadIdx.x;
-            if (rr[c] < 0) {
-                pr[c] = make_float2(0.0f, 0.0f);
-            } else if (LR[local] == rr[c]) {
-                pr[c] = LP[local];
-            } else {
-                pr[c] = __ldg(pairs_t + (size_t)rr[c] * TILE2 + local);
-                A.lpair[(size_t)t * TILE2 + local] = pr[c];
-                A.lrow[(size_t)t * TILE2 + local] = (uint8_t)rr[c];
-            }
+            const int local = (ty * 4 + c) * TILE + tx;
+            pr[c] = level_pair(A, pairs_t, LP, LR, local, C[c].row, (size_t)t * TILE2 + local, local);
         }
         // every thread has read the image and r: the next tile's copies land in it during this tile's gathers
         __syncthreads();
@@ -900,30 +993,11 @@ __global__ void __launch_bounds__(UPDATE_THREADS) update_kernel(const __grid_con
         int any = 0;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            const int jj = threadIdx.y * 4 + c, ii = threadIdx.x;
-            const int k = base + jj * px + ii;
-            const float hcv = hcs[c];
-            const float h = hn[c];
-            float dk, om = 1.0f;
-            if (hcv <= 0.0f) {
-                dk = h;
-            } else if (h >= hcv) {
-                dk = pr[c].y + (h - hcv);
-            } else {
-                const int r = rr[c];
-                const float2 q = pr[c];
-                if (A.P.level_fp64 && r == 0) {
-                    const double sd = sqrt((double)h / (double)hcv) * (double)last;
-                    dk = (float)((double)q.x + sd * ((double)q.y - (double)q.x));
-                } else {
-                    dk = q.x + (sv[c] - (float)r) * (q.y - q.x);
-                }
-                const float m = (float)last;
-                om = hcv * (float)(2 * r + 1) / (m * m) / fmax32(q.y - q.x, 1e-12f);
-            }
-            A.d[k] = dk;
+            const int k = base + (ty * 4 + c) * px + tx;
+            float om;
+            A.d[k] = cell_out_level(A, C[c], pr[c], om);
             if (want_plan) A.om[k] = om;
-            any |= h > 0.0f;
+            any |= C[c].hn > 0.0f;
         }
         if (want_wet) {
             const int w = __syncthreads_or(any);
@@ -944,7 +1018,319 @@ int update_occupancy() {
 }
 
 void launch_update(const TMaps& M, const StepArgs& A, int grid, cudaStream_t s) {
-    update_kernel<<<grid, dim3(32, 8), UPDATE_SMEM, s>>>(M, A);
+    update_kernel<<<grid, UPDATE_THREADS, UPDATE_SMEM, s>>>(M, A);
+}
+
+// ------------------------------------------------------------------ the resident loop
+
+// Shared-memory image of a strip of H rows for the resident loop's update: boxes of 40 x (H + 3) floats from one row
+// above the strip to two below (own cell (j, i) at box (j + 1, i + 4)), the own rows' residual, source and Hc, r of the
+// strip and its one-cell ring, and the level cache.
+template <int H>
+struct UpdateStrip {
+    static constexpr int BOXN = pad32(BOXW * (H + 3));
+    static constexpr int QX1 = 0, QY1 = BOXN, HB = 2 * BOXN, RES = 3 * BOXN, SRC = RES + TILE * H, HC = SRC + TILE * H;
+    static constexpr int R = HC + TILE * H, LP = pad32(R + (H + 2) * RPAD), LR = LP + 2 * TILE * H;
+    static constexpr int SMEM = 4 * LR + TILE * H;
+    static constexpr int BYTES = 4 * (3 * BOXW * (H + 3) + 3 * TILE * H) + 9 * TILE * H;
+    static constexpr int CELLS = H * TILE / RESIDENT_THREADS > 0 ? H * TILE / RESIDENT_THREADS : 1;  // a thread
+};
+
+// A unit of the resident loop, a strip of H rows of a tile: where it lies, and its run's settings.
+struct Unit {
+    int t, run, ts, tj, ti, row0, b0, b1;
+};
+struct UnitStep {
+    float dt, dx;
+    int flags, p;
+};
+constexpr int UNITS_HELD = 32;  // units whose places a CTA keeps from step to step
+
+template <int H>
+__device__ __forceinline__ Unit unit_place(const StepArgs& A, int u) {
+    constexpr int PER = TILE / H;
+    Unit U;
+    U.t = __ldcg(A.work + u / PER);
+    U.run = A.tile_run[U.t];
+    U.ts = table_of(A, U.t);
+    U.tj = A.tiles[2 * U.t];
+    U.ti = A.tiles[2 * U.t + 1];
+    U.row0 = (u % PER) * H;
+    U.b0 = A.bstart ? A.bstart[U.t] : 0;
+    U.b1 = A.bstart ? A.bstart[U.t + 1] : 0;
+    return U;
+}
+
+__device__ __forceinline__ UnitStep unit_step(const StepArgs& A, const StepView& V, int run) {
+    return UnitStep{__ldcg(V.dtf + run), A.R.dx[run], __ldcg(V.flags + run), __ldcg(V.parity + run)};
+}
+
+// The update of one strip with its boundary cells of a prescribed depth and its envelope; the update pass's arithmetic.
+// What does not depend on the copies (the boundary items, the envelope's entries) is loaded while they land. False: they
+// did not land (reported; the caller leaves).
+template <int H>
+__device__ __forceinline__ bool update_unit(const UpdateMaps& M, const StepArgs& A, const StepView& V, float* sm,
+                                            uint64_t* bar, uint32_t& phase, const Unit& U, const UnitStep& S) {
+    using L = UpdateStrip<H>;
+    const int tid = threadIdx.x, px = A.px;
+    const float dt = S.dt, area = S.dx * S.dx;
+    const int want_max = (S.flags & F_MAX) == F_MAX, n = 1 - S.p;
+    const int base = (U.tj * TILE + GY + U.row0) * px + U.ti * TILE + GX;  // the strip's first cell
+    const size_t fid0 = (size_t)U.t * TILE2 + U.row0 * TILE;
+    if ((tid & 31) == 0) {
+        const int x0 = U.ti * TILE + GX - 4, y0 = U.tj * TILE + GY + U.row0;
+        fence_proxy_async();
+        switch (tid >> 5) {
+            case 0:
+                mbar_expect_tx(bar, (uint32_t)L::BYTES);
+                tma_load_2d(sm + L::QX1, &M.qx1, x0, y0 - 1, bar);
+                break;
+            case 1: tma_load_2d(sm + L::QY1, &M.qy1, x0, y0 - 1, bar); break;
+            case 2: tma_load_2d(sm + L::HB, &M.h[S.p], x0, y0 - 1, bar); break;
+            case 3: tma_load_2d(sm + L::RES, &M.res, x0 + 4, y0, bar); break;
+            case 4: tma_load_2d(sm + L::SRC, &M.src, x0 + 4, y0, bar); break;
+            case 5:
+                bulk_load(sm + L::HC, A.hc + (size_t)U.ts * TILE2 + U.row0 * TILE, TILE * H * 4, bar);
+                break;
+            case 6: bulk_load(sm + L::LP, A.lpair + fid0, TILE * H * 8, bar); break;
+            case 7: bulk_load(sm + L::LR, A.lrow + fid0, TILE * H, bar); break;
+        }
+    }
+    // this thread's boundary item, if any: one of the tile's whose cell lies in the strip
+    int item = -1;
+    if (tid < U.b1 - U.b0) {
+        const int m = A.bitem[U.b0 + tid];
+        const int row = A.bcell[m] / px - GY - U.tj * TILE - U.row0;
+        if (A.bkind[m] < 2 && row >= 0 && row < H) item = m;
+    }
+    const bool mine = tid < H * TILE;
+    EnvelopeIn E[L::CELLS];
+    bool marked[L::CELLS];
+    if (want_max && mine) {
+#pragma unroll
+        for (int c = 0; c < L::CELLS; ++c) {
+            const int cell = tid + RESIDENT_THREADS * c, js = cell >> 5, ii = cell & 31;
+            marked[c] = (A.bmark[U.t * TILE + U.row0 + js] >> ii) & 1u;
+            E[c] = envelope_load(A, (int)fid0 + cell, base + js * px + ii, A.uu[0][n], A.uu[1][n]);
+        }
+    }
+    const bool ok = mbar_wait(bar, phase);
+    phase ^= 1u;
+    if (__syncthreads_or(!ok)) {
+        if (tid == 0) atomicExch(&A.ctl->status, W2B_ETIMEOUT);
+        mbar_wait(bar, phase ^ 1u);
+        return false;
+    }
+    const float *QX1 = sm + L::QX1, *QY1 = sm + L::QY1, *HB = sm + L::HB;
+    float* rs = sm + L::R;
+    for (int idx = tid; idx < (H + 2) * RING; idx += RESIDENT_THREADS) {
+        const int rj = idx / RING, ri = idx - rj * RING;
+        rs[rj * RPAD + ri] = positivity(QX1, QY1, HB, rj * BOXW + ri + 3, dt, area);  // cell (rj - 1, ri - 1)
+    }
+    __syncthreads();
+    const float2* pairs_t = A.dtab2 + (size_t)U.ts * (A.rows - 1) * TILE2 + U.row0 * TILE;
+    const float2* LP = reinterpret_cast<const float2*>(sm + L::LP);
+    const uint8_t* LR = reinterpret_cast<const uint8_t*>(sm + L::LR);
+    int any = 0;
+    if (mine) {
+        CellOut C[L::CELLS];
+        float2 pr[L::CELLS];
+#pragma unroll
+        for (int c = 0; c < L::CELLS; ++c) {
+            const int cell = tid + RESIDENT_THREADS * c, js = cell >> 5, ii = cell & 31;
+            C[c] = continuity(A, QX1, QY1, HB, rs + (js + 1) * RPAD + (ii + 1), (js + 1) * BOXW + ii + 4, cell,
+                              base + js * px + ii, sm + L::RES, sm + L::SRC, sm + L::HC, A.hh[n], dt, area);
+            pr[c] = level_pair(A, pairs_t, LP, LR, cell, C[c].row, fid0 + cell, cell);
+        }
+#pragma unroll
+        for (int c = 0; c < L::CELLS; ++c) {
+            const int cell = tid + RESIDENT_THREADS * c, k = base + (cell >> 5) * px + (cell & 31);
+            float om;
+            const float dk = cell_out_level(A, C[c], pr[c], om);
+            A.d[k] = dk;
+            if (S.flags & F_WAVE) A.om[k] = om;
+            any |= C[c].hn > 0.0f;
+            if (want_max && !marked[c])
+                envelope_apply(A, (int)fid0 + cell, E[c], dk, C[c].hn, __ldcg(V.max_time + U.run), A.ctl->arrive,
+                               A.ctl->deep);
+        }
+    }
+    // the strip's cells are written and its image is read; whether any is wet
+    const int w = __syncthreads_or(any);
+    if ((S.flags & F_WET) && w && tid == 0) atomicOr(A.wet + U.t, 1);
+    if (U.b0 < U.b1) {
+        if (item >= 0) boundary_cell(A, item, n, S.flags, __ldcg(V.max_time + U.run), A.ctl->arrive, A.ctl->deep);
+        for (int x = U.b0 + RESIDENT_THREADS + tid; x < U.b1; x += RESIDENT_THREADS) {
+            const int m = A.bitem[x], row = A.bcell[m] / px - GY - U.tj * TILE - U.row0;
+            if (A.bkind[m] < 2 && row >= 0 && row < H)
+                boundary_cell(A, m, n, S.flags, __ldcg(V.max_time + U.run), A.ctl->arrive, A.ctl->deep);
+        }
+    }
+    return true;
+}
+
+// Up to max_steps steps of the device loop in one cooperative launch. A step of the loop's kernels of their own is six
+// dependent launches, which on a few hundred tiles cost more than their work; here it is two grid barriers: the face
+// pass by strips of H rows (first barrier), then the update of the same strips with their boundary cells and envelope,
+// while one CTA of its own forms the next step's settings in the second set (second barrier); that CTA then takes the
+// tally and the lines while the next face pass runs. Boundary cells that follow another (one more barrier) and steps
+// that rebuild the lists (two or three more, one step in active_every) come after it. The same arithmetic in the same
+// order for every cell, face and sum as the kernels of their own. What CTAs hand one another between barriers is read
+// past L1 or by bulk copies. Latency bounds it on small grids, so strips of 4 rows (a warp a row and axis) serve the
+// smallest, and a CTA keeps the places of its strips from step to step. A step of the exact build, this way and as
+// kernels of their own: 62 x 62 cells 14 against 30 us (face pass 4.0, update 2.9, a barrier 2 to 3 us), 256 x 256 19 against
+// 31 us; the kernels also run the empty steps at the end of a graph of 16, about 8 us each. Where the passes' own work
+// fills the chip it gains nothing (1500 x 1101: 155 against 150 us), and the launch tuner keeps the kernels.
+template <int H, bool ON>
+__global__ void __launch_bounds__(RESIDENT_THREADS, RESIDENT_CTAS)
+    resident_kernel(const __grid_constant__ ResidentMaps M, const __grid_constant__ StepArgs A, int max_steps) {
+    constexpr int PER = TILE / H;
+    extern __shared__ __align__(128) float sm[];
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ float red[RESIDENT_THREADS / 32];
+    __shared__ float rowc[2 * 64 + 1];
+    __shared__ Unit places[UNITS_HELD];
+    __shared__ UnitStep steps[UNITS_HELD];
+    Ctl* ctl = A.ctl;
+    GridState* grid = grid_state(ctl);
+    const int workers = (int)gridDim.x - 1;  // the last CTA forms the next step's settings and rebuilds the lists
+    const bool control = (int)blockIdx.x == workers;
+    const int tid = threadIdx.x;
+    if (tid == 0) {
+        mbar_init(&bar, 1);
+        fence_barrier_init();
+    }
+    fill_rowc(rowc, A.rows);
+    uint32_t phase = 0, met = 0;
+    uint32_t any = ctl->any;
+    int nwork = ctl->nwork, mst = ctl->m_stored, b = 0;
+    bool moved = true;  // the work list is not the one `places` was taken from
+    const bool follow = A.bstart && A.bstart[A.ntiles + 1];
+    for (int step = 0; step < max_steps && (any & ANY_RUN); ++step) {
+        const StepView V = step_view(A.R, b);
+        const int left = PER * nwork - (int)blockIdx.x;
+        const int units = control || left <= 0 ? 0 : (left + workers - 1) / workers;  // this CTA's
+        // the places and settings of its units from c0 on (kept from the step before where they are all held and the
+        // lists have not moved; the settings then came with the step's flags)
+        auto take = [&](int c0) {
+            const int n = units - c0 < UNITS_HELD ? units - c0 : UNITS_HELD;
+            __syncthreads();
+            if (tid < n && (moved || units > UNITS_HELD)) {
+                places[tid] = unit_place<H>(A, (int)blockIdx.x + (c0 + tid) * workers);
+                steps[tid] = unit_step(A, V, places[tid].run);
+            }
+            __syncthreads();
+            return n;
+        };
+        for (int c0 = 0; c0 < units; c0 += UNITS_HELD) {
+            const int n = take(c0);
+            for (int i = 0; i < n; ++i) {
+                const Unit U = places[i];
+                const UnitStep S = steps[i];
+                if (!(S.flags & F_RUN)) continue;  // uniform over the CTA
+                if ((S.flags & F_WET) && U.row0 == 0 && tid == 0) A.wet[U.t] = 0;  // its strips' updates join their flags
+                if (!strip_unit<H, RESIDENT_THREADS / 32, ON, true>(M.s, A, sm, &bar, phase, rowc, red, U.t, U.ts, U.tj,
+                                                                    U.ti, U.row0, U.run, S.dt, S.dx,
+                                                                    (S.flags & F_WAVE) != 0, S.p, mst, V.wave_bits))
+                    return;
+            }
+        }
+        moved = false;
+        if (!grid_barrier(grid, ctl, met)) return;
+        if (control) next_settings(A, V, step_view(A.R, b ^ 1), any, grid);
+        for (int c0 = 0; c0 < units; c0 += UNITS_HELD) {
+            const int n = units > UNITS_HELD ? take(c0) : units;
+            for (int i = 0; i < n; ++i)
+                if (steps[i].flags & F_RUN)
+                    if (!update_unit<H>(M.u, A, V, sm, &bar, phase, places[i], steps[i])) return;
+        }
+        if (!grid_barrier(grid, ctl, met)) return;
+        const uint32_t next = __ldcg(&ctl->any);
+        const int rebuild = __ldcg(&grid->rebuild);
+        if (tid < units && units <= UNITS_HELD) steps[tid] = unit_step(A, step_view(A.R, b ^ 1), places[tid].run);
+        if (follow) {
+            boundary_items(A, V, (int)(blockIdx.x * RESIDENT_THREADS) + tid, (int)(gridDim.x * RESIDENT_THREADS), 2);
+            if (!grid_barrier(grid, ctl, met)) return;
+        }
+        if (control) tally_items(A, V, tid, RESIDENT_THREADS);
+        if (rebuild) {
+            if (!grid_barrier(grid, ctl, met)) return;
+            if (control) rebuild_lists(A, V, false, (any & ANY_ACT) != 0, true);
+            if (!grid_barrier(grid, ctl, met)) return;
+            nwork = __ldcg(&ctl->nwork);
+            const int woken = __ldcg(&ctl->nwoken);
+            if (woken) {
+                if (!control) plan_tiles(A, step_view(A.R, b ^ 1).parity, A.woken, woken, blockIdx.x, workers);
+                if (!grid_barrier(grid, ctl, met)) return;
+            }
+            moved = true;
+        }
+        b ^= 1;
+        mst = 0;
+        any = next;
+    }
+    // the settings of the step that comes next where the other forms of the loop read them
+    if (b) {
+        if (!grid_barrier(grid, ctl, met)) return;
+        if (control) adopt_settings(A);
+    }
+    grid_leave(grid);
+}
+
+template <int H>
+constexpr int resident_smem() {
+    return StripImage<H>::SMEM > UpdateStrip<H>::SMEM ? StripImage<H>::SMEM : UpdateStrip<H>::SMEM;
+}
+
+struct ResidentForm {
+    const void* kernel;
+    int smem;
+};
+static ResidentForm resident_form(int rows, bool on) {
+    switch (rows) {
+        case 16:
+            return {on ? (const void*)resident_kernel<16, true> : (const void*)resident_kernel<16, false>,
+                    resident_smem<16>()};
+        case 8:
+            return {on ? (const void*)resident_kernel<8, true> : (const void*)resident_kernel<8, false>,
+                    resident_smem<8>()};
+        default:
+            return {on ? (const void*)resident_kernel<4, true> : (const void*)resident_kernel<4, false>,
+                    resident_smem<4>()};
+    }
+}
+
+cudaError_t resident_setup() {
+    cudaError_t e = cudaSuccess;
+    for (const int rows : {16, 8, 4})
+        for (const bool on : {true, false}) {
+            const ResidentForm f = resident_form(rows, on);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(f.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, f.smem);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(f.kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+        }
+    return e;
+}
+
+// The resident CTAs a SM of the resident loop with strips of `rows` rows (16, 8 or 4).
+int resident_occupancy(int rows) {
+    int least = 1 << 20;
+    for (const bool on : {true, false}) {
+        const ResidentForm f = resident_form(rows, on);
+        int occ = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, f.kernel, RESIDENT_THREADS, f.smem);
+        least = occ < least ? occ : least;
+    }
+    return least;
+}
+
+// Up to max_steps steps in one cooperative launch of `grid` CTAs (at least two, at most as many as are resident at
+// once); the control block's grid state starts at zero.
+cudaError_t launch_resident(int rows, const ResidentMaps& M, const StepArgs& A, int grid, int max_steps, cudaStream_t s) {
+    const ResidentForm f = resident_form(rows, A.P.second && A.P.sheet && A.P.mirror && A.P.carry);
+    ResidentMaps maps = M;
+    StepArgs args = A;
+    void* params[] = {&maps, &args, &max_steps};
+    return cudaLaunchCooperativeKernel(f.kernel, dim3(grid), dim3(RESIDENT_THREADS), params, f.smem, s);
 }
 
 }  // namespace W2B_ARITH
@@ -1021,28 +1407,6 @@ void launch_momentum(const StepArgs& A, int sms, cudaStream_t s) {
 
 // ------------------------------------------------------------------ envelope pass
 
-// The envelope of one own cell (wadi2d/engine/maxima.py:75-92; the CPU twin forms the centre speed in float64) with
-// every load issued before any store, so that a thread's loads make one round trip; only the entries that change are
-// written. un, vn: the face velocities after the step.
-__device__ __forceinline__ void envelope_cell(const StepArgs& A, int fid, int k, float dk, float hk, float time,
-                                              float arrive, float deep, const float* un, const float* vn) {
-    const float d0 = A.env[0][fid], h0 = A.env[1][fid], s0 = A.env[2][fid], z0 = A.env[3][fid];
-    const float a0 = A.env[4][fid];
-    const float ue = un[k + 1], uw = un[k], vs = vn[k + A.px], vn0 = vn[k];
-    // max(old, new) as fmax32 forms it keeps old exactly when old >= new
-    if (!(d0 >= dk)) A.env[0][fid] = dk;
-    if (!(h0 >= hk)) A.env[1][fid] = hk;
-    if (dk > deep) {
-        const double uc = 0.5 * (double)(uw + ue);
-        const double vc = 0.5 * (double)(vn0 + vs);
-        const double sp = sqrt(uc * uc + vc * vc);
-        if (!((double)s0 >= sp)) A.env[2][fid] = (float)sp;
-        const double hz = sp * (double)dk;
-        if (!((double)z0 >= hz)) A.env[3][fid] = (float)hz;
-    }
-    if (a0 < 0.0f && dk >= arrive) A.env[4][fid] = time;
-}
-
 // The envelope after a step of the device loop, for the own cells of the work list's tiles whose runs record it at
 // this step (F_MAX); boundary cells are recorded by the boundary pass after its overwrite. A CTA a tile at a time, a
 // thread a cell; on steps that record no envelope every CTA returns at once.
@@ -1086,142 +1450,42 @@ __global__ void __launch_bounds__(TILE2, 2) envelope_kernel(StepArgs A) {
 
 // ------------------------------------------------------------------ boundary, tally, control (one CTA)
 
-// Boundary cells of every running run (wadi2d/solver/gpu/kernels/cells.cu:95-111) and their envelope entries after
-// the overwrite; in the device loop (control = 1) also the FP64 tally of every step and the design lines. Every item
-// is independent of the others (a follow boundary reads an interior cell), so the kernel is a grid-stride loop over
-// them: boundary cells, then tally faces, then one warp a line.
+// Boundary cells of every running run and their envelope entries after the overwrite; in the device loop (control = 1)
+// also the FP64 tally of every step and the design lines. Every item is independent of the others (a follow boundary
+// reads an interior cell), so the kernel is a grid-stride loop over them.
 __global__ void boundary_kernel(StepArgs A, int control) {
-    Ctl* ctl = A.ctl;
-    if (!(ctl->any & ANY_RUN)) return;
-    const RunTab& R = A.R;
+    if (!(A.ctl->any & ANY_RUN)) return;
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gstride = gridDim.x * blockDim.x;
-    for (int m = gtid; m < A.nb; m += gstride) {
-        const int k = A.bcell[m];
-        const int run = A.tile_run[tile_of_native(A, k)];
-        const int flags = R.flags[run];
-        if (!(flags & F_RUN)) continue;
-        const int n = 1 - R.parity[run];
-        float* h_next = A.hh[n];
-        const int kind = A.bkind[m];
-        if (kind == 0) {
-            h_next[k] = A.bh0[m];
-            A.d[k] = A.bd0[m];
-        } else if (kind == 1) {
-            h_next[k] = 0.0f;
-            A.d[k] = 0.0f;
-        } else {
-            const int r = A.bref[m];
-            h_next[k] = h_next[r];
-            A.d[k] = fmax32(A.d[r] + A.bd0[m], 0.0f);
-        }
-        if ((flags & F_MAX) == F_MAX)
-            envelope_cell(A, fid_of_native(A, k), k, A.d[k], h_next[k], R.max_time[run], ctl->arrive, ctl->deep,
-                          A.uu[0][n], A.uu[1][n]);
-    }
-    if (!control) return;
-    for (int m = gtid; m < A.ntally; m += gstride) {
-        const int face = A.tface[m];
-        const int run = A.tile_run[tile_of_native(A, face)];
-        if (!(R.flags[run] & F_RUN)) continue;
-        const float qv = A.taxis[m] ? A.q[1][face] : A.q[0][face];
-        A.ttotal[m] += R.dt_tally[run] * (double)(A.tsign[m] * qv);
-    }
-    // design lines (wadi2d/engine/monitor.py:229-232 at every step): Q = sum of sign q over the line's faces, FP64,
-    // lane-strided then a fixed shuffle tree; the running peak of |Q| and the time at the end of the step
-    const int lane = threadIdx.x & 31;
-    const int gwarp = gtid >> 5, nwarps = gstride >> 5;
-    for (int l = gwarp; l < A.nlines; l += nwarps) {
-        const int s = A.lstart[l], e = A.lstart[l + 1];
-        if (s >= e) continue;
-        const int run = A.tile_run[tile_of_native(A, A.lface[s])];
-        if (!(R.flags[run] & F_RUN)) continue;
-        double acc = 0.0;
-        for (int m = s + lane; m < e; m += 32) {
-            const int f = A.lface[m];
-            acc += (double)A.lsign[m] * (double)(A.laxis[m] ? A.q[1][f] : A.q[0][f]);
-        }
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-        if (lane == 0) {
-            A.lq[l] = acc;
-            const double a = fabs(acc);
-            if (a > A.lpeak[l]) {
-                A.lpeak[l] = a;
-                A.ltime[l] = R.t[run] + R.dt_step[run];
-            }
-        }
-    }
+    const StepView V = step_view(A.R, 0);
+    boundary_items(A, V, gtid, gstride, 0);
+    if (control) tally_items(A, V, gtid, gstride);
 }
 
-// Each running run's clock after its step (wadi2d/solver/stepper.py:113-124): the swap of its halves, t, the step
-// counts, the step rule on refresh steps (dt_min and non-finite checks); a run that stops marks the work list for
-// rebuilding. The threads of one CTA, after boundary_kernel.
+// The end of a step of the device loop, in the kernels of its own: each running run's clock and the next step's
+// settings. The threads of one CTA.
 __device__ void run_clocks(const StepArgs& A) {
     Ctl* ctl = A.ctl;
     if (!(ctl->any & ANY_RUN)) return;
-    const RunTab& R = A.R;
-    for (int r = threadIdx.x; r < A.nruns; r += blockDim.x) {
-        if (!(R.flags[r] & F_RUN)) continue;
-        R.parity[r] ^= 1;
-        R.t[r] = R.t[r] + R.dt_step[r];
-        R.nsteps[r] += 1;
-        R.steps_run[r] += 1;
-        if (R.flags[r] & F_WAVE) {
-            R.wave_last[r] = __uint_as_float(R.wave_bits[r]);
-            const double w = (double)__uint_as_float(R.wave_bits[r]);
-            if (!isfinite(w)) {
-                R.status[r] = W2B_ENONFINITE;
-            } else {
-                const double lim = ctl->cfl * (double)R.dx[r] / (ctl->wave_floor > w ? ctl->wave_floor : w);
-                R.dt[r] = ctl->dt_max < lim ? ctl->dt_max : lim;
-                if (R.dt[r] < ctl->dt_min) R.status[r] = W2B_EDTMIN;
-            }
-        }
-        if (!live_run(R, r, ctl)) ctl->prune = 1;  // its tiles leave the work list at this step's rebuild
-    }
+    const StepView V = step_view(A.R, 0);
+    for (int r = threadIdx.x; r < A.nruns; r += blockDim.x)
+        if (run_clock(A, V, V, r)) ctl->prune = 1;  // its tiles leave the work list at this step's rebuild
 }
 
 // Before a step of the device loop, for each run: the loop test and the step's settings
 // (wadi2d/solver/stepper.py:106-111). The threads of one CTA; ctl->any gathers the runs' flags.
 __device__ void step_settings(const StepArgs& A) {
     Ctl* ctl = A.ctl;
-    const RunTab& R = A.R;
     __shared__ uint32_t any;
     if (threadIdx.x == 0) any = 0u;
     __syncthreads();
+    const StepView V = step_view(A.R, 0);
     uint32_t mine = 0u;
-    for (int r = threadIdx.x; r < A.nruns; r += blockDim.x) {
-        if (!live_run(R, r, ctl)) {
-            R.flags[r] = 0;
-            continue;
-        }
-        const int refresh = R.refresh_due[r] || (R.nsteps[r] % ctl->dt_every == 0);
-        R.refresh_due[r] = 0;
-        const int activate = (int)(R.nsteps[r] % ctl->active_every == 0);
-        double dt = R.dt[r];
-        const double rest = R.t_end[r] - R.t[r];
-        if (rest < dt) dt = rest;
-        if (ctl->dt_max < dt) dt = ctl->dt_max;
-        R.dt_step[r] = dt;
-        R.dtf[r] = (float)dt;
-        const double t_new = R.t[r] + dt;
-        R.dt_tally[r] = t_new - R.t[r];
-        R.max_time[r] = (float)t_new;
-        const int want_max = ctl->max_every > 0 && ((R.nsteps[r] + 1) % ctl->max_every == 0);
-        const int act = activate && ctl->adaptive;
-        R.flags[r] = F_RUN | (refresh ? F_WAVE : 0) | (activate ? F_WET : 0) | (want_max ? F_MAX : 0) | (act ? F_ACT : 0);
-        if (refresh) R.wave_bits[r] = 0u;
-        mine |= ANY_RUN | (refresh ? ANY_WAVE : 0u) | (act ? ANY_ACT : 0u) | (want_max ? ANY_MAX : 0u);
-    }
+    for (int r = threadIdx.x; r < A.nruns; r += blockDim.x) mine |= run_settings(A, V, r);
     if (mine) atomicOr(&any, mine);
     __syncthreads();
     if (threadIdx.x == 0) ctl->any = any;
-    // the wave of each tile of a run that refreshes: the face pass's strip form takes each half's maximum into it
-    if (any & ANY_WAVE)
-        for (int t = threadIdx.x; t < A.ntiles; t += blockDim.x)
-            if (R.flags[A.tile_run[t]] & F_WAVE) A.wave[t] = 0.0f;
+    if (any & ANY_WAVE) clear_waves(A, V);
 }
-
-__global__ void prestep_kernel(StepArgs A) { step_settings(A); }
 
 // The end of a host-driven step of run 0: the swap of the ping-pong pairs (wadi2d/solver/gpu/backend.py:185-188).
 __global__ void endstep_kernel(StepArgs A) { A.R.parity[0] ^= 1; }
@@ -1237,116 +1501,41 @@ __global__ void setstep_kernel(StepArgs A, float dtf, int want_wave, int want_we
     if (want_wave) A.R.wave_bits[0] = 0u;
 }
 
-// ------------------------------------------------------------------ active-list rebuild (one CTA of 1024)
-
-// Exclusive scan of flags over one 1024-thread CTA; returns this thread's offset and the total in *total.
-__device__ __forceinline__ int block_scan(int flag, int* warp_sums, int* total) {
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    int v = flag;
-    for (int o = 1; o < 32; o <<= 1) {
-        const int n = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= o) v += n;
-    }
-    if (lane == 31) warp_sums[wid] = v;
-    __syncthreads();
-    if (wid == 0) {
-        int w = lane < (int)(blockDim.x >> 5) ? warp_sums[lane] : 0;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int n = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o) w += n;
-        }
-        warp_sums[lane] = w;  // inclusive sums of warps
-    }
-    __syncthreads();
-    const int before = (wid > 0 ? warp_sums[wid - 1] : 0) + v - flag;
-    *total = warp_sums[(blockDim.x >> 5) - 1];
-    __syncthreads();
-    return before;
-}
-
-// rebuild_active(check=True), wadi2d/solver/stepper.py:56-92, for the runs that rebuild at this step: wet or kept
-// tiles and their eight neighbours are active; a tile sleeps after SLEEP_CHECKS checks in a row that did not want it;
-// tiles that join the list are listed in woken for their wet share to be written. Then the work list: the active tiles
-// of the runs that take another step, rebuilt whenever the active list or the set of stepping runs changed.
-// only_work = 1: the work list alone, before the first step of the device loop.
-__device__ void rebuild_lists(const StepArgs& A, int only_work) {
-    Ctl* ctl = A.ctl;
-    const bool rebuild = !only_work && (ctl->any & ANY_ACT);
-    if (!only_work && !rebuild) {
-        // no tile woke at this step: the plan pass that follows has nothing to do
-        if (threadIdx.x == 0) ctl->nwoken = 0;
-        if (!ctl->prune) return;
-    }
-    const int nt = A.ntiles;
-    int* wet_eff = A.scratch;
-    int* flags = A.scratch + nt;
-    __shared__ int sums[32];
-    if (rebuild) {
-        for (int t = threadIdx.x; t < nt; t += blockDim.x) wet_eff[t] = t != 0 && (A.wet[t] != 0 || A.keep[t] != 0);
-        __syncthreads();
-        for (int t = threadIdx.x; t < nt; t += blockDim.x) {
-            if (t == 0) {
-                flags[0] = 0;
-                continue;
-            }
-            const int cur = A.is_act[t];
-            if (!(A.R.flags[A.tile_run[t]] & F_ACT)) {  // this tile's run does not rebuild at this step
-                flags[t] = cur;
-                continue;
-            }
-            int act = wet_eff[t];
-            for (int n = 0; n < 8; ++n) act |= wet_eff[A.nbr[8 * t + n]];
-            if (act)
-                A.idle[t] = 0;
-            else
-                A.idle[t] += 1;
-            act |= cur && A.idle[t] < SLEEP_CHECKS;
-            flags[t] = act | ((act && !cur) << 1);
-            A.is_act[t] = act;
-        }
-        __syncthreads();
-        int nact = 0, nwoken = 0;
-        for (int base = 0; base < nt; base += blockDim.x) {
-            const int t = base + threadIdx.x;
-            const int f = t < nt ? flags[t] : 0;
-            int tot_a, tot_w;
-            const int oa = block_scan(f & 1, sums, &tot_a);
-            const int ow = block_scan((f >> 1) & 1, sums, &tot_w);
-            if (f & 1) A.active[nact + oa] = t;
-            if (f & 2) A.woken[nwoken + ow] = t;
-            nact += tot_a;
-            nwoken += tot_w;
-        }
-        if (threadIdx.x == 0) {
-            ctl->nact = nact;
-            ctl->nwoken = nwoken;
-        }
-    }
-    // the work list, in tile order: active tiles whose run takes another step
-    int nwork = 0;
-    for (int base = 0; base < nt; base += blockDim.x) {
-        const int t = base + threadIdx.x;
-        const int f = t > 0 && t < nt && A.is_act[t] && live_run(A.R, A.tile_run[t], ctl);
-        int tot;
-        const int o = block_scan(f, sums, &tot);
-        if (f) A.work[nwork + o] = t;
-        nwork += tot;
-    }
+// Before the first step of the device loop, in one CTA of 1024 threads: the loop's settings (c; the stored-momenta flag
+// stays), each run's clock (clocks and t_ends, or a single run's by value), the work list of the runs that take a step,
+// and the first step's settings.
+__global__ void __launch_bounds__(1024) begin_kernel(const __grid_constant__ StepArgs A, Ctl c, W2BClock one, double t_end,
+                                                     long long max_steps, const W2BClock* clocks,
+                                                     const double* t_ends) {
+    const RunTab& R = A.R;
     if (threadIdx.x == 0) {
-        ctl->nwork = nwork;
-        ctl->prune = 0;
+        c.m_stored = A.ctl->m_stored;
+        *A.ctl = c;
     }
+    for (int r = threadIdx.x; r < A.nruns; r += blockDim.x) {
+        const W2BClock k = clocks ? clocks[r] : one;
+        R.t[r] = k.t;
+        R.dt[r] = k.dt;
+        R.t_end[r] = t_ends ? t_ends[r] : t_end;
+        R.nsteps[r] = k.nsteps;
+        R.steps_run[r] = 0;
+        R.max_steps[r] = max_steps;
+        R.refresh_due[r] = k.refresh_due;
+        R.status[r] = 0;
+    }
+    __syncthreads();
+    rebuild_lists(A, step_view(A.R, 0), true, false, false);
+    __syncthreads();
+    step_settings(A);
 }
-
-__global__ void __launch_bounds__(1024) activity_kernel(StepArgs A, int only_work) { rebuild_lists(A, only_work); }
 
 // The end of a step of the device loop and the settings of the next, in one CTA of 1024 threads: each running run's
 // clock, the active-list rebuild (for the runs that check at this step) with the woken tiles and the work list, then
 // the next step's loop test and settings. plan_kernel, after it, takes the woken tiles.
-__global__ void __launch_bounds__(1024) control_kernel(StepArgs A) {
+__global__ void __launch_bounds__(1024) control_kernel(const __grid_constant__ StepArgs A) {
     run_clocks(A);
     __syncthreads();
-    rebuild_lists(A, 0);
+    rebuild_lists(A, step_view(A.R, 0), false, (A.ctl->any & ANY_ACT) != 0, A.ctl->prune);
     __syncthreads();
     step_settings(A);
 }
@@ -1354,22 +1543,8 @@ __global__ void __launch_bounds__(1024) control_kernel(StepArgs A) {
 // refresh_plan of the listed tiles (wadi2d/solver/gpu/kernels/cells.cu:66-78) from the current mean depth. count < 0:
 // the tiles the device loop's last rebuild woke (ctl->nwoken, 0 when it did not rebuild).
 __global__ void __launch_bounds__(256) plan_kernel(StepArgs A, const int32_t* list, int count) {
-    Ctl* ctl = A.ctl;
-    if (count < 0) count = ctl->nwoken;
-    for (int a = blockIdx.x; a < count; a += gridDim.x) {
-        const int t = list[a];
-        const int tj = A.tiles[2 * t], ti = A.tiles[2 * t + 1];
-        const int base = (tj * TILE + GY) * A.px + ti * TILE + GX;
-        const int ts = table_of(A, t);
-        const float2* pairs_t = A.dtab2 + (size_t)ts * (A.rows - 1) * TILE2;
-        const float* h = A.hh[A.R.parity[A.tile_run[t]]];
-        for (int c = 0; c < 4; ++c) {
-            const int jj = threadIdx.y * 4 + c, ii = threadIdx.x;
-            const int local = jj * TILE + ii;
-            const int k = base + jj * A.px + ii;
-            A.om[k] = cell_plan(h[k], A.hc[ts * TILE2 + local], pairs_t + local, A.rows);
-        }
-    }
+    if (count < 0) count = A.ctl->nwoken;
+    plan_tiles(A, A.R.parity, list, count, blockIdx.x, gridDim.x);
 }
 
 // Maxima.update over the active tiles, host-driven (wadi2d/engine/maxima.py:118-130): the current halves are the
@@ -1445,6 +1620,32 @@ __global__ void pack_tables_kernel(const float* __restrict__ dtab, const float* 
         const float* b = ftaby + cell * rows * 2 + 2 * r;
         fy[o] = make_float4(b[0], b[1], b[2], b[3]);
     }
+}
+
+// The boundary cells by tile (StepArgs::bstart, bitem), from their NATIVE indices: counts, their running sum, then the
+// items; next: ntiles ints of scratch. One CTA of 1024 threads.
+__global__ void __launch_bounds__(1024) boundary_index_kernel(StepArgs A, int32_t* start, int32_t* item, int32_t* next) {
+    __shared__ int sums[32];
+    const int nt = A.ntiles, tid = threadIdx.x;
+    for (int t = tid; t < nt + 2; t += blockDim.x) start[t] = 0;
+    __syncthreads();
+    for (int m = tid; m < A.nb; m += blockDim.x) {
+        atomicAdd(start + tile_of_native(A, A.bcell[m]), 1);
+        if (A.bkind[m] > 1) start[nt + 1] = 1;
+    }
+    __syncthreads();
+    int before = 0;
+    for (int base = 0; base < nt; base += blockDim.x) {
+        const int t = base + tid;
+        const int n = t < nt ? start[t] : 0;
+        int total;
+        const int o = before + block_scan(n, sums, &total);
+        if (t < nt) start[t] = next[t] = o;
+        before += total;
+    }
+    if (tid == 0) start[nt] = before;
+    __syncthreads();
+    for (int m = tid; m < A.nb; m += blockDim.x) item[atomicAdd(next + tile_of_native(A, A.bcell[m]), 1)] = m;
 }
 
 // Boundary marks: clear, then one bit per boundary cell.
