@@ -3,6 +3,7 @@
 // The handle binds caller-owned device buffers; the only memory it allocates is its own host record (with a pinned copy
 // of the run table for the loop's read-back), the CUDA graphs of the device loop and the index of the boundary cells. Ping-pong pairs (h, u, v, mx, my) are resolved through the handle's parity, which
 // flips after every step: the reference swaps its arrays the same way (wadi2d/solver/gpu/backend.py:185-188).
+#include <cmath>
 #include <cstddef>
 #include <cstdio>
 #include <cstring>
@@ -70,7 +71,6 @@ __global__ void control_kernel(const __grid_constant__ StepArgs A);
 __global__ void begin_kernel(const __grid_constant__ StepArgs A, Ctl c, W2BClock one, double t_end, long long max_steps,
                              const W2BClock* clocks, const double* t_ends);
 __global__ void setstep_kernel(StepArgs A, float dtf, int want_wave, int want_wet, int nact);
-__global__ void endstep_kernel(StepArgs A);
 __global__ void plan_kernel(StepArgs A, const int32_t* list, int count);
 __global__ void maxima_kernel(StepArgs A, float time, float arrive, float deep, int nact);
 __global__ void tally_kernel(StepArgs A, double dt);
@@ -94,6 +94,7 @@ struct LoopConfig {
 };
 constexpr int TUNE_CANDIDATES = 7;  // the default, it with more steps a graph, two strip forms, three resident ones
 constexpr int FORCED = TUNE_CANDIDATES;          // the slot of a configuration the caller fixes
+constexpr int TAILS = 2, TAIL_STEPS[TAILS] = {4, 1};  // graphs of fewer steps, for the end of a call
 constexpr int TUNE_SAMPLES = 3;                  // timed launches a candidate before the tuner settles
 constexpr int MAX_GRAPH_STEPS = 64;
 constexpr double TUNE_MARGIN = 0.02;
@@ -107,8 +108,8 @@ constexpr double TUNE_MARGIN = 0.02;
 struct Loop {
     LoopConfig cand[TUNE_CANDIDATES + 1];
     int ncand = 0;
-    cudaGraphExec_t exec[TUNE_CANDIDATES + 1] = {};
-    unsigned version[TUNE_CANDIDATES + 1];
+    cudaGraphExec_t exec[TUNE_CANDIDATES + 1][TAILS + 1] = {};  // of the configuration's steps, and of TAIL_STEPS'
+    unsigned version[TUNE_CANDIDATES + 1][TAILS + 1];
     double sec[TUNE_CANDIDATES] = {};
     long long steps[TUNE_CANDIDATES] = {};
     int samples[TUNE_CANDIDATES] = {};
@@ -116,7 +117,8 @@ struct Loop {
     int tuning = 1;
     cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};  // a launch's start; the ends of two successive launches
     Loop() {
-        for (auto& v : version) v = ~0u;
+        for (auto& v : version)
+            for (auto& w : v) w = ~0u;
     }
 };
 
@@ -302,22 +304,23 @@ static int build_tmaps(Handle& H) {
     auto own = [&](CUtensorMap* m, const float* p) {
         if (st == W2B_OK) st = encode_2d(enc, m, p, H.g, H.L, 32, 32);
     };
-    box(&H.tmaps.d, B.d);
-    box(&H.tmaps.qx, B.qx);
-    box(&H.tmaps.qy, B.qy);
-    box(&H.tmaps.om, B.om);
-    box(&H.tmaps.zcx, B.zcx);
-    box(&H.tmaps.zcy, B.zcy);
-    box(&H.tmaps.qx1, B.qx1);
-    box(&H.tmaps.qy1, B.qy1);
-    own(&H.tmaps.res, B.res);
-    own(&H.tmaps.src, B.src);
+    box(&H.tmaps.tile.d, B.d);
+    box(&H.tmaps.tile.qx, B.qx);
+    box(&H.tmaps.tile.qy, B.qy);
+    box(&H.tmaps.tile.om, B.om);
+    box(&H.tmaps.tile.zcx, B.zcx);
+    box(&H.tmaps.tile.zcy, B.zcy);
+    box(&H.tmaps.update.qx1, B.qx1);
+    box(&H.tmaps.update.qy1, B.qy1);
+    own(&H.tmaps.update.res, B.res);
+    own(&H.tmaps.update.src, B.src);
     for (int p = 0; p < 2; ++p) {
-        box(&H.tmaps.h[p], B.h[p]);
-        box(&H.tmaps.u[p], B.u[p]);
-        box(&H.tmaps.v[p], B.v[p]);
-        own(&H.tmaps.mx[p], B.mx[p]);
-        own(&H.tmaps.my[p], B.my[p]);
+        box(&H.tmaps.tile.h[p], B.h[p]);
+        box(&H.tmaps.update.h[p], B.h[p]);
+        box(&H.tmaps.tile.u[p], B.u[p]);
+        box(&H.tmaps.tile.v[p], B.v[p]);
+        own(&H.tmaps.tile.mx[p], B.mx[p]);
+        own(&H.tmaps.tile.my[p], B.my[p]);
     }
     // the strip forms' boxes, 40 columns of the rows the face arithmetic reads around a strip of `rows` rows: the
     // velocities rows + 4 (two above, two below), the y discharge rows + 2, the x lip rows, depth, mean depth, x
@@ -355,12 +358,16 @@ static int build_tmaps(Handle& H) {
     return st;
 }
 
-static void drop_graph(Handle& H, int c) {
-    if (H.loop.exec[c]) {
-        cudaGraphExecDestroy(H.loop.exec[c]);
-        H.loop.exec[c] = nullptr;
+static void drop_graph(Handle& H, int c, int tail) {
+    if (H.loop.exec[c][tail]) {
+        cudaGraphExecDestroy(H.loop.exec[c][tail]);
+        H.loop.exec[c][tail] = nullptr;
     }
-    H.loop.version[c] = ~0u;
+    H.loop.version[c][tail] = ~0u;
+}
+
+static void drop_graph(Handle& H, int c) {
+    for (int k = 0; k <= TAILS; ++k) drop_graph(H, c, k);
 }
 
 static void drop_graphs(Handle& H) {
@@ -433,17 +440,20 @@ static size_t host_bytes(int nruns) {
 }
 
 // The face pass of a host-driven step (w2b_step, w2b_step_timed) over n tiles: in the form and at the CTAs a SM the
-// device loop's tuner settled on, the tile form while it tunes.
+// device loop's tuner settled on (strips of 8 rows for its resident loop of 8 or 4), and while it tunes in strips of 8
+// rows, which are within a percent of the fastest form at every size measured (81 tiles: 7.1 us against the tile form's
+// 12.4; 1,680 tiles: 74 against 88).
 static void launch_faces_host(Handle& H, const StepArgs& A, int n, cudaStream_t s) {
     const LoopConfig& C = H.loop.cand[H.loop.chosen];
-    if (!H.loop.tuning && C.strips) {
-        const int rows = C.strips == 16 ? 16 : 8;
-        const int occ = !C.resident ? C.faces_per_sm : (rows == 16 ? H.strips16_occ : H.strips8_occ);
-        const int g = H.sms * occ, units = (TILE / rows) * n;
-        passes(H.P).launch_strips(rows, H.tmaps, A, units < g ? units : g, s);
-    } else {
+    const bool settled = !H.loop.tuning;
+    if (settled && !C.strips) {
         passes(H.P).launch_faces(H.tmaps, A, faces_grid(H, n), s);
+        return;
     }
+    const int rows = settled && C.strips == 16 ? 16 : 8;
+    const int occ = settled && !C.resident ? C.faces_per_sm : (rows == 16 ? H.strips16_occ : H.strips8_occ);
+    const int g = H.sms * occ, units = (TILE / rows) * n;
+    passes(H.P).launch_strips(rows, H.tmaps, A, units < g ? units : g, s);
 }
 
 // One step of the device loop under launch configuration C: every running run advances by one of its own steps.
@@ -460,9 +470,11 @@ static int launch_loop_step(Handle& H, const LoopConfig& C, cudaStream_t s) {
         X.launch_faces(H.tmaps, A, tiles < fgrid ? tiles : fgrid, s);
     X.launch_update(H.tmaps, A, tiles < ugrid ? tiles : ugrid, s);
     envelope_kernel<<<H.sms * 2, TILE2, 0, s>>>(A);
-    boundary_kernel<<<boundary_grid(H, 1), 256, 0, s>>>(A, 1);
-    control_kernel<<<1, 1024, 0, s>>>(A);  // clocks, rebuild and work list, the next step's settings
-    plan_kernel<<<grid, 256, 0, s>>>(A, A.woken, -1);
+    // the small kernels start while the one before them ends (grid_wait); the passes do not: CTAs that start as others
+    // leave crowd onto the SMs that finish first, and the pass then waits for those (384 tiles: 57 us a step against 49)
+    CK(launch_next(boundary_kernel, boundary_grid(H, 1), 256, 0, s, A, 1));
+    CK(launch_next(control_kernel, 1, 1024, 0, s, A));  // clocks, rebuild and work list, the next step's settings
+    CK(launch_next(plan_kernel, grid, 256, 0, s, A, A.woken, -1));
     CKL("loop step");
     return W2B_OK;
 }
@@ -742,9 +754,8 @@ int32_t w2b_step(void* handle, float dt, int32_t want_wave, int32_t want_wet, vo
     Handle* H = static_cast<Handle*>(handle);
     cudaStream_t s = (cudaStream_t)stream;
     if (H->nruns != 1) return W2B_EINVAL;  // a batch steps in the device loop
-    if (want_wave) CK(cudaMemsetAsync(H->B.wave, 0, sizeof(float) * H->g.ntiles, s));
     const StepArgs A = make_args(*H);
-    setstep_kernel<<<1, 1, 0, s>>>(A, dt, want_wave, want_wet, H->nact);
+    setstep_kernel<<<1, want_wave ? 1024 : 32, 0, s>>>(A, dt, want_wave, want_wet, H->nact);
     if (H->nact == 0) {  // as the reference: no tiles, no swap
         CKL("w2b_step");
         return W2B_OK;
@@ -752,8 +763,7 @@ int32_t w2b_step(void* handle, float dt, int32_t want_wave, int32_t want_wet, vo
     const int grid = blocks_for(*H, H->nact);
     launch_faces_host(*H, A, H->nact, s);
     passes(H->P).launch_update(H->tmaps, A, grid, s);
-    if (H->nb) boundary_kernel<<<boundary_grid(*H, 0), 256, 0, s>>>(A, 0);
-    endstep_kernel<<<1, 1, 0, s>>>(A);
+    CK(launch_next(boundary_kernel, boundary_grid(*H, 0), 256, 0, s, A, 0));
     CKL("w2b_step");
     H->cur ^= 1;
     return W2B_OK;
@@ -766,17 +776,15 @@ int32_t w2b_step_timed(void* handle, float dt, int32_t want_wave, int32_t want_w
     if (H->nact == 0 || H->nruns != 1) return W2B_EINVAL;
     cudaEvent_t ev[4];
     for (auto& e : ev) CK(cudaEventCreate(&e));
-    if (want_wave) CK(cudaMemsetAsync(H->B.wave, 0, sizeof(float) * H->g.ntiles, s));
     const StepArgs A = make_args(*H);
-    setstep_kernel<<<1, 1, 0, s>>>(A, dt, want_wave, want_wet, H->nact);
+    setstep_kernel<<<1, 1024, 0, s>>>(A, dt, want_wave, want_wet, H->nact);
     const int grid = blocks_for(*H, H->nact);
     CK(cudaEventRecord(ev[0], s));
     launch_faces_host(*H, A, H->nact, s);
     CK(cudaEventRecord(ev[1], s));
     passes(H->P).launch_update(H->tmaps, A, grid, s);
     CK(cudaEventRecord(ev[2], s));
-    if (H->nb) boundary_kernel<<<boundary_grid(*H, 0), 256, 0, s>>>(A, 0);
-    endstep_kernel<<<1, 1, 0, s>>>(A);
+    boundary_kernel<<<boundary_grid(*H, 0), 256, 0, s>>>(A, 0);
     CK(cudaEventRecord(ev[3], s));
     CKL("w2b_step_timed");
     H->cur ^= 1;
@@ -789,11 +797,12 @@ int32_t w2b_step_timed(void* handle, float dt, int32_t want_wave, int32_t want_w
 int32_t w2b_max_wave(void* handle, float* out, void* stream) {
     if (!handle || !out) return W2B_EINVAL;
     Handle* H = static_cast<Handle*>(handle);
-    int32_t status = 0;
-    CK(cudaMemcpyAsync(out, H->R.wave_bits, sizeof(float), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
-    CK(cudaMemcpyAsync(&status, &H->ctl()->status, sizeof(int32_t), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
+    int32_t* const held = reinterpret_cast<int32_t*>(H->host);  // pinned: the two copies queue without the host
+    CK(cudaMemcpyAsync(held, H->R.wave_bits, sizeof(float), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
+    CK(cudaMemcpyAsync(held + 1, &H->ctl()->status, sizeof(int32_t), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
     CK(cudaStreamSynchronize((cudaStream_t)stream));
-    return status == W2B_ETIMEOUT ? W2B_ETIMEOUT : W2B_OK;
+    memcpy(out, held, sizeof(float));
+    return held[1] == W2B_ETIMEOUT ? W2B_ETIMEOUT : W2B_OK;
 }
 
 int32_t w2b_wet_flags(void* handle, int32_t* out, void* stream) {
@@ -949,26 +958,43 @@ int32_t w2b_tally(void* handle, double dt, void* stream) {
     return W2B_OK;
 }
 
-// The graph of configuration c, captured again when the arguments it would hold have changed.
-static int loop_graph(Handle& H, int c) {
+// The graph of configuration c, of its steps (tail 0) or of TAIL_STEPS[tail - 1], captured again when the arguments it
+// would hold have changed.
+static int loop_graph(Handle& H, int c, int tail) {
     Loop& L = H.loop;
-    if (L.exec[c] && L.version[c] == H.version) return W2B_OK;
-    drop_graph(H, c);
+    if (L.exec[c][tail] && L.version[c][tail] == H.version) return W2B_OK;
+    drop_graph(H, c, tail);
     cudaGraph_t graph;
     CK(cudaStreamBeginCapture(H.cap, cudaStreamCaptureModeThreadLocal));
     int stc = W2B_OK;
-    for (int k = 0; k < L.cand[c].steps && stc == W2B_OK; ++k) stc = launch_loop_step(H, L.cand[c], H.cap);
+    const int steps = tail ? TAIL_STEPS[tail - 1] : L.cand[c].steps;
+    for (int k = 0; k < steps && stc == W2B_OK; ++k) stc = launch_loop_step(H, L.cand[c], H.cap);
     cudaError_t e = cudaStreamEndCapture(H.cap, &graph);
     if (stc != W2B_OK) {
         if (e == cudaSuccess) cudaGraphDestroy(graph);
         return stc;
     }
     CK(e);
-    e = cudaGraphInstantiate(&L.exec[c], graph, 0);
+    e = cudaGraphInstantiate(&L.exec[c][tail], graph, 0);
     cudaGraphDestroy(graph);
-    if (e != cudaSuccess) L.exec[c] = nullptr;  // nothing to destroy later
+    if (e != cudaSuccess) L.exec[c][tail] = nullptr;  // nothing to destroy later
     CK(e);
-    L.version[c] = H.version;
+    L.version[c][tail] = H.version;
+    return W2B_OK;
+}
+
+// One launch of `steps` loop steps of configuration c, or of fewer: the resident loop stops by itself, and a graph of
+// the configuration's steps is made up of whole ones and of tails. Returns the status; *took: the steps launched.
+static int launch_chunk(Handle& H, int c, int64_t steps, int64_t* took, cudaStream_t s) {
+    Loop& L = H.loop;
+    const LoopConfig& C = L.cand[c];
+    *took = C.steps;
+    if (C.resident) return launch_loop_resident(H, C, s);
+    int tail = 0;
+    while (tail < TAILS && *took > steps) *took = TAIL_STEPS[tail++];
+    const int st = loop_graph(H, c, tail);
+    if (st != W2B_OK) return st;
+    CK(cudaGraphLaunch(L.exec[c][tail], s));
     return W2B_OK;
 }
 
@@ -995,9 +1021,11 @@ static void tune_sample(Handle& H, int c, long long live, float ms) {
         if (k != best) drop_graph(H, k);
 }
 
-// The device-resident loop. Steps run in chunks (a captured graph, or one launch of the resident loop, of the launch
-// configuration's steps), every running run advancing one of its own steps each loop step; after each chunk the host
-// reads the run table and the control block once, into pinned memory.
+// The device-resident loop. Steps run in chunks (a captured graph, or one launch of the resident loop), every running
+// run advancing one of its own steps each loop step; after a few chunks the host reads the run table and the control
+// block once, into pinned memory. Empty steps at the end of a call cost a launch of every kernel each (about 20 us for
+// 1,680 tiles), so the last chunks are graphs of fewer steps.
+constexpr int CHUNKS = 8;
 static int advance_runs(Handle* H, const W2BStepper* cfg, const double* t_end, int64_t max_steps, W2BClock* clocks,
                         cudaStream_t s) {
     const int n = H->nruns;
@@ -1033,24 +1061,39 @@ static int advance_runs(Handle* H, const W2BStepper* cfg, const double* t_end, i
     const RunTab T = run_table(held, n);
     Loop& L = H->loop;
     long long ran_before = 0;  // loop steps so far in this call (the largest steps_run of any run)
+    bool first_round = true;     // the runs' clocks are the caller's, not yet read back
     int end = 1, have_prev = 0;  // ev[end] takes this launch's end; ev[3 - end] holds the last one's, if have_prev
     if (L.tuning)  // every candidate's graph before the first timed launch: no capture falls inside a timing
         for (int k = 0; k < L.ncand; ++k) {
-            const int stc = L.cand[k].resident ? W2B_OK : loop_graph(*H, k);
+            const int stc = L.cand[k].resident ? W2B_OK : loop_graph(*H, k, 0);
             if (stc != W2B_OK) return stc;
         }
     for (;;) {
         const bool timed = L.tuning != 0;
         const int c = timed ? L.next : L.chosen;
-        const bool resident = L.cand[c].resident != 0;
-        int stc = resident ? W2B_OK : loop_graph(*H, c);
-        if (stc != W2B_OK) return stc;
         if (timed && !have_prev) CK(cudaEventRecord(L.ev[0], s));
-        if (resident)
-            stc = launch_loop_resident(*H, L.cand[c], s);
-        else
-            CK(cudaGraphLaunch(L.exec[c], s));
-        if (stc != W2B_OK) return stc;
+        // a timed launch is one of the candidate's steps; else as many as the runs will want at their current steps (a
+        // step rule that shortens them on the way takes another round), at most CHUNKS before the host looks
+        int64_t want = L.cand[c].steps;
+        if (!timed) {
+            want = 1;
+            for (int r = 0; r < n; ++r) {
+                double dt = first_round ? clocks[r].dt : T.dt[r];
+                dt = dt < cfg->dt_max ? dt : cfg->dt_max;
+                const double left = t_end[r] - (first_round ? clocks[r].t : T.t[r]);
+                const int64_t cap = max_steps - (first_round ? 0 : T.steps_run[r]);
+                const double est = dt > 0.0 ? ceil((left - 1e-9) / dt) : 1.0;
+                const int64_t need = est < (double)cap ? (int64_t)est : cap;
+                if ((first_round || T.status[r] == 0) && need > want) want = need;
+            }
+        }
+        first_round = false;
+        for (int k = 0; k < (timed ? 1 : CHUNKS) && want > 0; ++k) {
+            int64_t took = 0;
+            const int stc = launch_chunk(*H, c, want, &took, s);
+            if (stc != W2B_OK) return stc;
+            want -= took;
+        }
         if (timed) CK(cudaEventRecord(L.ev[end], s));
         CK(cudaMemcpyAsync(held, H->B.runs, run_table_bytes(n), cudaMemcpyDeviceToHost, s));
         CK(cudaMemcpyAsync(hctl, H->ctl(), sizeof(Ctl), cudaMemcpyDeviceToHost, s));

@@ -207,7 +207,8 @@ struct StepArgs {
 struct StripMaps {
     CUtensorMap d, h[2], u[2], v[2], qx, qy, zcx, zcy, mx[2], my[2];
 };
-// The update's boxes for a strip of H rows (the resident loop): 40 x (H + 3), one row above to two below, and 32 x H.
+// The update's boxes: for a whole tile 40 x 36, and 32 x 32 for the residual and the source; for a strip of H rows (the
+// resident loop) 40 x (H + 3), one row above to two below, and 32 x H.
 struct UpdateMaps {
     CUtensorMap qx1, qy1, h[2], res, src;
 };
@@ -215,11 +216,14 @@ struct ResidentMaps {
     StripMaps s;
     UpdateMaps u;
 };
-struct TMaps {
+struct TileMaps {
     CUtensorMap d, h[2], u[2], v[2], qx, qy, om, zcx, zcy, mx[2], my[2];
-    CUtensorMap qx1, qy1;  // 40 x 36 boxes for the update pass
-    CUtensorMap res, src;  // 32 x 32 boxes
-    StripMaps s16, s8;     // strips of 16 and of 8 rows
+};
+// Every kernel is launched with the maps it takes only: they are its parameters, copied with each launch.
+struct TMaps {
+    TileMaps tile;
+    UpdateMaps update;
+    StripMaps s16, s8;  // strips of 16 and of 8 rows
 };
 
 // ------------------------------------------------------------------ float32 helpers

@@ -409,15 +409,12 @@ __device__ __forceinline__ void fill_rowc(float* rowc, int rows) {
 // the tile's wave maximum goes to its run's maximum (an integer atomic max on the float bits). p is the parity of
 // the run's ping-pong halves.
 template <bool ON>
-__global__ void __launch_bounds__(FACES_THREADS, 2) faces_kernel(const __grid_constant__ TMaps M, StepArgs A) {
+__global__ void __launch_bounds__(FACES_THREADS, 2) faces_kernel(const __grid_constant__ TileMaps M, StepArgs A) {
     extern __shared__ __align__(128) float sm[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ float red[32];
     __shared__ float rowc[2 * 64 + 1];
     Ctl* ctl = A.ctl;
-    if (!(ctl->any & ANY_RUN)) return;
-    const int nwork = ctl->nwork;
-    const int mst = ctl->m_stored;
     const int tid = threadIdx.x;
     if (tid == 0) {
         mbar_init(&bar, 1);
@@ -425,6 +422,9 @@ __global__ void __launch_bounds__(FACES_THREADS, 2) faces_kernel(const __grid_co
     }
     fill_rowc(rowc, A.rows);
     __syncthreads();
+    if (!(ctl->any & ANY_RUN)) return;
+    const int nwork = ctl->nwork;
+    const int mst = ctl->m_stored;
     const float* statics[12] = {A.fl[0], A.fr[0], A.gl[0], A.gr[0], A.ef[0], A.cw[0],
                                 A.fl[1], A.fr[1], A.gl[1], A.gr[1], A.ef[1], A.cw[1]};
     uint32_t phase = 0;
@@ -685,7 +685,7 @@ __device__ __forceinline__ bool strip_unit(const StripMaps& SM_, const StepArgs&
 
 template <int H, bool ON>
 __global__ void __launch_bounds__(StripImage<H>::THREADS, StripImage<H>::CTAS)
-    strips_kernel(const __grid_constant__ TMaps M, StepArgs A) {
+    strips_kernel(const __grid_constant__ StripMaps M, StepArgs A) {
     using L = StripImage<H>;
     constexpr int PER = TILE / H;  // strips a tile
     extern __shared__ __align__(128) float sm[];
@@ -693,22 +693,22 @@ __global__ void __launch_bounds__(StripImage<H>::THREADS, StripImage<H>::CTAS)
     __shared__ float red[L::THREADS / 32];
     __shared__ float rowc[2 * 64 + 1];
     Ctl* ctl = A.ctl;
-    if (!(ctl->any & ANY_RUN)) return;
-    const int nunits = PER * ctl->nwork;
-    const int mst = ctl->m_stored;
     if (threadIdx.x == 0) {
         mbar_init(&bar, 1);
         fence_barrier_init();
     }
     fill_rowc(rowc, A.rows);
     __syncthreads();
+    if (!(ctl->any & ANY_RUN)) return;
+    const int nunits = PER * ctl->nwork;
+    const int mst = ctl->m_stored;
     uint32_t phase = 0;
     for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
         const int t = A.list[u / PER];
         const int run = A.tile_run[t];
         const int flags = A.R.flags[run];
         if (!(flags & F_RUN)) continue;  // the tile's run has finished: uniform over the CTA
-        if (!strip_unit<H, L::THREADS / 32, ON, false>(H == 16 ? M.s16 : M.s8, A, sm, &bar, phase, rowc, red, t,
+        if (!strip_unit<H, L::THREADS / 32, ON, false>(M, A, sm, &bar, phase, rowc, red, t,
                                                        table_of(A, t), A.tiles[2 * t], A.tiles[2 * t + 1], (u % PER) * H,
                                                        run, A.R.dtf[run], A.R.dx[run], (flags & F_WAVE) != 0,
                                                        A.R.parity[run], mst, A.R.wave_bits))
@@ -758,14 +758,14 @@ void launch_strips(int rows, const TMaps& M, const StepArgs& A, int grid, cudaSt
     const bool on = A.P.second && A.P.sheet && A.P.mirror && A.P.carry;
     if (rows == 16) {
         if (on)
-            strips_kernel<16, true><<<grid, StripImage<16>::THREADS, StripImage<16>::SMEM, s>>>(M, A);
+            strips_kernel<16, true><<<grid, StripImage<16>::THREADS, StripImage<16>::SMEM, s>>>(M.s16, A);
         else
-            strips_kernel<16, false><<<grid, StripImage<16>::THREADS, StripImage<16>::SMEM, s>>>(M, A);
+            strips_kernel<16, false><<<grid, StripImage<16>::THREADS, StripImage<16>::SMEM, s>>>(M.s16, A);
     } else {
         if (on)
-            strips_kernel<8, true><<<grid, StripImage<8>::THREADS, StripImage<8>::SMEM, s>>>(M, A);
+            strips_kernel<8, true><<<grid, StripImage<8>::THREADS, StripImage<8>::SMEM, s>>>(M.s8, A);
         else
-            strips_kernel<8, false><<<grid, StripImage<8>::THREADS, StripImage<8>::SMEM, s>>>(M, A);
+            strips_kernel<8, false><<<grid, StripImage<8>::THREADS, StripImage<8>::SMEM, s>>>(M.s8, A);
     }
 }
 
@@ -780,9 +780,9 @@ int faces_occupancy() {
 // The face pass, in its form with the numerics switches folded in when they are all on (the reference's defaults).
 void launch_faces(const TMaps& M, const StepArgs& A, int grid, cudaStream_t s) {
     if (A.P.second && A.P.sheet && A.P.mirror && A.P.carry)
-        faces_kernel<true><<<grid, FACES_THREADS, FACES_SMEM, s>>>(M, A);
+        faces_kernel<true><<<grid, FACES_THREADS, FACES_SMEM, s>>>(M.tile, A);
     else
-        faces_kernel<false><<<grid, FACES_THREADS, FACES_SMEM, s>>>(M, A);
+        faces_kernel<false><<<grid, FACES_THREADS, FACES_SMEM, s>>>(M.tile, A);
 }
 
 // ------------------------------------------------------------------ update pass
@@ -897,7 +897,7 @@ __device__ __forceinline__ int next_tile(const StepArgs& A, int a, int nwork) {
 
 // Issue (thread 0) the copies of tile t's update image against bar: the unscaled discharges and the old depth with
 // their ring, the residual, the source and Hc, and the tile's level cache (each cell's last level pair and its row).
-__device__ __forceinline__ void update_issue(float* sm, uint64_t* bar, const TMaps& M, const StepArgs& A, int t) {
+__device__ __forceinline__ void update_issue(float* sm, uint64_t* bar, const UpdateMaps& M, const StepArgs& A, int t) {
     const int p = A.R.parity[A.tile_run[t]];
     const int tj = A.tiles[2 * t], ti = A.tiles[2 * t + 1];
     fence_proxy_async();
@@ -919,21 +919,21 @@ __device__ __forceinline__ void update_issue(float* sm, uint64_t* bar, const TMa
 // level pairs from the cache, or for the cells whose row changed from the table (the gathers issued together). Once
 // every thread has read the image, thread 0 issues the next tile's copies into it, and they land while any gathers
 // return and the level, the wet share and the wet flag are finished.
-__global__ void __launch_bounds__(UPDATE_THREADS) update_kernel(const __grid_constant__ TMaps M, StepArgs A) {
+__global__ void __launch_bounds__(UPDATE_THREADS) update_kernel(const __grid_constant__ UpdateMaps M, StepArgs A) {
     extern __shared__ __align__(128) float sm[];
     __shared__ __align__(8) uint64_t bar;
     Ctl* ctl = A.ctl;
-    if (!(ctl->any & ANY_RUN)) return;
-    const int nwork = ctl->nwork;
     const int px = A.px;
     const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
-    // the face pass before this one has stepped: from now on the momenta are formed from the state (Ctl::m_stored)
-    if (blockIdx.x == 0 && tid == 0) ctl->m_stored = 0;
     if (tid == 0) {
         mbar_init(&bar, 1);
         fence_barrier_init();
     }
     __syncthreads();
+    if (!(ctl->any & ANY_RUN)) return;
+    const int nwork = ctl->nwork;
+    // the face pass before this one has stepped: from now on the momenta are formed from the state (Ctl::m_stored)
+    if (blockIdx.x == 0 && tid == 0) ctl->m_stored = 0;
     uint32_t phase = 0;
     const float* QX1 = sm + U_QX1 * BOX;
     const float* QY1 = sm + U_QY1 * BOX;
@@ -1018,7 +1018,7 @@ int update_occupancy() {
 }
 
 void launch_update(const TMaps& M, const StepArgs& A, int grid, cudaStream_t s) {
-    update_kernel<<<grid, UPDATE_THREADS, UPDATE_SMEM, s>>>(M, A);
+    update_kernel<<<grid, UPDATE_THREADS, UPDATE_SMEM, s>>>(M.update, A);
 }
 
 // ------------------------------------------------------------------ the resident loop
@@ -1380,8 +1380,7 @@ void launch_wait_check(uint32_t polls, long long* out, cudaStream_t s) { wait_ch
 // The face momenta into their arrays (each run's current half), as the face pass forms them once a face pass has
 // stepped: the last step's abar * u, abar from the other half of the mean depth pair (the depths that step started
 // from), rounded once. Every own face of every tile; nothing when the arrays already hold the momenta
-// (Ctl::m_stored), so it may run before any read or write of the state. momentum_mark_kernel, after it, records that
-// they do.
+// (Ctl::m_stored), so it may run before any read or write of the state; the last CTA to leave records that they do.
 __global__ void momentum_kernel(StepArgs A) {
     if (A.ctl->m_stored) return;
     const long long n = (long long)(A.ntiles - 1) * TILE2;
@@ -1396,13 +1395,16 @@ __global__ void momentum_kernel(StepArgs A) {
         A.mm[0][p][k] = __fmul_rn(0.5f * (ho[k - 1] + ho[k]) * dx, A.uu[0][p][k]);
         A.mm[1][p][k] = __fmul_rn(0.5f * (ho[k - A.px] + ho[k]) * dx, A.uu[1][p][k]);
     }
+    __syncthreads();
+    GridState* grid = grid_state(A.ctl);
+    if (threadIdx.x == 0 && atomicAdd(&grid->left, 1u) == gridDim.x - 1) {
+        A.ctl->m_stored = 1;
+        grid->left = 0;
+    }
 }
-
-__global__ void momentum_mark_kernel(Ctl* ctl) { ctl->m_stored = 1; }
 
 void launch_momentum(const StepArgs& A, int sms, cudaStream_t s) {
     momentum_kernel<<<sms * 4, 256, 0, s>>>(A);
-    momentum_mark_kernel<<<1, 1, 0, s>>>(A.ctl);
 }
 
 // ------------------------------------------------------------------ envelope pass
@@ -1418,6 +1420,7 @@ __global__ void __launch_bounds__(TILE2, 2) envelope_kernel(StepArgs A) {
     __shared__ int3 place[ENV_CHUNK];            // tile, run, native index of the tile's first own cell
     __shared__ uint32_t marks[ENV_CHUNK * TILE];  // the tile's boundary marks, a word a row
     Ctl* ctl = A.ctl;
+    grid_open();
     if (!(ctl->any & ANY_MAX)) return;
     const int nwork = ctl->nwork;
     const float arrive = ctl->arrive, deep = ctl->deep;
@@ -1451,14 +1454,26 @@ __global__ void __launch_bounds__(TILE2, 2) envelope_kernel(StepArgs A) {
 // ------------------------------------------------------------------ boundary, tally, control (one CTA)
 
 // Boundary cells of every running run and their envelope entries after the overwrite; in the device loop (control = 1)
-// also the FP64 tally of every step and the design lines. Every item is independent of the others (a follow boundary
-// reads an interior cell), so the kernel is a grid-stride loop over them.
+// also the FP64 tally of every step and the design lines; in a host-driven step (0) the swap of run 0's ping-pong pairs
+// at its end (wadi2d/solver/gpu/backend.py:185-188), by the last CTA to leave. Every item is independent of the others
+// (a follow boundary reads an interior cell), so the kernel is a grid-stride loop over them.
 __global__ void boundary_kernel(StepArgs A, int control) {
+    grid_open();
+    grid_wait();
     if (!(A.ctl->any & ANY_RUN)) return;
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gstride = gridDim.x * blockDim.x;
     const StepView V = step_view(A.R, 0);
     boundary_items(A, V, gtid, gstride, 0);
-    if (control) tally_items(A, V, gtid, gstride);
+    if (control) {
+        tally_items(A, V, gtid, gstride);
+        return;
+    }
+    __syncthreads();
+    GridState* grid = grid_state(A.ctl);
+    if (threadIdx.x == 0 && atomicAdd(&grid->left, 1u) == gridDim.x - 1) {
+        A.R.parity[0] ^= 1;
+        grid->left = 0;
+    }
 }
 
 // The end of a step of the device loop, in the kernels of its own: each running run's clock and the next step's
@@ -1487,18 +1502,20 @@ __device__ void step_settings(const StepArgs& A) {
     if (any & ANY_WAVE) clear_waves(A, V);
 }
 
-// The end of a host-driven step of run 0: the swap of the ping-pong pairs (wadi2d/solver/gpu/backend.py:185-188).
-__global__ void endstep_kernel(StepArgs A) { A.R.parity[0] ^= 1; }
-
-// A host-driven step of run 0 (the reference backend's step(dt, want_wave, want_wet)).
-__global__ void setstep_kernel(StepArgs A, float dtf, int want_wave, int want_wet, int nact) {
+// A host-driven step of run 0 (the reference backend's step(dt, want_wave, want_wet)), with the tiles' waves cleared when
+// it wants them. One CTA.
+__global__ void __launch_bounds__(1024) setstep_kernel(StepArgs A, float dtf, int want_wave, int want_wet, int nact) {
     Ctl* ctl = A.ctl;
-    ctl->nact = nact;
-    ctl->nwork = nact;
-    ctl->any = ANY_RUN | (want_wave ? ANY_WAVE : 0u);
-    A.R.dtf[0] = dtf;
-    A.R.flags[0] = F_RUN | (want_wave ? F_WAVE : 0) | (want_wet ? F_WET : 0);
-    if (want_wave) A.R.wave_bits[0] = 0u;
+    if (threadIdx.x == 0) {
+        ctl->nact = nact;
+        ctl->nwork = nact;
+        ctl->any = ANY_RUN | (want_wave ? ANY_WAVE : 0u);
+        A.R.dtf[0] = dtf;
+        A.R.flags[0] = F_RUN | (want_wave ? F_WAVE : 0) | (want_wet ? F_WET : 0);
+        if (want_wave) A.R.wave_bits[0] = 0u;
+    }
+    if (want_wave)
+        for (int t = threadIdx.x; t < A.ntiles; t += blockDim.x) A.wave[t] = 0.0f;
 }
 
 // Before the first step of the device loop, in one CTA of 1024 threads: the loop's settings (c; the stored-momenta flag
@@ -1533,6 +1550,8 @@ __global__ void __launch_bounds__(1024) begin_kernel(const __grid_constant__ Ste
 // clock, the active-list rebuild (for the runs that check at this step) with the woken tiles and the work list, then
 // the next step's loop test and settings. plan_kernel, after it, takes the woken tiles.
 __global__ void __launch_bounds__(1024) control_kernel(const __grid_constant__ StepArgs A) {
+    grid_open();
+    grid_wait();
     run_clocks(A);
     __syncthreads();
     rebuild_lists(A, step_view(A.R, 0), false, (A.ctl->any & ANY_ACT) != 0, A.ctl->prune);
@@ -1543,6 +1562,8 @@ __global__ void __launch_bounds__(1024) control_kernel(const __grid_constant__ S
 // refresh_plan of the listed tiles (wadi2d/solver/gpu/kernels/cells.cu:66-78) from the current mean depth. count < 0:
 // the tiles the device loop's last rebuild woke (ctl->nwoken, 0 when it did not rebuild).
 __global__ void __launch_bounds__(256) plan_kernel(StepArgs A, const int32_t* list, int count) {
+    grid_open();
+    grid_wait();
     if (count < 0) count = A.ctl->nwoken;
     plan_tiles(A, A.R.parity, list, count, blockIdx.x, gridDim.x);
 }

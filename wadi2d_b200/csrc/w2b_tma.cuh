@@ -4,6 +4,8 @@
 #pragma once
 
 #include <cuda.h>
+#include <cuda_runtime.h>
+
 #include <cstdint>
 
 namespace w2b {
@@ -49,6 +51,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t phase, uint32_
     return false;
 }
 
+// A kernel launched with programmatic serialisation starts while the one before it in the stream still runs, as soon as
+// that one's CTAs have all said grid_open: what it does before grid_wait must not touch what an earlier kernel writes.
+// grid_wait returns when every earlier kernel has finished. Both do nothing in a plain launch.
+__device__ __forceinline__ void grid_open() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // A 2D box of a tensor map into shared memory; x is the innermost coordinate (its byte offset is a multiple of 16).
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
     asm volatile(
@@ -62,6 +70,22 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
                  : "memory");
+}
+
+// Launch a kernel that says grid_wait itself, so that its start overlaps the end of the kernel before it.
+template <class... P, class... Q>
+inline cudaError_t launch_next(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Q&&... args) {
+    cudaLaunchAttribute serial;
+    serial.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    serial.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &serial;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
 }  // namespace w2b
