@@ -261,6 +261,12 @@ class B200Backend:
         self.hooks = None
         self.extra_wave = 0.0
         self.wet = TileFlags(self)
+        self._half_at = {pair[half].data_ptr(): pair[half] for pair in (t[k] for k in ("h", "u", "v", "mx", "my"))
+                         for half in (0, 1)}  # fmt: skip
+        self._w2b_step = _lib.lib().w2b_step
+        self._active: np.ndarray | None = None  # None: not read back since the device loop last moved it
+        self._held: np.ndarray | None = None  # what the device's list holds, as far as the host knows
+        self.nact = -1
         self.set_active(np.arange(1, nt, dtype=np.int32))
 
     # ------------------------------------------------------------------ plumbing
@@ -274,7 +280,9 @@ class B200Backend:
         )  # fmt: skip
 
     def _stream(self) -> int:
-        return self.torch.cuda.current_stream(self.device).cuda_stream
+        torch = self.torch
+        index = self.device.index
+        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
     def native(self, name: str):
         """The current device tensor of a field, NATIVE layout (for the velocities and momenta, with the momenta put in
@@ -283,13 +291,8 @@ class B200Backend:
             self.sync_momentum()
         p = ctypes.c_void_p()
         _lib.call("w2b_field_ptr", self.handle, _lib.FIELD_ID[name], ctypes.byref(p))
-        for key in ("h", "u", "v", "mx", "my"):
-            pair = self._t[key]
-            for half in (0, 1):
-                if pair[half].data_ptr() == p.value:
-                    return pair[half]
-        key = name
-        return self._t[key]
+        half = self._half_at.get(p.value)
+        return self._t[name] if half is None else half
 
     def sync_momentum(self) -> None:
         """The face momenta into their arrays, on the current stream, before the state is read or written directly
@@ -312,8 +315,29 @@ class B200Backend:
 
     # ------------------------------------------------------------------ the reference backend interface
 
+    @property
+    def active_tiles(self) -> np.ndarray:
+        """The active tiles; after the device loop, read back when first asked for."""
+        if self._active is None:
+            self._active = self._t["active"][: self.nact].cpu().numpy().astype(np.int32)
+            self._held = self._active.copy()
+        return self._active
+
+    @active_tiles.setter
+    def active_tiles(self, tiles: np.ndarray) -> None:
+        self._active = tiles
+
+    def lists_moved(self, nact: int) -> None:
+        """The device loop left nact active tiles."""
+        self.nact, self._active, self._held = nact, None, None
+
     def set_active(self, active: np.ndarray) -> None:
-        self.active_tiles = np.ascontiguousarray(active, np.int32)
+        active = np.ascontiguousarray(active, np.int32)
+        if self._held is not None and np.array_equal(active, self._held):
+            self.active_tiles, self.nact = active, int(active.size)
+            return
+        self._held = active.copy()
+        self.active_tiles = active
         self.nact = int(self.active_tiles.size)
         torch = self.torch
         act = self._t["active"]
@@ -370,7 +394,10 @@ class B200Backend:
         """Nothing to do: the NATIVE layout has no halo copies."""
 
     def step(self, dt: float, want_wave: bool, want_wet: bool) -> None:
-        _lib.call("w2b_step", self.handle, float(np.float32(dt)), int(want_wave), int(want_wet), self._stream())
+        # (ctypes rounds dt to float32)
+        status = self._w2b_step(self.handle, float(dt), int(want_wave), int(want_wet), self._stream())
+        if status != _lib.OK:
+            raise _lib.W2BError(status, "w2b_step")
 
     def loop_config(self) -> dict:
         """The device loop's launch schedule (w2b_loop_config): the face and update passes' CTAs a SM and the loop

@@ -259,11 +259,11 @@ class Batch:
     # ------------------------------------------------------------------ the reference model's setters, per run
 
     def _pull(self) -> None:
-        """The device's active list and idle counters into the host's copies, before a host rebuild."""
+        """The device's idle counters into the host's copy, before a host rebuild (the backend reads the active list back
+        when it is asked for)."""
         if not self._device_newer:
             return
         b = self.backend
-        b.active_tiles = b._t["active"][: b.nact].cpu().numpy().astype(np.int32)
         self.stepper.idle[:] = b._t["idle"].cpu().numpy()
         self._device_newer = False
 
@@ -395,7 +395,7 @@ class Batch:
         self.t[:], self.dt[:], self.nsteps[:] = clocks["t"], clocks["dt"], clocks["nsteps"]
         self.status[:] = clocks["status"]
         self.refresh_due[:] = 0
-        b.nact = int(clocks["nact"][0])
+        b.lists_moved(int(clocks["nact"][0]))
         self._device_newer = True
         if status not in (_lib.OK, _lib.ENONFINITE, _lib.EDTMIN):
             raise _lib.W2BError(status, "w2b_advance_runs")

@@ -42,12 +42,27 @@ class Stepper:
         self.dt = self.num.cfl * self.grid.dx / self.num.wave_floor
         self.kick = None
         self.wake_rules: list[Callable[[np.ndarray], np.ndarray]] = []
-        self.idle = np.zeros(self.grid.ntiles, np.int32)
+        self._idle = np.zeros(self.grid.ntiles, np.int32)
+        self._idle_there = False  # the device loop has counted on: its counts are read back when first asked for
         # what the device's keep flags and idle counts hold, as far as this stepper knows (None: unknown); the device
         # loop uploads them only when the host's copies differ, so that a window's advance issues no host-to-device
         # copy of its own while the next window's source is uploaded (run.SourceStager)
         self._dev_keep: np.ndarray | None = None
         self._dev_idle: np.ndarray | None = None
+
+    @property
+    def idle(self) -> np.ndarray:
+        """Checks in a row each tile was not wanted."""
+        if self._idle_there:
+            self._idle_there = False
+            self._idle[:] = self.backend._t["idle"].cpu().numpy()
+            self._dev_idle = self._idle.copy()
+        return self._idle
+
+    @idle.setter
+    def idle(self, counts: np.ndarray) -> None:
+        self._idle_there = False
+        self._idle = counts
 
     def pin(self, tiles: np.ndarray) -> None:
         """Tiles that must see every smallest step; the uniform step has no other kind."""
@@ -130,8 +145,8 @@ class Stepper:
         if self._dev_keep is None or not np.array_equal(keep, self._dev_keep):
             b._t["keep"].copy_(torch.as_tensor(keep, device=b.device))
             self._dev_keep = keep
-        if self._dev_idle is None or not np.array_equal(self.idle, self._dev_idle):
-            b._t["idle"].copy_(torch.as_tensor(self.idle, device=b.device))
+        if not self._idle_there and (self._dev_idle is None or not np.array_equal(self._idle, self._dev_idle)):
+            b._t["idle"].copy_(torch.as_tensor(self._idle, device=b.device))
         num = self.num
         cfg = _lib.Stepper(num.cfl, num.wave_floor, num.dt_max, num.dt_min, num.dt_every, num.active_every,
                            int(self.adaptive_active), int(max_every), arrive, deep)  # fmt: skip
@@ -140,11 +155,8 @@ class Stepper:
         status = b.advance_device(cfg, t_end, limit, clock)
         self.t, self.dt, self.nsteps = float(clock.t), float(clock.dt), int(clock.nsteps)
         self.refresh_due = False
-        nact = int(clock.nact)
-        b.active_tiles = b._t["active"][:nact].cpu().numpy().astype(np.int32)
-        b.nact = nact
-        self.idle[:] = b._t["idle"].cpu().numpy()
-        self._dev_idle = self.idle.copy()
+        b.lists_moved(int(clock.nact))
+        self._idle_there = True
         if status == _lib.ENONFINITE:
             raise NumericalFailure(f"non-finite wave speed at t = {self.t:.3f} s")
         if status == _lib.EDTMIN:
