@@ -68,3 +68,36 @@ def test_lists_are_the_devices():
     flags = np.zeros(m.grid.ntiles, np.int32)
     flags[fewer] = 1
     assert np.array_equal(b._t["is_act"].cpu().numpy(), flags)
+
+
+def test_host_steps_in_one_launch_equal_the_kernels_of_their_own():
+    """A grid small enough for one launch a step against a batch-sized one (the same run with a dry block of tiles beside
+    it that lifts it over the line), with fixed, free and following boundary cells."""
+    from wadi2d_b200.backend import BoundaryCells
+
+    def run(wide: bool):
+        n, m = 60, 60
+        grid = TileGrid.from_mask(np.ones((n, m if not wide else 4000), bool), 0.0, 0.0, 10.0)
+        k = 2
+        rng = np.random.default_rng(5)
+        z = np.full((grid.shape[0] * k, grid.shape[1] * k), 50.0)
+        z[: 64 * k, : 61 * k] = 0.05 * np.arange(61 * k)[None, ::-1] + 0.3 * rng.random((64 * k, 61 * k))
+        model = Model(build_tables(grid, ArrayBed(z, 5.0), Tables(face_conveyance="strips")), Numerics())
+        model.stepper.adaptive_active = False
+        depth = np.zeros(grid.shape)
+        depth[1:61, 1:61] = 0.4
+        model.set_depth(depth)
+        rows = np.arange(5, 25)
+        cell = np.array([model.cell_state_index(int(j), 1) for j in rows], np.int32)
+        ref = np.array([model.cell_state_index(int(j), 3) for j in rows], np.int32)
+        kind = np.arange(20, dtype=np.int32) % 3
+        model.set_boundary(BoundaryCells(cell, ref, kind, np.full(20, 0.3, np.float32), np.full(20, 0.2, np.float32)))
+        for s in range(30):
+            model.backend.step(0.4, s % 8 == 0, s % 5 == 0)
+        wave = model.backend.max_wave()
+        return [model.field(f)[:64, :61] for f in ("h", "d", "u", "v", "qx", "qy", "res")], wave
+
+    small, wide = run(False), run(True)
+    assert small[1] == wide[1]
+    for a, b in zip(small[0], wide[0], strict=True):
+        assert np.array_equal(a, b)

@@ -29,7 +29,8 @@ namespace w2b {
     void launch_strips(int rows, const TMaps& M, const StepArgs& A, int grid, cudaStream_t s); \
     cudaError_t resident_setup();                                                   \
     int resident_occupancy(int rows);                                               \
-    cudaError_t launch_resident(int rows, const ResidentMaps& M, const StepArgs& A, int grid, int max_steps, cudaStream_t s);
+    cudaError_t launch_resident(int rows, const ResidentMaps& M, const StepArgs& A, int grid, int max_steps, \
+                                const HostStep& host, cudaStream_t s);
 namespace exact {
 W2B_PASSES_DECL
 }
@@ -50,7 +51,7 @@ struct Passes {
     void (*launch_strips)(int, const TMaps&, const StepArgs&, int, cudaStream_t);
     cudaError_t (*resident_setup)();
     int (*resident_occupancy)(int);
-    cudaError_t (*launch_resident)(int, const ResidentMaps&, const StepArgs&, int, int, cudaStream_t);
+    cudaError_t (*launch_resident)(int, const ResidentMaps&, const StepArgs&, int, int, const HostStep&, cudaStream_t);
 };
 static const Passes EXACT_PASSES = {exact::faces_setup,  exact::launch_probe,     exact::faces_occupancy,
                                     exact::launch_faces, exact::update_setup,     exact::update_occupancy,
@@ -479,15 +480,22 @@ static int launch_loop_step(Handle& H, const LoopConfig& C, cudaStream_t s) {
     return W2B_OK;
 }
 
-// Up to C.steps steps of the resident loop. Its CTAs wait for one another, so two such launches of one process must
-// not share a GPU half resident each: every launch waits for the one before it on the device, whatever its stream.
-static int launch_loop_resident(Handle& H, const LoopConfig& C, cudaStream_t s) {
+// After a wait gave up: the grid barrier's counters may be anything.
+static cudaError_t clear_grid(Handle& H, cudaStream_t s) {
+    return cudaMemsetAsync(reinterpret_cast<char*>(H.ctl()) + GRID_STATE_AT, 0, sizeof(GridState), s);
+}
+
+// A launch of the resident loop over up to `tiles` tiles in strips of `rows` rows, at most per_sm CTAs a SM. Its CTAs wait
+// for one another, so two such launches of one process must not share a GPU half resident each: every launch waits for
+// the one before it on the device, whatever its stream.
+static int launch_resident(Handle& H, const StepArgs& A, int rows, int per_sm, int64_t tiles, int max_steps,
+                           const HostStep& host, cudaStream_t s) {
     static struct {
         std::mutex mutex;
         cudaEvent_t last = nullptr;
     } lanes[64];
-    const int64_t units = (int64_t)(TILE / C.strips) * (H.g.ntiles - 1);
-    const int64_t most = (int64_t)H.sms * C.faces_per_sm - 1;
+    const int64_t units = (int64_t)(TILE / rows) * tiles;
+    const int64_t most = (int64_t)H.sms * per_sm - 1;
     const int workers = (int)(units < most ? (units > 0 ? units : 1) : most);
     int dev = 0;
     CK(cudaGetDevice(&dev));
@@ -498,9 +506,30 @@ static int launch_loop_resident(Handle& H, const LoopConfig& C, cudaStream_t s) 
         CK(cudaEventCreateWithFlags(&lane.last, cudaEventDisableTiming));
     else
         CK(cudaStreamWaitEvent(s, lane.last, 0));
-    CK(passes(H.P).launch_resident(C.strips, H.rmaps[resident_index(C.strips)], make_args(H), workers + 1, C.steps, s));
+    CK(passes(H.P).launch_resident(rows, H.rmaps[resident_index(rows)], A, workers + 1, max_steps, host, s));
     CK(cudaEventRecord(lane.last, s));
     return W2B_OK;
+}
+
+// A host-driven step as one launch, where its strips of 8 rows are one wave of the resident kernel (then its two grid
+// barriers cost less than the gaps between the passes' kernels: 81 tiles 18 us of GPU time against 27; at 384 tiles they
+// are even) and the stream is not being captured (the launch waits for another stream's event). *done: whether it was.
+static int host_resident(Handle& H, float dt, int want_wave, int want_wet, cudaStream_t s, bool* done) {
+    *done = false;
+    const int occ = H.resident_occ[resident_index(8)];
+    if ((int64_t)(TILE / 8) * H.nact > (int64_t)H.sms * occ - 1) return W2B_OK;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(s, &cap));
+    if (cap != cudaStreamCaptureStatusNone) return W2B_OK;
+    if (want_wave) {
+        CK(cudaMemsetAsync(H.B.wave, 0, sizeof(float) * H.g.ntiles, s));
+        CK(cudaMemsetAsync(H.R.wave_bits, 0, sizeof(uint32_t), s));
+    }
+    StepArgs A = make_args(H);
+    A.work = H.B.active;
+    const HostStep host = {dt, F_RUN | (want_wave ? F_WAVE : 0) | (want_wet ? F_WET : 0), H.nact};
+    *done = true;
+    return launch_resident(H, A, 8, occ, H.nact, 1, host, s);
 }
 
 }  // namespace w2b
@@ -754,6 +783,15 @@ int32_t w2b_step(void* handle, float dt, int32_t want_wave, int32_t want_wet, vo
     Handle* H = static_cast<Handle*>(handle);
     cudaStream_t s = (cudaStream_t)stream;
     if (H->nruns != 1) return W2B_EINVAL;  // a batch steps in the device loop
+    if (H->nact > 0) {
+        bool done = false;
+        const int st = host_resident(*H, dt, want_wave, want_wet, s, &done);
+        if (st != W2B_OK) return st;
+        if (done) {
+            H->cur ^= 1;
+            return W2B_OK;
+        }
+    }
     const StepArgs A = make_args(*H);
     setstep_kernel<<<1, want_wave ? 1024 : 32, 0, s>>>(A, dt, want_wave, want_wet, H->nact);
     if (H->nact == 0) {  // as the reference: no tiles, no swap
@@ -802,7 +840,9 @@ int32_t w2b_max_wave(void* handle, float* out, void* stream) {
     CK(cudaMemcpyAsync(held + 1, &H->ctl()->status, sizeof(int32_t), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
     CK(cudaStreamSynchronize((cudaStream_t)stream));
     memcpy(out, held, sizeof(float));
-    return held[1] == W2B_ETIMEOUT ? W2B_ETIMEOUT : W2B_OK;
+    if (held[1] != W2B_ETIMEOUT) return W2B_OK;
+    clear_grid(*H, (cudaStream_t)stream);
+    return W2B_ETIMEOUT;
 }
 
 int32_t w2b_wet_flags(void* handle, int32_t* out, void* stream) {
@@ -989,7 +1029,8 @@ static int launch_chunk(Handle& H, int c, int64_t steps, int64_t* took, cudaStre
     Loop& L = H.loop;
     const LoopConfig& C = L.cand[c];
     *took = C.steps;
-    if (C.resident) return launch_loop_resident(H, C, s);
+    if (C.resident)
+        return launch_resident(H, make_args(H), C.strips, C.faces_per_sm, H.g.ntiles - 1, C.steps, HostStep{}, s);
     int tail = 0;
     while (tail < TAILS && *took > steps) *took = TAIL_STEPS[tail++];
     const int st = loop_graph(H, c, tail);
@@ -1119,8 +1160,7 @@ static int advance_runs(Handle* H, const W2BStepper* cfg, const double* t_end, i
         if (done) break;
     }
     const int32_t gstatus = hctl->status;
-    if (gstatus)  // a wait gave up: the grid barrier's counters may be anything
-        CK(cudaMemsetAsync(reinterpret_cast<char*>(H->ctl()) + GRID_STATE_AT, 0, sizeof(GridState), s));
+    if (gstatus) CK(clear_grid(*H, s));
     H->nact = hctl->nact;
     H->cur = T.parity[0];
     int32_t first = gstatus;

@@ -216,6 +216,11 @@ struct ResidentMaps {
     StripMaps s;
     UpdateMaps u;
 };
+// A host-driven step's settings (flags: F_* of run 0, 0 in the device loop) and its tiles.
+struct HostStep {
+    float dt;
+    int32_t flags, tiles;
+};
 struct TileMaps {
     CUtensorMap d, h[2], u[2], v[2], qx, qy, om, zcx, zcy, mx[2], my[2];
 };

@@ -1178,12 +1178,15 @@ __device__ __forceinline__ bool update_unit(const UpdateMaps& M, const StepArgs&
 // order for every cell, face and sum as the kernels of their own. What CTAs hand one another between barriers is read
 // past L1 or by bulk copies. Latency bounds it on small grids, so strips of 4 rows (a warp a row and axis) serve the
 // smallest, and a CTA keeps the places of its strips from step to step. A step of the exact build, this way and as
-// kernels of their own: 62 x 62 cells 14 against 30 us (face pass 4.0, update 2.9, a barrier 2 to 3 us), 256 x 256 19 against
-// 31 us; the kernels also run the empty steps at the end of a graph of 16, about 8 us each. Where the passes' own work
-// fills the chip it gains nothing (1500 x 1101: 155 against 150 us), and the launch tuner keeps the kernels.
+// kernels of their own: 62 x 62 cells 13 against 30 us (face pass 4.0, update 2.9, a barrier 2 to 3 us), 256 x 256 18
+// against 31 us, a valley of 190 awake tiles 22 against 33 us. Where the passes' own work fills the chip it gains nothing
+// (1500 x 1101: 155 against 136 us), and the launch tuner keeps the kernels.
+// A host-driven step (host.flags not 0) is one step of it: the settings come with the launch, the tiles are the active
+// list (in A.work's place, host.tiles of them), nothing but the swap of run 0's halves follows.
 template <int H, bool ON>
-__global__ void __launch_bounds__(RESIDENT_THREADS, RESIDENT_CTAS)
-    resident_kernel(const __grid_constant__ ResidentMaps M, const __grid_constant__ StepArgs A, int max_steps) {
+__global__ void __launch_bounds__(RESIDENT_THREADS, resident_ctas(H))
+    resident_kernel(const __grid_constant__ ResidentMaps M, const __grid_constant__ StepArgs A, int max_steps,
+                    HostStep host) {
     constexpr int PER = TILE / H;
     extern __shared__ __align__(128) float sm[];
     __shared__ __align__(8) uint64_t bar;
@@ -1202,8 +1205,8 @@ __global__ void __launch_bounds__(RESIDENT_THREADS, RESIDENT_CTAS)
     }
     fill_rowc(rowc, A.rows);
     uint32_t phase = 0, met = 0;
-    uint32_t any = ctl->any;
-    int nwork = ctl->nwork, mst = ctl->m_stored, b = 0;
+    uint32_t any = host.flags ? ANY_RUN : ctl->any;
+    int nwork = host.flags ? host.tiles : ctl->nwork, mst = ctl->m_stored, b = 0;
     bool moved = true;  // the work list is not the one `places` was taken from
     const bool follow = A.bstart && A.bstart[A.ntiles + 1];
     for (int step = 0; step < max_steps && (any & ANY_RUN); ++step) {
@@ -1217,7 +1220,8 @@ __global__ void __launch_bounds__(RESIDENT_THREADS, RESIDENT_CTAS)
             __syncthreads();
             if (tid < n && (moved || units > UNITS_HELD)) {
                 places[tid] = unit_place<H>(A, (int)blockIdx.x + (c0 + tid) * workers);
-                steps[tid] = unit_step(A, V, places[tid].run);
+                steps[tid] = host.flags ? UnitStep{host.dt, A.R.dx[0], host.flags, __ldcg(A.R.parity)}
+                                        : unit_step(A, V, places[tid].run);
             }
             __syncthreads();
             return n;
@@ -1237,7 +1241,11 @@ __global__ void __launch_bounds__(RESIDENT_THREADS, RESIDENT_CTAS)
         }
         moved = false;
         if (!grid_barrier(grid, ctl, met)) return;
-        if (control) next_settings(A, V, step_view(A.R, b ^ 1), any, grid);
+        if (control && host.flags) {
+            if (tid == 0) ctl->m_stored = 0;
+        } else if (control) {
+            next_settings(A, V, step_view(A.R, b ^ 1), any, grid);
+        }
         for (int c0 = 0; c0 < units; c0 += UNITS_HELD) {
             const int n = units > UNITS_HELD ? take(c0) : units;
             for (int i = 0; i < n; ++i)
@@ -1245,6 +1253,16 @@ __global__ void __launch_bounds__(RESIDENT_THREADS, RESIDENT_CTAS)
                     if (!update_unit<H>(M.u, A, V, sm, &bar, phase, places[i], steps[i])) return;
         }
         if (!grid_barrier(grid, ctl, met)) return;
+        if (host.flags) {
+            if (follow) {
+                const int n = 1 - __ldcg(A.R.parity);
+                for (int m = (int)(blockIdx.x * RESIDENT_THREADS) + tid; m < A.nb; m += gridDim.x * RESIDENT_THREADS)
+                    if (A.bkind[m] >= 2) boundary_cell(A, m, n, host.flags, 0.0f, 0.0f, 0.0f);
+                if (!grid_barrier(grid, ctl, met)) return;
+            }
+            if (control && tid == 0) A.R.parity[0] ^= 1;
+            break;
+        }
         const uint32_t next = __ldcg(&ctl->any);
         const int rebuild = __ldcg(&grid->rebuild);
         if (tid < units && units <= UNITS_HELD) steps[tid] = unit_step(A, step_view(A.R, b ^ 1), places[tid].run);
@@ -1325,11 +1343,13 @@ int resident_occupancy(int rows) {
 
 // Up to max_steps steps in one cooperative launch of `grid` CTAs (at least two, at most as many as are resident at
 // once); the control block's grid state starts at zero.
-cudaError_t launch_resident(int rows, const ResidentMaps& M, const StepArgs& A, int grid, int max_steps, cudaStream_t s) {
+cudaError_t launch_resident(int rows, const ResidentMaps& M, const StepArgs& A, int grid, int max_steps,
+                            const HostStep& host, cudaStream_t s) {
     const ResidentForm f = resident_form(rows, A.P.second && A.P.sheet && A.P.mirror && A.P.carry);
     ResidentMaps maps = M;
     StepArgs args = A;
-    void* params[] = {&maps, &args, &max_steps};
+    HostStep step = host;
+    void* params[] = {&maps, &args, &max_steps, &step};
     return cudaLaunchCooperativeKernel(f.kernel, dim3(grid), dim3(RESIDENT_THREADS), params, f.smem, s);
 }
 
