@@ -197,15 +197,21 @@ __device__ __forceinline__ double edge_weight(const TableArgs& A, int axis, int6
     return lined(zpix(A, fr, fc) > zpix(A, nr, nc) ? npix_at(A, fr, fc) : npix_at(A, nr, nc), nm);
 }
 
+// A pixel of a face's line: its bed, and half the length of the bed from the pixel before it.
+struct __align__(16) LinePixel {
+    double z, half_seg;
+};
+
 // One pixel's conveyance term weight d cbrt(R)^2 at one level (_local_radius_conveyance, wadi2d/tables/core.py:
-// 82-179): E is the face's conveyance line (n pixels), HS half the length of the bed between pixels t and t + 1. The
-// local radius R weighs depth and wetted perimeter by a tent of half-width w = beta d / pixel pixels around pixel i,
-// inside its wet stretch; its sums are differences of running sums taken from the line's start, so the sums run in
-// that order here too: over [0, i] with their values kept at the tent's first pixel lo, then over (i, hi]. A dry pixel
-// adds nothing to a sum and starts a new stretch, so lo moves behind it; the first dry pixel after i ends the sweep.
-__device__ __forceinline__ double local_term(const double* __restrict__ E, const double* __restrict__ HS, int n, int i,
-                                             double level, double pixel, double beta, double weight) {
-    const double di = level - E[i];
+// 82-179): L is the face's conveyance line (n pixels). The local radius R weighs depth and wetted perimeter by a tent of
+// half-width w = beta d / pixel pixels around pixel i, inside its wet stretch; its sums are differences of running sums
+// taken from the line's start, so the sums run in that order here too: over [0, i] with their values kept at the tent's
+// first pixel lo, then over (i, hi]. A dry pixel adds nothing to a sum and starts a new stretch, so lo moves behind it;
+// the first dry pixel after i ends the sweep. Almost every pixel swept lies between wet ones: that case is the loops'
+// first branch, and takes one 16-byte load.
+__device__ __forceinline__ double local_term(const LinePixel* __restrict__ L, int n, int i, double level, double pixel,
+                                             double beta, double weight) {
+    const double di = level - L[i].z;
     if (!(di > 0.0)) return 0.0;
     double w = beta * di / pixel;
     if (w < 1e-9) w = 1e-9;
@@ -214,56 +220,59 @@ __device__ __forceinline__ double local_term(const double* __restrict__ E, const
     hi = hi < n - 1 ? hi : n - 1;
     const double half = 0.5 * pixel;
     double s0 = 0.0, s1 = 0.0, p0 = 0.0, p1 = 0.0, ft = 0.0;
-    double da = level - E[0];  // depth of pixel t, and cr: the perimeter it has from its west segment or the line's end
-    da = da > 0.0 ? da : 0.0;
-    double cr = da > 0.0 ? half : 0.0;
-    if (n == 1) cr = da > 0.0 ? half + half : 0.0;
-    auto step = [&](int t) {
-        double db = 0.0, nr = 0.0, per = cr;
-        if (t + 1 < n) {
-            db = level - E[t + 1];
-            db = db > 0.0 ? db : 0.0;
-            if (da > 0.0 && db > 0.0) {
-                nr = HS[t];
-                per += nr;
-            } else if (da > 0.0) {
-                const double rise = E[t + 1] - E[t];
-                if (rise > 0.0) {
-                    const double f = da / rise;
-                    per += (f <= 1.0 ? f : 1.0) * (2.0 * HS[t]);
-                } else {
-                    per += half;
-                }
-            } else if (db > 0.0) {
-                const double rise = E[t + 1] - E[t];
-                if (-rise > 0.0) {
-                    const double f = db / -rise;
-                    nr = (f <= 1.0 ? f : 1.0) * (2.0 * HS[t]);
-                } else {
-                    nr = half;
-                }
-            }
-            if (t + 2 == n && db > 0.0) nr = half + nr;
-        }
-        if (da > 0.0) {
-            s0 += da;
-            s1 += ft * da;
-            p0 += per;
-            p1 += ft * per;
-        }
-        da = db;
-        cr = nr;
-        ft += 1.0;
+    double da = level - L[0].z;  // depth of pixel t (dry: not over 0), and cr: the perimeter it has from its west
+    double cr = 0.0;             // segment or the line's end
+    if (da > 0.0) cr = n == 1 ? half + half : half;
+    auto add = [&](double per) {
+        s0 += da;
+        s1 += ft * da;
+        p0 += per;
+        p1 += ft * per;
+    };
+    // the perimeter a wet pixel has from a segment to a dry one `rise` higher
+    auto partial = [&](double depth, double rise, double half_seg) {
+        if (!(rise > 0.0)) return half;
+        const double f = depth / rise;
+        return (f <= 1.0 ? f : 1.0) * (2.0 * half_seg);
     };
     double l0 = 0.0, l1 = 0.0, l2 = 0.0, l3 = 0.0;
-    for (int t = 0; t <= i; ++t) {
-        const bool dry = !(da > 0.0);
+    for (int t = 0; t < i; ++t) {
+        const LinePixel next = L[t + 1];
+        const double db = level - next.z;
         if (t == lo) l0 = s0, l1 = s1, l2 = p0, l3 = p1;
-        step(t);
-        if (dry && t >= lo) l0 = s0, l1 = s1, l2 = p0, l3 = p1;
+        if (da > 0.0 && db > 0.0) {
+            add(cr + next.half_seg);
+            cr = next.half_seg;
+        } else {
+            if (da > 0.0)
+                add(cr + partial(da, next.z - L[t].z, next.half_seg));
+            else if (t >= lo)
+                l0 = s0, l1 = s1, l2 = p0, l3 = p1;
+            cr = !(da > 0.0) && db > 0.0 ? partial(db, L[t].z - next.z, next.half_seg) : 0.0;
+        }
+        da = db;
+        ft += 1.0;
     }
-    const double m0 = s0, m1 = s1, m2 = p0, m3 = p1;
-    for (int t = i + 1; t <= hi && da > 0.0; ++t) step(t);
+    if (i == lo) l0 = s0, l1 = s1, l2 = p0, l3 = p1;
+    if (i == n - 1 && i > 0) cr = half + cr;
+    double m0 = 0.0, m1 = 0.0, m2 = 0.0, m3 = 0.0;
+    for (int t = i; t <= hi && da > 0.0; ++t) {
+        double db = 0.0, per = cr;
+        if (t + 1 < n) {
+            const LinePixel next = L[t + 1];
+            db = level - next.z;
+            if (db > 0.0) {
+                per += next.half_seg;
+                cr = t + 2 == n ? half + next.half_seg : next.half_seg;
+            } else {
+                per += partial(da, next.z - L[t].z, next.half_seg);
+            }
+        }
+        add(per);
+        if (t == i) m0 = s0, m1 = s1, m2 = p0, m3 = p1;
+        da = db;
+        ft += 1.0;
+    }
     const double fi = (double)i;
     double a_sum = (1.0 - fi / w) * (m0 - l0) + (m1 - l1) / w;
     a_sum += (1.0 + fi / w) * (s0 - m0) - (s1 - m1) / w;
@@ -277,23 +286,28 @@ __device__ __forceinline__ double local_term(const double* __restrict__ E, const
 // The face tables (_face_table, wadi2d/tables/core.py:44-79, and the local radius's conveyance), a group of GF faces
 // in a row along their own line at a time (GF divides 32: a column of a tile's west faces, a row of its north faces).
 // The faces of a group share one line of GF k + 2 margin pixels, read once; then every (face, row, pixel) is a thread's
-// own sweep along it (local_term), and every (face, row) a thread that adds its pixels' terms in order. The work is
-// FP64 and the sweeps' instructions bound it. A thread a face with its nine line arrays in shared memory, as this was
-// first written, left 63 threads a SM on lines of 44 pixels and 9 on lines of 298.
+// own sweep along it (local_term), and every (face, row) a thread that adds its pixels' terms in order. The sweeps'
+// instructions bound it: 2.1 M faces of 24- to 44-pixel lines (1024 x 1024 cells, 4 x 4 pixels) take 8.5 ms, 98 k faces of
+// up to 298 (10 x 10 pixels of 1 m) 2.9 ms. A thread a face with its nine line arrays in shared memory, as this was first
+// written, left 63 and 9 threads a SM and took 67 and 99 ms; the sweep with clamped depths and no branch of its own for
+// wet neighbours took 12.0 and 4.9; a thread four or five pixels at once (one sweep for all, 200 registers, 8 warps a SM)
+// 13.4 and 4.0. Three CTAs a SM (80 registers) against two: 8.5 against 9.2.
 // LINE_SMEM: the group's line in shared memory, else (a line too long for it) in the caller's workspace, GF = 1.
 struct FaceShape {
     int gf, fc;      // faces a group; of them, whose terms are held at a time
     int line;        // pixels of a group's line
 };
 template <bool LINE_SMEM>
-__global__ void __launch_bounds__(FACE_THREADS) face_tables_kernel(TableArgs A, FaceShape F) {
-    extern __shared__ double sws[];
+__global__ void __launch_bounds__(FACE_THREADS, 3) face_tables_kernel(TableArgs A, FaceShape F) {
+    extern __shared__ __align__(16) double sws[];
     __shared__ double s_zf[TILE], s_top[TILE];
     __shared__ int s_e[TILE];  // pixels the conveyance line reaches past the face's ends, -1: the strips' sum
     const int k = A.k, rows = A.rows, last = rows - 1, GF = F.gf, tid = threadIdx.x;
     double* terms = sws;
-    double* ext = LINE_SMEM ? sws + (size_t)F.fc * rows * k : A.ws + (size_t)blockIdx.x * 2 * F.line;
-    double* hs = ext + F.line;
+    // (the terms are an even count of doubles apart from the line's start: its pixels are 16 bytes)
+    LinePixel* line = reinterpret_cast<LinePixel*>(LINE_SMEM ? sws + (((size_t)F.fc * rows * k + 1) & ~(size_t)1)
+                                                             : (double*)(((uintptr_t)A.ws + 15) & ~(uintptr_t)15) +
+                                                                   (size_t)blockIdx.x * 2 * F.line);
     const int per = TILE / GF;
     const int64_t groups = (int64_t)(A.ntiles - 1) * 2 * TILE * per;
     for (int64_t g = blockIdx.x; g < groups; g += gridDim.x) {
@@ -303,12 +317,12 @@ __global__ void __launch_bounds__(FACE_THREADS) face_tables_kernel(TableArgs A, 
         const int jj0 = axis == 0 ? sub * GF : c, ii0 = axis == 0 ? c : sub * GF;
         const int64_t j0 = (int64_t)A.tiles[2 * t] * TILE + jj0, i0 = (int64_t)A.tiles[2 * t + 1] * TILE + ii0;
         const int dj = axis == 0, di = axis != 0;
-        for (int s = tid; s < F.line; s += FACE_THREADS) ext[s] = edge_pixel(A, axis, j0 * k, i0 * k, s - A.margin);
+        for (int s = tid; s < F.line; s += FACE_THREADS) line[s].z = edge_pixel(A, axis, j0 * k, i0 * k, s - A.margin);
         __syncthreads();
         if (A.local)
-            for (int s = tid; s < F.line - 1; s += FACE_THREADS) {
-                const double rise = ext[s + 1] - ext[s];
-                hs[s] = 0.5 * sqrt(A.pixel * A.pixel + rise * rise);
+            for (int s = tid + 1; s < F.line; s += FACE_THREADS) {
+                const double rise = line[s].z - line[s - 1].z;
+                line[s].half_seg = 0.5 * sqrt(A.pixel * A.pixel + rise * rise);
             }
         const double* crests = axis == 0 ? A.xcrest : A.ycrest;
         for (int f = tid >> 5; f < GF; f += FACE_THREADS / 32) {
@@ -319,7 +333,7 @@ __global__ void __launch_bounds__(FACE_THREADS) face_tables_kernel(TableArgs A, 
             double hi = -INFINITY;
             if (A.local && natural) {
                 for (int s = lane; s < A.nmax; s += 32) {
-                    const double v = ext[f * k + s];
+                    const double v = line[f * k + s].z;
                     hi = v > hi ? v : hi;
                 }
                 for (int o = 16; o > 0; o >>= 1) {
@@ -328,8 +342,8 @@ __global__ void __launch_bounds__(FACE_THREADS) face_tables_kernel(TableArgs A, 
                 }
             }
             if (lane == 0) {
-                const double* prof = ext + f * k + A.margin;
-                auto at = [&](int q) { return natural || prof[q] >= crest ? prof[q] : crest; };
+                const LinePixel* prof = line + f * k + A.margin;
+                auto at = [&](int q) { return natural || prof[q].z >= crest ? prof[q].z : crest; };
                 double zf = at(0);
                 for (int q = 1; q < k; ++q) zf = at(q) < zf ? at(q) : zf;
                 double relmax = at(0) - zf;
@@ -369,7 +383,7 @@ __global__ void __launch_bounds__(FACE_THREADS) face_tables_kernel(TableArgs A, 
                 const int at = f * k + A.margin - e;
                 const int64_t j = j0 + f * dj, i = i0 + f * di;
                 const double weight = A.npix ? edge_weight(A, axis, j * k, i * k, q, A.nman[j * A.nx + i]) : 1.0;
-                terms[x] = local_term(ext + at, hs + at, k + 2 * e, e + q, level, A.pixel, A.beta, weight);
+                terms[x] = local_term(line + at, k + 2 * e, e + q, level, A.pixel, A.beta, weight);
             }
             __syncthreads();
             for (int x = tid; x < nf * rows; x += FACE_THREADS) {
@@ -379,13 +393,13 @@ __global__ void __launch_bounds__(FACE_THREADS) face_tables_kernel(TableArgs A, 
                 const double crest = crests ? crests[cell] : NAN;
                 const double* lengths = axis == 0 ? A.xlen : A.ylen;
                 const double length = lengths ? lengths[cell] : 1.0;
-                const double* prof = ext + f * k + A.margin;
+                const LinePixel* prof = line + f * k + A.margin;
                 const double zf = s_zf[f], xr = (double)r / (double)last;
                 const double e = s_top[f] * (xr * xr);
                 const bool strips = s_e[f] < 0;
                 double area = 0.0, conv = 0.0;
                 for (int q = 0; q < k; ++q) {
-                    const double v = prof[q] >= crest || isnan(crest) ? prof[q] : crest;
+                    const double v = prof[q].z >= crest || isnan(crest) ? prof[q].z : crest;
                     const double dep = e - (v - zf);
                     if (dep > 0.0) {
                         area += dep;
@@ -533,11 +547,11 @@ static int32_t build(const W2BTableIn* in, const W2BTableOut* out, void* stream)
     int64_t term_faces = FACE_TERM_BYTES / face_terms;
     term_faces = term_faces < 1 ? 1 : (term_faces > TILE ? TILE : term_faces);
     auto line_bytes = [&](int gf) { return 2 * ((int64_t)gf * in->k + 2 * A.margin) * (int64_t)sizeof(double); };
-    while (F.gf > 1 && line_bytes(F.gf) + term_faces * face_terms > FACE_SMEM_BYTES) F.gf /= 2;
+    while (F.gf > 1 && line_bytes(F.gf) + term_faces * face_terms + 8 > FACE_SMEM_BYTES) F.gf /= 2;
     F.fc = (int)(term_faces < F.gf ? term_faces : F.gf);
     F.line = (int)(F.gf * in->k + 2 * A.margin);
-    const bool line_smem = line_bytes(F.gf) + F.fc * face_terms <= FACE_SMEM_BYTES;
-    const size_t bytes = (size_t)(F.fc * face_terms + (line_smem ? line_bytes(F.gf) : 0));
+    const bool line_smem = line_bytes(F.gf) + F.fc * face_terms + 8 <= FACE_SMEM_BYTES;
+    const size_t bytes = (size_t)(F.fc * face_terms + 8 + (line_smem ? line_bytes(F.gf) : 0));
     int dev = 0, sms = 148, occ = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -550,7 +564,7 @@ static int32_t build(const W2BTableIn* in, const W2BTableOut* out, void* stream)
     const int64_t groups = (int64_t)(in->ntiles - 1) * 2 * TILE * (TILE / F.gf);
     int64_t fblocks = (int64_t)sms * (occ > 0 ? occ : 1);
     if (!line_smem) {
-        const int64_t held = out->ws_threads * 9 * (int64_t)(A.nmax + 1) / (2 * (int64_t)F.line);
+        const int64_t held = (out->ws_threads * 9 * (int64_t)(A.nmax + 1) - 1) / (2 * (int64_t)F.line);
         fblocks = fblocks < held ? fblocks : held;
     }
     if (groups > 0) kernel<<<(unsigned)(fblocks < groups ? fblocks : groups), FACE_THREADS, bytes, s>>>(A, F);
