@@ -423,16 +423,16 @@ int32_t w2b_mma_gemm(const void* a, const void* b, int32_t m, int32_t n, int32_t
  * row rows[*step * batch + r] (step NULL: 0); rows from `valid` on are zero; h0 (m x k, BF16, or NULL) takes them.
  * Then, v being the product plus bias (n, or NULL), each of these that is not NULL:
  *  - w, mw, vw, wb: one Adam step of the weights w (m x n) with gradient v (step size lr, or lr_table[*step]), wb their
- *    BF16 copy; and with gb, mb, vb one of the biases gb (m) with the column sums of A (a_mn), rows in order;
+ *    BF16 copy (h and t are then NULL); and with gb, mb, vb one of the biases gb (m) with the column sums of A (a_mn), rows in order;
  *  - gb without w: those column sums into gb;
  *  - c: v (FP32);
  *  - h (BF16): with t, scale (v - t) on the valid rows of the targets t (rows of n, picked as x's), 0 on the rest, and
  *    partial[tile] (FP64) the squared errors of each 128 x 32 tile; else v where z (with z NULL, v itself) is positive,
  *    0 elsewhere.
- * x, h0, a, b, h, z, t, w, mw, vw and wb 16-byte aligned. */
+ * b_early (w2b_mlp_train): the launch before does not write b. x, h0, a, b, h, z, t, w, mw, vw and wb 16-byte aligned. */
 typedef struct {
     const void *a, *b;
-    int32_t m, n, k, a_mn, b_mn;
+    int32_t m, n, k, a_mn, b_mn, b_early;
     int32_t valid, batch;
     const float* x;
     const int64_t *rows, *step;
@@ -449,8 +449,9 @@ typedef struct {
 #define W2B_MLP_OPS_MAX 4
 /* Up to W2B_MLP_OPS_MAX products (host array; none reads what another writes) in one launch. */
 int32_t w2b_mlp_ops(const W2BMlpOp* ops, int32_t count, int32_t* status, void* stream);
-/* iters training steps back to back without the host: each launches the products of `ops` in `launches` launches of
- * sizes[l] products, in order, then w2b_mlp_tick. ops and sizes are host arrays, read before the call returns. */
+/* iters training steps without the host: each the products of `ops` in `launches` launches of sizes[l] products, in
+ * order, then w2b_mlp_tick's arithmetic; up to 12 launches a step all in one cooperative launch. ops and sizes are host
+ * arrays, read before the call returns. status: 3 device int32, zero at the first call; [0] as above. */
 int32_t w2b_mlp_train(const W2BMlpOp* ops, const int32_t* sizes, int32_t launches, int32_t iters,
                       const double* partial, int32_t n, double count, double* loss, int64_t* step, int32_t* status,
                       void* stream);

@@ -114,3 +114,18 @@ def test_epilogues():
     for _, got, want in layers:
         for p, q in zip(got, want, strict=True):
             assert torch.equal(p, q)
+
+
+@pytest.mark.parametrize("dims,iters,batch", [((16, 16), 2, 1), ((16, 48, 16), 513, 40), ((16,) + (32,) * 7 + (16,), 5, 144)])
+def test_training_in_one_launch(dims, iters, batch):
+    """Steps of a fit in the cooperative launch (one layer; more steps than a launch takes) and, with more products than
+    it takes, launched one by one, against the host's step after step: losses, weights and biases bit for bit."""
+    from wadi2d_b200.surrogate import Network
+
+    rng = np.random.default_rng(11)
+    x, t = (rng.standard_normal((150, 16)).astype(np.float32) for _ in range(2))
+    nets = [Network(dims=dims, seed=4), Network(dims=dims, seed=4)]
+    losses = [net.fit(x, t, iters=iters, batch=batch, seed=6, graph=graph) for net, graph in zip(nets, (True, False), strict=True)]
+    assert losses[0] == losses[1]
+    for (wa, ba), (wb, bb) in zip(nets[0].weights(), nets[1].weights(), strict=True):
+        assert np.array_equal(wa, wb) and np.array_equal(ba, bb)

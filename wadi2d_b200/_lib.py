@@ -80,7 +80,7 @@ class Inflow(ctypes.Structure):
 class MlpOp(ctypes.Structure):
     _fields_ = (
         [("a", c_vp), ("b", c_vp)]
-        + [(n, c_i32) for n in ("m", "n", "k", "a_mn", "b_mn", "valid", "batch")]
+        + [(n, c_i32) for n in ("m", "n", "k", "a_mn", "b_mn", "b_early", "valid", "batch")]
         + [(n, c_vp) for n in ("x", "rows", "step", "h0", "bias", "z", "t", "c", "h", "partial", "w", "mw", "vw", "gb",
                                "mb", "vb", "wb", "lr_table")]
         + [(n, c_f32) for n in ("scale", "lr", "b1", "b2", "eps")]

@@ -485,29 +485,31 @@ static cudaError_t clear_grid(Handle& H, cudaStream_t s) {
     return cudaMemsetAsync(reinterpret_cast<char*>(H.ctl()) + GRID_STATE_AT, 0, sizeof(GridState), s);
 }
 
-// A launch of the resident loop over up to `tiles` tiles in strips of `rows` rows, at most per_sm CTAs a SM. Its CTAs wait
-// for one another, so two such launches of one process must not share a GPU half resident each: every launch waits for
-// the one before it on the device, whatever its stream.
-static int launch_resident(Handle& H, const StepArgs& A, int rows, int per_sm, int64_t tiles, int max_steps,
-                           const HostStep& host, cudaStream_t s) {
+cudaError_t launch_in_turn(const void* kernel, int grid, int block, void** params, size_t smem, cudaStream_t s) {
     static struct {
         std::mutex mutex;
         cudaEvent_t last = nullptr;
     } lanes[64];
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    auto& lane = lanes[dev];
+    std::lock_guard<std::mutex> lock(lane.mutex);
+    e = lane.last ? cudaStreamWaitEvent(s, lane.last, 0) : cudaEventCreateWithFlags(&lane.last, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(block), params, smem, s);
+    if (e == cudaSuccess) e = cudaEventRecord(lane.last, s);
+    return e;
+}
+
+// A launch of the resident loop over up to `tiles` tiles in strips of `rows` rows, at most per_sm CTAs a SM.
+static int launch_resident(Handle& H, const StepArgs& A, int rows, int per_sm, int64_t tiles, int max_steps,
+                           const HostStep& host, cudaStream_t s) {
     const int64_t units = (int64_t)(TILE / rows) * tiles;
     const int64_t most = (int64_t)H.sms * per_sm - 1;
     const int workers = (int)(units < most ? (units > 0 ? units : 1) : most);
-    int dev = 0;
-    CK(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64 || workers < 1) return W2B_EINVAL;
-    auto& lane = lanes[dev];
-    std::lock_guard<std::mutex> lock(lane.mutex);
-    if (!lane.last)
-        CK(cudaEventCreateWithFlags(&lane.last, cudaEventDisableTiming));
-    else
-        CK(cudaStreamWaitEvent(s, lane.last, 0));
+    if (workers < 1) return W2B_EINVAL;
     CK(passes(H.P).launch_resident(rows, H.rmaps[resident_index(rows)], A, workers + 1, max_steps, host, s));
-    CK(cudaEventRecord(lane.last, s));
     return W2B_OK;
 }
 

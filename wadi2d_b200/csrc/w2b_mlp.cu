@@ -9,12 +9,11 @@
 // chunk's copies (cp.async, 16 B each) in flight at once, and the element-wise work that follows a product (bias and
 // activation, the loss gradient, the activation's gradient, bias gradients, Adam) is its epilogue. A 256 x 256 x 256
 // product takes 8.4 us where a CTA a 128-row tile, staging 128 of K at a time by loads through registers with
-// 8-way bank conflicts, took 39 us; a training step at a batch of 256 is 9 launches and
-// 94 us instead of 50 launches and 700 us.
+// 8-way bank conflicts, took 39 us; a training step at a batch of 256 is 68 us (mlp_train_kernel; as 9 launches 94 us)
+// instead of 50 launches and 700 us.
 // Operands sit in shared memory in the canonical layout without swizzle: core matrices of 8 rows of 16 bytes (K-major:
-// 8 rows of 8 K; MN-major: 8 K of 8 rows), the next 8 of K 128 B on, the next 8 rows (K chunk / 8) x 128 B on, in both
-// orders. Thread 0 issues one MMA per 16 of K against the accumulator in tensor memory and commits it to an mbarrier;
-// the CTA waits (bounded) before the next chunk overwrites the tiles. The epilogue reads the accumulator with
+// 8 rows of 8 K; MN-major: 8 K of 8 rows), core_strides apart. Thread 0
+// issues one MMA per 16 of K against the accumulator in tensor memory and commits it to an mbarrier; the CTA waits (bounded) before the next chunk overwrites the tiles. The epilogue reads the accumulator with
 // tcgen05.ld.32x32b (warp w owns tensor-memory lanes 32 (w mod 4) .. + 31, one row each, and half of the columns).
 // A wait that gives up sets the status word, waits once more for the MMAs in flight, frees the tensor memory and
 // returns.
@@ -27,6 +26,7 @@
 #include <vector>
 
 #include "w2b_common.cuh"
+#include "w2b_loop.cuh"
 #include "w2b_tma.cuh"
 
 namespace w2b {
@@ -34,7 +34,9 @@ namespace w2b {
 constexpr int GEMM_M = 128, GEMM_N = 32;
 constexpr int GEMM_KC = 256;  // K staged a chunk at a time
 constexpr int GEMM_THREADS = 256;
-constexpr int GEMM_SMEM = (GEMM_M + GEMM_N) * GEMM_KC * 2;  // 80 KB: two CTAs a SM
+constexpr int GEMM_A = GEMM_M / 8 * (GEMM_KC / 8) * 144;  // bytes of A's part of shared memory (core_strides)
+constexpr int GEMM_SMEM = GEMM_A + GEMM_N / 8 * (GEMM_KC / 8) * 144;  // 90 KB: two CTAs a SM
+static_assert(GEMM_M / 8 * (GEMM_KC / 8 * 128 + 16) <= GEMM_A, "either order fits");
 
 __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
     // shared-memory matrix descriptor: start address, leading and stride byte offsets (16-byte units), version 1 for
@@ -51,27 +53,35 @@ __device__ __forceinline__ void copy16(uint32_t dst, const void* src, bool valid
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
 
+// Where an operand's core matrices lie in shared memory: their stride from one 8 of K to the next (lead) and from 8 rows
+// to the next (step), for a chunk of kc pieces of 8 K. A warp copies whole source lines, which run along K (K-major) or
+// along the rows (MN-major): the stride in that direction is 16 bytes over a multiple of 128, so that a line's pieces
+// fall into different banks.
+struct CoreStrides {
+    int lead, step;
+};
+__device__ __forceinline__ CoreStrides core_strides(int kc, bool mn) {
+    return mn ? CoreStrides{128, kc * 128 + 16} : CoreStrides{144, kc * 144};
+}
+
 // A K chunk (kw of it from k0) of `rows` rows of an operand, from row r0 on, into shared memory; rows at or past
-// `limit` are zero. mn: the operand is K x ld row-major (ld its rows' count), else rows of ld = K. A warp's 32 copies
-// are 8 rows (or 8 K) of 64 contiguous bytes each, and fill contiguous shared memory: no bank conflicts.
+// `limit` are zero. mn: the operand is K x ld row-major (ld its rows' count), else rows of ld = K. The threads take a
+// line's 16-byte pieces one after another, line after line, stepped without a division.
 __device__ __forceinline__ void stage(uint32_t dst, const __nv_bfloat16* src, int ld, int rows, int r0, int limit,
                                       int k0, int kw, bool mn) {
-    const int kc = kw / 8, sbo = kc * 128;
-    const int inner = mn ? rows / 8 : kc, outer = mn ? kw : rows;  // 16-byte pieces of a source line; source lines
-    const int spans = (inner + 3) / 4, items = spans * outer * 4;
-    for (int idx = threadIdx.x; idx < items; idx += GEMM_THREADS) {
-        const int lane = idx & 31, at = idx >> 5;
-        const int line = (at / spans) * 8 + (lane & 7), piece = (at % spans) * 4 + (lane >> 3);
-        if (piece >= inner) continue;
-        if (mn) {
-            const int r = r0 + piece * 8;
-            copy16(dst + piece * sbo + (line >> 3) * 128 + (line & 7) * 16,
-                   src + (r < limit ? (size_t)(k0 + line) * ld + r : 0), r < limit);
-        } else {
-            const int r = r0 + line;
-            copy16(dst + (line >> 3) * sbo + piece * 128 + (line & 7) * 16,
-                   src + (r < limit ? (size_t)r * ld + k0 + piece * 8 : 0), r < limit);
-        }
+    const CoreStrides S = core_strides(kw / 8, mn);
+    const int inner = (mn ? rows : kw) / 8, lines = mn ? kw : rows;
+    const int across = mn ? S.step : S.lead, down = mn ? S.lead : S.step;  // from a piece, from 8 lines to the next
+    const int by = GEMM_THREADS / inner, rest = GEMM_THREADS - by * inner;
+    int line = threadIdx.x / inner, piece = threadIdx.x - line * inner;
+    const __nv_bfloat16* base = src + (size_t)(mn ? k0 : r0) * ld + (mn ? r0 : k0);
+    while (line < lines) {
+        const bool valid = (mn ? r0 + piece * 8 : r0 + line) < limit;
+        copy16(dst + piece * across + (line >> 3) * down + (line & 7) * 16,
+               valid ? base + (size_t)line * ld + piece * 8 : src, valid);
+        line += by;
+        piece += rest;
+        if (piece >= inner) piece -= inner, ++line;
     }
 }
 
@@ -81,24 +91,26 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
 }
 
 // The row of the data set that row r of a batch is: its own, or the one this step's draw names.
-__device__ __forceinline__ int64_t batch_row(const W2BMlpOp& G, int r) {
-    return G.rows ? G.rows[(G.step ? *G.step : 0) * G.batch + r] : r;
+__device__ __forceinline__ int64_t batch_row(const W2BMlpOp& G, int64_t at, int r) {
+    return G.rows ? G.rows[at * G.batch + r] : r;
 }
 
 // stage for the network's input: FP32 rows (the batch's rows of the data set, zero past its valid ones), rounded to
 // BF16; the first column of CTAs also writes them out, for the backward pass.
-__device__ __forceinline__ void stage_input(uint8_t* dst, const W2BMlpOp& G, int m0, int k0, int kw, bool write) {
-    const int kc = kw / 8, sbo = kc * 128;
+__device__ __forceinline__ void stage_input(uint8_t* dst, const W2BMlpOp& G, int64_t at, int m0, int k0, int kw,
+                                            bool write) {
+    const int kc = kw / 8;
+    const CoreStrides S = core_strides(kc, false);
     for (int idx = threadIdx.x; idx < GEMM_M * kc; idx += GEMM_THREADS) {
         const int r = idx / kc, c = idx - r * kc;
         float4 lo = make_float4(0.0f, 0.0f, 0.0f, 0.0f), hi = lo;
         if (m0 + r < G.valid) {
-            const float4* x = reinterpret_cast<const float4*>(G.x + batch_row(G, m0 + r) * G.k + k0 + c * 8);
+            const float4* x = reinterpret_cast<const float4*>(G.x + batch_row(G, at, m0 + r) * G.k + k0 + c * 8);
             lo = x[0];
             hi = x[1];
         }
         const uint4 v = make_uint4(pack2(lo.x, lo.y), pack2(lo.z, lo.w), pack2(hi.x, hi.y), pack2(hi.z, hi.w));
-        *reinterpret_cast<uint4*>(dst + (r >> 3) * sbo + c * 128 + (r & 7) * 16) = v;
+        *reinterpret_cast<uint4*>(dst + (r >> 3) * S.step + c * S.lead + (r & 7) * 16) = v;
         if (write && m0 + r < G.m)
             *reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(G.h0) + (size_t)(m0 + r) * G.k + k0 + c * 8) = v;
     }
@@ -112,56 +124,111 @@ __device__ __forceinline__ void adam_one(float& w, float& m, float& v, float gi,
     w = w - lr_t * m / (sqrtf(v) + eps);
 }
 
+// Products of one launch: their first tiles, and where the last one's end.
 struct MlpGroup {
     W2BMlpOp op[W2B_MLP_OPS_MAX];
-    int first[W2B_MLP_OPS_MAX + 1];  // each product's first CTA
+    int first[W2B_MLP_OPS_MAX + 1];
     int count;
 };
 
-__global__ void __launch_bounds__(GEMM_THREADS) mlp_kernel(const __grid_constant__ MlpGroup P, int32_t* status) {
-    extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ __align__(8) uint64_t bar;
-    __shared__ uint32_t tmem_base;
-    __shared__ double red[GEMM_THREADS / 32];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    int o = 0;
-    while (o + 1 < P.count && (int)blockIdx.x >= P.first[o + 1]) ++o;
-    const W2BMlpOp& G = P.op[o];
-    const int M = G.m, N = G.n, K = G.k;
-    const int ntn = (N + GEMM_N - 1) / GEMM_N;
-    const int tile = (int)blockIdx.x - P.first[o];
-    const int m0 = tile / ntn * GEMM_M, n0 = tile % ntn * GEMM_N;
-    const int nt = N - n0 < GEMM_N ? N - n0 : GEMM_N;
-    uint8_t* sA = smem;
-    uint8_t* sB = smem + GEMM_M * GEMM_KC * 2;
-    constexpr uint32_t NCOLS = 32;
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
-                     "r"(NCOLS)
+// What a CTA works in: shared memory (A's tile, then B's), the barrier its MMAs commit to with its phase, a scratch of
+// one double a warp, and its accumulator in tensor memory.
+struct MlpCta {
+    uint8_t* smem;
+    uint64_t* bar;
+    double* red;
+    uint32_t phase, tmem;
+};
+constexpr uint32_t MLP_COLS = 32;
+
+// Tensor memory and the barrier of a CTA; and back (every thread, on every way out).
+__device__ __forceinline__ void mlp_begin(MlpCta& C, uint32_t* tmem_base) {
+    if (threadIdx.x < 32) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_base)),
+                     "r"(MLP_COLS)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    if (tid == 0) {
-        mbar_init(&bar, 1);
+    if (threadIdx.x == 0) {
+        mbar_init(C.bar, 1);
         fence_barrier_init();
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = tmem_base;
+    C.phase = 0;
+    C.tmem = *tmem_base;
+}
+__device__ __forceinline__ void mlp_end(MlpCta& C) {
+    tc_fence_before();
+    __syncthreads();
+    if (threadIdx.x < 32)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(C.tmem), "r"(MLP_COLS) : "memory");
+}
+
+// The first K chunk of B of a product's tile into shared memory (asynchronously).
+__device__ __forceinline__ void stage_b(const MlpCta& C, const W2BMlpOp& G, int tile, int k0) {
+    const int ntn = (G.n + GEMM_N - 1) / GEMM_N, n0 = tile % ntn * GEMM_N;
+    const int nt = G.n - n0 < GEMM_N ? G.n - n0 : GEMM_N, kw = G.k - k0 < GEMM_KC ? G.k - k0 : GEMM_KC;
+    stage(smem_u32(C.smem + GEMM_A), static_cast<const __nv_bfloat16*>(G.b), G.b_mn ? G.n : G.k, nt, n0, G.n,
+          k0, kw, G.b_mn);
+}
+
+// One tile of a product. at: the training step (what *G.step holds); b_staged: stage_b has begun for it. next: what to
+// begin once the MMAs are done with shared memory's B (the next tile's, while this one's epilogue runs). False: a wait gave
+// up (reported; the caller frees the tensor memory and leaves).
+template <class Next>
+__device__ __forceinline__ bool mlp_tile(MlpCta& C, const W2BMlpOp& G, int tile, int64_t at, bool b_staged, int32_t* status,
+                                         Next next) {
+    uint8_t* const smem = C.smem;
+    double* const red = C.red;
+    const uint32_t tmem = C.tmem;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int M = G.m, N = G.n, K = G.k;
+    const int ntn = (N + GEMM_N - 1) / GEMM_N;
+    const int m0 = tile / ntn * GEMM_M, n0 = tile % ntn * GEMM_N;
+    const int nt = N - n0 < GEMM_N ? N - n0 : GEMM_N;
+    uint8_t* sA = smem;
+    uint8_t* sB = smem + GEMM_A;
     // instruction descriptor: FP32 accumulator, BF16 A and B, their orders, N / 8, M / 16
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((G.a_mn ? 1u : 0u) << 15) |
                            ((G.b_mn ? 1u : 0u) << 16) | ((uint32_t)(nt >> 3) << 17) | ((uint32_t)(GEMM_M >> 4) << 24);
     const bool bias_grad = G.gb && n0 == 0;  // the column sums of A (K x M), rows in order
     float gb = 0.0f;
-    uint32_t phase = 0;
     bool ok = true;
+    // what the epilogue reads: a thread's quads of four columns, 32 rows (or 64) apart, the same columns in each; loaded
+    // while the MMAs run
+    const int shift = nt == GEMM_N ? 3 : 2;  // quads of columns in a row of the tile: 8, or 4
+    const int c = (tid & ((1 << shift) - 1)) * 4;
+    constexpr int QUADS = GEMM_M * GEMM_N / 4 / GEMM_THREADS;
+    float4 z[QUADS], m4[QUADS], v4[QUADS];
+    float bias[4], lr = G.lr;
+    const float* zs = G.w ? G.w : (G.h && !G.t ? G.z : nullptr);
+    auto ahead = [&] {
+        if (G.lr_table) lr = G.lr_table[at];
+        if (G.bias)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) bias[j] = G.bias[n0 + c + j];
+#pragma unroll
+        for (int x = 0; x < QUADS; ++x) {
+            const int r = (tid + x * GEMM_THREADS) >> shift, row = m0 + r;
+            if (r >= GEMM_M || row >= M) continue;
+            const size_t e0 = (size_t)row * N + n0 + c;
+            if (zs) z[x] = *reinterpret_cast<const float4*>(zs + e0);
+            if (G.w) {
+                m4[x] = *reinterpret_cast<const float4*>(G.mw + e0);
+                v4[x] = *reinterpret_cast<const float4*>(G.vw + e0);
+            }
+            if (G.t && row < G.valid)
+                z[x] = *reinterpret_cast<const float4*>(G.t + batch_row(G, at, row) * N + n0 + c);
+        }
+    };
     for (int k0 = 0; k0 < K && ok; k0 += GEMM_KC) {
         const int kw = K - k0 < GEMM_KC ? K - k0 : GEMM_KC;  // this chunk's K, a multiple of 16
-        const uint32_t sbo = (uint32_t)(kw / 8) * 128u;
-        stage(smem_u32(sB), static_cast<const __nv_bfloat16*>(G.b), G.b_mn ? N : K, nt, n0, N, k0, kw, G.b_mn);
+        const CoreStrides SA = core_strides(kw / 8, G.a_mn), SB = core_strides(kw / 8, G.b_mn);
+        if (k0 > 0 || !b_staged) stage_b(C, G, tile, k0);
         if (G.x)
-            stage_input(sA, G, m0, k0, kw, n0 == 0 && G.h0);
+            stage_input(sA, G, at, m0, k0, kw, n0 == 0 && G.h0);
         else
             stage(smem_u32(sA), static_cast<const __nv_bfloat16*>(G.a), G.a_mn ? M : K, GEMM_M, m0, M, k0, kw, G.a_mn);
         asm volatile("cp.async.wait_all;" ::: "memory");
@@ -169,10 +236,10 @@ __global__ void __launch_bounds__(GEMM_THREADS) mlp_kernel(const __grid_constant
         __syncthreads();
         if (tid == 0) {
             tc_fence_after();
-            const uint32_t a0 = smem_u32(sA), b0 = smem_u32(sB);
+            // (a step of 16 K is two core matrices on; a descriptor's address field counts 16 bytes)
+            const uint64_t a0 = umma_desc(smem_u32(sA), SA.lead, SA.step), b0 = umma_desc(smem_u32(sB), SB.lead, SB.step);
             for (int s = 0; s < kw / 16; ++s) {
-                const uint64_t da = umma_desc(a0 + s * 256, 128, sbo);
-                const uint64_t db = umma_desc(b0 + s * 256, 128, sbo);
+                const uint64_t da = a0 + s * SA.lead / 8, db = b0 + s * SB.lead / 8;
                 const uint32_t acc = (k0 > 0 || s > 0) ? 1u : 0u;
                 asm volatile(
                     "{\n\t.reg .pred p;\n\t"
@@ -182,90 +249,86 @@ __global__ void __launch_bounds__(GEMM_THREADS) mlp_kernel(const __grid_constant
                     : "memory");
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                             smem_u32(&bar))
+                             smem_u32(C.bar))
                          : "memory");
         }
+        if (k0 + GEMM_KC >= K) ahead();
         if (bias_grad && tid >= GEMM_M) {
+            // a thread a row, in the order of K
             const int r = tid - GEMM_M;
-            const __nv_bfloat16* col = reinterpret_cast<const __nv_bfloat16*>(sA + (r >> 3) * sbo) + (r & 7);
+            const __nv_bfloat16* col = reinterpret_cast<const __nv_bfloat16*>(sA + (r >> 3) * SA.step) + (r & 7);
 #pragma unroll 16
-            for (int kk = 0; kk < kw; ++kk) gb += __bfloat162float(col[(kk >> 3) * 64 + (kk & 7) * 8]);
+            for (int kk = 0; kk < kw; ++kk) gb += __bfloat162float(col[kk * 8]);
         }
-        ok = mbar_wait(&bar, phase);
-        if (!ok) mbar_wait(&bar, phase);  // once more for the MMAs in flight before anything is freed
-        phase ^= 1u;
+        ok = mbar_wait(C.bar, C.phase);
+        if (!ok) mbar_wait(C.bar, C.phase);  // once more for the MMAs in flight before anything is freed
+        C.phase ^= 1u;
         ok = !__syncthreads_or(!ok);
         tc_fence_after();
     }
+    if (ok) next();
     if (ok) {
         // the tile through shared memory, so that the epilogue's loads and stores are whole row segments
         constexpr int PITCH = GEMM_N + 4;
         float* acc = reinterpret_cast<float*>(smem);
         const int c1 = (warp >> 2) * (nt / 2);  // this warp's columns of the tile: nt / 2 of them, 8 or 16
-        for (int c = c1; c < c1 + nt / 2; c += 8) {
+        for (int d = c1; d < c1 + nt / 2; d += 8) {
             uint32_t u[8];
             asm volatile(
                 "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                 : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7])
-                : "r"(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c));
+                : "r"(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)d));
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            uint4* to = reinterpret_cast<uint4*>(acc + ((warp & 3) * 32 + lane) * PITCH + c);
+            uint4* to = reinterpret_cast<uint4*>(acc + ((warp & 3) * 32 + lane) * PITCH + d);
             to[0] = make_uint4(u[0], u[1], u[2], u[3]);
             to[1] = make_uint4(u[4], u[5], u[6], u[7]);
         }
         __syncthreads();
-        const float lr = G.lr_table ? G.lr_table[*G.step] : G.lr;
         double loss = 0.0;
-        const int quads = nt / 4;
-#pragma unroll 4
-        for (int idx = tid; idx < GEMM_M * quads; idx += GEMM_THREADS) {
-            const int r = idx / quads, row = m0 + r, col = n0 + (idx - r * quads) * 4;
-            if (row >= M) continue;
-            float v[4];
-            const float4 q = *reinterpret_cast<const float4*>(acc + r * PITCH + col - n0);
-            v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+#pragma unroll
+        for (int x = 0; x < QUADS; ++x) {
+            const int r = (tid + x * GEMM_THREADS) >> shift, row = m0 + r;
+            if (r >= GEMM_M || row >= M) continue;
+            const size_t e0 = (size_t)row * N + n0 + c;
+            const float4 q = *reinterpret_cast<const float4*>(acc + r * PITCH + c);
+            float v[4] = {q.x, q.y, q.z, q.w};
             if (G.bias)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) v[j] += G.bias[col + j];
-            const size_t at = (size_t)row * N + col;
+                for (int j = 0; j < 4; ++j) v[j] += bias[j];
             if (G.w) {  // the gradient of four weights: their Adam step
-                const float4 w4 = *reinterpret_cast<const float4*>(G.w + at);
-                const float4 m4 = *reinterpret_cast<const float4*>(G.mw + at);
-                const float4 v4 = *reinterpret_cast<const float4*>(G.vw + at);
-                float w[4] = {w4.x, w4.y, w4.z, w4.w}, m[4] = {m4.x, m4.y, m4.z, m4.w}, s[4] = {v4.x, v4.y, v4.z, v4.w};
+                float w[4] = {z[x].x, z[x].y, z[x].z, z[x].w}, m[4] = {m4[x].x, m4[x].y, m4[x].z, m4[x].w};
+                float s[4] = {v4[x].x, v4[x].y, v4[x].z, v4[x].w};
 #pragma unroll
                 for (int j = 0; j < 4; ++j) adam_one(w[j], m[j], s[j], v[j], lr, G.b1, G.b2, G.eps);
-                *reinterpret_cast<float4*>(G.w + at) = make_float4(w[0], w[1], w[2], w[3]);
-                *reinterpret_cast<float4*>(G.mw + at) = make_float4(m[0], m[1], m[2], m[3]);
-                *reinterpret_cast<float4*>(G.vw + at) = make_float4(s[0], s[1], s[2], s[3]);
-                *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(G.wb) + at) =
+                *reinterpret_cast<float4*>(G.w + e0) = make_float4(w[0], w[1], w[2], w[3]);
+                *reinterpret_cast<float4*>(G.mw + e0) = make_float4(m[0], m[1], m[2], m[3]);
+                *reinterpret_cast<float4*>(G.vw + e0) = make_float4(s[0], s[1], s[2], s[3]);
+                *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(G.wb) + e0) =
                     make_uint2(pack2(w[0], w[1]), pack2(w[2], w[3]));
             }
             if (G.c) {
                 if (!((uintptr_t)G.c & 15)) {
-                    *reinterpret_cast<float4*>(G.c + at) = make_float4(v[0], v[1], v[2], v[3]);
+                    *reinterpret_cast<float4*>(G.c + e0) = make_float4(v[0], v[1], v[2], v[3]);
                 } else {
-                    for (int j = 0; j < 4; ++j) G.c[at + j] = v[j];
+                    for (int j = 0; j < 4; ++j) G.c[e0 + j] = v[j];
                 }
             }
             if (G.h) {  // the loss's gradient, the gradient behind an activation, or the next layer's input (relu)
                 if (G.t) {
-                    float4 t = make_float4(v[0], v[1], v[2], v[3]);
-                    if (row < G.valid) t = *reinterpret_cast<const float4*>(G.t + batch_row(G, row) * N + col);
-                    const float e[4] = {v[0] - t.x, v[1] - t.y, v[2] - t.z, v[3] - t.w};
+                    const float e[4] = {v[0] - z[x].x, v[1] - z[x].y, v[2] - z[x].z, v[3] - z[x].w};
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         loss += row < G.valid ? (double)e[j] * (double)e[j] : 0.0;
                         v[j] = row < G.valid ? G.scale * e[j] : 0.0f;
                     }
                 } else {
-                    const float4 z = G.z ? *reinterpret_cast<const float4*>(G.z + at) : make_float4(v[0], v[1], v[2], v[3]);
-                    v[0] = z.x > 0.0f ? v[0] : 0.0f;
-                    v[1] = z.y > 0.0f ? v[1] : 0.0f;
-                    v[2] = z.z > 0.0f ? v[2] : 0.0f;
-                    v[3] = z.w > 0.0f ? v[3] : 0.0f;
+                    const float4 y = zs ? z[x] : make_float4(v[0], v[1], v[2], v[3]);
+                    v[0] = y.x > 0.0f ? v[0] : 0.0f;
+                    v[1] = y.y > 0.0f ? v[1] : 0.0f;
+                    v[2] = y.z > 0.0f ? v[2] : 0.0f;
+                    v[3] = y.w > 0.0f ? v[3] : 0.0f;
                 }
-                *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(G.h) + at) =
+                *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(G.h) + e0) =
                     make_uint2(pack2(v[0], v[1]), pack2(v[2], v[3]));
             }
         }
@@ -285,14 +348,102 @@ __global__ void __launch_bounds__(GEMM_THREADS) mlp_kernel(const __grid_constant
             else
                 G.gb[r] = gb;
         }
+        tc_fence_before();
+        __syncthreads();  // the accumulator and the tile in shared memory are read: the next tile may write them
+        tc_fence_after();
     } else if (tid == 0) {
         atomicExch(status, W2B_ETIMEOUT);
     }
-    tc_fence_before();
-    __syncthreads();
-    if (warp == 0) {
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(NCOLS) : "memory");
+    return ok;
+}
+
+__device__ __forceinline__ const W2BMlpOp& mlp_op(const MlpGroup& P, int tile, int& local) {
+    int o = 0;
+    while (o + 1 < P.count && tile >= P.first[o + 1]) ++o;
+    local = tile - P.first[o];
+    return P.op[o];
+}
+
+__global__ void __launch_bounds__(GEMM_THREADS) mlp_kernel(const __grid_constant__ MlpGroup P, int32_t* status) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ uint32_t tmem_base;
+    __shared__ double red[GEMM_THREADS / 32];
+    MlpCta C{smem, &bar, red};
+    mlp_begin(C, &tmem_base);
+    int tile;
+    const W2BMlpOp& G = mlp_op(P, blockIdx.x, tile);
+    mlp_tile(C, G, tile, G.step ? *G.step : 0, false, status, [] {});
+    mlp_end(C);
+}
+
+// Training steps in one cooperative launch: each step's groups of products in order, a grid barrier after each. A group is
+// a few tiles and as kernels of their own cost 8.4 us and a gap of 1.8 each, most of it starting up; here a CTA keeps its
+// tensor memory and its code, and while a tile's epilogue and the barrier run the next one's B is on its way (b_early).
+// A step at a batch of 256 (four products of 256 x 256 among them) is 8 groups and 68 us instead of 94. Of a group's 8.8 us
+// 2.5 are A's 64 KB on their way from L2 (one SM takes in 26 B a clock), 0.7-1.5 the MMAs and the epilogue's operands,
+// 1.7 the epilogue, 0.9 the next B, 1.8 the barrier.
+constexpr int TRAIN_GROUPS_MAX = 12;
+constexpr int TRAIN_ITERS_MAX = 512;  // steps a launch, so that none holds the GPU for long
+struct MlpTrain {
+    MlpGroup group[TRAIN_GROUPS_MAX];
+    int groups, iters, partials;
+    const double* partial;
+    double count;
+    double* loss;
+    int64_t* step;
+    int32_t* status;  // [1], [2]: the barrier's arrivals, the CTAs that have left
+};
+__global__ void __launch_bounds__(GEMM_THREADS, 2) mlp_train_kernel(const __grid_constant__ MlpTrain T) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    __shared__ __align__(8) uint64_t bar;
+    __shared__ uint32_t tmem_base;
+    __shared__ double red[GEMM_THREADS / 32];
+    MlpCta C{smem, &bar, red};
+    mlp_begin(C, &tmem_base);
+    const int64_t step0 = *T.step;
+    uint32_t* const arrived = reinterpret_cast<uint32_t*>(T.status + 1);
+    uint32_t met = 0;
+    bool staged = false, ok = true;  // staged: the B of this CTA's first tile of the group has begun
+    for (int it = 0; it < T.iters && ok; ++it) {
+        for (int g = 0; g < T.groups && ok; ++g) {
+            const MlpGroup& P = T.group[g];
+            const int tiles = P.first[P.count];
+            const MlpGroup& Q = T.group[g + 1 < T.groups ? g + 1 : 0];
+            bool begun = false;
+            auto ahead = [&] {  // the first tile of the next group
+                int local;
+                if ((int)blockIdx.x >= Q.first[Q.count]) return;
+                const W2BMlpOp& N = mlp_op(Q, blockIdx.x, local);
+                if (!N.b_early) return;
+                stage_b(C, N, local, 0);
+                begun = true;
+            };
+            for (int x = blockIdx.x; x < tiles && ok; x += gridDim.x) {
+                int tile;
+                const W2BMlpOp& G = mlp_op(P, x, tile);
+                const bool last = x + (int)gridDim.x >= tiles;
+                ok = mlp_tile(C, G, tile, step0 + it, staged && x == (int)blockIdx.x, T.status, [&] {
+                    if (last) ahead();
+                });
+            }
+            if ((int)blockIdx.x >= tiles && !staged) ahead();
+            staged = begun;
+            if (ok && g == T.groups - 1 && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+                double s = 0.0;
+                for (int i = 0; i < T.partials; ++i) s += __ldcg(T.partial + i);
+                T.loss[step0 + it] = s / T.count;
+            }
+            if (ok) ok = grid_barrier(arrived, T.status, met);
+        }
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    if (ok && threadIdx.x == 0 && atomicAdd(arrived + 1, 1u) == gridDim.x - 1) {  // the last CTA to leave
+        *T.step = step0 + T.iters;
+        arrived[0] = 0;
+        arrived[1] = 0;
+    }
+    mlp_end(C);
 }
 
 // The end of a training step: its loss (the partial sums in order, over the outputs' count) into loss[*step],
@@ -318,6 +469,7 @@ static int mlp_group(const W2BMlpOp* ops, int count, MlpGroup& P) {
         if ((G.t && (!G.partial || !G.h)) || (G.rows && G.batch < 1) || (G.lr_table && !G.step))
             return W2B_EINVAL;
         if (G.w && (!G.mw || !G.vw || !G.wb || (G.gb && (!G.mb || !G.vb)))) return W2B_EINVAL;
+        if (G.w && (G.h || G.t)) return W2B_EINVAL;
         if (G.gb && !G.a_mn) return W2B_EINVAL;
         P.op[i] = G;
         P.first[i + 1] = P.first[i] + (G.m + GEMM_M - 1) / GEMM_M * ((G.n + GEMM_N - 1) / GEMM_N);
@@ -454,16 +606,53 @@ int32_t w2b_mlp_train(const W2BMlpOp* ops, const int32_t* sizes, int32_t launche
                       void* stream) {
     if (!ops || !sizes || launches < 1 || iters < 0 || !partial || n < 1 || !(count > 0.0) || !loss || !step || !status)
         return W2B_EINVAL;
+    cudaStream_t s = (cudaStream_t)stream;
     try {
         std::vector<MlpGroup> groups(launches);
+        int widest = 1;
         for (int l = 0; l < launches; ops += sizes[l], ++l) {
             if (sizes[l] < 1 || sizes[l] > W2B_MLP_OPS_MAX) return W2B_EINVAL;
             const int st = mlp_group(ops, sizes[l], groups[l]);
             if (st != W2B_OK) return st;
+            const int tiles = groups[l].first[sizes[l]];
+            widest = tiles > widest ? tiles : widest;
+        }
+        if (!iters) return W2B_OK;
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (mlp_status(cudaStreamIsCapturing(s, &cap)) != W2B_OK) return W2B_ECUDA;
+        if (launches <= TRAIN_GROUPS_MAX && cap == cudaStreamCaptureStatusNone) {
+            // one launch of every step; a stream being captured cannot wait for another stream's
+            MlpTrain T;
+            memset(&T, 0, sizeof(T));
+            memcpy(T.group, groups.data(), sizeof(MlpGroup) * launches);
+            T.groups = launches;
+            T.partials = n;
+            T.partial = partial;
+            T.count = count;
+            T.loss = loss;
+            T.step = step;
+            T.status = status;
+            int dev = 0, sms = 0, occ = 0;
+            if (cudaGetDevice(&dev) != cudaSuccess ||
+                cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+                cudaFuncSetAttribute(mlp_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM) !=
+                    cudaSuccess ||
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mlp_train_kernel, GEMM_THREADS, GEMM_SMEM) !=
+                    cudaSuccess)
+                return mlp_status(cudaGetLastError());
+            if (occ < 1) return W2B_ECUDA;
+            const int ctas = widest < sms * occ ? widest : sms * occ;
+            for (int done = 0; done < iters; done += T.iters) {
+                T.iters = iters - done < TRAIN_ITERS_MAX ? iters - done : TRAIN_ITERS_MAX;
+                void* params[] = {&T};
+                const int st =
+                    mlp_status(launch_in_turn((const void*)mlp_train_kernel, ctas, GEMM_THREADS, params, GEMM_SMEM, s));
+                if (st != W2B_OK) return st;
+            }
+            return W2B_OK;
         }
         if (cudaFuncSetAttribute(mlp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM) != cudaSuccess)
             return W2B_ECUDA;
-        cudaStream_t s = (cudaStream_t)stream;
         for (int it = 0; it < iters; ++it) {
             for (const MlpGroup& P : groups) mlp_kernel<<<P.first[P.count], GEMM_THREADS, GEMM_SMEM, s>>>(P, status);
             mlp_tick_kernel<<<1, 1, 0, s>>>(partial, n, count, loss, step);

@@ -1350,7 +1350,7 @@ cudaError_t launch_resident(int rows, const ResidentMaps& M, const StepArgs& A, 
     StepArgs args = A;
     HostStep step = host;
     void* params[] = {&maps, &args, &max_steps, &step};
-    return cudaLaunchCooperativeKernel(f.kernel, dim3(grid), dim3(RESIDENT_THREADS), params, f.smem, s);
+    return launch_in_turn(f.kernel, grid, RESIDENT_THREADS, params, f.smem, s);
 }
 
 }  // namespace W2B_ARITH

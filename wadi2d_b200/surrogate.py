@@ -73,7 +73,7 @@ class Network:
             self._sync(i)
         self.lr = lr
         self.t = 0
-        self.status = torch.zeros(1, dtype=torch.int32, device=dev)
+        self.status = torch.zeros(3, dtype=torch.int32, device=dev)  # the status, and w2b_mlp_train's barrier
 
     # ------------------------------------------------------------------ plumbing
 
@@ -128,7 +128,7 @@ class Network:
         zs, h, ops = [], None, []
         for i in range(L):
             out, inp = self.W[i].shape
-            op = dict(b=self.Wb[i], m=npad, n=out, k=inp, bias=self.b[i])
+            op = dict(b=self.Wb[i], m=npad, n=out, k=inp, bias=self.b[i], b_early=int(i > 0))
             op.update(first if i == 0 else dict(a=h))
             if keep or i == L - 1:
                 zs.append(torch.empty((npad, out), dtype=torch.float32, device=dev))
@@ -165,10 +165,11 @@ class Network:
         ends = []
         for i in range(len(self.W) - 1, -1, -1):
             out, inp = self.W[i].shape
-            ends.append(dict(a=dz, b=hs[i], m=out, n=inp, k=npad, a_mn=1, b_mn=1))
+            ends.append(dict(a=dz, b=hs[i], m=out, n=inp, k=npad, a_mn=1, b_mn=1, b_early=int(len(self.W) > 1)))
             if i > 0:
                 back = torch.empty((npad, inp), dtype=torch.bfloat16, device=dev)
-                ops.append(dict(a=dz, b=self.Wb[i], m=npad, n=inp, k=out, b_mn=1, z=zs[i - 1], h=back))
+                ops.append(dict(a=dz, b=self.Wb[i], m=npad, n=inp, k=out, b_mn=1, z=zs[i - 1], h=back,
+                                b_early=1))  # fmt: skip
                 dz = back
         return ops, partial, ends[::-1]
 
@@ -204,8 +205,9 @@ class Network:
             self._sync(i)
 
     def _check(self) -> None:
-        if int(self.status.item()) != 0:
-            raise _lib.W2BError(int(self.status.item()), "w2b_mlp_ops")
+        status = int(self.status[0].item())
+        if status != 0:
+            raise _lib.W2BError(status, "w2b_mlp_ops")
 
     def step(self, x, t):
         """One Adam step on the batch (x, t); returns the loss before the step (a device scalar)."""
@@ -219,8 +221,8 @@ class Network:
         """Adam over random batches of (x, t), standardised; returns the loss every 100 steps.
 
         With ``graph`` (the default) the batches are drawn up front (the same draws, in the same order, as one step
-        at a time draws them), the training set goes to the device once, and the library launches every step (gather,
-        forward, backward, Adam with the step's own size, all read on the device) back to back: the same arithmetic on
+        at a time draws them), the training set goes to the device once, and the library takes every step (gather,
+        forward, backward, Adam with the step's own size, all read on the device) in one launch: the same arithmetic on
         the same data in the same order as stepping from the host, without a host round trip a step."""
         rng = np.random.default_rng(seed)
         x, t = np.asarray(x, np.float32), np.asarray(t, np.float32)
