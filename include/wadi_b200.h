@@ -427,7 +427,7 @@ int32_t w2b_mma_gemm(const void* a, const void* b, int32_t m, int32_t n, int32_t
  *  - gb without w: those column sums into gb;
  *  - c: v (FP32);
  *  - h (BF16): with t, scale (v - t) on the valid rows of the targets t (rows of n, picked as x's), 0 on the rest, and
- *    partial[tile] (FP64) the squared errors of each 128 x 32 tile; else v where z (with z NULL, v itself) is positive,
+ *    partial[tile] (FP64) the squared errors of each 64 x 32 tile; else v where z (with z NULL, v itself) is positive,
  *    0 elsewhere.
  * b_early (w2b_mlp_train): the launch before does not write b. x, h0, a, b, h, z, t, w, mw, vw and wb 16-byte aligned. */
 typedef struct {

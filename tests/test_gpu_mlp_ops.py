@@ -1,5 +1,5 @@
 """The network's fused products (w2b_mlp_ops) on the B200 against FP64 products of the same BF16 values: every pair of
-operand orders at the edges of the 128 x 32 tile and of the 256-wide K chunk, and each epilogue against its definition
+operand orders at the edges of the tiles (64 or 128 rows by 32) and of the 256-wide K chunk, and each epilogue against its definition
 applied to the product the plain epilogue gives."""
 
 from __future__ import annotations
@@ -32,7 +32,7 @@ def _operands(rng, m, n, k):
     return make((m, k)), make((n, k))
 
 
-@pytest.mark.parametrize("m,n,k", [(16, 16, 16), (128, 32, 256), (144, 48, 272), (304, 256, 512), (256, 16, 1040)])
+@pytest.mark.parametrize("m,n,k", [(16, 16, 16), (128, 32, 256), (144, 48, 272), (304, 256, 512), (256, 16, 1040), (2400, 256, 272)])
 @pytest.mark.parametrize("a_mn", [0, 1])
 @pytest.mark.parametrize("b_mn", [0, 1])
 def test_products_in_every_order(m, n, k, a_mn, b_mn):
@@ -84,7 +84,7 @@ def test_epilogues():
     assert torch.equal(h, torch.where(z > 0, plain, torch.zeros_like(plain)).to(torch.bfloat16))
     # the loss and its gradient
     t = torch.as_tensor(rng.standard_normal((200, n)), dtype=torch.float32, device="cuda")
-    partial = torch.full((4,), np.nan, dtype=torch.float64, device="cuda")
+    partial = torch.full((6,), np.nan, dtype=torch.float64, device="cuda")
     _run(dict(pick, b=b, m=m, n=n, k=k, bias=bias, t=t, scale=0.25, h=h, partial=partial))
     off = torch.zeros_like(plain)
     off[:valid] = plain[:valid] - t[rows[2]]

@@ -25,13 +25,16 @@ __device__ __forceinline__ GridState* grid_state(Ctl* ctl) {
 // Every CTA of a cooperative launch: what each wrote before it, in either proxy's eyes, is what all read after it.
 // met: this launch's arrivals so far, the same in every CTA. False: some CTA did not come in time (reported; the
 // caller leaves, and so does every other CTA, each by its own count).
-__device__ __forceinline__ bool grid_barrier(uint32_t* arrived, int32_t* status, uint32_t& met) {
+// meanwhile: what every thread does after its CTA has arrived, before it waits.
+template <class Meanwhile>
+__device__ __forceinline__ bool grid_barrier(uint32_t* arrived, int32_t* status, uint32_t& met, Meanwhile meanwhile) {
     met += gridDim.x;
     asm volatile("fence.proxy.async;" ::: "memory");  // the state is written by threads and read by bulk copies
     __syncthreads();
     bool late = false;
+    if (threadIdx.x == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrived) : "memory");
+    meanwhile();
     if (threadIdx.x == 0) {
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrived) : "memory");
         uint32_t seen, polls = 0;
         do {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(arrived) : "memory");
@@ -43,7 +46,7 @@ __device__ __forceinline__ bool grid_barrier(uint32_t* arrived, int32_t* status,
     return !__syncthreads_or(late);
 }
 __device__ __forceinline__ bool grid_barrier(GridState* grid, Ctl* ctl, uint32_t& met) {
-    return grid_barrier(&grid->arrived, &ctl->status, met);
+    return grid_barrier(&grid->arrived, &ctl->status, met, [] {});
 }
 
 // The end of a resident launch: the last CTA to leave puts the barrier's counters back to zero.

@@ -1,20 +1,21 @@
 // The surrogate's network on the tensor cores: C = A B^T with BF16 operands and an FP32 accumulator in tensor memory
-// (tcgen05.mma, kind::f16, one CTA a 128-row tile), and the element-wise kernels of training (activation, its
+// (tcgen05.mma, kind::f16, a CTA a tile of 64 or 128 rows), and the element-wise kernels of training (activation, its
 // gradient, transposes, the mean-square-error gradient, column sums, Adam).
 //
 // The products: C (M x N) = A B^T, 16 <= N <= 256, N and K multiples of 16, each operand K-major (row-major M x K or
 // N x K) or MN-major (row-major K x M or K x N: what a backward pass has in hand, so nothing is transposed in memory).
 // They are a few megaflops each, so latency bounds them: launches, one trip to L2 for the operands, one for the
-// epilogue's. A CTA of 8 warps therefore takes a tile of 128 x 32 (a product of 256 x 256 is 16 CTAs), all of a K
+// epilogue's. A CTA of 8 warps therefore takes a tile of 64 x 32 (a product of 256 x 256 is 32 CTAs), all of a K
 // chunk's copies (cp.async, 16 B each) in flight at once, and the element-wise work that follows a product (bias and
 // activation, the loss gradient, the activation's gradient, bias gradients, Adam) is its epilogue. A 256 x 256 x 256
-// product takes 8.4 us where a CTA a 128-row tile, staging 128 of K at a time by loads through registers with
-// 8-way bank conflicts, took 39 us; a training step at a batch of 256 is 68 us (mlp_train_kernel; as 9 launches 94 us)
+// product takes 7.8 us where a CTA a 128-row tile, staging 128 of K at a time by loads through registers with
+// 8-way bank conflicts, took 39 us; a training step at a batch of 256 is 50 us (mlp_train_kernel; as 9 launches 94 us)
 // instead of 50 launches and 700 us.
 // Operands sit in shared memory in the canonical layout without swizzle: core matrices of 8 rows of 16 bytes (K-major:
-// 8 rows of 8 K; MN-major: 8 K of 8 rows), core_strides apart. Thread 0
-// issues one MMA per 16 of K against the accumulator in tensor memory and commits it to an mbarrier; the CTA waits (bounded) before the next chunk overwrites the tiles. The epilogue reads the accumulator with
-// tcgen05.ld.32x32b (warp w owns tensor-memory lanes 32 (w mod 4) .. + 31, one row each, and half of the columns).
+// 8 rows of 8 K; MN-major: 8 K of 8 rows), core_strides apart. Thread 0 issues one MMA per 16 of K against the
+// accumulator in tensor memory and commits it to an mbarrier; the CTA waits (bounded) before the next chunk overwrites
+// the tiles. The epilogue reads the accumulator with tcgen05.ld.32x32b (warp w sees tensor-memory lanes 32 (w mod 4) ..
+// + 31, one row a lane, of a tile of 64 rows in the first 16 of them, and takes half of the columns).
 // A wait that gives up sets the status word, waits once more for the MMAs in flight, frees the tensor memory and
 // returns.
 #include <cuda_bf16.h>
@@ -31,12 +32,12 @@
 
 namespace w2b {
 
-constexpr int GEMM_M = 128, GEMM_N = 32;
+constexpr int GEMM_N = 32;  // a tile's columns; its rows (TM) are 64 or 128: tile_rows
 constexpr int GEMM_KC = 256;  // K staged a chunk at a time
 constexpr int GEMM_THREADS = 256;
-constexpr int GEMM_A = GEMM_M / 8 * (GEMM_KC / 8) * 144;  // bytes of A's part of shared memory (core_strides)
-constexpr int GEMM_SMEM = GEMM_A + GEMM_N / 8 * (GEMM_KC / 8) * 144;  // 90 KB: two CTAs a SM
-static_assert(GEMM_M / 8 * (GEMM_KC / 8 * 128 + 16) <= GEMM_A, "either order fits");
+// bytes of `rows` rows of an operand in shared memory (core_strides; the other order takes less)
+__host__ __device__ constexpr int gemm_bytes(int rows) { return rows / 8 * (GEMM_KC / 8) * 144; }
+__host__ __device__ constexpr int gemm_smem(int tm) { return gemm_bytes(tm) + gemm_bytes(GEMM_N); }  // 54 or 90 KB: two CTAs a SM
 
 __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
     // shared-memory matrix descriptor: start address, leading and stride byte offsets (16-byte units), version 1 for
@@ -97,11 +98,12 @@ __device__ __forceinline__ int64_t batch_row(const W2BMlpOp& G, int64_t at, int 
 
 // stage for the network's input: FP32 rows (the batch's rows of the data set, zero past its valid ones), rounded to
 // BF16; the first column of CTAs also writes them out, for the backward pass.
+template <int TM>
 __device__ __forceinline__ void stage_input(uint8_t* dst, const W2BMlpOp& G, int64_t at, int m0, int k0, int kw,
                                             bool write) {
     const int kc = kw / 8;
     const CoreStrides S = core_strides(kc, false);
-    for (int idx = threadIdx.x; idx < GEMM_M * kc; idx += GEMM_THREADS) {
+    for (int idx = threadIdx.x; idx < TM * kc; idx += GEMM_THREADS) {
         const int r = idx / kc, c = idx - r * kc;
         float4 lo = make_float4(0.0f, 0.0f, 0.0f, 0.0f), hi = lo;
         if (m0 + r < G.valid) {
@@ -127,11 +129,11 @@ __device__ __forceinline__ void adam_one(float& w, float& m, float& v, float gi,
 // Products of one launch: their first tiles, and where the last one's end.
 struct MlpGroup {
     W2BMlpOp op[W2B_MLP_OPS_MAX];
-    int first[W2B_MLP_OPS_MAX + 1];
-    int count;
+    int first[W2B_MLP_OPS_MAX + 1];  // for tiles of tm rows
+    int count, tm;
 };
 
-// What a CTA works in: shared memory (A's tile, then B's), the barrier its MMAs commit to with its phase, a scratch of
+// What a CTA works in: shared memory (B's tile, then A's), the barrier its MMAs commit to with its phase, a scratch of
 // one double a warp, and its accumulator in tensor memory.
 struct MlpCta {
     uint8_t* smem;
@@ -170,37 +172,35 @@ __device__ __forceinline__ void mlp_end(MlpCta& C) {
 __device__ __forceinline__ void stage_b(const MlpCta& C, const W2BMlpOp& G, int tile, int k0) {
     const int ntn = (G.n + GEMM_N - 1) / GEMM_N, n0 = tile % ntn * GEMM_N;
     const int nt = G.n - n0 < GEMM_N ? G.n - n0 : GEMM_N, kw = G.k - k0 < GEMM_KC ? G.k - k0 : GEMM_KC;
-    stage(smem_u32(C.smem + GEMM_A), static_cast<const __nv_bfloat16*>(G.b), G.b_mn ? G.n : G.k, nt, n0, G.n,
-          k0, kw, G.b_mn);
+    stage(smem_u32(C.smem), static_cast<const __nv_bfloat16*>(G.b), G.b_mn ? G.n : G.k, nt, n0, G.n, k0, kw, G.b_mn);
 }
 
-// One tile of a product. at: the training step (what *G.step holds); b_staged: stage_b has begun for it. next: what to
-// begin once the MMAs are done with shared memory's B (the next tile's, while this one's epilogue runs). False: a wait gave
-// up (reported; the caller frees the tensor memory and leaves).
-template <class Next>
-__device__ __forceinline__ bool mlp_tile(MlpCta& C, const W2BMlpOp& G, int tile, int64_t at, bool b_staged, int32_t* status,
-                                         Next next) {
+// One tile of a product. at: the training step (what *G.step holds); b_staged: stage_b has begun for it. False: a wait
+// gave up (reported; the caller frees the tensor memory and leaves).
+template <int TM>
+__device__ __forceinline__ bool mlp_tile(MlpCta& C, const W2BMlpOp& G, int tile, int64_t at, bool b_staged,
+                                         int32_t* status) {
     uint8_t* const smem = C.smem;
     double* const red = C.red;
     const uint32_t tmem = C.tmem;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int M = G.m, N = G.n, K = G.k;
     const int ntn = (N + GEMM_N - 1) / GEMM_N;
-    const int m0 = tile / ntn * GEMM_M, n0 = tile % ntn * GEMM_N;
+    const int m0 = tile / ntn * TM, n0 = tile % ntn * GEMM_N;
     const int nt = N - n0 < GEMM_N ? N - n0 : GEMM_N;
-    uint8_t* sA = smem;
-    uint8_t* sB = smem + GEMM_A;
+    uint8_t* sB = smem;
+    uint8_t* sA = smem + gemm_bytes(GEMM_N);
     // instruction descriptor: FP32 accumulator, BF16 A and B, their orders, N / 8, M / 16
     const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((G.a_mn ? 1u : 0u) << 15) |
-                           ((G.b_mn ? 1u : 0u) << 16) | ((uint32_t)(nt >> 3) << 17) | ((uint32_t)(GEMM_M >> 4) << 24);
+                           ((G.b_mn ? 1u : 0u) << 16) | ((uint32_t)(nt >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
     const bool bias_grad = G.gb && n0 == 0;  // the column sums of A (K x M), rows in order
     float gb = 0.0f;
     bool ok = true;
     // what the epilogue reads: a thread's quads of four columns, 32 rows (or 64) apart, the same columns in each; loaded
-    // while the MMAs run
+    // while A lands
     const int shift = nt == GEMM_N ? 3 : 2;  // quads of columns in a row of the tile: 8, or 4
     const int c = (tid & ((1 << shift) - 1)) * 4;
-    constexpr int QUADS = GEMM_M * GEMM_N / 4 / GEMM_THREADS;
+    constexpr int QUADS = TM * GEMM_N / 4 / GEMM_THREADS;
     float4 z[QUADS], m4[QUADS], v4[QUADS];
     float bias[4], lr = G.lr;
     const float* zs = G.w ? G.w : (G.h && !G.t ? G.z : nullptr);
@@ -212,7 +212,7 @@ __device__ __forceinline__ bool mlp_tile(MlpCta& C, const W2BMlpOp& G, int tile,
 #pragma unroll
         for (int x = 0; x < QUADS; ++x) {
             const int r = (tid + x * GEMM_THREADS) >> shift, row = m0 + r;
-            if (r >= GEMM_M || row >= M) continue;
+            if (r >= TM || row >= M) continue;
             const size_t e0 = (size_t)row * N + n0 + c;
             if (zs) z[x] = *reinterpret_cast<const float4*>(zs + e0);
             if (G.w) {
@@ -228,9 +228,10 @@ __device__ __forceinline__ bool mlp_tile(MlpCta& C, const W2BMlpOp& G, int tile,
         const CoreStrides SA = core_strides(kw / 8, G.a_mn), SB = core_strides(kw / 8, G.b_mn);
         if (k0 > 0 || !b_staged) stage_b(C, G, tile, k0);
         if (G.x)
-            stage_input(sA, G, at, m0, k0, kw, n0 == 0 && G.h0);
+            stage_input<TM>(sA, G, at, m0, k0, kw, n0 == 0 && G.h0);
         else
-            stage(smem_u32(sA), static_cast<const __nv_bfloat16*>(G.a), G.a_mn ? M : K, GEMM_M, m0, M, k0, kw, G.a_mn);
+            stage(smem_u32(sA), static_cast<const __nv_bfloat16*>(G.a), G.a_mn ? M : K, TM, m0, M, k0, kw, G.a_mn);
+        if (k0 + GEMM_KC >= K) ahead();
         asm volatile("cp.async.wait_all;" ::: "memory");
         fence_proxy_async();  // these writes, before the tensor cores read the tiles
         __syncthreads();
@@ -252,10 +253,9 @@ __device__ __forceinline__ bool mlp_tile(MlpCta& C, const W2BMlpOp& G, int tile,
                              smem_u32(C.bar))
                          : "memory");
         }
-        if (k0 + GEMM_KC >= K) ahead();
-        if (bias_grad && tid >= GEMM_M) {
+        if (bias_grad && tid >= GEMM_THREADS - TM) {
             // a thread a row, in the order of K
-            const int r = tid - GEMM_M;
+            const int r = tid - (GEMM_THREADS - TM);
             const __nv_bfloat16* col = reinterpret_cast<const __nv_bfloat16*>(sA + (r >> 3) * SA.step) + (r & 7);
 #pragma unroll 16
             for (int kk = 0; kk < kw; ++kk) gb += __bfloat162float(col[kk * 8]);
@@ -266,11 +266,10 @@ __device__ __forceinline__ bool mlp_tile(MlpCta& C, const W2BMlpOp& G, int tile,
         ok = !__syncthreads_or(!ok);
         tc_fence_after();
     }
-    if (ok) next();
     if (ok) {
         // the tile through shared memory, so that the epilogue's loads and stores are whole row segments
         constexpr int PITCH = GEMM_N + 4;
-        float* acc = reinterpret_cast<float*>(smem);
+        float* acc = reinterpret_cast<float*>(sA);
         const int c1 = (warp >> 2) * (nt / 2);  // this warp's columns of the tile: nt / 2 of them, 8 or 16
         for (int d = c1; d < c1 + nt / 2; d += 8) {
             uint32_t u[8];
@@ -279,16 +278,18 @@ __device__ __forceinline__ bool mlp_tile(MlpCta& C, const W2BMlpOp& G, int tile,
                 : "=r"(u[0]), "=r"(u[1]), "=r"(u[2]), "=r"(u[3]), "=r"(u[4]), "=r"(u[5]), "=r"(u[6]), "=r"(u[7])
                 : "r"(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)d));
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            uint4* to = reinterpret_cast<uint4*>(acc + ((warp & 3) * 32 + lane) * PITCH + d);
-            to[0] = make_uint4(u[0], u[1], u[2], u[3]);
-            to[1] = make_uint4(u[4], u[5], u[6], u[7]);
+            if (lane < TM / 4) {  // 64 rows are in the first 16 lanes of each warp's 32
+                uint4* to = reinterpret_cast<uint4*>(acc + ((warp & 3) * (TM / 4) + lane) * PITCH + d);
+                to[0] = make_uint4(u[0], u[1], u[2], u[3]);
+                to[1] = make_uint4(u[4], u[5], u[6], u[7]);
+            }
         }
         __syncthreads();
-        double loss = 0.0;
+        double loss[TM / 64] = {};  // of each 64 rows: the sums are the same for either tile
 #pragma unroll
         for (int x = 0; x < QUADS; ++x) {
             const int r = (tid + x * GEMM_THREADS) >> shift, row = m0 + r;
-            if (r >= GEMM_M || row >= M) continue;
+            if (r >= TM || row >= M) continue;
             const size_t e0 = (size_t)row * N + n0 + c;
             const float4 q = *reinterpret_cast<const float4*>(acc + r * PITCH + c);
             float v[4] = {q.x, q.y, q.z, q.w};
@@ -318,7 +319,11 @@ __device__ __forceinline__ bool mlp_tile(MlpCta& C, const W2BMlpOp& G, int tile,
                     const float e[4] = {v[0] - z[x].x, v[1] - z[x].y, v[2] - z[x].z, v[3] - z[x].w};
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
-                        loss += row < G.valid ? (double)e[j] * (double)e[j] : 0.0;
+                        const double sq = row < G.valid ? (double)e[j] * (double)e[j] : 0.0;
+                        if (TM == 64 || r < 64)
+                            loss[0] += sq;
+                        else
+                            loss[TM / 64 - 1] += sq;
                         v[j] = row < G.valid ? G.scale * e[j] : 0.0f;
                     }
                 } else {
@@ -333,16 +338,21 @@ __device__ __forceinline__ bool mlp_tile(MlpCta& C, const W2BMlpOp& G, int tile,
             }
         }
         if (G.t) {  // the CTA's share of the squared error
-            for (int q = 16; q > 0; q >>= 1) loss += __shfl_down_sync(0xffffffffu, loss, q);
-            if (lane == 0) red[warp] = loss;
+#pragma unroll
+            for (int b = 0; b < TM / 64; ++b) {
+                for (int q = 16; q > 0; q >>= 1) loss[b] += __shfl_down_sync(0xffffffffu, loss[b], q);
+                if (lane == 0) red[b * (GEMM_THREADS / 32) + warp] = loss[b];
+            }
             __syncthreads();
-            if (tid == 0) {
-                for (int q = 1; q < GEMM_THREADS / 32; ++q) loss += red[q];
-                G.partial[tile] = loss;
+            if (tid < TM / 64 && m0 + tid * 64 < M) {
+                const double* part = red + tid * (GEMM_THREADS / 32);
+                double sum = part[0];
+                for (int q = 1; q < GEMM_THREADS / 32; ++q) sum += part[q];
+                G.partial[(m0 / 64 + tid) * ntn + n0 / GEMM_N] = sum;
             }
         }
-        if (bias_grad && tid >= GEMM_M && m0 + tid - GEMM_M < M) {
-            const int r = m0 + tid - GEMM_M;
+        if (bias_grad && tid >= GEMM_THREADS - TM && m0 + tid - (GEMM_THREADS - TM) < M) {
+            const int r = m0 + tid - (GEMM_THREADS - TM);
             if (G.w)
                 adam_one(G.gb[r], G.mb[r], G.vb[r], gb, lr, G.b1, G.b2, G.eps);
             else
@@ -364,25 +374,25 @@ __device__ __forceinline__ const W2BMlpOp& mlp_op(const MlpGroup& P, int tile, i
     return P.op[o];
 }
 
+template <int TM>
 __global__ void __launch_bounds__(GEMM_THREADS) mlp_kernel(const __grid_constant__ MlpGroup P, int32_t* status) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t tmem_base;
-    __shared__ double red[GEMM_THREADS / 32];
+    __shared__ double red[TM / 64 * (GEMM_THREADS / 32)];
     MlpCta C{smem, &bar, red};
     mlp_begin(C, &tmem_base);
     int tile;
     const W2BMlpOp& G = mlp_op(P, blockIdx.x, tile);
-    mlp_tile(C, G, tile, G.step ? *G.step : 0, false, status, [] {});
+    mlp_tile<TM>(C, G, tile, G.step ? *G.step : 0, false, status);
     mlp_end(C);
 }
 
 // Training steps in one cooperative launch: each step's groups of products in order, a grid barrier after each. A group is
 // a few tiles and as kernels of their own cost 8.4 us and a gap of 1.8 each, most of it starting up; here a CTA keeps its
-// tensor memory and its code, and while a tile's epilogue and the barrier run the next one's B is on its way (b_early).
-// A step at a batch of 256 (four products of 256 x 256 among them) is 8 groups and 68 us instead of 94. Of a group's 8.8 us
-// 2.5 are A's 64 KB on their way from L2 (one SM takes in 26 B a clock), 0.7-1.5 the MMAs and the epilogue's operands,
-// 1.7 the epilogue, 0.9 the next B, 1.8 the barrier.
+// tensor memory and its code, and while it waits at the barrier its next tile's B is on its way (b_early).
+// A step at a batch of 256 (four products of 256 x 256 among them) is 8 groups and 50 us instead of 94. Of a group's 6 us
+// 1.6 are A's 32 KB on their way from L2 (one SM takes in 26 B a clock), 0.9 the MMAs, 0.9 the epilogue, 2.2 the barrier.
 constexpr int TRAIN_GROUPS_MAX = 12;
 constexpr int TRAIN_ITERS_MAX = 512;  // steps a launch, so that none holds the GPU for long
 struct MlpTrain {
@@ -394,11 +404,12 @@ struct MlpTrain {
     int64_t* step;
     int32_t* status;  // [1], [2]: the barrier's arrivals, the CTAs that have left
 };
+template <int TM>
 __global__ void __launch_bounds__(GEMM_THREADS, 2) mlp_train_kernel(const __grid_constant__ MlpTrain T) {
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t tmem_base;
-    __shared__ double red[GEMM_THREADS / 32];
+    __shared__ double red[TM / 64 * (GEMM_THREADS / 32)];
     MlpCta C{smem, &bar, red};
     mlp_begin(C, &tmem_base);
     const int64_t step0 = *T.step;
@@ -409,32 +420,26 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2) mlp_train_kernel(const __grid
         for (int g = 0; g < T.groups && ok; ++g) {
             const MlpGroup& P = T.group[g];
             const int tiles = P.first[P.count];
-            const MlpGroup& Q = T.group[g + 1 < T.groups ? g + 1 : 0];
-            bool begun = false;
-            auto ahead = [&] {  // the first tile of the next group
-                int local;
-                if ((int)blockIdx.x >= Q.first[Q.count]) return;
-                const W2BMlpOp& N = mlp_op(Q, blockIdx.x, local);
-                if (!N.b_early) return;
-                stage_b(C, N, local, 0);
-                begun = true;
-            };
             for (int x = blockIdx.x; x < tiles && ok; x += gridDim.x) {
                 int tile;
                 const W2BMlpOp& G = mlp_op(P, x, tile);
-                const bool last = x + (int)gridDim.x >= tiles;
-                ok = mlp_tile(C, G, tile, step0 + it, staged && x == (int)blockIdx.x, T.status, [&] {
-                    if (last) ahead();
-                });
+                ok = mlp_tile<TM>(C, G, tile, step0 + it, staged && x == (int)blockIdx.x, T.status);
             }
-            if ((int)blockIdx.x >= tiles && !staged) ahead();
-            staged = begun;
             if (ok && g == T.groups - 1 && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
                 double s = 0.0;
                 for (int i = 0; i < T.partials; ++i) s += __ldcg(T.partial + i);
                 T.loss[step0 + it] = s / T.count;
             }
-            if (ok) ok = grid_barrier(arrived, T.status, met);
+            if (!ok) break;
+            ok = grid_barrier(arrived, T.status, met, [&] {
+                const MlpGroup& Q = T.group[g + 1 < T.groups ? g + 1 : 0];
+                staged = (int)blockIdx.x < Q.first[Q.count];
+                if (!staged) return;
+                int tile;
+                const W2BMlpOp& G = mlp_op(Q, blockIdx.x, tile);
+                staged = G.b_early;
+                if (staged) stage_b(C, G, tile, 0);
+            });
         }
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
@@ -456,6 +461,14 @@ __global__ void mlp_tick_kernel(const double* __restrict__ partial, int n, doubl
     *step += 1;
 }
 
+// The tiles of a launch's products, at tm rows each.
+static int tile_rows(MlpGroup& P, int tm) {
+    P.tm = tm;
+    for (int i = 0; i < P.count; ++i)
+        P.first[i + 1] = P.first[i] + (P.op[i].m + tm - 1) / tm * ((P.op[i].n + GEMM_N - 1) / GEMM_N);
+    return P.first[P.count];
+}
+
 // The products of one launch; W2B_EINVAL if the shapes, orders or alignments are not what the kernel takes.
 static int mlp_group(const W2BMlpOp* ops, int count, MlpGroup& P) {
     memset(&P, 0, sizeof(P));
@@ -472,8 +485,8 @@ static int mlp_group(const W2BMlpOp* ops, int count, MlpGroup& P) {
         if (G.w && (G.h || G.t)) return W2B_EINVAL;
         if (G.gb && !G.a_mn) return W2B_EINVAL;
         P.op[i] = G;
-        P.first[i + 1] = P.first[i] + (G.m + GEMM_M - 1) / GEMM_M * ((G.n + GEMM_N - 1) / GEMM_N);
     }
+    tile_rows(P, 128);
     return W2B_OK;
 }
 
@@ -483,14 +496,64 @@ static int mlp_status(cudaError_t e) {
     return W2B_ECUDA;
 }
 
+// The rows of a tile: 64 while tiles of 128 would leave SMs without one, for a CTA is bound by what one SM takes in of A
+// and by its share of the epilogue. A product of 256 x 256 x 256 takes 7.8 us against 8.7 (1024 rows 8.2
+// against 9.2, 2304 rows the same 10.3), a training step at a batch of 256 50 us against 66, 1024 63 against 84, 2304 117
+// against 121.
+static int pick_rows(int tiles128, int* sms) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 0;
+    return tiles128 <= *sms ? 64 : 128;
+}
+
+template <int TM>
+static cudaError_t launch_group(const MlpGroup& P, int32_t* status, cudaStream_t s) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(mlp_kernel<TM>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_smem(TM));
+    if (e != cudaSuccess) return e;
+    mlp_kernel<TM><<<P.first[P.count], GEMM_THREADS, gemm_smem(TM), s>>>(P, status);
+    return cudaGetLastError();
+}
+
+static int launch_group(MlpGroup& P, int32_t* status, cudaStream_t s) {
+    int sms = 0;
+    const int tm = pick_rows(tile_rows(P, 128), &sms);
+    if (!tm) return W2B_ECUDA;
+    tile_rows(P, tm);
+    return mlp_status(tm == 64 ? launch_group<64>(P, status, s) : launch_group<128>(P, status, s));
+}
+
 static int launch_mlp(const W2BMlpOp* ops, int count, int32_t* status, cudaStream_t s) {
     MlpGroup P;
     const int st = mlp_group(ops, count, P);
-    if (st != W2B_OK) return st;
-    if (cudaFuncSetAttribute(mlp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM) != cudaSuccess)
-        return W2B_ECUDA;
-    mlp_kernel<<<P.first[count], GEMM_THREADS, GEMM_SMEM, s>>>(P, status);
-    return mlp_status(cudaGetLastError());
+    return st != W2B_OK ? st : launch_group(P, status, s);
+}
+
+// Every step of T in cooperative launches of at most TRAIN_ITERS_MAX.
+template <int TM>
+static int launch_train(MlpTrain& T, int iters, int sms, cudaStream_t s) {
+    int widest = 1, occ = 0;
+    for (int l = 0; l < T.groups; ++l) {
+        const int tiles = tile_rows(T.group[l], TM);
+        widest = tiles > widest ? tiles : widest;
+    }
+    if (cudaFuncSetAttribute(mlp_train_kernel<TM>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_smem(TM)) !=
+            cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mlp_train_kernel<TM>, GEMM_THREADS, gemm_smem(TM)) !=
+            cudaSuccess)
+        return mlp_status(cudaGetLastError());
+    if (occ < 1) return W2B_ECUDA;
+    const int ctas = widest < sms * occ ? widest : sms * occ;
+    for (int done = 0; done < iters; done += T.iters) {
+        T.iters = iters - done < TRAIN_ITERS_MAX ? iters - done : TRAIN_ITERS_MAX;
+        void* params[] = {&T};
+        const int st = mlp_status(
+            launch_in_turn((const void*)mlp_train_kernel<TM>, ctas, GEMM_THREADS, params, gemm_smem(TM), s));
+        if (st != W2B_OK) return st;
+    }
+    return W2B_OK;
 }
 
 // ------------------------------------------------------------------ element-wise kernels of training
@@ -614,7 +677,7 @@ int32_t w2b_mlp_train(const W2BMlpOp* ops, const int32_t* sizes, int32_t launche
             if (sizes[l] < 1 || sizes[l] > W2B_MLP_OPS_MAX) return W2B_EINVAL;
             const int st = mlp_group(ops, sizes[l], groups[l]);
             if (st != W2B_OK) return st;
-            const int tiles = groups[l].first[sizes[l]];
+            const int tiles = tile_rows(groups[l], 128);
             widest = tiles > widest ? tiles : widest;
         }
         if (!iters) return W2B_OK;
@@ -632,29 +695,16 @@ int32_t w2b_mlp_train(const W2BMlpOp* ops, const int32_t* sizes, int32_t launche
             T.loss = loss;
             T.step = step;
             T.status = status;
-            int dev = 0, sms = 0, occ = 0;
-            if (cudaGetDevice(&dev) != cudaSuccess ||
-                cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-                cudaFuncSetAttribute(mlp_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM) !=
-                    cudaSuccess ||
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mlp_train_kernel, GEMM_THREADS, GEMM_SMEM) !=
-                    cudaSuccess)
-                return mlp_status(cudaGetLastError());
-            if (occ < 1) return W2B_ECUDA;
-            const int ctas = widest < sms * occ ? widest : sms * occ;
-            for (int done = 0; done < iters; done += T.iters) {
-                T.iters = iters - done < TRAIN_ITERS_MAX ? iters - done : TRAIN_ITERS_MAX;
-                void* params[] = {&T};
-                const int st =
-                    mlp_status(launch_in_turn((const void*)mlp_train_kernel, ctas, GEMM_THREADS, params, GEMM_SMEM, s));
+            int sms = 0;
+            const int tm = pick_rows(widest, &sms);
+            if (!tm) return W2B_ECUDA;
+            return tm == 64 ? launch_train<64>(T, iters, sms, s) : launch_train<128>(T, iters, sms, s);
+        }
+        for (int it = 0; it < iters; ++it) {
+            for (MlpGroup& P : groups) {
+                const int st = launch_group(P, status, s);
                 if (st != W2B_OK) return st;
             }
-            return W2B_OK;
-        }
-        if (cudaFuncSetAttribute(mlp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM) != cudaSuccess)
-            return W2B_ECUDA;
-        for (int it = 0; it < iters; ++it) {
-            for (const MlpGroup& P : groups) mlp_kernel<<<P.first[P.count], GEMM_THREADS, GEMM_SMEM, s>>>(P, status);
             mlp_tick_kernel<<<1, 1, 0, s>>>(partial, n, count, loss, step);
             const int st = mlp_status(cudaGetLastError());
             if (st != W2B_OK) return st;

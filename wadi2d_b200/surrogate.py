@@ -158,7 +158,7 @@ class Network:
         torch, dev = self.torch, self.device
         npad, nout = _pad16(max(n, 1)), self.dims[-1]
         dz = torch.empty((npad, nout), dtype=torch.bfloat16, device=dev)
-        tiles = ((npad + 127) // 128) * ((nout + 31) // 32)
+        tiles = ((npad + 63) // 64) * ((nout + 31) // 32)
         partial = torch.empty(tiles, dtype=torch.float64, device=dev)
         loss = dict(t=t, valid=n, scale=2.0 / (n * nout), h=dz, partial=partial, **(pick or {}))
         npad, hs, zs, ops = self._forward(x, n, True, loss, pick)
