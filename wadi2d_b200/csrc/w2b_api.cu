@@ -24,7 +24,7 @@ namespace w2b {
     void launch_faces(const TMaps& M, const StepArgs& A, int grid, cudaStream_t s); \
     cudaError_t update_setup();                                                     \
     int update_occupancy();                                                         \
-    void launch_update(const TMaps& M, const StepArgs& A, int grid, cudaStream_t s); \
+    void launch_update(const TMaps& M, const StepArgs& A, int grid, int control, cudaStream_t s); \
     int strips_occupancy(int rows);                                                 \
     void launch_strips(int rows, const TMaps& M, const StepArgs& A, int grid, cudaStream_t s); \
     cudaError_t resident_setup();                                                   \
@@ -46,7 +46,7 @@ struct Passes {
     void (*launch_faces)(const TMaps&, const StepArgs&, int, cudaStream_t);
     cudaError_t (*update_setup)();
     int (*update_occupancy)();
-    void (*launch_update)(const TMaps&, const StepArgs&, int, cudaStream_t);
+    void (*launch_update)(const TMaps&, const StepArgs&, int, int, cudaStream_t);
     int (*strips_occupancy)(int);
     void (*launch_strips)(int, const TMaps&, const StepArgs&, int, cudaStream_t);
     cudaError_t (*resident_setup)();
@@ -66,9 +66,9 @@ static const Passes& passes(const W2BParams& P) { return P.arith == W2B_ARITH_FA
 void launch_cbrt_check(uint32_t first, uint32_t count, unsigned long long* out, cudaStream_t s);
 void launch_wait_check(uint32_t polls, long long* out, cudaStream_t s);
 void launch_momentum(const StepArgs& A, int sms, cudaStream_t s);
-__global__ void boundary_kernel(StepArgs A, int control);
-__global__ void envelope_kernel(StepArgs A);
-__global__ void control_kernel(const __grid_constant__ StepArgs A);
+__global__ void boundary_kernel(StepArgs A);
+__global__ void step_end_kernel(StepArgs A);
+__global__ void rebuild_kernel(const __grid_constant__ StepArgs A, int adopt);
 __global__ void begin_kernel(const __grid_constant__ StepArgs A, Ctl c, W2BClock one, double t_end, long long max_steps,
                              const W2BClock* clocks, const double* t_ends);
 __global__ void setstep_kernel(StepArgs A, float dtf, int want_wave, int want_wet, int nact);
@@ -238,6 +238,8 @@ static StepArgs make_args(const Handle& H) {
     A.lpeak = H.lpeak;
     A.ltime = H.ltime;
     A.ctl = H.ctl();
+    A.any = &A.ctl->any;
+    A.any_next = &A.ctl->any2;
     A.tile_run = H.B.tile_run;
     A.lpair = reinterpret_cast<float2*>(H.B.lpair);
     A.lrow = H.B.lrow;
@@ -398,15 +400,9 @@ static void init_loop(Handle& H) {
     L.tuning = 1;
 }
 
-// CTAs of boundary_kernel: enough for its items (boundary cells; with control, tally faces and a warp a line), at
-// most four a SM.
-static int boundary_grid(const Handle& H, int control) {
-    int64_t items = H.nb;
-    if (control) {
-        items = items > H.ntally ? items : H.ntally;
-        items = items > (int64_t)H.nlines * 32 ? items : (int64_t)H.nlines * 32;
-    }
-    int64_t g = (items + 255) / 256;
+// CTAs of boundary_kernel: enough for its cells, at most four a SM.
+static int boundary_grid(const Handle& H) {
+    const int64_t g = (H.nb + 255) / 256;
     const int64_t cap = 4 * (int64_t)(H.sms > 0 ? H.sms : 148);
     return (int)(g < 1 ? 1 : (g > cap ? cap : g));
 }
@@ -457,10 +453,13 @@ static void launch_faces_host(Handle& H, const StepArgs& A, int n, cudaStream_t 
     passes(H.P).launch_strips(rows, H.tmaps, A, units < g ? units : g, s);
 }
 
-// One step of the device loop under launch configuration C: every running run advances by one of its own steps.
-static int launch_loop_step(Handle& H, const LoopConfig& C, cudaStream_t s) {
+// Step k of `steps` of a launch of the device loop under launch configuration C: every running run advances by one of its
+// own steps. The steps take the two sets of settings in turn, the first step the first; the last leaves the next one's
+// there.
+static int launch_loop_step(Handle& H, const LoopConfig& C, int k, int steps, cudaStream_t s) {
     StepArgs A = make_args(H);
     A.list = A.work;
+    if (k & 1) A = other_set(A);
     const int grid = blocks_for(H, H.g.ntiles - 1);
     const int tiles = H.g.ntiles - 1 > 0 ? H.g.ntiles - 1 : 1;
     const int fgrid = H.sms * C.faces_per_sm, ugrid = H.sms * C.update_per_sm;
@@ -469,12 +468,13 @@ static int launch_loop_step(Handle& H, const LoopConfig& C, cudaStream_t s) {
         X.launch_strips(C.strips, H.tmaps, A, (TILE / C.strips) * tiles < fgrid ? (TILE / C.strips) * tiles : fgrid, s);
     else
         X.launch_faces(H.tmaps, A, tiles < fgrid ? tiles : fgrid, s);
-    X.launch_update(H.tmaps, A, tiles < ugrid ? tiles : ugrid, s);
-    envelope_kernel<<<H.sms * 2, TILE2, 0, s>>>(A);
+    X.launch_update(H.tmaps, A, (tiles < ugrid - 1 ? tiles : ugrid - 1) + 1, 1, s);
+    // A step is five kernels; with the boundary cells, the clocks and settings as two more in a row it was 80 us instead of
+    // 65 for ten catchments of 90 to 500 cells a side, 139 instead of 130 at 1500 x 1101, 865 instead of 840 at 4096^2.
     // the small kernels start while the one before them ends (grid_wait); the passes do not: CTAs that start as others
     // leave crowd onto the SMs that finish first, and the pass then waits for those (384 tiles: 57 us a step against 49)
-    CK(launch_next(boundary_kernel, boundary_grid(H, 1), 256, 0, s, A, 1));
-    CK(launch_next(control_kernel, 1, 1024, 0, s, A));  // clocks, rebuild and work list, the next step's settings
+    CK(launch_next(step_end_kernel, H.sms * 2, TILE2, 0, s, A));
+    CK(launch_next(rebuild_kernel, 1, 1024, 0, s, A, k == steps - 1 && !(k & 1)));
     CK(launch_next(plan_kernel, grid, 256, 0, s, A, A.woken, -1));
     CKL("loop step");
     return W2B_OK;
@@ -802,8 +802,8 @@ int32_t w2b_step(void* handle, float dt, int32_t want_wave, int32_t want_wet, vo
     }
     const int grid = blocks_for(*H, H->nact);
     launch_faces_host(*H, A, H->nact, s);
-    passes(H->P).launch_update(H->tmaps, A, grid, s);
-    CK(launch_next(boundary_kernel, boundary_grid(*H, 0), 256, 0, s, A, 0));
+    passes(H->P).launch_update(H->tmaps, A, grid, 0, s);
+    CK(launch_next(boundary_kernel, boundary_grid(*H), 256, 0, s, A));
     CKL("w2b_step");
     H->cur ^= 1;
     return W2B_OK;
@@ -822,9 +822,9 @@ int32_t w2b_step_timed(void* handle, float dt, int32_t want_wave, int32_t want_w
     CK(cudaEventRecord(ev[0], s));
     launch_faces_host(*H, A, H->nact, s);
     CK(cudaEventRecord(ev[1], s));
-    passes(H->P).launch_update(H->tmaps, A, grid, s);
+    passes(H->P).launch_update(H->tmaps, A, grid, 0, s);
     CK(cudaEventRecord(ev[2], s));
-    boundary_kernel<<<boundary_grid(*H, 0), 256, 0, s>>>(A, 0);
+    boundary_kernel<<<boundary_grid(*H), 256, 0, s>>>(A);
     CK(cudaEventRecord(ev[3], s));
     CKL("w2b_step_timed");
     H->cur ^= 1;
@@ -1010,7 +1010,7 @@ static int loop_graph(Handle& H, int c, int tail) {
     CK(cudaStreamBeginCapture(H.cap, cudaStreamCaptureModeThreadLocal));
     int stc = W2B_OK;
     const int steps = tail ? TAIL_STEPS[tail - 1] : L.cand[c].steps;
-    for (int k = 0; k < steps && stc == W2B_OK; ++k) stc = launch_loop_step(H, L.cand[c], H.cap);
+    for (int k = 0; k < steps && stc == W2B_OK; ++k) stc = launch_loop_step(H, L.cand[c], k, steps, H.cap);
     cudaError_t e = cudaStreamEndCapture(H.cap, &graph);
     if (stc != W2B_OK) {
         if (e == cudaSuccess) cudaGraphDestroy(graph);

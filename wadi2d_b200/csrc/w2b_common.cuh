@@ -23,8 +23,8 @@ constexpr int SLEEP_CHECKS = 2;  // wadi2d/solver/stepper.py:12
 struct Ctl {
     int32_t nact;       // active tiles (all runs)
     int32_t nwork;      // entries of the work list the face and update passes take
-    int32_t prune;      // a run stopped stepping: the work list is to be rebuilt
-    uint32_t any;       // ANY_* bits: OR over the runs of this step's flags
+    uint32_t any;       // ANY_* bits: OR over the runs of the step's flags, of the first set of settings
+    uint32_t any2;      // of the second
     int32_t nwoken;     // tiles the last rebuild woke
     int32_t status;     // a failure no single run owns (W2B_ETIMEOUT)
     int32_t nruns;
@@ -60,7 +60,7 @@ struct RunTab {
     uint32_t* wave_bits;  // max wave speed of the run's tiles, as float bits (waves are never negative)
     int32_t* parity;      // the run's current half of the ping-pong pairs
     float* wave_last;     // the wave maximum of the run's last refresh step (what the clock reports)
-    // a second set of the step's settings: the resident loop forms the next step's while this one's are read
+    // a second set of the step's settings: the next step's are formed while this one's are read
     double *dt_tally2, *t_new, *t_new2;  // t_new: the clock at the end of the step
     float *dtf2, *max_time2;
     int32_t *flags2, *parity2;
@@ -191,6 +191,7 @@ struct StepArgs {
     double* __restrict__ lpeak;
     double* __restrict__ ltime;
     Ctl* ctl;
+    uint32_t *any, *any_next;  // the step's ANY_* bits, and the next step's
     // runs: the run of each tile, and the run table
     const int32_t* __restrict__ tile_run;
     RunTab R;
@@ -199,6 +200,25 @@ struct StepArgs {
     uint8_t* __restrict__ lrow;
     int32_t nruns;
 };
+
+// The arguments of a step that reads the second set of settings and forms the next step's in the first.
+inline StepArgs other_set(StepArgs A) {
+    RunTab& R = A.R;
+    auto swap = [](auto& a, auto& b) {
+        const auto c = a;
+        a = b;
+        b = c;
+    };
+    swap(R.dt_tally, R.dt_tally2);
+    swap(R.t_new, R.t_new2);
+    swap(R.dtf, R.dtf2);
+    swap(R.max_time, R.max_time2);
+    swap(R.flags, R.flags2);
+    swap(R.parity, R.parity2);
+    swap(R.wave_bits, R.wave_bits2);
+    swap(A.any, A.any_next);
+    return A;
+}
 
 // Tensor maps of the NATIVE state arrays for the face pass's TMA boxes: 40 x 36 floats (the tile, two cells of halo
 // north and south, four west and east so that the box's first column stays 16-byte aligned), and 32 x 32 for the

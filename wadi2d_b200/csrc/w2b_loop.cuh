@@ -111,12 +111,17 @@ __device__ __forceinline__ void boundary_cell(const StepArgs& A, int m, int n, i
         envelope_cell(A, fid_of_native(A, k), k, A.d[k], h_next[k], time, arrive, deep, A.uu[0][n], A.uu[1][n]);
 }
 
+// The run that native cell k belongs to.
+__device__ __forceinline__ int run_of_native(const StepArgs& A, int k) {
+    return A.nruns == 1 ? 0 : A.tile_run[tile_of_native(A, k)];
+}
+
 // The boundary cells of at least this kind of every running run.
 __device__ __forceinline__ void boundary_items(const StepArgs& A, const StepView& V, int gtid, int gstride,
                                                int least_kind) {
     for (int m = gtid; m < A.nb; m += gstride) {
         if (A.bkind[m] < least_kind) continue;
-        const int run = A.tile_run[tile_of_native(A, A.bcell[m])];
+        const int run = run_of_native(A, A.bcell[m]);
         const int flags = __ldcg(V.flags + run);
         if (!(flags & F_RUN)) continue;
         boundary_cell(A, m, 1 - __ldcg(V.parity + run), flags, __ldcg(V.max_time + run), A.ctl->arrive, A.ctl->deep);
@@ -129,7 +134,7 @@ __device__ __forceinline__ void boundary_items(const StepArgs& A, const StepView
 __device__ __forceinline__ void tally_items(const StepArgs& A, const StepView& V, int gtid, int gstride) {
     for (int m = gtid; m < A.ntally; m += gstride) {
         const int face = A.tface[m];
-        const int run = A.tile_run[tile_of_native(A, face)];
+        const int run = run_of_native(A, face);
         if (!(__ldcg(V.flags + run) & F_RUN)) continue;
         const float qv = __ldcg((A.taxis[m] ? A.q[1] : A.q[0]) + face);
         A.ttotal[m] = __dadd_rn(A.ttotal[m], __dmul_rn(__ldcg(V.dt_tally + run), (double)(A.tsign[m] * qv)));
@@ -139,7 +144,7 @@ __device__ __forceinline__ void tally_items(const StepArgs& A, const StepView& V
     for (int l = gwarp; l < A.nlines; l += nwarps) {
         const int s = A.lstart[l], e = A.lstart[l + 1];
         if (s >= e) continue;
-        const int run = A.tile_run[tile_of_native(A, A.lface[s])];
+        const int run = run_of_native(A, A.lface[s]);
         if (!(__ldcg(V.flags + run) & F_RUN)) continue;
         double acc = 0.0;
         for (int m = s + lane; m < e; m += 32) {
@@ -226,10 +231,11 @@ __device__ __forceinline__ void clear_waves(const StepArgs& A, const StepView& W
         if (W.flags[A.tile_run[t]] & F_WAVE) A.wave[t] = 0.0f;
 }
 
-// The resident loop, one CTA, while the others update the state: every run's clock after the step of settings V, the
-// settings of the next step into W, and whether this step ends with a rebuild of the lists (any: this step's flags).
+// The device loop, one CTA, while the others update the state: every run's clock after the step of settings V, the
+// settings of the next step into W, their flags into *to, and whether this step ends with a rebuild of the lists (any:
+// this step's flags). A step that no run takes hands each run's half on.
 __device__ __forceinline__ void next_settings(const StepArgs& A, const StepView& V, const StepView& W, uint32_t any,
-                                              GridState* grid) {
+                                              uint32_t* to, GridState* grid) {
     uint32_t mine = 0u;
     bool prune = false;
     for (int r = threadIdx.x; r < A.nruns; r += blockDim.x) {
@@ -241,8 +247,8 @@ __device__ __forceinline__ void next_settings(const StepArgs& A, const StepView&
         if (__syncthreads_or(mine & bit)) next |= bit;
     prune = __syncthreads_or(prune);
     if (threadIdx.x == 0) {
-        A.ctl->any = next;
-        A.ctl->m_stored = 0;
+        *to = next;
+        if (any & ANY_RUN) A.ctl->m_stored = 0;
         grid->rebuild = prune || (any & ANY_ACT);
     }
     if (next & ANY_WAVE) clear_waves(A, W);
@@ -358,10 +364,7 @@ static __device__ __noinline__ void rebuild_lists(const StepArgs& A, const StepV
         if (f) A.work[nwork + o] = t;
         nwork += tot;
     }
-    if (threadIdx.x == 0) {
-        ctl->nwork = nwork;
-        ctl->prune = 0;
-    }
+    if (threadIdx.x == 0) ctl->nwork = nwork;
 }
 
 // refresh_plan (wadi2d/solver/gpu/kernels/cells.cu:66-78) of the listed tiles from entry `first` on, `stride` apart,

@@ -422,7 +422,7 @@ __global__ void __launch_bounds__(FACES_THREADS, 2) faces_kernel(const __grid_co
     }
     fill_rowc(rowc, A.rows);
     __syncthreads();
-    if (!(ctl->any & ANY_RUN)) return;
+    if (!(*A.any & ANY_RUN)) return;
     const int nwork = ctl->nwork;
     const int mst = ctl->m_stored;
     const float* statics[12] = {A.fl[0], A.fr[0], A.gl[0], A.gr[0], A.ef[0], A.cw[0],
@@ -699,7 +699,7 @@ __global__ void __launch_bounds__(StripImage<H>::THREADS, StripImage<H>::CTAS)
     }
     fill_rowc(rowc, A.rows);
     __syncthreads();
-    if (!(ctl->any & ANY_RUN)) return;
+    if (!(*A.any & ANY_RUN)) return;
     const int nunits = PER * ctl->nwork;
     const int mst = ctl->m_stored;
     uint32_t phase = 0;
@@ -889,8 +889,8 @@ __device__ __forceinline__ float cell_out_level(const StepArgs& A, const CellOut
 }
 
 // The first entry at or after a, in steps of the grid, whose run is stepping (the same for every thread of a CTA).
-__device__ __forceinline__ int next_tile(const StepArgs& A, int a, int nwork) {
-    for (; a < nwork; a += gridDim.x)
+__device__ __forceinline__ int next_tile(const StepArgs& A, int a, int nwork, int stride) {
+    for (; a < nwork; a += stride)
         if (A.R.flags[A.tile_run[A.list[a]]] & F_RUN) break;
     return a;
 }
@@ -919,21 +919,31 @@ __device__ __forceinline__ void update_issue(float* sm, uint64_t* bar, const Upd
 // level pairs from the cache, or for the cells whose row changed from the table (the gathers issued together). Once
 // every thread has read the image, thread 0 issues the next tile's copies into it, and they land while any gathers
 // return and the level, the wet share and the wet flag are finished.
-__global__ void __launch_bounds__(UPDATE_THREADS) update_kernel(const __grid_constant__ UpdateMaps M, StepArgs A) {
+// control: a step of the device loop, whose first CTA takes no tiles but forms the next step's settings meanwhile (they
+// need the face pass's wave maxima only). As a kernel of its own at the step's end that work, a chain of loads and FP64
+// in one CTA, was 8-14 us of every step.
+__global__ void __launch_bounds__(UPDATE_THREADS) update_kernel(const __grid_constant__ UpdateMaps M, StepArgs A,
+                                                                int control) {
     extern __shared__ __align__(128) float sm[];
     __shared__ __align__(8) uint64_t bar;
     Ctl* ctl = A.ctl;
     const int px = A.px;
     const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
+    grid_open();
+    const int worker = (int)blockIdx.x - control, workers = (int)gridDim.x - control;
+    if (worker < 0) {
+        next_settings(A, step_view(A.R, 0), step_view(A.R, 1), *A.any, A.any_next, grid_state(ctl));
+        return;
+    }
     if (tid == 0) {
         mbar_init(&bar, 1);
         fence_barrier_init();
     }
     __syncthreads();
-    if (!(ctl->any & ANY_RUN)) return;
+    if (!(*A.any & ANY_RUN)) return;
     const int nwork = ctl->nwork;
     // the face pass before this one has stepped: from now on the momenta are formed from the state (Ctl::m_stored)
-    if (blockIdx.x == 0 && tid == 0) ctl->m_stored = 0;
+    if (worker == 0 && tid == 0) ctl->m_stored = 0;
     uint32_t phase = 0;
     const float* QX1 = sm + U_QX1 * BOX;
     const float* QY1 = sm + U_QY1 * BOX;
@@ -942,7 +952,7 @@ __global__ void __launch_bounds__(UPDATE_THREADS) update_kernel(const __grid_con
     const float* SRC = sm + U_OWN + TILE2;
     const float* HC = sm + U_OWN + 2 * TILE2;
     float* rs = sm + U_R;
-    int a = next_tile(A, blockIdx.x, nwork);
+    int a = next_tile(A, worker, nwork, workers);
     if (tid == 0 && a < nwork) update_issue(sm, &bar, M, A, A.list[a]);
     while (a < nwork) {
         const int t = A.list[a];
@@ -988,7 +998,7 @@ __global__ void __launch_bounds__(UPDATE_THREADS) update_kernel(const __grid_con
         }
         // every thread has read the image and r: the next tile's copies land in it during this tile's gathers
         __syncthreads();
-        const int an = next_tile(A, a + gridDim.x, nwork);
+        const int an = next_tile(A, a + workers, nwork, workers);
         if (tid == 0 && an < nwork) update_issue(sm, &bar, M, A, A.list[an]);
         int any = 0;
 #pragma unroll
@@ -1017,8 +1027,9 @@ int update_occupancy() {
     return occ;
 }
 
-void launch_update(const TMaps& M, const StepArgs& A, int grid, cudaStream_t s) {
-    update_kernel<<<grid, UPDATE_THREADS, UPDATE_SMEM, s>>>(M.update, A);
+// grid: the CTAs, with control (a step of the device loop) at least two.
+void launch_update(const TMaps& M, const StepArgs& A, int grid, int control, cudaStream_t s) {
+    update_kernel<<<grid, UPDATE_THREADS, UPDATE_SMEM, s>>>(M.update, A, control);
 }
 
 // ------------------------------------------------------------------ the resident loop
@@ -1244,7 +1255,7 @@ __global__ void __launch_bounds__(RESIDENT_THREADS, resident_ctas(H))
         if (control && host.flags) {
             if (tid == 0) ctl->m_stored = 0;
         } else if (control) {
-            next_settings(A, V, step_view(A.R, b ^ 1), any, grid);
+            next_settings(A, V, step_view(A.R, b ^ 1), any, &ctl->any, grid);
         }
         for (int c0 = 0; c0 < units; c0 += UNITS_HELD) {
             const int n = units > UNITS_HELD ? take(c0) : units;
@@ -1427,21 +1438,31 @@ void launch_momentum(const StepArgs& A, int sms, cudaStream_t s) {
     momentum_kernel<<<sms * 4, 256, 0, s>>>(A);
 }
 
-// ------------------------------------------------------------------ envelope pass
+// ------------------------------------------------------------------ the end of a step
 
-// The envelope after a step of the device loop, for the own cells of the work list's tiles whose runs record it at
-// this step (F_MAX); boundary cells are recorded by the boundary pass after its overwrite. A CTA a tile at a time, a
-// thread a cell; on steps that record no envelope every CTA returns at once.
+// After the update of a step of the device loop: the boundary cells of every running run with their envelope entries, the
+// FP64 tally and the design lines, and, at a step that records it (F_MAX), the envelope of the own cells of the work
+// list's tiles. Each item is independent of the others (a follow boundary reads an interior cell), so one kernel takes
+// them all: the first as a grid-stride loop, then a CTA a tile at a time, a thread a cell.
 // A tile's place (work list -> tile -> its run, its first own cell, its rows' boundary marks) is a chain of dependent
 // loads, each from L2; the CTA stages it for ENV_CHUNK of its tiles at once in shared memory (all chains in flight
 // together), so that a tile's own work waits on its run's flags (L1-resident) and then on its cells' data only.
 constexpr int ENV_CHUNK = 64;
-__global__ void __launch_bounds__(TILE2, 2) envelope_kernel(StepArgs A) {
+__global__ void __launch_bounds__(TILE2, 2) step_end_kernel(StepArgs A) {
     __shared__ int3 place[ENV_CHUNK];            // tile, run, native index of the tile's first own cell
     __shared__ uint32_t marks[ENV_CHUNK * TILE];  // the tile's boundary marks, a word a row
     Ctl* ctl = A.ctl;
     grid_open();
-    if (!(ctl->any & ANY_MAX)) return;
+    grid_wait();
+    const uint32_t any = *A.any;
+    if (any & ANY_RUN) {
+        const StepView V = step_view(A.R, 0);
+        const int gtid = blockIdx.x * TILE2 + threadIdx.x, gstride = gridDim.x * TILE2;
+        boundary_items(A, V, gtid, gstride, 0);
+        // (from the other end, so that few threads have both a boundary cell and a tally face)
+        tally_items(A, V, (gridDim.x - 1 - blockIdx.x) * TILE2 + threadIdx.x, gstride);
+    }
+    if (!(any & ANY_MAX)) return;
     const int nwork = ctl->nwork;
     const float arrive = ctl->arrive, deep = ctl->deep;
     const int tid = threadIdx.x, jj = tid >> 5, ii = tid & 31;
@@ -1471,23 +1492,13 @@ __global__ void __launch_bounds__(TILE2, 2) envelope_kernel(StepArgs A) {
     }
 }
 
-// ------------------------------------------------------------------ boundary, tally, control (one CTA)
-
-// Boundary cells of every running run and their envelope entries after the overwrite; in the device loop (control = 1)
-// also the FP64 tally of every step and the design lines; in a host-driven step (0) the swap of run 0's ping-pong pairs
-// at its end (wadi2d/solver/gpu/backend.py:185-188), by the last CTA to leave. Every item is independent of the others
-// (a follow boundary reads an interior cell), so the kernel is a grid-stride loop over them.
-__global__ void boundary_kernel(StepArgs A, int control) {
+// The boundary cells after a host-driven step, and the swap of run 0's ping-pong pairs at its end
+// (wadi2d/solver/gpu/backend.py:185-188), by the last CTA to leave.
+__global__ void boundary_kernel(StepArgs A) {
     grid_open();
     grid_wait();
-    if (!(A.ctl->any & ANY_RUN)) return;
-    const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gstride = gridDim.x * blockDim.x;
-    const StepView V = step_view(A.R, 0);
-    boundary_items(A, V, gtid, gstride, 0);
-    if (control) {
-        tally_items(A, V, gtid, gstride);
-        return;
-    }
+    if (!(*A.any & ANY_RUN)) return;
+    boundary_items(A, step_view(A.R, 0), blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, 0);
     __syncthreads();
     GridState* grid = grid_state(A.ctl);
     if (threadIdx.x == 0 && atomicAdd(&grid->left, 1u) == gridDim.x - 1) {
@@ -1496,15 +1507,7 @@ __global__ void boundary_kernel(StepArgs A, int control) {
     }
 }
 
-// The end of a step of the device loop, in the kernels of its own: each running run's clock and the next step's
-// settings. The threads of one CTA.
-__device__ void run_clocks(const StepArgs& A) {
-    Ctl* ctl = A.ctl;
-    if (!(ctl->any & ANY_RUN)) return;
-    const StepView V = step_view(A.R, 0);
-    for (int r = threadIdx.x; r < A.nruns; r += blockDim.x)
-        if (run_clock(A, V, V, r)) ctl->prune = 1;  // its tiles leave the work list at this step's rebuild
-}
+// ------------------------------------------------------------------ settings and lists (one CTA)
 
 // Before a step of the device loop, for each run: the loop test and the step's settings
 // (wadi2d/solver/stepper.py:106-111). The threads of one CTA; ctl->any gathers the runs' flags.
@@ -1566,26 +1569,29 @@ __global__ void __launch_bounds__(1024) begin_kernel(const __grid_constant__ Ste
     step_settings(A);
 }
 
-// The end of a step of the device loop and the settings of the next, in one CTA of 1024 threads: each running run's
-// clock, the active-list rebuild (for the runs that check at this step) with the woken tiles and the work list, then
-// the next step's loop test and settings. plan_kernel, after it, takes the woken tiles.
-__global__ void __launch_bounds__(1024) control_kernel(const __grid_constant__ StepArgs A) {
+// The end of a step of the device loop, in one CTA of 1024 threads: at a step that checks (or after which some run has
+// stopped) the active-list rebuild with the woken tiles and the work list, which plan_kernel takes after it; and with
+// adopt (the last of a launch of an odd number of steps) the next step's settings where the first step of a launch reads
+// them.
+__global__ void __launch_bounds__(1024) rebuild_kernel(const __grid_constant__ StepArgs A, int adopt) {
     grid_open();
     grid_wait();
-    run_clocks(A);
-    __syncthreads();
-    rebuild_lists(A, step_view(A.R, 0), false, (A.ctl->any & ANY_ACT) != 0, A.ctl->prune);
-    __syncthreads();
-    step_settings(A);
+    if (grid_state(A.ctl)->rebuild) rebuild_lists(A, step_view(A.R, 0), false, (*A.any & ANY_ACT) != 0, true);
+    if (adopt) {
+        __syncthreads();
+        adopt_settings(A);
+        if (threadIdx.x == 0) *A.any = *A.any_next;
+    }
 }
 
 // refresh_plan of the listed tiles (wadi2d/solver/gpu/kernels/cells.cu:66-78) from the current mean depth. count < 0:
-// the tiles the device loop's last rebuild woke (ctl->nwoken, 0 when it did not rebuild).
+// the tiles that a rebuild at the end of this step of the device loop woke, by the next step's halves.
 __global__ void __launch_bounds__(256) plan_kernel(StepArgs A, const int32_t* list, int count) {
     grid_open();
     grid_wait();
-    if (count < 0) count = A.ctl->nwoken;
-    plan_tiles(A, A.R.parity, list, count, blockIdx.x, gridDim.x);
+    const bool loop = count < 0;
+    if (loop) count = grid_state(A.ctl)->rebuild ? A.ctl->nwoken : 0;
+    plan_tiles(A, loop ? A.R.parity2 : A.R.parity, list, count, blockIdx.x, gridDim.x);
 }
 
 // Maxima.update over the active tiles, host-driven (wadi2d/engine/maxima.py:118-130): the current halves are the
