@@ -683,6 +683,29 @@ __device__ __forceinline__ bool strip_unit(const StripMaps& SM_, const StepArgs&
     return true;
 }
 
+// Where a CTA's next tiles or strips lie, with their runs' settings: a chain of dependent loads (work list -> tile -> its
+// run -> its settings), each from L2. A CTA takes the chains of several at once into shared memory, a thread each, so that
+// a unit's copies are issued as soon as the one before it is done: a step at 4096^2 takes 843 us against 860 with each
+// unit's chain before its copies, at 1500 x 1101 125.2 against 126.2.
+struct Place {
+    int t, ts, run, tj, ti;
+    int flags_p;  // the run's flags and its half (bit 31)
+    float dt, dx;
+};
+__device__ __forceinline__ Place take_place(const StepArgs& A, int t) {
+    Place W;
+    W.t = t;
+    W.run = A.tile_run[t];
+    W.ts = table_of(A, t);
+    W.tj = A.tiles[2 * t];
+    W.ti = A.tiles[2 * t + 1];
+    W.flags_p = A.R.flags[W.run] | (A.R.parity[W.run] << 31);
+    W.dt = A.R.dtf[W.run];
+    W.dx = A.R.dx[W.run];
+    return W;
+}
+constexpr int STRIP_PLACES = 8;  // as many as leave eight CTAs of eight rows on a SM
+
 template <int H, bool ON>
 __global__ void __launch_bounds__(StripImage<H>::THREADS, StripImage<H>::CTAS)
     strips_kernel(const __grid_constant__ StripMaps M, StepArgs A) {
@@ -692,6 +715,7 @@ __global__ void __launch_bounds__(StripImage<H>::THREADS, StripImage<H>::CTAS)
     __shared__ __align__(8) uint64_t bar;
     __shared__ float red[L::THREADS / 32];
     __shared__ float rowc[2 * 64 + 1];
+    __shared__ Place places[STRIP_PLACES];
     Ctl* ctl = A.ctl;
     if (threadIdx.x == 0) {
         mbar_init(&bar, 1);
@@ -703,16 +727,21 @@ __global__ void __launch_bounds__(StripImage<H>::THREADS, StripImage<H>::CTAS)
     const int nunits = PER * ctl->nwork;
     const int mst = ctl->m_stored;
     uint32_t phase = 0;
-    for (int u = blockIdx.x; u < nunits; u += gridDim.x) {
-        const int t = A.list[u / PER];
-        const int run = A.tile_run[t];
-        const int flags = A.R.flags[run];
-        if (!(flags & F_RUN)) continue;  // the tile's run has finished: uniform over the CTA
-        if (!strip_unit<H, L::THREADS / 32, ON, false>(M, A, sm, &bar, phase, rowc, red, t,
-                                                       table_of(A, t), A.tiles[2 * t], A.tiles[2 * t + 1], (u % PER) * H,
-                                                       run, A.R.dtf[run], A.R.dx[run], (flags & F_WAVE) != 0,
-                                                       A.R.parity[run], mst, A.R.wave_bits))
-            return;
+    const int G = gridDim.x;
+    for (int u0 = blockIdx.x; u0 < nunits; u0 += STRIP_PLACES * G) {
+        if (threadIdx.x < STRIP_PLACES && u0 + (int)threadIdx.x * G < nunits)
+            places[threadIdx.x] = take_place(A, A.list[(u0 + (int)threadIdx.x * G) / PER]);
+        __syncthreads();
+        for (int i = 0; i < STRIP_PLACES && u0 + i * G < nunits; ++i) {
+            const Place& W = places[i];
+            const int flags = W.flags_p & 0x7fffffff;
+            if (!(flags & F_RUN)) continue;  // the tile's run has finished: uniform over the CTA
+            if (!strip_unit<H, L::THREADS / 32, ON, false>(M, A, sm, &bar, phase, rowc, red, W.t, W.ts, W.tj, W.ti,
+                                                           ((u0 + i * G) % PER) * H, W.run, W.dt, W.dx,
+                                                           (flags & F_WAVE) != 0, W.flags_p < 0, mst, A.R.wave_bits))
+                return;
+        }
+        __syncthreads();  // every thread has read the places
     }
 }
 
@@ -888,18 +917,11 @@ __device__ __forceinline__ float cell_out_level(const StepArgs& A, const CellOut
     return dk;
 }
 
-// The first entry at or after a, in steps of the grid, whose run is stepping (the same for every thread of a CTA).
-__device__ __forceinline__ int next_tile(const StepArgs& A, int a, int nwork, int stride) {
-    for (; a < nwork; a += stride)
-        if (A.R.flags[A.tile_run[A.list[a]]] & F_RUN) break;
-    return a;
-}
-
-// Issue (thread 0) the copies of tile t's update image against bar: the unscaled discharges and the old depth with
+// Issue (thread 0) the copies of a tile's update image against bar: the unscaled discharges and the old depth with
 // their ring, the residual, the source and Hc, and the tile's level cache (each cell's last level pair and its row).
-__device__ __forceinline__ void update_issue(float* sm, uint64_t* bar, const UpdateMaps& M, const StepArgs& A, int t) {
-    const int p = A.R.parity[A.tile_run[t]];
-    const int tj = A.tiles[2 * t], ti = A.tiles[2 * t + 1];
+__device__ __forceinline__ void update_issue(float* sm, uint64_t* bar, const UpdateMaps& M, const StepArgs& A,
+                                             const Place& W) {
+    const int p = W.flags_p < 0, tj = W.tj, ti = W.ti, t = W.t;
     fence_proxy_async();
     mbar_expect_tx(bar, (uint32_t)(3 * BOX + 3 * TILE2) * 4u + (uint32_t)TILE2 * 9u);
     const int x0 = ti * TILE + GX - 4, y0 = tj * TILE + GY - 2;
@@ -908,7 +930,7 @@ __device__ __forceinline__ void update_issue(float* sm, uint64_t* bar, const Upd
     tma_load_2d(sm + U_H * BOX, &M.h[p], x0, y0, bar);
     tma_load_2d(sm + U_OWN, &M.res, x0 + 4, y0 + 2, bar);
     tma_load_2d(sm + U_OWN + TILE2, &M.src, x0 + 4, y0 + 2, bar);
-    bulk_load(sm + U_OWN + 2 * TILE2, A.hc + (size_t)table_of(A, t) * TILE2, TILE2 * 4, bar);
+    bulk_load(sm + U_OWN + 2 * TILE2, A.hc + (size_t)W.ts * TILE2, TILE2 * 4, bar);
     bulk_load(sm + U_LP, A.lpair + (size_t)t * TILE2, TILE2 * 8, bar);
     bulk_load(sm + U_LR, A.lrow + (size_t)t * TILE2, TILE2, bar);
 }
@@ -919,13 +941,16 @@ __device__ __forceinline__ void update_issue(float* sm, uint64_t* bar, const Upd
 // level pairs from the cache, or for the cells whose row changed from the table (the gathers issued together). Once
 // every thread has read the image, thread 0 issues the next tile's copies into it, and they land while any gathers
 // return and the level, the wet share and the wet flag are finished.
+// Four CTAs a SM: 64 registers. Three (69) took half of the places' gain, five (48, with spills) 3 % of a step.
+constexpr int UPDATE_PLACES = 16;
 // control: a step of the device loop, whose first CTA takes no tiles but forms the next step's settings meanwhile (they
 // need the face pass's wave maxima only). As a kernel of its own at the step's end that work, a chain of loads and FP64
 // in one CTA, was 8-14 us of every step.
-__global__ void __launch_bounds__(UPDATE_THREADS) update_kernel(const __grid_constant__ UpdateMaps M, StepArgs A,
+__global__ void __launch_bounds__(UPDATE_THREADS, 4) update_kernel(const __grid_constant__ UpdateMaps M, StepArgs A,
                                                                 int control) {
     extern __shared__ __align__(128) float sm[];
     __shared__ __align__(8) uint64_t bar;
+    __shared__ Place places[2 * UPDATE_PLACES];
     Ctl* ctl = A.ctl;
     const int px = A.px;
     const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
@@ -952,26 +977,37 @@ __global__ void __launch_bounds__(UPDATE_THREADS) update_kernel(const __grid_con
     const float* SRC = sm + U_OWN + TILE2;
     const float* HC = sm + U_OWN + 2 * TILE2;
     float* rs = sm + U_R;
-    int a = next_tile(A, worker, nwork, workers);
-    if (tid == 0 && a < nwork) update_issue(sm, &bar, M, A, A.list[a]);
-    while (a < nwork) {
-        const int t = A.list[a];
-        const int run = A.tile_run[t];
-        const int flags = A.R.flags[run];
-        const float dt = A.R.dtf[run];
-        const float dxr = A.R.dx[run];
+    const int n = worker < nwork ? (nwork - worker + workers - 1) / workers : 0;  // this CTA's tiles
+    // the places of UPDATE_PLACES of them from `first` on, into their half of the ring
+    auto take = [&](int first) {
+        const int i = first + tid;
+        if (tid < UPDATE_PLACES && i < n)
+            places[i % (2 * UPDATE_PLACES)] = take_place(A, A.list[worker + i * workers]);
+    };
+    take(0);
+    __syncthreads();
+    if (tid == 0 && n > 0) update_issue(sm, &bar, M, A, places[0]);
+    for (int i = 0; i < n; ++i) {
+        if (i % UPDATE_PLACES == 0) take(i + UPDATE_PLACES);  // (their half was last read at tile i - 1)
+        const Place& W = places[i % (2 * UPDATE_PLACES)];
+        const int t = W.t, ts = W.ts, tj = W.tj, ti = W.ti, p = W.flags_p < 0;
+        const int flags = W.flags_p & 0x7fffffff;
+        const float dt = W.dt, dxr = W.dx;
         const float area = dxr * dxr;
         const int want_plan = (flags & F_WAVE) != 0;
         const int want_wet = (flags & F_WET) != 0;
-        const int p = A.R.parity[run];
         float* __restrict__ h_next = A.hh[1 - p];
-        const int tj = A.tiles[2 * t], ti = A.tiles[2 * t + 1];
         const bool ok = mbar_wait(&bar, phase);
         phase ^= 1u;
         if (__syncthreads_or(!ok)) {
             if (tid == 0) atomicExch(&ctl->status, W2B_ETIMEOUT);
             mbar_wait(&bar, phase ^ 1u);
             return;
+        }
+        if (!(flags & F_RUN)) {  // the tile's run has finished: uniform over the CTA
+            __syncthreads();
+            if (tid == 0 && i + 1 < n) update_issue(sm, &bar, M, A, places[(i + 1) % (2 * UPDATE_PLACES)]);
+            continue;
         }
         // r of the tile and its ring, from the old h
         for (int idx = tid; idx < RING * RING; idx += UPDATE_THREADS) {
@@ -980,7 +1016,7 @@ __global__ void __launch_bounds__(UPDATE_THREADS) update_kernel(const __grid_con
         }
         __syncthreads();
         const int base = (tj * TILE + GY) * px + ti * TILE + GX;
-        const float2* __restrict__ pairs_t = A.dtab2 + (size_t)table_of(A, t) * (A.rows - 1) * TILE2;
+        const float2* __restrict__ pairs_t = A.dtab2 + (size_t)ts * (A.rows - 1) * TILE2;
         CellOut C[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
@@ -998,8 +1034,7 @@ __global__ void __launch_bounds__(UPDATE_THREADS) update_kernel(const __grid_con
         }
         // every thread has read the image and r: the next tile's copies land in it during this tile's gathers
         __syncthreads();
-        const int an = next_tile(A, a + workers, nwork, workers);
-        if (tid == 0 && an < nwork) update_issue(sm, &bar, M, A, A.list[an]);
+        if (tid == 0 && i + 1 < n) update_issue(sm, &bar, M, A, places[(i + 1) % (2 * UPDATE_PLACES)]);
         int any = 0;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
@@ -1013,7 +1048,6 @@ __global__ void __launch_bounds__(UPDATE_THREADS) update_kernel(const __grid_con
             const int w = __syncthreads_or(any);
             if (tid == 0) A.wet[t] = w;
         }
-        a = an;
     }
 }
 
