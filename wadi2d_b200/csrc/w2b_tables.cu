@@ -3,8 +3,9 @@
 // Restates wadi2d/tables/core.py (cell tables :16-41, face tables :44-79, local hydraulic radius :82-179 and
 // :324-371, centre beds :267-279) and wadi2d/tables/builder.py (the per-tile windows :199-238, inverts, closed faces
 // and natural crests :290-308) in FP64 with the reference's summation order: every running sum is taken by one
-// thread in the reference's sequence, so the only difference from the CPU build is the last-ulp rounding of CUDA's
-// double cbrt and pow against glibc's, which the float32 tables almost never see.
+// thread in the reference's sequence, so the only differences from the CPU build are the last-ulp rounding of CUDA's
+// double cbrt and pow against glibc's, which the float32 tables almost never see, and of the local radius's sums, which
+// are taken over its tent alone (local_term).
 //
 // Pixels are read from the whole bed with clipped indices, which is what the reference's per-tile windows of an
 // ArrayBed hold (wadi2d/tables/builder.py:47-50): a window that reaches past the bed repeats its edge pixel.
@@ -204,58 +205,60 @@ struct __align__(16) LinePixel {
 
 // One pixel's conveyance term weight d cbrt(R)^2 at one level (_local_radius_conveyance, wadi2d/tables/core.py:
 // 82-179): L is the face's conveyance line (n pixels). The local radius R weighs depth and wetted perimeter by a tent of
-// half-width w = beta d / pixel pixels around pixel i, inside its wet stretch; its sums are differences of running sums
-// taken from the line's start, so the sums run in that order here too: over [0, i] with their values kept at the tent's
-// first pixel lo, then over (i, hi]. A dry pixel adds nothing to a sum and starts a new stretch, so lo moves behind it;
-// the first dry pixel after i ends the sweep. Almost every pixel swept lies between wet ones: that case is the loops'
-// first branch, and takes one 16-byte load.
+// half-width w = beta d / pixel (tent: beta / pixel) pixels around pixel i, inside its wet stretch. The reference takes the tent's sums as
+// differences of running sums from the line's start; here they run over the tent alone, with the distance from pixel i as
+// the argument, which needs no difference (so it rounds less) and sweeps 2 w pixels instead of i + w: w goes with the
+// level, so most table rows' tents are far shorter than the line. A dry pixel before i starts the sums again; the first dry
+// pixel after i ends them. Almost every pixel swept lies between wet ones: that case is the loops' first branch, and takes
+// one 16-byte load.
 __device__ __forceinline__ double local_term(const LinePixel* __restrict__ L, int n, int i, double level, double pixel,
-                                             double beta, double weight) {
+                                             double tent, double weight) {
     const double di = level - L[i].z;
     if (!(di > 0.0)) return 0.0;
-    double w = beta * di / pixel;
+    double w = tent * di;
     if (w < 1e-9) w = 1e-9;
-    const int lo = (int)ceil((double)i - w);
-    int hi = (int)floor((double)i + w);
+    int lo = (int)ceil((double)i - w), hi = (int)floor((double)i + w);
+    lo = lo > 0 ? lo : 0;
     hi = hi < n - 1 ? hi : n - 1;
     const double half = 0.5 * pixel;
-    double s0 = 0.0, s1 = 0.0, p0 = 0.0, p1 = 0.0, ft = 0.0;
-    double da = level - L[0].z;  // depth of pixel t (dry: not over 0), and cr: the perimeter it has from its west
-    double cr = 0.0;             // segment or the line's end
-    if (da > 0.0) cr = n == 1 ? half + half : half;
-    auto add = [&](double per) {
-        s0 += da;
-        s1 += ft * da;
-        p0 += per;
-        p1 += ft * per;
-    };
     // the perimeter a wet pixel has from a segment to a dry one `rise` higher
     auto partial = [&](double depth, double rise, double half_seg) {
         if (!(rise > 0.0)) return half;
         const double f = depth / rise;
         return (f <= 1.0 ? f : 1.0) * (2.0 * half_seg);
     };
-    double l0 = 0.0, l1 = 0.0, l2 = 0.0, l3 = 0.0;
-    for (int t = 0; t < i; ++t) {
+    double s0 = 0.0, s1 = 0.0, p0 = 0.0, p1 = 0.0;  // sums of depth and perimeter, and of u times them
+    double u = (double)(lo - i);                    // minus the distance of pixel t from pixel i
+    double da = level - L[lo].z;  // depth of pixel t (dry: not over 0), and cr: the perimeter it has from its west
+    double cr = 0.0;              // segment or the line's end
+    if (da > 0.0) {
+        if (lo == 0)
+            cr = n == 1 ? half + half : half;
+        else
+            cr = level - L[lo - 1].z > 0.0 ? L[lo].half_seg : partial(da, L[lo - 1].z - L[lo].z, L[lo].half_seg);
+    }
+    auto add = [&](double per) {
+        s0 += da;
+        s1 = fma(u, da, s1);
+        p0 += per;
+        p1 = fma(u, per, p1);
+    };
+    for (int t = lo; t < i; ++t) {
         const LinePixel next = L[t + 1];
         const double db = level - next.z;
-        if (t == lo) l0 = s0, l1 = s1, l2 = p0, l3 = p1;
         if (da > 0.0 && db > 0.0) {
             add(cr + next.half_seg);
             cr = next.half_seg;
+        } else if (da > 0.0) {  // the next pixel, dry, starts the sums again
+            cr = 0.0;
         } else {
-            if (da > 0.0)
-                add(cr + partial(da, next.z - L[t].z, next.half_seg));
-            else if (t >= lo)
-                l0 = s0, l1 = s1, l2 = p0, l3 = p1;
-            cr = !(da > 0.0) && db > 0.0 ? partial(db, L[t].z - next.z, next.half_seg) : 0.0;
+            s0 = s1 = p0 = p1 = 0.0;
+            cr = db > 0.0 ? partial(db, L[t].z - next.z, next.half_seg) : 0.0;
         }
         da = db;
-        ft += 1.0;
+        u += 1.0;
     }
-    if (i == lo) l0 = s0, l1 = s1, l2 = p0, l3 = p1;
     if (i == n - 1 && i > 0) cr = half + cr;
-    double m0 = 0.0, m1 = 0.0, m2 = 0.0, m3 = 0.0;
     for (int t = i; t <= hi && da > 0.0; ++t) {
         double db = 0.0, per = cr;
         if (t + 1 < n) {
@@ -269,15 +272,10 @@ __device__ __forceinline__ double local_term(const LinePixel* __restrict__ L, in
             }
         }
         add(per);
-        if (t == i) m0 = s0, m1 = s1, m2 = p0, m3 = p1;
         da = db;
-        ft += 1.0;
+        u -= 1.0;
     }
-    const double fi = (double)i;
-    double a_sum = (1.0 - fi / w) * (m0 - l0) + (m1 - l1) / w;
-    a_sum += (1.0 + fi / w) * (s0 - m0) - (s1 - m1) / w;
-    double p_sum = (1.0 - fi / w) * (m2 - l2) + (m3 - l3) / w;
-    p_sum += (1.0 + fi / w) * (p0 - m2) - (p1 - m3) / w;
+    const double a_sum = fma(s0, w, s1), p_sum = fma(p0, w, p1);  // both w times the tent's sum: one division in all
     const double radius = p_sum > 0.0 ? pixel * a_sum / p_sum : di;
     const double cb = cbrt(radius);
     return weight * di * (cb * cb);
@@ -286,12 +284,14 @@ __device__ __forceinline__ double local_term(const LinePixel* __restrict__ L, in
 // The face tables (_face_table, wadi2d/tables/core.py:44-79, and the local radius's conveyance), a group of GF faces
 // in a row along their own line at a time (GF divides 32: a column of a tile's west faces, a row of its north faces).
 // The faces of a group share one line of GF k + 2 margin pixels, read once; then every (face, row, pixel) is a thread's
-// own sweep along it (local_term), and every (face, row) a thread that adds its pixels' terms in order. The sweeps'
-// instructions bound it: 2.1 M faces of 24- to 44-pixel lines (1024 x 1024 cells, 4 x 4 pixels) take 8.5 ms, 98 k faces of
-// up to 298 (10 x 10 pixels of 1 m) 2.9 ms. A thread a face with its nine line arrays in shared memory, as this was first
-// written, left 63 and 9 threads a SM and took 67 and 99 ms; the sweep with clamped depths and no branch of its own for
-// wet neighbours took 12.0 and 4.9; a thread four or five pixels at once (one sweep for all, 200 registers, 8 warps a SM)
-// 13.4 and 4.0. Three CTAs a SM (80 registers) against two: 8.5 against 9.2.
+// own sweep along it (local_term), and every (face, row) a thread that adds its pixels' terms in order. FP64 instructions
+// bound it (the sweeps, a division, a cbrt and four conversions a term): 2.1 M faces of 24- to 44-pixel lines (1024 x 1024
+// cells, 4 x 4 pixels) take 4.3 ms, 98 k faces of up to 298 (10 x 10 pixels of 1 m) 1.2 ms. A thread a face with its nine
+// line arrays in shared memory, as this was first written, left 63 and 9 threads a SM and took 67 and 99 ms; sweeps from
+// the line's start 8.5 and 2.9; the tent's sweeps with four divisions a term, the rows' levels and the indices divided out
+// for each term, 5.2 and 1.26. A thread four or five pixels at once (one sweep for all, 200 registers, 8 warps a SM) was
+// slower. Three CTAs of 256 threads a SM (80 registers): four (64, with spills) 5.3 and 1.39 against 5.2 and 1.26; six of
+// 128 threads the same.
 // LINE_SMEM: the group's line in shared memory, else (a line too long for it) in the caller's workspace, GF = 1.
 struct FaceShape {
     int gf, fc;      // faces a group; of them, whose terms are held at a time
@@ -300,7 +300,8 @@ struct FaceShape {
 template <bool LINE_SMEM>
 __global__ void __launch_bounds__(FACE_THREADS, 3) face_tables_kernel(TableArgs A, FaceShape F) {
     extern __shared__ __align__(16) double sws[];
-    __shared__ double s_zf[TILE], s_top[TILE];
+    __shared__ double s_zf[TILE], s_top[TILE], s_scale[TILE], s_len[TILE], s_crest[TILE], s_nm[TILE];
+    __shared__ double s_xx[ROWS_MAX];  // a row's level over the invert, of the face's full depth
     __shared__ int s_e[TILE];  // pixels the conveyance line reaches past the face's ends, -1: the strips' sum
     const int k = A.k, rows = A.rows, last = rows - 1, GF = F.gf, tid = threadIdx.x;
     double* terms = sws;
@@ -308,6 +309,11 @@ __global__ void __launch_bounds__(FACE_THREADS, 3) face_tables_kernel(TableArgs 
     LinePixel* line = reinterpret_cast<LinePixel*>(LINE_SMEM ? sws + (((size_t)F.fc * rows * k + 1) & ~(size_t)1)
                                                              : (double*)(((uintptr_t)A.ws + 15) & ~(uintptr_t)15) +
                                                                    (size_t)blockIdx.x * 2 * F.line);
+    for (int r = tid; r < rows; r += FACE_THREADS) {
+        const double xr = (double)r / (double)last;
+        s_xx[r] = xr * xr;
+    }
+    const double tent = A.beta / A.pixel;
     const int per = TILE / GF;
     const int64_t groups = (int64_t)(A.ntiles - 1) * 2 * TILE * per;
     for (int64_t g = blockIdx.x; g < groups; g += gridDim.x) {
@@ -363,6 +369,12 @@ __global__ void __launch_bounds__(FACE_THREADS, 3) face_tables_kernel(TableArgs 
                     e = (int)ceil(A.beta * top / A.pixel);
                     e = e > A.margin ? A.margin : e;
                 }
+                const double* lengths = axis == 0 ? A.xlen : A.ylen;
+                const double nm = A.nman[cell];
+                s_nm[f] = nm;
+                s_scale[f] = A.pixel * (1.0 / nm);
+                s_len[f] = lengths ? lengths[cell] : 1.0;
+                s_crest[f] = crest;
                 s_zf[f] = zf;
                 s_top[f] = top;
                 s_e[f] = e;
@@ -374,28 +386,31 @@ __global__ void __launch_bounds__(FACE_THREADS, 3) face_tables_kernel(TableArgs 
         __syncthreads();
         for (int f0 = 0; f0 < GF; f0 += F.fc) {
             const int nf = GF - f0 < F.fc ? GF - f0 : F.fc;
-            for (int x = tid; x < nf * rows * k && A.local; x += FACE_THREADS) {
-                const int q = x % k, f = f0 + x / k % nf, r = x / (k * nf);
-                const int e = s_e[f];
-                if (e < 0) continue;
-                const double xr = (double)r / (double)last;
-                const double level = s_zf[f] + s_top[f] * (xr * xr);
-                const int at = f * k + A.margin - e;
-                const int64_t j = j0 + f * dj, i = i0 + f * di;
-                const double weight = A.npix ? edge_weight(A, axis, j * k, i * k, q, A.nman[j * A.nx + i]) : 1.0;
-                terms[x] = local_term(line + at, k + 2 * e, e + q, level, A.pixel, A.beta, weight);
+            // term x is pixel q of face f at row r, q fastest; stepped without a division
+            const int kf = k * nf, dr = FACE_THREADS / kf, rest = FACE_THREADS % kf, df = rest / k, dq = rest % k;
+            int r = tid / kf, fl = tid % kf / k, q = tid % k;
+            for (int x = tid; x < kf * rows && A.local; x += FACE_THREADS) {
+                const int f = f0 + fl, e = s_e[f];
+                if (e >= 0) {
+                    const double level = s_zf[f] + s_top[f] * s_xx[r];
+                    const int at = f * k + A.margin - e;
+                    const int64_t j = j0 + f * dj, i = i0 + f * di;
+                    const double weight = A.npix ? edge_weight(A, axis, j * k, i * k, q, s_nm[f]) : 1.0;
+                    terms[x] = local_term(line + at, k + 2 * e, e + q, level, A.pixel, tent, weight);
+                }
+                q += dq;
+                if (q >= k) q -= k, ++fl;
+                fl += df;
+                if (fl >= nf) fl -= nf, ++r;
+                r += dr;
             }
             __syncthreads();
             for (int x = tid; x < nf * rows; x += FACE_THREADS) {
                 const int r = x % rows, fl = x / rows, f = f0 + fl;
-                const int64_t j = j0 + f * dj, i = i0 + f * di, cell = j * A.nx + i;
-                const double nm = A.nman[cell];
-                const double crest = crests ? crests[cell] : NAN;
-                const double* lengths = axis == 0 ? A.xlen : A.ylen;
-                const double length = lengths ? lengths[cell] : 1.0;
+                const int64_t j = j0 + f * dj, i = i0 + f * di;
+                const double crest = s_crest[f], length = s_len[f];
                 const LinePixel* prof = line + f * k + A.margin;
-                const double zf = s_zf[f], xr = (double)r / (double)last;
-                const double e = s_top[f] * (xr * xr);
+                const double zf = s_zf[f], e = s_top[f] * s_xx[r];
                 const bool strips = s_e[f] < 0;
                 double area = 0.0, conv = 0.0;
                 for (int q = 0; q < k; ++q) {
@@ -405,7 +420,7 @@ __global__ void __launch_bounds__(FACE_THREADS, 3) face_tables_kernel(TableArgs 
                         area += dep;
                         if (strips) {
                             const double cb = cbrt(dep);
-                            conv += edge_weight(A, axis, j * k, i * k, q, nm) * dep * (cb * cb);
+                            conv += edge_weight(A, axis, j * k, i * k, q, s_nm[f]) * dep * (cb * cb);
                         }
                     }
                     if (!strips) conv += terms[(r * nf + fl) * k + q];
@@ -413,7 +428,7 @@ __global__ void __launch_bounds__(FACE_THREADS, 3) face_tables_kernel(TableArgs 
                 const size_t o = (size_t)t * TILE2 + (jj0 + f * dj) * TILE + ii0 + f * di;
                 float* out = (axis == 0 ? A.ftabx : A.ftaby) + (o * rows + r) * 2;
                 out[0] = (float)(A.pixel * area * length);
-                out[1] = (float)pow(A.pixel * (1.0 / nm) * conv * length, 0.6);
+                out[1] = (float)pow(s_scale[f] * conv * length, 0.6);
             }
             __syncthreads();  // the terms, and at the end the line and the faces' numbers, are read by every thread
         }
