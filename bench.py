@@ -1051,9 +1051,9 @@ def main() -> None:
                        "arith": args.arith, "loop": "device-resident, CUDA graphs", "launch": launch,
                        "tuning_steps": tune_steps},
             "roofline": roofline, "cpu_baseline": cpu, "parity": parity, "e2e": e2e, "sweep": sweep, "clocks": clk,
-            # the device loop's launches: the work list and the first step's settings, then graphs of 16 steps of
-            # six kernels (faces, update, envelope, boundary, control, plan)
-            "gpu_launches": 2 + 6 * launch["steps_per_graph"] * -(-ran // launch["steps_per_graph"]),
+            # the device loop's launches: the work list and the first step's settings, then graphs of steps of five
+            # kernels (faces, update, step end, rebuild, plan), or the resident loop's
+            "gpu_launches": 1 + (-(-ran // launch["steps_per_graph"]) if launch["resident"] else 5 * ran),
         }  # fmt: skip
         print(json.dumps(line), flush=True)
     if world > 1:

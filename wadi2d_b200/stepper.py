@@ -3,7 +3,7 @@
 ``advance`` is the reference's host loop, statement for statement (one ``backend.step`` per step, the host reading
 the wave speed back on refresh steps and the wet flags on active-list steps). ``run`` is the same loop resident on
 the device (``w2b_advance``): step rule, refresh cadence, sleeping tiles, the envelope every ``max_every`` steps and
-the boundary tally every step, captured as CUDA graphs, with one host read per graph of 16 steps.
+the boundary tally every step, as CUDA graphs or one resident kernel, with one host read per some launches.
 """
 
 from __future__ import annotations
