@@ -66,6 +66,7 @@ static const Passes& passes(const W2BParams& P) { return P.arith == W2B_ARITH_FA
 void launch_cbrt_check(uint32_t first, uint32_t count, unsigned long long* out, cudaStream_t s);
 void launch_wait_check(uint32_t polls, long long* out, cudaStream_t s);
 void launch_momentum(const StepArgs& A, int sms, cudaStream_t s);
+void launch_asleep(const StepArgs& A, int sms, cudaStream_t s);
 __global__ void boundary_kernel(StepArgs A);
 __global__ void step_end_kernel(StepArgs A);
 __global__ void rebuild_kernel(const __grid_constant__ StepArgs A, int adopt);
@@ -133,6 +134,7 @@ struct Handle {
     W2BBuffers B{};
     int cur = 0;  // run 0's current half (the device keeps it in R.parity[0])
     int nact = 0;
+    bool touched = false;  // a state array has been in a caller's hands since the last step (asleep_kernel)
     int nruns = 1;
     RunTab R;
     int nb = 0;
@@ -434,6 +436,16 @@ static int set_passes(Handle& H) {
 // The pinned buffer: the run table, the control block, a batch's clocks and end times.
 static size_t host_bytes(int nruns) {
     return run_table_bytes(nruns) + W2B_CTL_BYTES + (sizeof(W2BClock) + sizeof(double)) * (size_t)nruns;
+}
+
+// Before steps: the sleeping tiles' other halves, if a caller may have written their current ones.
+static int settle_asleep(Handle& H, cudaStream_t s) {
+    if (H.touched && H.nact < H.g.ntiles - 1) {
+        launch_asleep(make_args(H), H.sms, s);
+        CKL("sleeping tiles");
+    }
+    H.touched = false;
+    return W2B_OK;
 }
 
 // The face pass of a host-driven step (w2b_step, w2b_step_timed) over n tiles: in the form and at the CTAs a SM the
@@ -787,7 +799,8 @@ int32_t w2b_step(void* handle, float dt, int32_t want_wave, int32_t want_wet, vo
     if (H->nruns != 1) return W2B_EINVAL;  // a batch steps in the device loop
     if (H->nact > 0) {
         bool done = false;
-        const int st = host_resident(*H, dt, want_wave, want_wet, s, &done);
+        int st = settle_asleep(*H, s);
+        if (st == W2B_OK) st = host_resident(*H, dt, want_wave, want_wet, s, &done);
         if (st != W2B_OK) return st;
         if (done) {
             H->cur ^= 1;
@@ -814,6 +827,8 @@ int32_t w2b_step_timed(void* handle, float dt, int32_t want_wave, int32_t want_w
     Handle* H = static_cast<Handle*>(handle);
     cudaStream_t s = (cudaStream_t)stream;
     if (H->nact == 0 || H->nruns != 1) return W2B_EINVAL;
+    const int st = settle_asleep(*H, s);
+    if (st != W2B_OK) return st;
     cudaEvent_t ev[4];
     for (auto& e : ev) CK(cudaEventCreate(&e));
     const StepArgs A = make_args(*H);
@@ -902,6 +917,7 @@ int32_t w2b_field_ptr(void* handle, int32_t field, float** out) {
     float* p = field_ptr(static_cast<Handle*>(handle), field);
     if (!p) return W2B_EINVAL;
     *out = p;
+    if (field == W2B_H || field == W2B_U || field == W2B_V) static_cast<Handle*>(handle)->touched = true;
     return W2B_OK;
 }
 
@@ -950,6 +966,7 @@ int32_t w2b_set_field(void* handle, int32_t field, const float* src, int32_t lay
     Handle* H = static_cast<Handle*>(handle);
     float* dst = field_ptr(H, field);
     if (!dst) return W2B_EINVAL;
+    if (field == W2B_H || field == W2B_U || field == W2B_V) H->touched = true;
     cudaStream_t s = (cudaStream_t)stream;
     if (momentum_field(field)) {
         const int st = sync_momentum(*H, s);
@@ -1097,6 +1114,8 @@ static int advance_runs(Handle* H, const W2BStepper* cfg, const double* t_end, i
         memcpy(hclocks, clocks, sizeof(W2BClock) * n);
         memcpy(hends, t_end, sizeof(double) * n);
     }
+    const int settled = settle_asleep(*H, s);
+    if (settled != W2B_OK) return settled;
     // the work list of the runs that take a step, and the first step's settings; each step sets the next's
     begin_kernel<<<1, 1024, 0, s>>>(make_args(*H), c, clocks[0], t_end[0], (long long)max_steps,
                                     n > 1 ? hclocks : nullptr, n > 1 ? hends : nullptr);

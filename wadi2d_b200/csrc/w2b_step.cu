@@ -1474,6 +1474,25 @@ __global__ void __launch_bounds__(256) momentum_kernel(StepArgs A) {
     }
 }
 
+// The other halves of the sleeping tiles from their current ones, after a caller has had the state arrays in hand: the
+// passes never write a sleeping tile, so what it holds has to be the same in both halves of its pairs (as it is where a
+// tile has fallen asleep by itself: dry and still), or the step after next would find in it what a write to the current
+// half meant to replace. A CTA a tile, a thread four cells in a row.
+__global__ void __launch_bounds__(256) asleep_kernel(StepArgs A) {
+    const int jj = threadIdx.x >> 3, ii = (threadIdx.x & 7) * 4;
+    for (int t = 1 + blockIdx.x; t < A.ntiles; t += gridDim.x) {
+        if (A.is_act[t]) continue;
+        const size_t k = (size_t)(A.tiles[2 * t] * TILE + GY + jj) * A.px + A.tiles[2 * t + 1] * TILE + GX + ii;
+        const int p = A.R.parity[A.tile_run[t]];
+        float* const pairs[3][2] = {{A.hh[p], A.hh[1 - p]}, {A.uu[0][p], A.uu[0][1 - p]}, {A.uu[1][p], A.uu[1][1 - p]}};
+#pragma unroll
+        for (int f = 0; f < 3; ++f)
+            *reinterpret_cast<float4*>(pairs[f][1] + k) = *reinterpret_cast<const float4*>(pairs[f][0] + k);
+    }
+}
+
+void launch_asleep(const StepArgs& A, int sms, cudaStream_t s) { asleep_kernel<<<sms * 8, 256, 0, s>>>(A); }
+
 void launch_momentum(const StepArgs& A, int sms, cudaStream_t s) {
     momentum_kernel<<<sms * 8, 256, 0, s>>>(A);
 }
