@@ -167,11 +167,14 @@ __device__ __forceinline__ void tally_items(const StepArgs& A, const StepView& V
 
 // A running run's clock after its step of settings V (wadi2d/solver/stepper.py:113-124): the swap of its halves (into
 // W, which may be V), t, the step counts, the step rule on refresh steps (dt_min and non-finite checks). True: the run
-// stops, so its tiles leave the work list at this step's rebuild.
+// stops, so its tiles leave the work list at this step's rebuild. Every run's wave maximum goes on to W, for either set
+// holds the last refresh step's (run_settings clears it where the next step refreshes).
 __device__ __forceinline__ bool run_clock(const StepArgs& A, const StepView& V, const StepView& W, int r) {
     Ctl* ctl = A.ctl;
     const RunTab& R = A.R;
     const int flags = V.flags[r];
+    const uint32_t bits = __ldcg(V.wave_bits + r);
+    W.wave_bits[r] = bits;
     if (!(flags & F_RUN)) {
         W.parity[r] = V.parity[r];
         return false;
@@ -181,7 +184,7 @@ __device__ __forceinline__ bool run_clock(const StepArgs& A, const StepView& V, 
     R.nsteps[r] += 1;
     R.steps_run[r] += 1;
     if (flags & F_WAVE) {
-        const float wave = __uint_as_float(__ldcg(V.wave_bits + r));
+        const float wave = __uint_as_float(bits);
         R.wave_last[r] = wave;
         const double w = (double)wave;
         if (!isfinite(w)) {
