@@ -90,41 +90,36 @@ __device__ __forceinline__ void envelope_cell(const StepArgs& A, int fid, int k,
     envelope_apply(A, fid, envelope_load(A, fid, k, un, vn), dk, hk, time, arrive, deep);
 }
 
-// Boundary cell m after a step to half n (wadi2d/solver/gpu/kernels/cells.cu:95-111), and its envelope entry.
-__device__ __forceinline__ void boundary_cell(const StepArgs& A, int m, int n, int flags, float time, float arrive,
-                                              float deep) {
-    const int k = A.bcell[m];
-    float* h_next = A.hh[n];
-    const int kind = A.bkind[m];
-    if (kind == 0) {
-        h_next[k] = A.bh0[m];
-        A.d[k] = A.bd0[m];
-    } else if (kind == 1) {
-        h_next[k] = 0.0f;
-        A.d[k] = 0.0f;
-    } else {
-        const int r = A.bref[m];
-        h_next[k] = h_next[r];
-        A.d[k] = fmax32(A.d[r] + A.bd0[m], 0.0f);
-    }
-    if ((flags & F_MAX) == F_MAX)
-        envelope_cell(A, fid_of_native(A, k), k, A.d[k], h_next[k], time, arrive, deep, A.uu[0][n], A.uu[1][n]);
-}
-
 // The run that native cell k belongs to.
 __device__ __forceinline__ int run_of_native(const StepArgs& A, int k) {
     return A.nruns == 1 ? 0 : A.tile_run[tile_of_native(A, k)];
 }
 
-// The boundary cells of at least this kind of every running run.
+// The boundary cells of every running run after its step (wadi2d/solver/gpu/kernels/cells.cu:95-111), whether their tile is
+// stepped or asleep, and their envelope entries. host_flags: a host-driven step's of run 0 (0 in the device loop). What a
+// cell needs is a chain of loads from L2, so all that do not depend on one another are issued together.
 __device__ __forceinline__ void boundary_items(const StepArgs& A, const StepView& V, int gtid, int gstride,
-                                               int least_kind) {
+                                               int host_flags = 0) {
     for (int m = gtid; m < A.nb; m += gstride) {
-        if (A.bkind[m] < least_kind) continue;
-        const int run = run_of_native(A, A.bcell[m]);
-        const int flags = __ldcg(V.flags + run);
+        const int k = A.bcell[m], kind = A.bkind[m];
+        const float h0 = A.bh0[m], d0 = A.bd0[m];
+        const float arrive = A.ctl->arrive, deep = A.ctl->deep;
+        const int fid = fid_of_native(A, k);
+        const int run = A.nruns == 1 ? 0 : A.tile_run[fid / TILE2];
+        const int flags = host_flags ? host_flags : __ldcg(V.flags + run);
+        const int n = 1 - __ldcg(V.parity + run);
+        const float time = __ldcg(V.max_time + run);
         if (!(flags & F_RUN)) continue;
-        boundary_cell(A, m, 1 - __ldcg(V.parity + run), flags, __ldcg(V.max_time + run), A.ctl->arrive, A.ctl->deep);
+        float* h_next = A.hh[n];
+        float hk = kind == 0 ? h0 : 0.0f, dk = kind == 0 ? d0 : 0.0f;
+        if (kind > 1) {
+            const int r = A.bref[m];
+            hk = h_next[r];
+            dk = fmax32(A.d[r] + d0, 0.0f);
+        }
+        h_next[k] = hk;
+        A.d[k] = dk;
+        if (flags & F_MAX) envelope_cell(A, fid, k, dk, hk, time, arrive, deep, A.uu[0][n], A.uu[1][n]);
     }
 }
 
@@ -174,8 +169,8 @@ __device__ __forceinline__ bool run_clock(const StepArgs& A, const StepView& V, 
     const RunTab& R = A.R;
     const int flags = V.flags[r];
     const uint32_t bits = __ldcg(V.wave_bits + r);
-    W.wave_bits[r] = bits;
     if (!(flags & F_RUN)) {
+        W.wave_bits[r] = bits;
         W.parity[r] = V.parity[r];
         return false;
     }
@@ -195,6 +190,7 @@ __device__ __forceinline__ bool run_clock(const StepArgs& A, const StepView& V, 
             if (R.dt[r] < ctl->dt_min) R.status[r] = W2B_EDTMIN;
         }
     }
+    W.wave_bits[r] = bits;
     return !live_run(R, r, ctl);
 }
 

@@ -848,10 +848,11 @@ struct CellOut {
 
 // Continuity (cells.cu:219-232) of the cell at box index b, own index `local` and native index k: the scaled discharges,
 // the residual and the mean depth written, and the level table's row (common.cuh cell_level): the top row above Hc.
-// row: r of the cell in the ring's image.
+// row: r of the cell in the ring's image. prescribed: a boundary cell whose depths another thread writes.
 __device__ __forceinline__ CellOut continuity(const StepArgs& A, const float* QX1, const float* QY1, const float* H,
                                               const float* row, int b, int local, int k, const float* RES,
-                                              const float* SRC, const float* HC, float* h_next, float dt, float area) {
+                                              const float* SRC, const float* HC, float* h_next, float dt, float area,
+                                              bool prescribed = false) {
     const int last = A.rows - 1;
     CellOut C;
     const float rc = row[0];
@@ -866,7 +867,7 @@ __device__ __forceinline__ CellOut continuity(const StepArgs& A, const float* QX
     const float total = h0 + inc;
     C.hn = fmax32(total, 0.0f);
     A.res[k] = total > 0.0f ? inc - (total - h0) : 0.0f;
-    h_next[k] = C.hn;
+    if (!prescribed) h_next[k] = C.hn;
     const float hcv = HC[local];
     C.hc = hcv;
     if (hcv <= 0.0f) {
@@ -1083,7 +1084,7 @@ struct UpdateStrip {
 
 // A unit of the resident loop, a strip of H rows of a tile: where it lies, and its run's settings.
 struct Unit {
-    int t, run, ts, tj, ti, row0, b0, b1;
+    int t, run, ts, tj, ti, row0;
 };
 struct UnitStep {
     float dt, dx;
@@ -1101,8 +1102,6 @@ __device__ __forceinline__ Unit unit_place(const StepArgs& A, int u) {
     U.tj = A.tiles[2 * U.t];
     U.ti = A.tiles[2 * U.t + 1];
     U.row0 = (u % PER) * H;
-    U.b0 = A.bstart ? A.bstart[U.t] : 0;
-    U.b1 = A.bstart ? A.bstart[U.t + 1] : 0;
     return U;
 }
 
@@ -1110,12 +1109,14 @@ __device__ __forceinline__ UnitStep unit_step(const StepArgs& A, const StepView&
     return UnitStep{__ldcg(V.dtf + run), A.R.dx[run], __ldcg(V.flags + run), __ldcg(V.parity + run)};
 }
 
-// The update of one strip with its boundary cells of a prescribed depth and its envelope; the update pass's arithmetic.
-// What does not depend on the copies (the boundary items, the envelope's entries) is loaded while they land. False: they
-// did not land (reported; the caller leaves).
-template <int H>
+// The update of one strip with its envelope; the update pass's arithmetic. leave: the depths of a boundary cell (bmark) are
+// left to whoever takes it (boundary_items), so that neither waits for the other. What does not depend on the copies (the
+// marks, the envelope's entries, and `meanwhile`) is done while they land. False: they did not land (reported; the caller
+// leaves).
+template <int H, class Meanwhile>
 __device__ __forceinline__ bool update_unit(const UpdateMaps& M, const StepArgs& A, const StepView& V, float* sm,
-                                            uint64_t* bar, uint32_t& phase, const Unit& U, const UnitStep& S) {
+                                            uint64_t* bar, uint32_t& phase, const Unit& U, const UnitStep& S, bool leave,
+                                            Meanwhile meanwhile) {
     using L = UpdateStrip<H>;
     const int tid = threadIdx.x, px = A.px;
     const float dt = S.dt, area = S.dx * S.dx;
@@ -1141,24 +1142,18 @@ __device__ __forceinline__ bool update_unit(const UpdateMaps& M, const StepArgs&
             case 7: bulk_load(sm + L::LR, A.lrow + fid0, TILE * H, bar); break;
         }
     }
-    // this thread's boundary item, if any: one of the tile's whose cell lies in the strip
-    int item = -1;
-    if (tid < U.b1 - U.b0) {
-        const int m = A.bitem[U.b0 + tid];
-        const int row = A.bcell[m] / px - GY - U.tj * TILE - U.row0;
-        if (A.bkind[m] < 2 && row >= 0 && row < H) item = m;
-    }
     const bool mine = tid < H * TILE;
     EnvelopeIn E[L::CELLS];
-    bool marked[L::CELLS];
-    if (want_max && mine) {
+    uint32_t marked[L::CELLS];
 #pragma unroll
-        for (int c = 0; c < L::CELLS; ++c) {
-            const int cell = tid + RESIDENT_THREADS * c, js = cell >> 5, ii = cell & 31;
-            marked[c] = (A.bmark[U.t * TILE + U.row0 + js] >> ii) & 1u;
-            E[c] = envelope_load(A, (int)fid0 + cell, base + js * px + ii, A.uu[0][n], A.uu[1][n]);
-        }
+    for (int c = 0; c < L::CELLS; ++c) {
+        const int cell = tid + RESIDENT_THREADS * c, js = cell >> 5, ii = cell & 31;
+        marked[c] = mine && A.nb ? (A.bmark[U.t * TILE + U.row0 + js] >> ii) & 1u : 0u;
+        if (mine && want_max) E[c] = envelope_load(A, (int)fid0 + cell, base + js * px + ii, A.uu[0][n], A.uu[1][n]);
     }
+    float time = 0.0f, arrive = 0.0f, deep = 0.0f;
+    if (want_max) time = __ldcg(V.max_time + U.run), arrive = A.ctl->arrive, deep = A.ctl->deep;
+    meanwhile();
     const bool ok = mbar_wait(bar, phase);
     phase ^= 1u;
     if (__syncthreads_or(!ok)) {
@@ -1184,7 +1179,8 @@ __device__ __forceinline__ bool update_unit(const UpdateMaps& M, const StepArgs&
         for (int c = 0; c < L::CELLS; ++c) {
             const int cell = tid + RESIDENT_THREADS * c, js = cell >> 5, ii = cell & 31;
             C[c] = continuity(A, QX1, QY1, HB, rs + (js + 1) * RPAD + (ii + 1), (js + 1) * BOXW + ii + 4, cell,
-                              base + js * px + ii, sm + L::RES, sm + L::SRC, sm + L::HC, A.hh[n], dt, area);
+                              base + js * px + ii, sm + L::RES, sm + L::SRC, sm + L::HC, A.hh[n], dt, area,
+                              leave && marked[c]);
             pr[c] = level_pair(A, pairs_t, LP, LR, cell, C[c].row, fid0 + cell, cell);
         }
 #pragma unroll
@@ -1192,33 +1188,25 @@ __device__ __forceinline__ bool update_unit(const UpdateMaps& M, const StepArgs&
             const int cell = tid + RESIDENT_THREADS * c, k = base + (cell >> 5) * px + (cell & 31);
             float om;
             const float dk = cell_out_level(A, C[c], pr[c], om);
-            A.d[k] = dk;
+            if (!(leave && marked[c])) A.d[k] = dk;
             if (S.flags & F_WAVE) A.om[k] = om;
             any |= C[c].hn > 0.0f;
             if (want_max && !marked[c])
-                envelope_apply(A, (int)fid0 + cell, E[c], dk, C[c].hn, __ldcg(V.max_time + U.run), A.ctl->arrive,
-                               A.ctl->deep);
+                envelope_apply(A, (int)fid0 + cell, E[c], dk, C[c].hn, time, arrive, deep);
         }
     }
     // the strip's cells are written and its image is read; whether any is wet
     const int w = __syncthreads_or(any);
     if ((S.flags & F_WET) && w && tid == 0) atomicOr(A.wet + U.t, 1);
-    if (U.b0 < U.b1) {
-        if (item >= 0) boundary_cell(A, item, n, S.flags, __ldcg(V.max_time + U.run), A.ctl->arrive, A.ctl->deep);
-        for (int x = U.b0 + RESIDENT_THREADS + tid; x < U.b1; x += RESIDENT_THREADS) {
-            const int m = A.bitem[x], row = A.bcell[m] / px - GY - U.tj * TILE - U.row0;
-            if (A.bkind[m] < 2 && row >= 0 && row < H)
-                boundary_cell(A, m, n, S.flags, __ldcg(V.max_time + U.run), A.ctl->arrive, A.ctl->deep);
-        }
-    }
     return true;
 }
 
 // Up to max_steps steps of the device loop in one cooperative launch. A step of the loop's kernels of their own is six
 // dependent launches, which on a few hundred tiles cost more than their work; here it is two grid barriers: the face
-// pass by strips of H rows (first barrier), then the update of the same strips with their boundary cells and envelope,
-// while one CTA of its own forms the next step's settings in the second set (second barrier); that CTA then takes the
-// tally and the lines while the next face pass runs. Boundary cells that follow another (one more barrier) and steps
+// pass by strips of H rows (first barrier), then the update of the same strips with their envelope, the boundary cells
+// shared out over the CTAs, while one CTA of its own forms the next step's settings in the second set (second barrier);
+// that CTA then takes the tally and the lines while the next face pass runs. Where some boundary cell follows another, all
+// of them (one more barrier), and steps
 // that rebuild the lists (two or three more, one step in active_every) come after it. The same arithmetic in the same
 // order for every cell, face and sum as the kernels of their own. What CTAs hand one another between barriers is read
 // past L1 or by bulk copies. Latency bounds it on small grids, so strips of 4 rows (a warp a row and axis) serve the
@@ -1291,18 +1279,29 @@ __global__ void __launch_bounds__(RESIDENT_THREADS, resident_ctas(H))
         } else if (control) {
             next_settings(A, V, step_view(A.R, b ^ 1), any, &ctl->any, grid);
         }
+        // this CTA's boundary cells, before or during its first strip: 32 a CTA (they lie apart in memory, and one SM takes
+        // in few such lines at once), the first ones in the last CTAs, which are those without a strip where there are any
+        bool bounds = !control && A.nb && !follow;
+        auto bound = [&] {
+            if (bounds)
+                boundary_items(A, V, ((tid >> 5) * workers + workers - 1 - (int)blockIdx.x) * 32 + (tid & 31),
+                               workers * RESIDENT_THREADS, host.flags);
+            bounds = false;
+        };
+        if (!units) bound();
         for (int c0 = 0; c0 < units; c0 += UNITS_HELD) {
             const int n = units > UNITS_HELD ? take(c0) : units;
             for (int i = 0; i < n; ++i)
-                if (steps[i].flags & F_RUN)
-                    if (!update_unit<H>(M.u, A, V, sm, &bar, phase, places[i], steps[i])) return;
+                if (!(steps[i].flags & F_RUN))
+                    bound();
+                else if (!update_unit<H>(M.u, A, V, sm, &bar, phase, places[i], steps[i], !follow, bound))
+                    return;
         }
         if (!grid_barrier(grid, ctl, met)) return;
         if (host.flags) {
             if (follow) {
-                const int n = 1 - __ldcg(A.R.parity);
-                for (int m = (int)(blockIdx.x * RESIDENT_THREADS) + tid; m < A.nb; m += gridDim.x * RESIDENT_THREADS)
-                    if (A.bkind[m] >= 2) boundary_cell(A, m, n, host.flags, 0.0f, 0.0f, 0.0f);
+                boundary_items(A, V, (int)(blockIdx.x * RESIDENT_THREADS) + tid, (int)(gridDim.x * RESIDENT_THREADS),
+                               host.flags);
                 if (!grid_barrier(grid, ctl, met)) return;
             }
             if (control && tid == 0) A.R.parity[0] ^= 1;
@@ -1312,7 +1311,7 @@ __global__ void __launch_bounds__(RESIDENT_THREADS, resident_ctas(H))
         const int rebuild = __ldcg(&grid->rebuild);
         if (tid < units && units <= UNITS_HELD) steps[tid] = unit_step(A, step_view(A.R, b ^ 1), places[tid].run);
         if (follow) {
-            boundary_items(A, V, (int)(blockIdx.x * RESIDENT_THREADS) + tid, (int)(gridDim.x * RESIDENT_THREADS), 2);
+            boundary_items(A, V, (int)(blockIdx.x * RESIDENT_THREADS) + tid, (int)(gridDim.x * RESIDENT_THREADS));
             if (!grid_barrier(grid, ctl, met)) return;
         }
         if (control) tally_items(A, V, tid, RESIDENT_THREADS);
@@ -1522,7 +1521,7 @@ __global__ void __launch_bounds__(TILE2, 2) step_end_kernel(StepArgs A) {
     if (any & ANY_RUN) {
         const StepView V = step_view(A.R, 0);
         const int gtid = blockIdx.x * TILE2 + threadIdx.x, gstride = gridDim.x * TILE2;
-        boundary_items(A, V, gtid, gstride, 0);
+        boundary_items(A, V, gtid, gstride);
         // (from the other end, so that few threads have both a boundary cell and a tally face)
         tally_items(A, V, (gridDim.x - 1 - blockIdx.x) * TILE2 + threadIdx.x, gstride);
     }
@@ -1562,7 +1561,7 @@ __global__ void boundary_kernel(StepArgs A) {
     grid_open();
     grid_wait();
     if (!(*A.any & ANY_RUN)) return;
-    boundary_items(A, step_view(A.R, 0), blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, 0);
+    boundary_items(A, step_view(A.R, 0), blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
     __syncthreads();
     GridState* grid = grid_state(A.ctl);
     if (threadIdx.x == 0 && atomicAdd(&grid->left, 1u) == gridDim.x - 1) {
