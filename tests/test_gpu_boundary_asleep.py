@@ -89,3 +89,26 @@ def test_host_steps_agree(kinds):
 
     for a, b in zip(go(True), go(False), strict=True):
         assert np.array_equal(a, b)
+
+
+def test_cells_set_again():
+    """Sets with and without following cells, one after the other, and none."""
+
+    def go(timed: bool):
+        m, _ = _model((0, 1, 2))
+        b, ms, states = m.backend, (ctypes.c_float * 3)(), []
+        every = b.bc
+        few = np.nonzero(every.kind < 2)[0]
+        own = BoundaryCells(*(getattr(every, f)[few] for f in ("cell", "ref", "kind", "d0", "h0")))
+        for bc in (every, own, BoundaryCells.empty(), every):
+            b.set_boundary(bc)
+            for s in range(3):
+                if timed:
+                    _lib.call("w2b_step_timed", b.handle, 0.2, int(s == 0), 0, b._stream(), ms)
+                else:
+                    b.step(0.2, s == 0, False)
+            states += _state(m)
+        return states
+
+    for a, b in zip(go(True), go(False), strict=True):
+        assert np.array_equal(a, b)

@@ -1,8 +1,8 @@
 // extern "C" entry points of libwadi_b200 (declared in include/wadi_b200.h) and the host side of the handle.
 //
 // The handle binds caller-owned device buffers; the only memory it allocates is its own host record (with a pinned copy
-// of the run table for the loop's read-back), the CUDA graphs of the device loop and the index of the boundary cells. Ping-pong pairs (h, u, v, mx, my) are resolved through the handle's parity, which
-// flips after every step: the reference swaps its arrays the same way (wadi2d/solver/gpu/backend.py:185-188).
+// of the run table for the loop's read-back) and the CUDA graphs of the device loop. Ping-pong pairs (h, u, v, mx, my) are
+// resolved through the handle's parity, which flips after every step: the reference swaps its arrays the same way (wadi2d/solver/gpu/backend.py:185-188).
 #include <cmath>
 #include <cstddef>
 #include <cstdio>
@@ -82,7 +82,6 @@ __global__ void native_to_ref_kernel(const float* nat, float* ref, const int32_t
 __global__ void pack_tables_kernel(const float* dtab, const float* ftabx, const float* ftaby, float2* dtab2,
                                    float4* fx, float4* fy, int ntiles, int rows);
 __global__ void bmark_kernel(StepArgs A, int clear_words);
-__global__ void boundary_index_kernel(StepArgs A, int32_t* start, int32_t* item, int32_t* next);
 
 // A launch configuration of the device loop: the face pass's form (whole tiles, or the strip form: half tiles in
 // smaller CTAs), its CTAs a SM, the update pass's CTAs a SM, and loop steps a launch: a captured graph of the passes'
@@ -154,8 +153,6 @@ struct Handle {
     int faces_occ = 2, update_occ = 1;  // resident CTAs a SM of the two passes
     int strips16_occ = 4, strips8_occ = 8;  // resident CTAs a SM of the face pass's strip forms
     int resident_occ[3] = {1, 1, 1};  // and of the resident loop's, in the order of RESIDENT_ROWS
-    int32_t *bstart = nullptr, *bitem = nullptr;  // the boundary cells by tile (StepArgs::bstart, bitem)
-    int bitem_held = 0;
     char* host = nullptr;  // pinned: the run table and the control block as read back, and a batch's clocks and ends
     TMaps tmaps;
     ResidentMaps rmaps[3];
@@ -224,8 +221,6 @@ static StepArgs make_args(const Handle& H) {
     A.bkind = H.bkind;
     A.bd0 = H.bd0;
     A.bh0 = H.bh0;
-    A.bstart = H.nb ? H.bstart : nullptr;
-    A.bitem = H.bitem;
     A.ntally = H.ntally;
     A.tface = H.tface;
     A.taxis = H.taxis;
@@ -690,8 +685,6 @@ int32_t w2b_destroy(void* handle) {
         if (e) cudaEventDestroy(e);
     if (H->cap) cudaStreamDestroy(H->cap);
     if (H->host) cudaFreeHost(H->host);
-    if (H->bstart) cudaFree(H->bstart);
-    if (H->bitem) cudaFree(H->bitem);
     delete H;
     return W2B_OK;
 }
@@ -739,14 +732,6 @@ int32_t w2b_set_boundary(void* handle, int32_t n, const int32_t* cell, const int
                          const float* d0, const float* h0) {
     if (!handle || n < 0 || (n && (!cell || !ref || !kind || !d0 || !h0))) return W2B_EINVAL;
     Handle* H = static_cast<Handle*>(handle);
-    if (n && !H->bstart) CK(cudaMalloc(&H->bstart, sizeof(int32_t) * (2 * (size_t)H->g.ntiles + 2)));
-    if (n > H->bitem_held) {  // the index may be in use by steps in flight: cudaFree waits for them
-        if (H->bitem) CK(cudaFree(H->bitem));
-        H->bitem = nullptr;
-        H->bitem_held = 0;
-        CK(cudaMalloc(&H->bitem, sizeof(int32_t) * (size_t)n));
-        H->bitem_held = n;
-    }
     H->nb = n;
     H->bcell = cell;
     H->bref = ref;
@@ -756,10 +741,7 @@ int32_t w2b_set_boundary(void* handle, int32_t n, const int32_t* cell, const int
     H->version++;
     const StepArgs A = make_args(*H);
     bmark_kernel<<<64, 256>>>(A, H->g.ntiles * TILE);
-    if (n) {
-        bmark_kernel<<<64, 256>>>(A, 0);
-        boundary_index_kernel<<<1, 1024>>>(A, H->bstart, H->bitem, H->bstart + H->g.ntiles + 2);
-    }
+    if (n) bmark_kernel<<<64, 256>>>(A, 0);
     CKL("w2b_set_boundary");
     return W2B_OK;
 }

@@ -44,7 +44,10 @@ struct GridState {
     int32_t rebuild;
 };
 constexpr int GRID_STATE_AT = 512;
-static_assert(sizeof(Ctl) <= GRID_STATE_AT && GRID_STATE_AT + sizeof(GridState) <= W2B_CTL_BYTES,
+// And on another line: whether some boundary cell follows another (bmark_kernel).
+constexpr int FOLLOW_AT = 768;
+static_assert(sizeof(Ctl) <= GRID_STATE_AT && GRID_STATE_AT + sizeof(GridState) <= FOLLOW_AT &&
+                  FOLLOW_AT + sizeof(int32_t) <= W2B_CTL_BYTES,
               "control block too large");
 
 constexpr uint32_t ANY_RUN = 1u, ANY_WAVE = 2u, ANY_ACT = 4u, ANY_MAX = 8u;
@@ -172,10 +175,6 @@ struct StepArgs {
     const int32_t* __restrict__ bkind;
     const float* __restrict__ bd0;
     const float* __restrict__ bh0;
-    // the boundary cells by tile: tile t's are bitem[bstart[t] .. bstart[t + 1]); bstart[ntiles + 1]: whether any
-    // follows another cell. Null without boundary cells.
-    const int32_t* __restrict__ bstart;
-    const int32_t* __restrict__ bitem;
     int32_t ntally;
     const int32_t* __restrict__ tface;
     const int32_t* __restrict__ taxis;

@@ -21,6 +21,9 @@ constexpr uint32_t GRID_WAIT_LIMIT = 1u << 21;  // polls of a barrier before a C
 __device__ __forceinline__ GridState* grid_state(Ctl* ctl) {
     return reinterpret_cast<GridState*>(reinterpret_cast<char*>(ctl) + GRID_STATE_AT);
 }
+__device__ __forceinline__ int32_t* follow_flag(Ctl* ctl) {
+    return reinterpret_cast<int32_t*>(reinterpret_cast<char*>(ctl) + FOLLOW_AT);
+}
 
 // Every CTA of a cooperative launch: what each wrote before it, in either proxy's eyes, is what all read after it.
 // met: this launch's arrivals so far, the same in every CTA. False: some CTA did not come in time (reported; the

@@ -1241,7 +1241,7 @@ __global__ void __launch_bounds__(RESIDENT_THREADS, resident_ctas(H))
     uint32_t any = host.flags ? ANY_RUN : ctl->any;
     int nwork = host.flags ? host.tiles : ctl->nwork, mst = ctl->m_stored, b = 0;
     bool moved = true;  // the work list is not the one `places` was taken from
-    const bool follow = A.bstart && A.bstart[A.ntiles + 1];
+    const bool follow = A.nb && *follow_flag(ctl);
     for (int step = 0; step < max_steps && (any & ANY_RUN); ++step) {
         const StepView V = step_view(A.R, b);
         const int left = PER * nwork - (int)blockIdx.x;
@@ -1732,42 +1732,19 @@ __global__ void pack_tables_kernel(const float* __restrict__ dtab, const float* 
     }
 }
 
-// The boundary cells by tile (StepArgs::bstart, bitem), from their NATIVE indices: counts, their running sum, then the
-// items; next: ntiles ints of scratch. One CTA of 1024 threads.
-__global__ void __launch_bounds__(1024) boundary_index_kernel(StepArgs A, int32_t* start, int32_t* item, int32_t* next) {
-    __shared__ int sums[32];
-    const int nt = A.ntiles, tid = threadIdx.x;
-    for (int t = tid; t < nt + 2; t += blockDim.x) start[t] = 0;
-    __syncthreads();
-    for (int m = tid; m < A.nb; m += blockDim.x) {
-        atomicAdd(start + tile_of_native(A, A.bcell[m]), 1);
-        if (A.bkind[m] > 1) start[nt + 1] = 1;
-    }
-    __syncthreads();
-    int before = 0;
-    for (int base = 0; base < nt; base += blockDim.x) {
-        const int t = base + tid;
-        const int n = t < nt ? start[t] : 0;
-        int total;
-        const int o = before + block_scan(n, sums, &total);
-        if (t < nt) start[t] = next[t] = o;
-        before += total;
-    }
-    if (tid == 0) start[nt] = before;
-    __syncthreads();
-    for (int m = tid; m < A.nb; m += blockDim.x) item[atomicAdd(next + tile_of_native(A, A.bcell[m]), 1)] = m;
-}
-
-// Boundary marks: clear, then one bit per boundary cell.
+// Boundary marks: clear, then one bit per boundary cell; and whether some of them follows another.
 __global__ void bmark_kernel(StepArgs A, int clear_words) {
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t* mark = const_cast<uint32_t*>(A.bmark);
+    int32_t* follow = follow_flag(A.ctl);
     if (clear_words > 0) {
+        if (tid == 0) *follow = 0;
         for (int w = tid; w < clear_words; w += gridDim.x * blockDim.x) mark[w] = 0u;
         return;
     }
     for (int m = tid; m < A.nb; m += gridDim.x * blockDim.x) {
         const int fid = fid_of_native(A, A.bcell[m]);
+        if (A.bkind[m] > 1) *follow = 1;
         atomicOr(mark + fid / TILE, 1u << (fid % TILE));
     }
 }
