@@ -100,7 +100,7 @@ typedef struct {
     int32_t *wet;
     int32_t *keep;    /* tiles kept active whatever the water: sources and boundaries */
     int32_t *idle;    /* checks in a row a tile was not wanted */
-    int32_t *is_act;  /* 1 on active tiles */
+    int32_t *is_act;  /* 1 on active tiles (w2b_set_active writes it) */
     int32_t *woken;   /* tiles that joined the list at the last rebuild */
     int32_t *work;    /* the device loop's work list: active tiles of the runs still stepping */
     int32_t *scratch; /* 2 * ntiles */
@@ -185,7 +185,8 @@ int32_t w2b_set_params(void* handle, const W2BParams* params);
 int32_t w2b_pack_tables(const W2BGridDesc* grid, const float* dtab, const float* ftabx, const float* ftaby,
                         float* dtab2, float* ftab4x, float* ftab4y, void* stream);
 
-/* Replaces set_active (wadi2d/solver/gpu/backend.py:116-119): tiles is a device array of n tile ids. */
+/* Replaces set_active (wadi2d/solver/gpu/backend.py:116-119): tiles is a device array of n tile ids. The list and the
+ * tiles' flags (W2BBuffers.is_act) both follow it. */
 int32_t w2b_set_active(void* handle, const int32_t* tiles, int32_t n, void* stream);
 
 /* Replaces set_boundary (wadi2d/solver/gpu/backend.py:127-132). Device arrays of n entries; cell and ref are NATIVE
@@ -225,7 +226,9 @@ int32_t w2b_refresh_plan(void* handle, const int32_t* tiles, int32_t n, void* st
  * step started from, so the next step forms it from the other half of the mean depth pair and the face velocity
  * instead of reading it (12 bytes a cell less HBM traffic a step, the same bits). Before reading or writing U, V, MX,
  * MY (or their other halves) through this pointer, call w2b_sync_momentum on the stream that will access them; the
- * next step then starts from the arrays, written or not. MX1 and MY1 (the other halves) hold nothing between steps. */
+ * next step then starts from the arrays, written or not. MX1 and MY1 (the other halves) hold nothing between steps.
+ * Fetch the pointer of H, U or V again before each write after a step, even where it is the same: the next step after
+ * this call puts what it finds in the sleeping tiles into the other halves too, where they would find it later. */
 int32_t w2b_field_ptr(void* handle, int32_t field, float** out);
 
 /* The face momenta into their arrays (the current half of every run) and a record that the next step starts from

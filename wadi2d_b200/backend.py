@@ -286,7 +286,7 @@ class B200Backend:
 
     def native(self, name: str):
         """The current device tensor of a field, NATIVE layout (for the velocities and momenta, with the momenta put in
-        their arrays first: w2b_sync_momentum)."""
+        their arrays first: w2b_sync_momentum). Asked for again before each write after a step (w2b_field_ptr)."""
         if name in MOMENTUM_FIELDS:
             self.sync_momentum()
         p = ctypes.c_void_p()
@@ -336,6 +336,8 @@ class B200Backend:
         if self._held is not None and np.array_equal(active, self._held):
             self.active_tiles, self.nact = active, int(active.size)
             return
+        if active.size and not 0 <= int(active.min()) <= int(active.max()) < self.grid.ntiles:
+            raise IndexError(f"set_active: tiles outside [0, {self.grid.ntiles})")
         self._held = active.copy()
         self.active_tiles = active
         self.nact = int(self.active_tiles.size)
@@ -343,9 +345,6 @@ class B200Backend:
         act = self._t["active"]
         if self.nact:
             act[: self.nact] = torch.as_tensor(self.active_tiles, device=self.device)
-        flags = np.zeros(self.grid.ntiles, np.int32)
-        flags[self.active_tiles] = 1
-        self._t["is_act"].copy_(torch.as_tensor(flags, device=self.device))
         _lib.call("w2b_set_active", self.handle, act.data_ptr(), self.nact, self._stream())
 
     @property

@@ -82,6 +82,7 @@ __global__ void native_to_ref_kernel(const float* nat, float* ref, const int32_t
 __global__ void pack_tables_kernel(const float* dtab, const float* ftabx, const float* ftaby, float2* dtab2,
                                    float4* fx, float4* fy, int ntiles, int rows);
 __global__ void bmark_kernel(StepArgs A, int clear_words);
+__global__ void active_flags_kernel(StepArgs A, int n);
 
 // A launch configuration of the device loop: the face pass's form (whole tiles, or the strip form: half tiles in
 // smaller CTAs), its CTAs a SM, the update pass's CTAs a SM, and loop steps a launch: a captured graph of the passes'
@@ -435,7 +436,7 @@ static size_t host_bytes(int nruns) {
 
 // Before steps: the sleeping tiles' other halves, if a caller may have written their current ones.
 static int settle_asleep(Handle& H, cudaStream_t s) {
-    if (H.touched && H.nact < H.g.ntiles - 1) {
+    if (H.touched && H.B.is_act && H.nact < H.g.ntiles - 1) {
         launch_asleep(make_args(H), H.sms, s);
         CKL("sleeping tiles");
     }
@@ -725,6 +726,8 @@ int32_t w2b_set_active(void* handle, const int32_t* tiles, int32_t n, void* stre
     if (n && tiles != H->B.active)
         CK(cudaMemcpyAsync(H->B.active, tiles, sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, s));
     H->nact = n;
+    if (H->B.is_act) active_flags_kernel<<<1, 1024, 0, s>>>(make_args(*H), n);
+    CKL("w2b_set_active");
     return W2B_OK;
 }
 

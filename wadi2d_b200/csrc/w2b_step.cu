@@ -1732,6 +1732,16 @@ __global__ void pack_tables_kernel(const float* __restrict__ dtab, const float* 
     }
 }
 
+// The flags of the active list's tiles (is_act). One CTA; a list entry outside the tiles is passed over.
+__global__ void __launch_bounds__(1024) active_flags_kernel(StepArgs A, int n) {
+    for (int t = threadIdx.x; t < A.ntiles; t += blockDim.x) A.is_act[t] = 0;
+    __syncthreads();
+    for (int a = threadIdx.x; a < n; a += blockDim.x) {
+        const int t = A.active[a];
+        if (t >= 0 && t < A.ntiles) A.is_act[t] = 1;
+    }
+}
+
 // Boundary marks: clear, then one bit per boundary cell; and whether some of them follows another.
 __global__ void bmark_kernel(StepArgs A, int clear_words) {
     const int tid = blockIdx.x * blockDim.x + threadIdx.x;
