@@ -231,6 +231,9 @@ int32_t w2b_refresh_plan(void* handle, const int32_t* tiles, int32_t n, void* st
  * this call puts what it finds in the sleeping tiles into the other halves too, where they would find it later. */
 int32_t w2b_field_ptr(void* handle, int32_t field, float** out);
 
+/* The same pointer for reading only: the next step does not go over the sleeping tiles for it. */
+int32_t w2b_field_read(void* handle, int32_t field, const float** out);
+
 /* The face momenta into their arrays (the current half of every run) and a record that the next step starts from
  * them (no work if they are there already). No counterpart in the reference, which stores the momenta every step.
  * In a batch, a momentum written for a run that does not step at the next loop step is formed from the state again

@@ -80,19 +80,16 @@ class Field:
     def __init__(self, backend: B200Backend, name: str) -> None:
         self.b, self.name = backend, name
 
-    def _tensor(self):
-        return self.b.native(self.name)
-
     def _index(self, idx):
         if isinstance(idx, slice) or idx is Ellipsis:
             raise TypeError("index a state field with reference state indices, or use get_field/set_field")
         return self.b.torch.as_tensor(native_of_ref(self.b.grid.tiles, idx, self.b.grid.shape[1]), device=self.b.device)
 
     def __getitem__(self, idx) -> np.ndarray:
-        return self._tensor()[self._index(idx)].cpu().numpy()
+        return self.b.reading(self.name)[self._index(idx)].cpu().numpy()
 
     def __setitem__(self, idx, value) -> None:
-        t = self._tensor()
+        t = self.b.native(self.name)
         t[self._index(idx)] = self.b.torch.as_tensor(np.asarray(value, np.float32), device=self.b.device)
 
     def __array__(self, dtype=None, copy=None):
@@ -287,10 +284,17 @@ class B200Backend:
     def native(self, name: str):
         """The current device tensor of a field, NATIVE layout (for the velocities and momenta, with the momenta put in
         their arrays first: w2b_sync_momentum). Asked for again before each write after a step (w2b_field_ptr)."""
+        return self._current("w2b_field_ptr", name)
+
+    def reading(self, name: str):
+        """``native`` for reading only: the next step does not look for what was written into sleeping tiles."""
+        return self._current("w2b_field_read", name)
+
+    def _current(self, entry: str, name: str):
         if name in MOMENTUM_FIELDS:
             self.sync_momentum()
         p = ctypes.c_void_p()
-        _lib.call("w2b_field_ptr", self.handle, _lib.FIELD_ID[name], ctypes.byref(p))
+        _lib.call(entry, self.handle, _lib.FIELD_ID[name], ctypes.byref(p))
         half = self._half_at.get(p.value)
         return self._t[name] if half is None else half
 

@@ -899,11 +899,20 @@ int32_t w2b_cell_size(void* handle, float* dx) {
     return W2B_OK;
 }
 
-int32_t w2b_field_ptr(void* handle, int32_t field, float** out) {
+int32_t w2b_field_read(void* handle, int32_t field, const float** out) {
     if (!handle || !out) return W2B_EINVAL;
-    float* p = field_ptr(static_cast<Handle*>(handle), field);
+    const float* p = field_ptr(static_cast<Handle*>(handle), field);
     if (!p) return W2B_EINVAL;
     *out = p;
+    return W2B_OK;
+}
+
+int32_t w2b_field_ptr(void* handle, int32_t field, float** out) {
+    if (!handle || !out) return W2B_EINVAL;
+    const float* p = nullptr;
+    const int st = w2b_field_read(handle, field, &p);
+    if (st != W2B_OK) return st;
+    *out = const_cast<float*>(p);
     if (field == W2B_H || field == W2B_U || field == W2B_V) static_cast<Handle*>(handle)->touched = true;
     return W2B_OK;
 }
