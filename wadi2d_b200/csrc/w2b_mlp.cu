@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2) mlp_train_kernel(const __grid
             for (int x = blockIdx.x; x < tiles && ok; x += gridDim.x) {
                 int tile;
                 const W2BMlpOp& G = mlp_op(P, x, tile);
-                ok = mlp_tile<TM>(C, G, tile, step0 + it, staged && x == (int)blockIdx.x, T.status);
+                ok = mlp_tile<TM>(C, G, tile, G.step ? step0 + it : 0, staged && x == (int)blockIdx.x, T.status);
             }
             if (ok && g == T.groups - 1 && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
                 double s = 0.0;
@@ -673,18 +673,21 @@ int32_t w2b_mlp_train(const W2BMlpOp* ops, const int32_t* sizes, int32_t launche
     try {
         std::vector<MlpGroup> groups(launches);
         int widest = 1;
+        bool counted = true;  // every product's step is this call's, or none
         for (int l = 0; l < launches; ops += sizes[l], ++l) {
             if (sizes[l] < 1 || sizes[l] > W2B_MLP_OPS_MAX) return W2B_EINVAL;
             const int st = mlp_group(ops, sizes[l], groups[l]);
             if (st != W2B_OK) return st;
+            for (int o = 0; o < sizes[l]; ++o) counted = counted && (!ops[o].step || ops[o].step == step);
             const int tiles = tile_rows(groups[l], 128);
             widest = tiles > widest ? tiles : widest;
         }
         if (!iters) return W2B_OK;
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         if (mlp_status(cudaStreamIsCapturing(s, &cap)) != W2B_OK) return W2B_ECUDA;
-        if (launches <= TRAIN_GROUPS_MAX && cap == cudaStreamCaptureStatusNone) {
-            // one launch of every step; a stream being captured cannot wait for another stream's
+        if (launches <= TRAIN_GROUPS_MAX && counted && cap == cudaStreamCaptureStatusNone) {
+            // one launch of every step, which counts the steps itself; a stream being captured cannot wait for another
+            // stream's
             MlpTrain T;
             memset(&T, 0, sizeof(T));
             memcpy(T.group, groups.data(), sizeof(MlpGroup) * launches);
