@@ -457,7 +457,7 @@ typedef struct {
 int32_t w2b_mlp_ops(const W2BMlpOp* ops, int32_t count, int32_t* status, void* stream);
 /* iters training steps without the host: each the products of `ops` in `launches` launches of sizes[l] products, in
  * order, then w2b_mlp_tick's arithmetic; up to 12 launches a step all in one cooperative launch, where each product's step
- * is NULL or this call's. ops and sizes are host
+ * is NULL or this call's and the last launch has no targets t. ops and sizes are host
  * arrays, read before the call returns. status: 3 device int32, zero at the first call; [0] as above. */
 int32_t w2b_mlp_train(const W2BMlpOp* ops, const int32_t* sizes, int32_t launches, int32_t iters,
                       const double* partial, int32_t n, double count, double* loss, int64_t* step, int32_t* status,

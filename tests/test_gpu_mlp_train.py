@@ -1,5 +1,6 @@
 """w2b_mlp_train through its own interface, against the same products launched one by one (w2b_mlp_ops, w2b_mlp_tick), bit for
-bit: a draw of rows that is the same every step (no step counter), and a step counter that is not the call's."""
+bit: a draw of rows that is the same every step (no step counter), a step counter that is not the call's, and a loss that
+the last launch of a step writes."""
 
 from __future__ import annotations
 
@@ -81,3 +82,12 @@ def test_rows_are_the_step_counters(step):
 
     for a, b in zip(Layer(step).fit(False), Layer(step).fit(True), strict=True):
         assert torch.equal(a, b)
+
+
+def test_a_loss_that_the_last_launch_writes():
+    import torch
+
+    a, b = Layer("own", train=False).fit(False), Layer("own", train=False).fit(True)
+    assert len(set(a[0].tolist())) == ITERS
+    for p, q in zip(a, b, strict=True):
+        assert torch.equal(p, q)

@@ -674,20 +674,24 @@ int32_t w2b_mlp_train(const W2BMlpOp* ops, const int32_t* sizes, int32_t launche
         std::vector<MlpGroup> groups(launches);
         int widest = 1;
         bool counted = true;  // every product's step is this call's, or none
+        bool summed = true;   // no loss in the last launch: its sums are there when that one begins
         for (int l = 0; l < launches; ops += sizes[l], ++l) {
             if (sizes[l] < 1 || sizes[l] > W2B_MLP_OPS_MAX) return W2B_EINVAL;
             const int st = mlp_group(ops, sizes[l], groups[l]);
             if (st != W2B_OK) return st;
-            for (int o = 0; o < sizes[l]; ++o) counted = counted && (!ops[o].step || ops[o].step == step);
+            for (int o = 0; o < sizes[l]; ++o) {
+                counted = counted && (!ops[o].step || ops[o].step == step);
+                summed = summed && !(ops[o].t && l == launches - 1);
+            }
             const int tiles = tile_rows(groups[l], 128);
             widest = tiles > widest ? tiles : widest;
         }
         if (!iters) return W2B_OK;
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         if (mlp_status(cudaStreamIsCapturing(s, &cap)) != W2B_OK) return W2B_ECUDA;
-        if (launches <= TRAIN_GROUPS_MAX && counted && cap == cudaStreamCaptureStatusNone) {
-            // one launch of every step, which counts the steps itself; a stream being captured cannot wait for another
-            // stream's
+        if (launches <= TRAIN_GROUPS_MAX && counted && summed && cap == cudaStreamCaptureStatusNone) {
+            // one launch of every step, which counts the steps itself and adds up the loss beside the last group; a stream
+            // being captured cannot wait for another stream's
             MlpTrain T;
             memset(&T, 0, sizeof(T));
             memcpy(T.group, groups.data(), sizeof(MlpGroup) * launches);
