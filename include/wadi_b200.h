@@ -9,7 +9,9 @@
  * Status codes (every call returns one):
  *   W2B_OK 0, W2B_EINVAL -1 (bad argument), W2B_ECUDA -2 (a CUDA call failed), W2B_ENONFINITE -3 (a non-finite
  *   wave speed: the reference's NumericalFailure, wadi2d/solver/stepper.py:116-118), W2B_EDTMIN -4 (the step fell
- *   below dt_min, wadi2d/solver/stepper.py:119-123), W2B_ETIMEOUT -5 (a bounded device wait gave up).
+ *   below dt_min, wadi2d/solver/stepper.py:119-123), W2B_ETIMEOUT -5 (a bounded device wait gave up: the state is torn.
+ *   w2b_advance reports it by itself, a host-driven step through the next w2b_max_wave, and from every one after it; the
+ *   next w2b_advance begins anew, from whatever state the caller has put back).
  *
  * Layouts. REF_TILE is the reference's tile-with-halo state layout (wadi2d/solver/layout.py:19-50): ntiles * 1296
  * floats, tile t, row j, column i (2-cell halo). NATIVE is this library's dense layout: the padded grid with GY guard
@@ -458,7 +460,7 @@ int32_t w2b_mlp_ops(const W2BMlpOp* ops, int32_t count, int32_t* status, void* s
 /* iters training steps without the host: each the products of `ops` in `launches` launches of sizes[l] products, in
  * order, then w2b_mlp_tick's arithmetic; up to 12 launches a step all in one cooperative launch, where each product's step
  * is NULL or this call's and the last launch has no targets t. ops and sizes are host
- * arrays, read before the call returns. status: 3 device int32, zero at the first call; [0] as above. */
+ * arrays, read before the call returns. status: 3 device int32, zero at the first call and to begin again after W2B_ETIMEOUT; [0] as above. */
 int32_t w2b_mlp_train(const W2BMlpOp* ops, const int32_t* sizes, int32_t launches, int32_t iters,
                       const double* partial, int32_t n, double count, double* loss, int64_t* step, int32_t* status,
                       void* stream);

@@ -488,11 +488,6 @@ static int launch_loop_step(Handle& H, const LoopConfig& C, int k, int steps, cu
     return W2B_OK;
 }
 
-// After a wait gave up: the grid barrier's counters may be anything.
-static cudaError_t clear_grid(Handle& H, cudaStream_t s) {
-    return cudaMemsetAsync(reinterpret_cast<char*>(H.ctl()) + GRID_STATE_AT, 0, sizeof(GridState), s);
-}
-
 cudaError_t launch_in_turn(const void* kernel, int grid, int block, void** params, size_t smem, cudaStream_t s) {
     static struct {
         std::mutex mutex;
@@ -845,7 +840,10 @@ int32_t w2b_max_wave(void* handle, float* out, void* stream) {
     CK(cudaStreamSynchronize((cudaStream_t)stream));
     memcpy(out, held, sizeof(float));
     if (held[1] != W2B_ETIMEOUT) return W2B_OK;
-    clear_grid(*H, (cudaStream_t)stream);
+    // the device's half: a step that gave up, and one that a failure kept from beginning, swapped nothing there
+    CK(cudaMemcpyAsync(held, H->R.parity, sizeof(int32_t), cudaMemcpyDeviceToHost, (cudaStream_t)stream));
+    CK(cudaStreamSynchronize((cudaStream_t)stream));
+    H->cur = held[0];
     return W2B_ETIMEOUT;
 }
 
@@ -1177,7 +1175,6 @@ static int advance_runs(Handle* H, const W2BStepper* cfg, const double* t_end, i
         if (done) break;
     }
     const int32_t gstatus = hctl->status;
-    if (gstatus) CK(clear_grid(*H, s));
     H->nact = hctl->nact;
     H->cur = T.parity[0];
     int32_t first = gstatus;

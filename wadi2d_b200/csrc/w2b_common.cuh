@@ -38,10 +38,13 @@ struct Ctl {
     int32_t m_stored;
 };
 // Behind it in the control block, on a line of its own: the resident loop's grid barrier (arrivals, counted up, and the
-// CTAs that have left; zero between launches) and whether the step in flight ends with a rebuild of the lists.
+// CTAs that have left; zero between launches, unless a wait gave up: then Ctl::status says so and no resident launch
+// begins until they are cleared), whether the step in flight ends with a rebuild of the lists, and the CTAs that are done
+// in a kernel that waits for nothing.
 struct GridState {
     uint32_t arrived, left;
     int32_t rebuild;
+    uint32_t done;
 };
 constexpr int GRID_STATE_AT = 512;
 // And on another line: whether some boundary cell follows another (bmark_kernel).

@@ -410,6 +410,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 2) mlp_train_kernel(const __grid
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t tmem_base;
     __shared__ double red[TM / 64 * (GEMM_THREADS / 32)];
+    if (*T.status) return;  // a wait before this launch gave up: the barrier's counters may be anything
     MlpCta C{smem, &bar, red};
     mlp_begin(C, &tmem_base);
     const int64_t step0 = *T.step;

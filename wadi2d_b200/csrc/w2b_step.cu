@@ -1242,6 +1242,7 @@ __global__ void __launch_bounds__(RESIDENT_THREADS, resident_ctas(H))
     int nwork = host.flags ? host.tiles : ctl->nwork, mst = ctl->m_stored, b = 0;
     bool moved = true;  // the work list is not the one `places` was taken from
     const bool follow = A.nb && *follow_flag(ctl);
+    if (ctl->status) return;  // a wait before this launch gave up: the barrier's counters may be anything
     for (int step = 0; step < max_steps && (any & ANY_RUN); ++step) {
         const StepView V = step_view(A.R, b);
         const int left = PER * nwork - (int)blockIdx.x;
@@ -1467,9 +1468,9 @@ __global__ void __launch_bounds__(256) momentum_kernel(StepArgs A) {
     }
     __syncthreads();
     GridState* grid = grid_state(A.ctl);
-    if (threadIdx.x == 0 && atomicAdd(&grid->left, 1u) == gridDim.x - 1) {
+    if (threadIdx.x == 0 && atomicAdd(&grid->done, 1u) == gridDim.x - 1) {
         A.ctl->m_stored = 1;
-        grid->left = 0;
+        grid->done = 0;
     }
 }
 
@@ -1564,9 +1565,9 @@ __global__ void boundary_kernel(StepArgs A) {
     boundary_items(A, step_view(A.R, 0), blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
     __syncthreads();
     GridState* grid = grid_state(A.ctl);
-    if (threadIdx.x == 0 && atomicAdd(&grid->left, 1u) == gridDim.x - 1) {
+    if (threadIdx.x == 0 && atomicAdd(&grid->done, 1u) == gridDim.x - 1) {
         A.R.parity[0] ^= 1;
-        grid->left = 0;
+        grid->done = 0;
     }
 }
 
@@ -1614,6 +1615,9 @@ __global__ void __launch_bounds__(1024) begin_kernel(const __grid_constant__ Ste
     if (threadIdx.x == 0) {
         c.m_stored = A.ctl->m_stored;
         *A.ctl = c;
+        GridState* grid = grid_state(A.ctl);  // whatever a wait that gave up has left
+        grid->arrived = grid->left = 0;
+        grid->rebuild = 0;
     }
     for (int r = threadIdx.x; r < A.nruns; r += blockDim.x) {
         const W2BClock k = clocks ? clocks[r] : one;
