@@ -29,8 +29,8 @@ namespace w2b {
     void launch_strips(int rows, const TMaps& M, const StepArgs& A, int grid, cudaStream_t s); \
     cudaError_t resident_setup();                                                   \
     int resident_occupancy(int rows);                                               \
-    cudaError_t launch_resident(int rows, const ResidentMaps& M, const StepArgs& A, int grid, int max_steps, \
-                                const HostStep& host, cudaStream_t s);
+    cudaError_t launch_resident(int rows, const ResidentMaps& M, const StepArgs& A, int grid, int occupancy, \
+                                int max_steps, const HostStep& host, cudaStream_t s);
 namespace exact {
 W2B_PASSES_DECL
 }
@@ -51,7 +51,8 @@ struct Passes {
     void (*launch_strips)(int, const TMaps&, const StepArgs&, int, cudaStream_t);
     cudaError_t (*resident_setup)();
     int (*resident_occupancy)(int);
-    cudaError_t (*launch_resident)(int, const ResidentMaps&, const StepArgs&, int, int, const HostStep&, cudaStream_t);
+    cudaError_t (*launch_resident)(int, const ResidentMaps&, const StepArgs&, int, int, int, const HostStep&,
+                                   cudaStream_t);
 };
 static const Passes EXACT_PASSES = {exact::faces_setup,  exact::launch_probe,     exact::faces_occupancy,
                                     exact::launch_faces, exact::update_setup,     exact::update_occupancy,
@@ -488,21 +489,94 @@ static int launch_loop_step(Handle& H, const LoopConfig& C, int k, int steps, cu
     return W2B_OK;
 }
 
-cudaError_t launch_in_turn(const void* kernel, int grid, int block, void** params, size_t smem, cudaStream_t s) {
-    static struct {
-        std::mutex mutex;
-        cudaEvent_t last = nullptr;
-    } lanes[64];
+// Cooperative launches on one device, whatever their streams: one may start beside others in flight only where all their
+// CTAs are sure to find a place, for CTAs that wait at a grid barrier hold theirs until the last has come. A CTA of a kernel
+// of which k are resident a SM takes at most 1 / k of everything a SM has, so a launch takes its CTAs / k SMs in all. While
+// the launches in flight and this one take at most (1 - w) of the SMs together, w the largest 1 / k among them, some SM always
+// has w of itself free, so every CTA finds room, in whatever order they come; with one k for all of them, a SM has room
+// until it holds k CTAs, so they may take all the SMs. Else this launch waits, on the device, for the oldest ones. Calls of 20
+// steps of eight models, a thread and a stream each: 328 us for all eight of 62 x 62 cells, 997 of 126 x 126 (two at a time),
+// where 1,836 and 1,900 with every launch behind the one before it.
+// A launch stands in the list, oldest first, under its stream (the stream's own order keeps it behind the ones before it on
+// that), with what may run until it ends: what it takes, or what those it waits for take.
+namespace {
+struct Flight {
+    unsigned long long stream;
+    cudaEvent_t done;
+    double sms, widest, narrowest;  // the SMs it takes; the largest and the smallest 1 / k
+};
+struct Lane {
+    static constexpr int HELD = 16;
+    std::mutex mutex;
+    Flight held[HELD];
+    cudaEvent_t spare[HELD] = {};
+    int count = 0, spares = 0, sms = 0;
+    void drop(int i) {
+        spare[spares++] = held[i].done;
+        for (--count; i < count; ++i) held[i] = held[i + 1];
+    }
+};
+}  // namespace
+
+cudaError_t launch_in_turn(const void* kernel, int grid, int block, void** params, size_t smem, int per_sm, cudaStream_t s) {
+    static Lane lanes[64];
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-    auto& lane = lanes[dev];
-    std::lock_guard<std::mutex> lock(lane.mutex);
-    e = lane.last ? cudaStreamWaitEvent(s, lane.last, 0) : cudaEventCreateWithFlags(&lane.last, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(block), params, smem, s);
-    if (e == cudaSuccess) e = cudaEventRecord(lane.last, s);
-    return e;
+    if (dev < 0 || dev >= 64 || per_sm < 1) return cudaErrorInvalidValue;
+    Lane& L = lanes[dev];
+    Flight mine = {0, nullptr, (double)grid / per_sm, 1.0 / per_sm, 1.0 / per_sm};
+    e = cudaStreamGetId(s, &mine.stream);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lock(L.mutex);
+    if (!L.sms) e = cudaDeviceGetAttribute(&L.sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    double ahead = 0.0;  // SMs of launches that end before this one starts
+    auto join = [](Flight& to, const Flight& f) {
+        to.widest = f.widest > to.widest ? f.widest : to.widest;
+        to.narrowest = f.narrowest < to.narrowest ? f.narrowest : to.narrowest;
+    };
+    auto behind = [&](int i) {
+        ahead += L.held[i].sms;
+        join(mine, L.held[i]);
+        L.drop(i);
+    };
+    if (L.count > 1 || (L.count == 1 && L.held[0].stream != mine.stream)) {
+        // the launches that have ended leave the list (a query would end another thread's capture in the default mode)
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        for (int i = L.count - 1; i >= 0; --i) {
+            const cudaError_t ended = cudaEventQuery(L.held[i].done);
+            if (ended == cudaSuccess) L.drop(i);
+            if (ended == cudaErrorNotReady) cudaGetLastError();  // not an error to report
+        }
+        cudaThreadExchangeStreamCaptureMode(&mode);
+    }
+    for (int i = L.count - 1; i >= 0; --i)
+        if (L.held[i].stream == mine.stream) behind(i);
+    auto fits = [&] {
+        Flight all = mine;
+        for (int i = 0; i < L.count; ++i) {
+            all.sms += L.held[i].sms;
+            join(all, L.held[i]);
+        }
+        return all.sms <= L.sms * (all.widest == all.narrowest ? 1.0 : 1.0 - all.widest);
+    };
+    while (L.count && (L.count == Lane::HELD || !fits())) {
+        e = cudaStreamWaitEvent(s, L.held[0].done, 0);
+        if (e != cudaSuccess) return e;
+        behind(0);
+    }
+    mine.sms = mine.sms > ahead ? mine.sms : ahead;
+    if (L.spares)
+        mine.done = L.spare[--L.spares];
+    else
+        e = cudaEventCreateWithFlags(&mine.done, cudaEventDisableTiming);
+    if (e != cudaSuccess) return e;
+    e = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(block), params, smem, s);
+    const cudaError_t noted = cudaEventRecord(mine.done, s);  // (of a launch that failed too: it stands for those ahead)
+    L.held[L.count++] = mine;
+    return e != cudaSuccess ? e : noted;
 }
 
 // A launch of the resident loop over up to `tiles` tiles in strips of `rows` rows, at most per_sm CTAs a SM; where there is
@@ -514,7 +588,8 @@ static int launch_resident(Handle& H, const StepArgs& A, int rows, int per_sm, i
     const int64_t most = (int64_t)H.sms * per_sm - 1;
     const int workers = (int)(units < most ? (units > 0 ? units : 1) : most);
     if (workers < 1) return W2B_EINVAL;
-    CK(passes(H.P).launch_resident(rows, H.rmaps[resident_index(rows)], A, workers + 1, max_steps, host, s));
+    const int form = resident_index(rows);
+    CK(passes(H.P).launch_resident(rows, H.rmaps[form], A, workers + 1, H.resident_occ[form], max_steps, host, s));
     return W2B_OK;
 }
 

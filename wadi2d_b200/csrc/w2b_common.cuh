@@ -480,9 +480,9 @@ __device__ __forceinline__ int fid_of_native(const StepArgs& A, int k) {
     return t * TILE2 + (j % TILE) * TILE + (i % TILE);
 }
 
-// A cooperative launch (CTAs that wait for one another). Two such launches of one process must not share a GPU half
-// resident each, so every one waits for the one before it on the device, whatever its stream.
-cudaError_t launch_in_turn(const void* kernel, int grid, int block, void** params, size_t smem, cudaStream_t s);
+// A cooperative launch (CTAs that wait for one another; per_sm of them resident a SM). Two such launches of one process must
+// not share a GPU half resident each, so one that might not fit beside those in flight waits for them on the device.
+cudaError_t launch_in_turn(const void* kernel, int grid, int block, void** params, size_t smem, int per_sm, cudaStream_t s);
 
 // The step arguments of a handle (for kernels of other translation units); false on a null handle.
 bool handle_args(void* handle, StepArgs* out);

@@ -540,8 +540,10 @@ static int launch_train(MlpTrain& T, int iters, int sms, cudaStream_t s) {
         const int tiles = tile_rows(T.group[l], TM);
         widest = tiles > widest ? tiles : widest;
     }
+    // (the largest carveout, as the resident loop's: a SM set up for one of them has room for the other)
     if (cudaFuncSetAttribute(mlp_train_kernel<TM>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_smem(TM)) !=
             cudaSuccess ||
+        cudaFuncSetAttribute(mlp_train_kernel<TM>, cudaFuncAttributePreferredSharedMemoryCarveout, 100) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, mlp_train_kernel<TM>, GEMM_THREADS, gemm_smem(TM)) !=
             cudaSuccess)
         return mlp_status(cudaGetLastError());
@@ -551,7 +553,7 @@ static int launch_train(MlpTrain& T, int iters, int sms, cudaStream_t s) {
         T.iters = iters - done < TRAIN_ITERS_MAX ? iters - done : TRAIN_ITERS_MAX;
         void* params[] = {&T};
         const int st = mlp_status(
-            launch_in_turn((const void*)mlp_train_kernel<TM>, ctas, GEMM_THREADS, params, gemm_smem(TM), s));
+            launch_in_turn((const void*)mlp_train_kernel<TM>, ctas, GEMM_THREADS, params, gemm_smem(TM), occ, s));
         if (st != W2B_OK) return st;
     }
     return W2B_OK;

@@ -1387,15 +1387,15 @@ int resident_occupancy(int rows) {
 }
 
 // Up to max_steps steps in one cooperative launch of `grid` CTAs (at least two, at most as many as are resident at
-// once); the control block's grid state starts at zero.
-cudaError_t launch_resident(int rows, const ResidentMaps& M, const StepArgs& A, int grid, int max_steps,
+// once, `occupancy` a SM); the control block's grid state starts at zero.
+cudaError_t launch_resident(int rows, const ResidentMaps& M, const StepArgs& A, int grid, int occupancy, int max_steps,
                             const HostStep& host, cudaStream_t s) {
     const ResidentForm f = resident_form(rows, A.P.second && A.P.sheet && A.P.mirror && A.P.carry);
     ResidentMaps maps = M;
     StepArgs args = A;
     HostStep step = host;
     void* params[] = {&maps, &args, &max_steps, &step};
-    return launch_in_turn(f.kernel, grid, RESIDENT_THREADS, params, f.smem, s);
+    return launch_in_turn(f.kernel, grid, RESIDENT_THREADS, params, f.smem, occupancy, s);
 }
 
 }  // namespace W2B_ARITH
