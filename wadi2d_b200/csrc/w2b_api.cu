@@ -1128,8 +1128,9 @@ static int launch_chunk(Handle& H, int c, int64_t steps, int64_t* took, cudaStre
 }
 
 // One timed launch of candidate c ran `live` loop steps in `ms`: add it, move to the next candidate, and settle on the
-// fastest once every candidate has its samples.
-static void tune_sample(Handle& H, int c, long long live, float ms) {
+// fastest once every candidate has its samples; then with the graphs of fewer steps that it will take, so that the first
+// call to end in one does not pay for them (222 us of a call of 13 steps of 484 tiles, which takes 663).
+static int tune_sample(Handle& H, int c, long long live, float ms, cudaStream_t s) {
     Loop& L = H.loop;
     if (live > 0) {
         L.sec[c] += 1e-3 * (double)ms;
@@ -1138,7 +1139,7 @@ static void tune_sample(Handle& H, int c, long long live, float ms) {
     }
     L.next = (c + 1) % L.ncand;
     for (int k = 0; k < L.ncand; ++k)
-        if (L.samples[k] < TUNE_SAMPLES) return;
+        if (L.samples[k] < TUNE_SAMPLES) return W2B_OK;
     auto per_step = [&](int k) { return L.sec[k] / (double)(L.steps[k] > 0 ? L.steps[k] : 1); };
     int best = 0;
     for (int k = 1; k < L.ncand; ++k)
@@ -1148,6 +1149,12 @@ static void tune_sample(Handle& H, int c, long long live, float ms) {
     L.tuning = 0;
     for (int k = 0; k < L.ncand; ++k)
         if (k != best) drop_graph(H, k);
+    int st = W2B_OK;
+    for (int tail = 1; tail <= TAILS && st == W2B_OK && !L.cand[best].resident; ++tail) {
+        st = loop_graph(H, best, tail);
+        if (st == W2B_OK) st = cuda_status(cudaGraphUpload(L.exec[best][tail], s), "cudaGraphUpload");
+    }
+    return st;
 }
 
 // The device-resident loop. Steps run in chunks (a captured graph, or one launch of the resident loop), every running
@@ -1234,7 +1241,8 @@ static int advance_runs(Handle* H, const W2BStepper* cfg, const double* t_end, i
             for (int r = 0; r < n; ++r) ran = T.steps_run[r] > ran ? T.steps_run[r] : ran;
             float ms = 0.0f;
             CK(cudaEventElapsedTime(&ms, have_prev ? L.ev[3 - end] : L.ev[0], L.ev[end]));
-            tune_sample(*H, c, ran - ran_before, ms);
+            const int stc = tune_sample(*H, c, ran - ran_before, ms, s);
+            if (stc != W2B_OK) return stc;
             ran_before = ran;
             have_prev = 1;
             end = 3 - end;
