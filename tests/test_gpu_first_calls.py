@@ -44,3 +44,14 @@ def test_the_first_call_after_tuning_takes_what_later_ones_take():
         first.append(call(m))
         later += [call(m) for _ in range(8)]
     assert min(first) < 1.15 * float(np.median(later))
+
+
+@pytest.mark.parametrize("side, tried", [(62, {0, 1}), (1000, {0})])
+def test_the_tuner_leaves_out_what_cannot_win(side, tried):
+    m = _model(side)
+    seen = set()
+    while m.backend.loop_config()["tuning"]:
+        seen.add(m.backend.loop_config()["resident"])
+        m.run(1e9, max_steps=1)
+    assert seen == tried
+    assert m.backend.loop_config()["resident"] in tried

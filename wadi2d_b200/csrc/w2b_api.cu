@@ -1127,10 +1127,28 @@ static int launch_chunk(Handle& H, int c, int64_t steps, int64_t* took, cudaStre
     return W2B_OK;
 }
 
+// Whether the tuner tries candidate k on `nact` active tiles: the resident loop only up to two waves of its strips. Beyond
+// them its launches cost more than the step's kernels everywhere measured, all cells wet, exact (us a step, kernels | 16- | 8-
+// | 4-row strips; waves in brackets): 121 tiles 22.9 | 19.3 (0.8) | 25.5 (1.1) | 25.8 (3.3); 196 26.1 | 30.5 (1.3) | 26.0
+// (1.8) | 35.1 (5.3); 256 28.8 | 31.0 (1.7) | 35.1 (2.3) | 41.2; 484 44.5 | 56.2 (3.3) | 54.1 (4.4) | 77.6; 1,645 112 | 161 |
+// 150 | 250. At 4096 x 4096 trying them made the first 900 steps of a handle 842 ms instead of 650.
+static bool tried(const Handle& H, int k, int64_t nact) {
+    const LoopConfig& C = H.loop.cand[k];
+    return !C.resident || (int64_t)(TILE / C.strips) * nact <= 2 * ((int64_t)H.sms * C.faces_per_sm - 1);
+}
+
+// The candidate that the tuner times next.
+static int next_candidate(const Handle& H, int64_t nact) {
+    const Loop& L = H.loop;
+    int c = L.next;
+    while (!tried(H, c, nact)) c = (c + 1) % L.ncand;  // (the first candidates are not resident)
+    return c;
+}
+
 // One timed launch of candidate c ran `live` loop steps in `ms`: add it, move to the next candidate, and settle on the
-// fastest once every candidate has its samples; then with the graphs of fewer steps that it will take, so that the first
+// fastest once every candidate that is tried on `nact` tiles has its samples; then with the graphs of fewer steps that it will take, so that the first
 // call to end in one does not pay for them (222 us of a call of 13 steps of 484 tiles, which takes 663).
-static int tune_sample(Handle& H, int c, long long live, float ms, cudaStream_t s) {
+static int tune_sample(Handle& H, int c, int64_t nact, long long live, float ms, cudaStream_t s) {
     Loop& L = H.loop;
     if (live > 0) {
         L.sec[c] += 1e-3 * (double)ms;
@@ -1139,11 +1157,11 @@ static int tune_sample(Handle& H, int c, long long live, float ms, cudaStream_t 
     }
     L.next = (c + 1) % L.ncand;
     for (int k = 0; k < L.ncand; ++k)
-        if (L.samples[k] < TUNE_SAMPLES) return W2B_OK;
+        if (tried(H, k, nact) && L.samples[k] < TUNE_SAMPLES) return W2B_OK;
     auto per_step = [&](int k) { return L.sec[k] / (double)(L.steps[k] > 0 ? L.steps[k] : 1); };
     int best = 0;
     for (int k = 1; k < L.ncand; ++k)
-        if (per_step(k) < per_step(best)) best = k;
+        if (tried(H, k, nact) && per_step(k) < per_step(best)) best = k;
     if (best != 0 && !(per_step(best) < (1.0 - TUNE_MARGIN) * per_step(0))) best = 0;
     L.chosen = best;
     L.tuning = 0;
@@ -1198,6 +1216,7 @@ static int advance_runs(Handle* H, const W2BStepper* cfg, const double* t_end, i
     CKL("advance begin");
     const RunTab T = run_table(held, n);
     Loop& L = H->loop;
+    int64_t nact = H->nact;
     long long ran_before = 0;  // loop steps so far in this call (the largest steps_run of any run)
     bool first_round = true;     // the runs' clocks are the caller's, not yet read back
     int end = 1, have_prev = 0;  // ev[end] takes this launch's end; ev[3 - end] holds the last one's, if have_prev
@@ -1208,7 +1227,7 @@ static int advance_runs(Handle* H, const W2BStepper* cfg, const double* t_end, i
         }
     for (;;) {
         const bool timed = L.tuning != 0;
-        const int c = timed ? L.next : L.chosen;
+        const int c = timed ? next_candidate(*H, nact) : L.chosen;
         if (timed && !have_prev) CK(cudaEventRecord(L.ev[0], s));
         // a timed launch is one of the candidate's steps; else as many as the runs will want at their current steps (a
         // step rule that shortens them on the way takes another round), at most CHUNKS before the host looks
@@ -1236,12 +1255,13 @@ static int advance_runs(Handle* H, const W2BStepper* cfg, const double* t_end, i
         CK(cudaMemcpyAsync(held, H->B.runs, run_table_bytes(n), cudaMemcpyDeviceToHost, s));
         CK(cudaMemcpyAsync(hctl, H->ctl(), sizeof(Ctl), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
+        nact = hctl->nact;
         if (timed) {
             long long ran = 0;
             for (int r = 0; r < n; ++r) ran = T.steps_run[r] > ran ? T.steps_run[r] : ran;
             float ms = 0.0f;
             CK(cudaEventElapsedTime(&ms, have_prev ? L.ev[3 - end] : L.ev[0], L.ev[end]));
-            const int stc = tune_sample(*H, c, ran - ran_before, ms, s);
+            const int stc = tune_sample(*H, c, nact, ran - ran_before, ms, s);
             if (stc != W2B_OK) return stc;
             ran_before = ran;
             have_prev = 1;
@@ -1316,7 +1336,7 @@ int32_t w2b_loop_config(void* handle, int32_t* out) {
     if (!handle || !out) return W2B_EINVAL;
     const Handle* H = static_cast<const Handle*>(handle);
     const Loop& L = H->loop;
-    const LoopConfig& C = L.cand[L.tuning ? L.next : L.chosen];
+    const LoopConfig& C = L.cand[L.tuning ? next_candidate(*H, H->nact) : L.chosen];
     out[0] = C.faces_per_sm;
     out[1] = C.update_per_sm;
     out[2] = C.steps;
@@ -1333,7 +1353,7 @@ int32_t w2b_loop_resident(void* handle, int32_t* out) {
     if (!handle || !out) return W2B_EINVAL;
     const Handle* H = static_cast<const Handle*>(handle);
     const Loop& L = H->loop;
-    out[0] = L.cand[L.tuning ? L.next : L.chosen].resident;
+    out[0] = L.cand[L.tuning ? next_candidate(*H, H->nact) : L.chosen].resident;
     for (int i = 0; i < 3; ++i) out[1 + i] = H->resident_occ[i];
     return W2B_OK;
 }
