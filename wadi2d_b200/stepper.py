@@ -8,6 +8,7 @@ the boundary tally every step, as CUDA graphs or one resident kernel, with one h
 
 from __future__ import annotations
 
+import sys
 from collections.abc import Callable
 from dataclasses import dataclass
 
@@ -157,6 +158,8 @@ class Stepper:
         self.refresh_due = False
         b.lists_moved(int(clock.nact))
         self._idle_there = True
+        if sys.getrefcount(self._idle) > 2:  # someone else holds the array: it keeps the counts, as it would if read back
+            self.idle  # noqa: B018
         if status == _lib.ENONFINITE:
             raise NumericalFailure(f"non-finite wave speed at t = {self.t:.3f} s")
         if status == _lib.EDTMIN:
