@@ -104,6 +104,8 @@ class Network:
             x = torch.as_tensor(np.asarray(x, np.float32), device=self.device)
         x = x.to(device=self.device, dtype=torch.float32)
         n = x.shape[0] if n is None else n
+        while x.dim() > 2 and x.shape[0] == 1:  # leading dimensions of one, as an assignment takes them
+            x = x[0]
         x = torch.broadcast_to(x, (n, width)).contiguous()
         if n == 0:
             return torch.zeros((1, width), dtype=torch.float32, device=self.device), 0
