@@ -948,8 +948,7 @@ def main() -> None:
     # end to end through the C-ABI with host buffers, as the reference's run driver and monitor take a run: per 30 s
     # window the window's rain from pinned memory (uploaded on a side stream while the window before steps, then put
     # in place by a device copy: run.SourceStager), the window stepped, then what the monitor reads each window (the
-    # clock and the active list, the design line's discharge, the outfall volume, the FP64 storage); at the end the
-    # five envelope maps
+    # clock, the design line's discharge, the outfall volume, the FP64 storage); at the end the five envelope maps
     from wadi2d_b200.maxima import Lines, faces_across
     from wadi2d_b200.run import DeviceStorage, MonitorReads, SourceStager
     from wadi2d_b200.state import state_index
@@ -980,7 +979,7 @@ def main() -> None:
         if w + 1 < args.e2e_windows:
             h2d += stager.stage(src_native)  # the next window's, crossing while this one steps
         m.run(m.stepper.t + win, maxima=maxima, tally=tally)
-        d2h += ctypes.sizeof(_lib.Clock) + 4 * (int(b.nact) + grid.ntiles)  # the clock, the active list, idle counts
+        d2h += int(_lib.lib().w2b_run_table_bytes(1))  # the loop's run table with the clock, once a window at least
         q, outflow, stored = monitor()
         series.append((m.stepper.t, float(q[0]), outflow, stored))
         d2h += monitor.host.numel() * 8
@@ -995,7 +994,7 @@ def main() -> None:
            "windows": args.e2e_windows, "steps": e2e_steps,
            "upload": "each window's rain from pinned host memory on a side stream while the window before steps, "
                      "then a device copy into place (run.SourceStager)",
-           "read_back": "per window: clock, active list, design-line discharge, outfall volume, storage; at the end: "
+           "read_back": "per window: the loop's run table, design-line discharge, outfall volume, storage; at the end: "
                         "the five envelope maps",
            "last_window": {"t_s": series[-1][0], "line_q_m3s": series[-1][1], "outflow_m3": series[-1][2],
                            "storage_m3": series[-1][3]} if series else None}  # fmt: skip
