@@ -281,6 +281,79 @@ __device__ __forceinline__ double local_term(const LinePixel* __restrict__ L, in
     return weight * di * (cb * cb);
 }
 
+// The same term where the line holds an infinite pixel: the reference's own running sums from the line's start. What is not
+// finite in them (a perimeter against an infinite wall, a depth over an infinite hole) stays in every sum behind it, and the
+// radius is then the depth; sums over the tent alone would forget it. No line of a real bed comes here: its cost, a sweep
+// from the line's start a term, does not matter.
+__device__ double running_term(const LinePixel* __restrict__ L, int n, int i, double level, double pixel,
+                                            double beta, double weight) {
+    auto depth = [&](int t) {
+        const double d = level - L[t].z;
+        return d > 0.0 ? d : 0.0;
+    };
+    const double di = depth(i);
+    if (!(di > 0.0)) return 0.0;
+    double w = beta * di / pixel;
+    if (w < 1e-9) w = 1e-9;
+    int first = i, last = i;  // the wet stretch around pixel i
+    while (first > 0 && depth(first - 1) > 0.0) --first;
+    while (last < n - 1 && depth(last + 1) > 0.0) ++last;
+    int lo = (int)ceil((double)i - w), hi = (int)floor((double)i + w);
+    lo = first > lo ? first : lo;
+    hi = last < hi ? last : hi;
+    // the perimeter that a wet pixel has from the segment to its neighbour of depth `other`, `rise` higher
+    auto share = [&](double d, double other, double rise, double half_seg) {
+        if (other > 0.0) return half_seg;
+        if (!(rise > 0.0)) return 0.5 * pixel;
+        const double f = d / rise;
+        return (f <= 1.0 ? f : 1.0) * (2.0 * half_seg);
+    };
+    double s0 = 0.0, s1 = 0.0, p0 = 0.0, p1 = 0.0;        // sums over the pixels before t
+    double ls0 = 0.0, ls1 = 0.0, lp0 = 0.0, lp1 = 0.0;    // before pixel lo
+    double is0 = 0.0, is1 = 0.0, ip0 = 0.0, ip1 = 0.0;    // up to pixel i
+    for (int t = 0; t <= hi; ++t) {
+        if (t == lo) ls0 = s0, ls1 = s1, lp0 = p0, lp1 = p1;
+        const double d = depth(t);
+        double per = 0.0;
+        if (d > 0.0) {
+            if (t == 0) per += 0.5 * pixel;
+            if (t == n - 1) per += 0.5 * pixel;
+            if (t > 0) per += share(d, depth(t - 1), L[t - 1].z - L[t].z, L[t].half_seg);
+            if (t < n - 1) per += share(d, depth(t + 1), L[t + 1].z - L[t].z, L[t + 1].half_seg);
+        }
+        s0 += d;
+        s1 += (double)t * d;
+        p0 += per;
+        p1 += (double)t * per;
+        if (t == i) is0 = s0, is1 = s1, ip0 = p0, ip1 = p1;
+    }
+    const double fi = (double)i;
+    double a_sum = (1.0 - fi / w) * (is0 - ls0) + (is1 - ls1) / w;
+    a_sum += (1.0 + fi / w) * (s0 - is0) - (s1 - is1) / w;
+    double p_sum = (1.0 - fi / w) * (ip0 - lp0) + (ip1 - lp1) / w;
+    p_sum += (1.0 + fi / w) * (p0 - ip0) - (p1 - ip1) / w;
+    const double radius = p_sum > 0.0 ? pixel * a_sum / p_sum : di;
+    const double cb = cbrt(radius);
+    return weight * di * (cb * cb);
+}
+
+// Whether the bed holds an infinite pixel, in a place of its own only until close_faces_kernel writes it (the first cell's
+// entry; zero before). A pass over the pixels that the faces' lines can reach: 25 us for 16 M of them.
+__device__ __forceinline__ float* infinite_word(const TableArgs& A) { return A.flx + TILE2; }
+__global__ void __launch_bounds__(256) infinite_kernel(TableArgs A) {
+    auto row = [&](int64_t r) { return r < 0 ? 0 : (r >= A.zh ? A.zh - 1 : r); };
+    auto col = [&](int64_t c) { return c < 0 ? 0 : (c >= A.zw ? A.zw - 1 : c); };
+    const int64_t r0 = row((int64_t)A.roff - A.margin - 1), r1 = row((int64_t)A.roff + (int64_t)A.ny * A.k + A.margin);
+    const int64_t c0 = col((int64_t)A.coff - A.margin - 1), c1 = col((int64_t)A.coff + (int64_t)A.nx * A.k + A.margin);
+    bool found = false;
+    for (int64_t r = r0 + blockIdx.x; r <= r1; r += gridDim.x) {
+        const double* z = A.z + r * A.zw;
+#pragma unroll 8
+        for (int64_t c = c0 + threadIdx.x; c <= c1; c += blockDim.x) found |= isinf(z[c]);
+    }
+    if (found) *infinite_word(A) = 1.0f;
+}
+
 // The face tables (_face_table, wadi2d/tables/core.py:44-79, and the local radius's conveyance), a group of GF faces
 // in a row along their own line at a time (GF divides 32: a column of a tile's west faces, a row of its north faces).
 // The faces of a group share one line of GF k + 2 margin pixels, read once; then every (face, row, pixel) is a thread's
@@ -293,16 +366,19 @@ __device__ __forceinline__ double local_term(const LinePixel* __restrict__ L, in
 // slower. Three CTAs of 256 threads a SM (80 registers): four (64, with spills) 5.3 and 1.39 against 5.2 and 1.26; six of
 // 128 threads the same.
 // LINE_SMEM: the group's line in shared memory, else (a line too long for it) in the caller's workspace, GF = 1.
+// INFINITE: once more the groups whose line holds an infinite pixel, by running_term, if infinite_kernel has found any (both
+// forms in one kernel, or a look for infinities in the other one, cost it 3 to 6 % of a build).
 struct FaceShape {
     int gf, fc;      // faces a group; of them, whose terms are held at a time
     int line;        // pixels of a group's line
 };
-template <bool LINE_SMEM>
+template <bool LINE_SMEM, bool INFINITE>
 __global__ void __launch_bounds__(FACE_THREADS, 3) face_tables_kernel(TableArgs A, FaceShape F) {
     extern __shared__ __align__(16) double sws[];
     __shared__ double s_zf[TILE], s_top[TILE], s_scale[TILE], s_len[TILE], s_crest[TILE], s_nm[TILE];
     __shared__ double s_xx[ROWS_MAX];  // a row's level over the invert, of the face's full depth
     __shared__ int s_e[TILE];  // pixels the conveyance line reaches past the face's ends, -1: the strips' sum
+    if (INFINITE && *infinite_word(A) == 0.0f) return;
     const int k = A.k, rows = A.rows, last = rows - 1, GF = F.gf, tid = threadIdx.x;
     double* terms = sws;
     // (the terms are an even count of doubles apart from the line's start: its pixels are 16 bytes)
@@ -325,6 +401,11 @@ __global__ void __launch_bounds__(FACE_THREADS, 3) face_tables_kernel(TableArgs 
         const int dj = axis == 0, di = axis != 0;
         for (int s = tid; s < F.line; s += FACE_THREADS) line[s].z = edge_pixel(A, axis, j0 * k, i0 * k, s - A.margin);
         __syncthreads();
+        if (INFINITE) {
+            bool found = false;
+            for (int s = tid; s < F.line; s += FACE_THREADS) found |= isinf(line[s].z);
+            if (!__syncthreads_or(found)) continue;
+        }
         if (A.local)
             for (int s = tid + 1; s < F.line; s += FACE_THREADS) {
                 const double rise = line[s].z - line[s - 1].z;
@@ -396,7 +477,10 @@ __global__ void __launch_bounds__(FACE_THREADS, 3) face_tables_kernel(TableArgs 
                     const int at = f * k + A.margin - e;
                     const int64_t j = j0 + f * dj, i = i0 + f * di;
                     const double weight = A.npix ? edge_weight(A, axis, j * k, i * k, q, s_nm[f]) : 1.0;
-                    terms[x] = local_term(line + at, k + 2 * e, e + q, level, A.pixel, tent, weight);
+                    if (INFINITE)
+                        terms[x] = running_term(line + at, k + 2 * e, e + q, level, A.pixel, A.beta, weight);
+                    else
+                        terms[x] = local_term(line + at, k + 2 * e, e + q, level, A.pixel, tent, weight);
                 }
                 q += dq;
                 if (q >= k) q -= k, ++fl;
@@ -570,8 +654,10 @@ static int32_t build(const W2BTableIn* in, const W2BTableOut* out, void* stream)
     int dev = 0, sms = 148, occ = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    auto kernel = line_smem ? face_tables_kernel<true> : face_tables_kernel<false>;
+    auto kernel = line_smem ? face_tables_kernel<true, false> : face_tables_kernel<false, false>;
+    auto infinite = line_smem ? face_tables_kernel<true, true> : face_tables_kernel<false, true>;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess ||
+        cudaFuncSetAttribute(infinite, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, FACE_THREADS, bytes) != cudaSuccess) {
         fprintf(stderr, "libwadi_b200: w2b_build_tables: face tables: %s\n", cudaGetErrorString(cudaGetLastError()));
         return W2B_ECUDA;
@@ -582,7 +668,15 @@ static int32_t build(const W2BTableIn* in, const W2BTableOut* out, void* stream)
         const int64_t held = (out->ws_threads * 9 * (int64_t)(A.nmax + 1) - 1) / (2 * (int64_t)F.line);
         fblocks = fblocks < held ? fblocks : held;
     }
-    if (groups > 0) kernel<<<(unsigned)(fblocks < groups ? fblocks : groups), FACE_THREADS, bytes, s>>>(A, F);
+    if (groups > 0) {
+        const unsigned grid = (unsigned)(fblocks < groups ? fblocks : groups);
+        kernel<<<grid, FACE_THREADS, bytes, s>>>(A, F);
+        if (A.local) {
+            if (cudaMemsetAsync(A.flx + TILE2, 0, sizeof(float), s) != cudaSuccess) return W2B_ECUDA;
+            infinite_kernel<<<sms * 8, 256, 0, s>>>(A);
+            infinite<<<grid, FACE_THREADS, bytes, s>>>(A, F);
+        }
+    }
     close_faces_kernel<<<148 * 8, 256, 0, s>>>(A);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
