@@ -377,21 +377,23 @@ int32_t w2b_build_tables_noalloc(const W2BTableIn* in, const W2BTableOut* out, v
  * with one fixed grid; the tile shape stays the reference's 32 x 32 (its table layout), so what is tuned is the
  * schedule: the face pass's form, CTAs a SM of the face pass and of the update pass, and loop steps a captured graph.
  * Every configuration gives the same results bit for bit. By default the handle tunes online during its first
- * w2b_advance / w2b_advance_runs calls: successive launches rotate through seven candidates (the default, it with 32
- * steps a graph, the face pass's two strip forms, and the resident loop with strips of 16, 8 and 4 rows), each timed with CUDA events from the end of the launch before it (the host's clock read between graphs
- * included) per loop step that ran; after three launches each the fastest is kept for the handle's life, the default
- * unless another is more than 2 % faster. The strip forms of the face pass take strips of 16 rows of a tile (CTAs of
- * 256 threads and 51 KB, four a SM) or of 8 rows (128 threads and 27 KB, eight a SM): the same faces bit for bit. The resident loop takes up to the
- * configuration's steps in one cooperative launch (CTAs of 256 threads, four a SM) instead of a graph of six launches a
- * step; such launches of one process on one GPU run beside one another as
- * long as all their CTAs are sure to fit, else one after another.
+ * w2b_advance / w2b_advance_runs calls: successive launches rotate through up to seven candidates (the default, it with
+ * 32 steps a graph, the face pass's two strip forms, and the resident loop with strips of 16, 8 and 4 rows where the
+ * strips of the tiles awake are at most two waves of it), each timed with CUDA events from the end of the launch before
+ * it (the host's clock read between launches included) per loop step that ran; after three launches each the fastest is
+ * kept for the handle's life, the default unless another is more than 2 % faster. The strip forms of the face pass take
+ * strips of 16 rows of a tile (CTAs of 256 threads and 51 KB, four a SM) or of 8 rows (128 threads and 27 KB, eight a
+ * SM): the same faces bit for bit. The resident loop takes up to the configuration's steps in one cooperative launch
+ * (CTAs of 256 threads; two a SM, with 8-row strips three) instead of a graph of five launches a step; such launches of
+ * one process on one GPU run beside one another as long as all their CTAs are sure to fit, else one after another.
  * w2b_loop_tuning(h, 1, ...) starts tuning again; w2b_loop_tuning(h, tune, f, u, s) with tune 0, 2 or 3 fixes a
- * configuration with the tile form, the 16-row or the 8-row strips, 4, 5 or 6 the resident loop with 16-, 8- or 4-row strips (1 <= f <= the form's resident CTAs a SM, 1 <= u <=
- * the update pass's, 1 <= s <= 64), W2B_EINVAL outside that. w2b_loop_config(h, out) fills out[9]: faces CTAs a SM,
+ * configuration with the tile form, the 16-row or the 8-row strips, 4, 5 or 6 the resident loop with 16-, 8- or 4-row
+ * strips (1 <= f <= the form's resident CTAs a SM, 1 <= u <= the update pass's, 1 <= s <= 64), W2B_EINVAL outside that.
+ * w2b_loop_config(h, out) fills out[9]: faces CTAs a SM,
  * update CTAs a SM, steps a graph (while tuning: the next launch's), tuning (1/0), the tile form's and the update
  * pass's resident CTAs a SM, the form (0 tiles, else the strip rows), and the 16-row and 8-row strip forms' resident
- * CTAs a SM. Host-driven steps (w2b_step) take the form and face-pass CTAs the tuner settled on, the tile form while
- * it tunes. */
+ * CTAs a SM. A host-driven step (w2b_step) is one launch of the resident kernel where its 8-row strips are one wave of
+ * it, else kernels of its own with the form and face-pass CTAs the tuner settled on, the 8-row strips while it tunes. */
 int32_t w2b_loop_tuning(void* handle, int32_t tune, int32_t faces_per_sm, int32_t update_per_sm, int32_t steps);
 int32_t w2b_loop_config(void* handle, int32_t* out);
 /* The resident loop: out[0] 1 while the configuration w2b_loop_config reports is it, out[1 .. 3] its resident CTAs

@@ -12,9 +12,10 @@ namespace w2b {
 
 constexpr int RESIDENT_THREADS = 256;
 // CTAs a SM the launch bound plans for, by the strips' height. Fewer leave more registers a thread: 4-row strips serve
-// the smallest grids, where nothing but a warp's own chain counts (62 x 62 cells: 13.0 us a step with two, 14.9 with
-// four); 8-row ones need their CTAs (256 x 256: 18.1 with three, 19.6 with four, 21.6 with two); 16-row ones do best with
-// two where the resident loop is the best form at all (a valley of 190 tiles: 22.2 against 30.1 with four).
+// the smallest grids, where nothing but a warp's own chain counts (62 x 62 cells: 11.4 us a step with two, 11.9 with
+// three, 13.2 with four); 8-row ones need their CTAs (256 x 256: 17.1 with three, 18.6 with four, 19.2 with two); 16-row
+// ones do best with two where the resident loop is the best form at all (a valley of 108 tiles: 20.7 against 25.0 with
+// three and 27.0 with four).
 constexpr int resident_ctas(int rows) { return rows == 8 ? 3 : 2; }
 constexpr uint32_t GRID_WAIT_LIMIT = 1u << 21;  // polls of a barrier before a CTA gives up, one to two seconds
 

@@ -1,15 +1,16 @@
-// The uniform-grid step on sm_100a: face pass, update pass (positivity ratio, continuity, level lookup), envelope pass,
-// boundary/tally/control pass, active-list rebuild, and the layout converters.
+// The uniform-grid step on sm_100a: face pass, update pass (positivity ratio, continuity, level lookup; in the device loop
+// also the clocks and the next step's settings), the step's end (boundary cells, tally, lines, envelope), active-list
+// rebuild; all of them in one kernel (the resident loop); and the layout converters.
 //
-// A CTA takes one 32 x 32 tile at a time, looping over its share of the work list (grid-stride, so a graph-captured
-// launch serves any list length): the face pass with 512 threads (a thread a column, two rows), the update pass with
-// 256 (a thread a column, four rows). State sits in the dense NATIVE layout, so a neighbour is an address offset and
+// A CTA takes one 32 x 32 tile, or a strip of one, at a time, looping over its share of the work list (grid-stride, so a
+// graph-captured launch serves any list length): the face pass with 512 threads (a thread a column, two rows; 256 or 128
+// in its strip forms), the update pass with 256 (a thread a column, four rows). State sits in the dense NATIVE layout, so a neighbour is an address offset and
 // the reference's halo exchanges (wadi2d/solver/gpu/kernels/cells.cu:80-93) disappear; the guard ring is zero like
 // the reference's void tile. In a batch every tile reads its run's clock, cell size, flags and current half.
 //
 // The face pass restates wadi2d/solver/gpu/kernels/faces.cu:10-175 (= wadi2d/solver/cpu/kernels.py:86-244); the
 // update pass fuses limit and update (cells.cu:4-63, kernels.py:247-299) by computing the positivity ratio r of the
-// tile and its one-cell ring in shared memory; the boundary pass restates cells.cu:95-111 and engine/maxima.py:53-62.
+// tile and its one-cell ring in shared memory; the step's end restates cells.cu:95-111 and engine/maxima.py:53-92.
 #include <cstdio>
 
 #include "w2b_common.cuh"
@@ -1201,19 +1202,18 @@ __device__ __forceinline__ bool update_unit(const UpdateMaps& M, const StepArgs&
     return true;
 }
 
-// Up to max_steps steps of the device loop in one cooperative launch. A step of the loop's kernels of their own is six
+// Up to max_steps steps of the device loop in one cooperative launch. A step of the loop's kernels of their own is five
 // dependent launches, which on a few hundred tiles cost more than their work; here it is two grid barriers: the face
 // pass by strips of H rows (first barrier), then the update of the same strips with their envelope, the boundary cells
 // shared out over the CTAs, while one CTA of its own forms the next step's settings in the second set (second barrier);
 // that CTA then takes the tally and the lines while the next face pass runs. Where some boundary cell follows another, all
-// of them (one more barrier), and steps
-// that rebuild the lists (two or three more, one step in active_every) come after it. The same arithmetic in the same
-// order for every cell, face and sum as the kernels of their own. What CTAs hand one another between barriers is read
-// past L1 or by bulk copies. Latency bounds it on small grids, so strips of 4 rows (a warp a row and axis) serve the
+// of them (one more barrier), and steps that rebuild the lists (two or three more, one step in active_every) come after it.
+// The same arithmetic in the same order for every cell, face and sum as the kernels of their own. What CTAs hand one
+// another between barriers is read past L1 or by bulk copies. Latency bounds it on small grids (issue active 11 % at 62 x
+// 62, 27 % at 256 x 256, a warp's time mostly at barriers), so strips of 4 rows (a warp a row and axis) serve the
 // smallest, and a CTA keeps the places of its strips from step to step. A step of the exact build, this way and as
-// kernels of their own: 62 x 62 cells 13 against 30 us (face pass 4.0, update 2.9, a barrier 2 to 3 us), 256 x 256 18
-// against 31 us, a valley of 190 awake tiles 22 against 33 us. Where the passes' own work fills the chip it gains nothing
-// (1500 x 1101: 155 against 136 us), and the launch tuner keeps the kernels.
+// kernels of their own: 4 tiles 11.2 against 20.3 us, 64 tiles 16.6 against 21.1, 121 tiles 19.7 against 22.6. Where the
+// passes' own work fills the chip it loses (1,645 tiles: 149 against 109 us), and the launch tuner leaves it out.
 // A host-driven step (host.flags not 0) is one step of it: the settings come with the launch, the tiles are the active
 // list (in A.work's place, host.tiles of them), nothing but the swap of run 0's halves follows.
 template <int H, bool ON>

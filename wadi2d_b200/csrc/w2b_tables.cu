@@ -357,9 +357,11 @@ __global__ void __launch_bounds__(256) infinite_kernel(TableArgs A) {
 // The face tables (_face_table, wadi2d/tables/core.py:44-79, and the local radius's conveyance), a group of GF faces
 // in a row along their own line at a time (GF divides 32: a column of a tile's west faces, a row of its north faces).
 // The faces of a group share one line of GF k + 2 margin pixels, read once; then every (face, row, pixel) is a thread's
-// own sweep along it (local_term), and every (face, row) a thread that adds its pixels' terms in order. FP64 instructions
-// bound it (the sweeps, a division, a cbrt and four conversions a term): 2.1 M faces of 24- to 44-pixel lines (1024 x 1024
-// cells, 4 x 4 pixels) take 4.3 ms, 98 k faces of up to 298 (10 x 10 pixels of 1 m) 1.2 ms. A thread a face with its nine
+// own sweep along it (local_term), and every (face, row) a thread that adds its pixels' terms in order. Instruction issue and
+// a thread's own chain bound it together (the sweeps, a division, a cbrt and four conversions a term: issue active 66 %, 56
+// % at 10 x 10 pixels, FP64 28 and 37 %, 36 % of the warps a SM could hold, most of their waiting on the result before): 2.1
+// M faces of 24- to 44-pixel lines (1024 x 1024 cells, 4 x 4 pixels) take 4.3 ms, 98 k faces of up to 298 (10 x 10 pixels
+// of 1 m) 1.2 ms. A thread a face with its nine
 // line arrays in shared memory, as this was first written, left 63 and 9 threads a SM and took 67 and 99 ms; sweeps from
 // the line's start 8.5 and 2.9; the tent's sweeps with four divisions a term, the rows' levels and the indices divided out
 // for each term, 5.2 and 1.26. A thread four or five pixels at once (one sweep for all, 200 registers, 8 warps a SM) was
